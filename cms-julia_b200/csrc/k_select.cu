@@ -8,7 +8,7 @@
 // cells before it), so it walks the cells in order within an event, one warp per
 // event, taking 32 cells at once when they share no track. The triplet cleaner only
 // ever writes "dup" and tests "!= bad", so its hits run in parallel. Vertex sums keep
-// the reference's track order (one thread per vertex walks its tracks in order).
+// the reference's track order (a warp per vertex hands its tracks' terms over in order).
 #include <cstddef>
 
 #include "pxl_internal.cuh"
@@ -340,9 +340,19 @@ __global__ void k_triplet_cleaner(Dev d) {
 }
 
 // ---------------------------------------------------------------- vertices
-constexpr int kVtxThreads = 256;
+// One CTA per event. What bounds it is latency: the sums of the fits and of the 2-means splits are
+// taken in the reference's track order, so they are serial chains. A warp takes a vertex: its lanes
+// read 32 tracks and form their terms (weights, residuals, divisions) at once, and only the
+// additions follow one another, handed over by shuffles. With a thread per vertex, each term's
+// loads and division sat in the chain too, and an event above the shared-memory capacity (2048
+// tracks then) paid global latency for them: an event of pileup 170 (4.3 k tracks) took 5.66 ms
+// and one of pileup 50 326 us.
 constexpr int kMaxVtx = 1024;
-constexpr int kVtxSmemTracks = 2048;  // selected tracks whose vertex arrays fit shared memory
+constexpr int kVtxWideThreads = 1024, kVtxNarrowThreads = 256;
+// Selected tracks whose arrays fit shared memory. The narrow form (46 KB, four or five CTAs per SM)
+// serves batches that fill the SMs with one CTA per event; the wide form (one CTA per SM) serves
+// small batches and the few events above the narrow capacity; above both, global memory.
+constexpr uint32_t kVtxWideTracks = 12288, kVtxNarrowTracks = 2048;
 
 struct VtxShared {
   uint32_t sh[33];
@@ -353,95 +363,141 @@ struct VtxShared {
   uint16_t parent[kMaxVtx];
 };
 
-// cluster_tracks_by_density, fit_vertices, split_vertices and sort_by_pt2 on the selected
-// tracks of one event (one CTA). TI / TB: types of the per-track vertex ids and neighbour
-// counts and of the histogram / list entries; the arrays are in shared memory for events of
-// up to kVtxSmemTracks selected tracks (16-bit entries) and in global memory above.
+// per-track arrays of one event, in shared or global memory
 template <typename TI, typename TB>
-__device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, int e, uint32_t nt, const float* __restrict__ zt,
-                                            const float* __restrict__ ezt2, const float* ptt2, const uint32_t* itrk,
-                                            TI* iv, TI* nn, uint8_t* izt, TB* B, float* zv, float* wv, float* vchi2,
-                                            float* ptv2, uint16_t* sort_ind, VtxShared& S) {
+struct VtxTracks {
+  const float* zt;
+  const float* ezt2;
+  TI* iv;        // 1-based values as the reference stores them
+  TI* nn;
+  TB* B;         // z histogram, then the vertices' track lists
+  TB* C;         // unordered form of B
+  uint8_t* izt;
+};
+
+constexpr size_t vtx_smem_bytes(uint32_t tracks) { return (sizeof(VtxShared) + 15) / 16 * 16 + size_t(tracks) * 17; }
+
+// entries [lo, hi) of C put in order into B: ascending, or descending with kDown. Each entry counts
+// the ones before it; the runs are short (a z bin, a vertex) and all entries count at once.
+template <bool kDown, typename TB>
+__device__ __forceinline__ void place_by_rank(const TB* C, TB* B, uint32_t p, uint32_t lo, uint32_t hi) {
+  const TB x = C[p];
+  uint32_t r = lo;
+  for (uint32_t q = lo; q < hi; ++q) r += kDown ? C[q] > x : C[q] < x;
+  B[r] = x;
+}
+
+// acc0 + a[0] + a[1] + ... and acc1 + b[0] + ... over the lanes of a warp in lane order (lanes that
+// take no part hold +0, which leaves a sum that is never -0 as it is); every lane gets the sums
+__device__ __forceinline__ void ordered_add2(float a, float b, uint32_t n, float& acc0, float& acc1) {
+  if (n >= 32) {
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      acc0 = __fadd_rn(acc0, __shfl_sync(0xffffffffu, a, k));
+      acc1 = __fadd_rn(acc1, __shfl_sync(0xffffffffu, b, k));
+    }
+  } else {
+#pragma unroll 4
+    for (uint32_t k = 0; k < n; ++k) {
+      acc0 = __fadd_rn(acc0, __shfl_sync(0xffffffffu, a, k));
+      acc1 = __fadd_rn(acc1, __shfl_sync(0xffffffffu, b, k));
+    }
+  }
+}
+
+__device__ __forceinline__ float ordered_add(float a, uint32_t n, float acc) {
+  if (n >= 32) {
+#pragma unroll
+    for (int k = 0; k < 32; ++k) acc = __fadd_rn(acc, __shfl_sync(0xffffffffu, a, k));
+  } else {
+#pragma unroll 4
+    for (uint32_t k = 0; k < n; ++k) acc = __fadd_rn(acc, __shfl_sync(0xffffffffu, a, k));
+  }
+  return acc;
+}
+
+// cluster_tracks_by_density, fit_vertices, split_vertices and sort_by_pt2 on the nt selected
+// tracks of one event (one CTA).
+template <typename TI, typename TB>
+__device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, const VtxTracks<TI, TB>& A,
+                                            const float* ptt2, const uint32_t* itrk, float* zv, float* wv,
+                                            float* vchi2, float* ptv2, uint16_t* sort_ind, VtxShared& S) {
   const uint64_t tb = E.tuple_base;
-  uint32_t* sh = S.sh;
-  uint32_t* s_off = S.off;
-  uint32_t* s_cur = S.cur;
-  uint32_t& s_nv = S.nv;
-  uint32_t& s_nvi = S.nvi;
-  uint32_t& s_warn = S.warn;
-  uint32_t* s_vcnt = S.vcnt;
-  uint32_t* s_voff = S.voff;
-  uint16_t* s_parent = S.parent;
+  const float* zt = A.zt;
+  const float* ezt2 = A.ezt2;
+  TI* iv = A.iv;
+  TI* nn = A.nn;
+  TB* B = A.B;
+  TB* C = A.C;
+  uint8_t* izt = A.izt;
+  const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   // cluster_tracks_by_density (:84-206), HisToContainer{UInt8,256,16000,8,UInt16}
-  for (int b = threadIdx.x; b < 257; b += blockDim.x) s_off[b] = 0;
+  for (uint32_t b = threadIdx.x; b < 257; b += blockDim.x) S.off[b] = 0;
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
     int32_t iz = int32_t(trunc(__dmul_rn(double(zt[i]), 10.)));
     iz = iz < -128 ? -128 : (iz > 127 ? 127 : iz);
     izt[i] = uint8_t(iz + 128);
-    atomicAdd(&s_off[izt[i]], 1u);
+    atomicAdd(&S.off[izt[i]], 1u);
     iv[i] = TI(i + 1);
   }
   __syncthreads();
   {  // exclusive starts of the 256 bins
-    const uint32_t v = threadIdx.x < 256 ? s_off[threadIdx.x] : 0u;
+    const uint32_t v = threadIdx.x < 256 ? S.off[threadIdx.x] : 0u;
     uint32_t tot;
-    const uint32_t ex = block_excl_scan(v, sh, &tot);
-    if (threadIdx.x < 256) { s_off[threadIdx.x] = ex; s_cur[threadIdx.x] = ex; }
-    if (threadIdx.x == 0) s_off[256] = tot;
+    const uint32_t ex = block_excl_scan(v, S.sh, &tot);
+    if (threadIdx.x < 256) { S.off[threadIdx.x] = ex; S.cur[threadIdx.x] = ex; }
+    if (threadIdx.x == 0) S.off[256] = tot;
   }
   __syncthreads();
-  // histogram contents (1-based track indices), decreasing track index within a bin: one
-  // warp walks the tracks from the last down, 32 at a time, ranking equal bins by lane
-  if (threadIdx.x < 32) {
-    const unsigned lane = threadIdx.x, lt = (1u << lane) - 1u;
-    for (uint32_t b0 = 0; b0 < nt; b0 += 32) {
-      const bool ok = b0 + lane < nt;
-      const uint32_t i = ok ? nt - 1 - (b0 + lane) : 0u;
-      const uint32_t bin = ok ? uint32_t(izt[i]) : 0xffffffffu;
-      const uint32_t peers = __match_any_sync(0xffffffffu, bin);
-      const uint32_t start = ok ? s_cur[bin] : 0u;
-      __syncwarp();
-      if (ok) {
-        const uint32_t rank = __popc(peers & lt);
-        B[start + rank] = TB(i + 1);
-        if (rank == uint32_t(__popc(peers)) - 1u) s_cur[bin] = start + rank + 1;
-      }
-      __syncwarp();
-    }
+  // histogram contents (1-based track indices), decreasing track index within a bin
+  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) C[atomicAdd(&S.cur[izt[i]], 1u)] = TB(i + 1);
+  __syncthreads();
+  for (uint32_t p = threadIdx.x; p < nt; p += blockDim.x) {
+    const uint32_t b = izt[C[p] - 1];
+    place_by_rank<true>(C, B, p, S.off[b], S.off[b + 1]);
   }
   __syncthreads();
+  // the density loops go over the tracks in histogram order: the lanes of a warp then scan the
+  // same few bins
   const float eps = 0.07f, err2_max = __fmul_rn(0.01f, 0.01f), chi2_max = 9.0f;
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
-    if (ezt2[i] > err2_max) continue;
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) {
+    const uint32_t i = B[s] - 1;
+    const float e2 = ezt2[i], z = zt[i];
+    if (e2 > err2_max) continue;
     const int bs0 = int(izt[i]) + 1;
     const int be = bs0 + 1 < 256 ? bs0 + 1 : 256;
     const int bs = bs0 - 1 > 1 ? bs0 - 1 : 1;
     int32_t cnt = 0;
-    for (uint32_t p = s_off[bs - 1]; p < s_off[be]; ++p) {
+    for (uint32_t p = S.off[bs - 1], pe = S.off[be]; p < pe; ++p) {
       const uint32_t j = B[p] - 1;
       if (j == i) continue;
-      const float dist = fabsf(__fsub_rn(zt[i], zt[j]));
+      const float dist = fabsf(__fsub_rn(z, zt[j]));
       if (dist > eps) continue;
-      if (__fmul_rn(dist, dist) > __fmul_rn(chi2_max, __fadd_rn(ezt2[i], ezt2[j]))) continue;
+      if (__fmul_rn(dist, dist) > __fmul_rn(chi2_max, __fadd_rn(e2, ezt2[j]))) continue;
       ++cnt;
     }
     nn[i] = TI(cnt);
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) {
+    const uint32_t i = B[s] - 1;
+    const float e2 = ezt2[i], z = zt[i];
+    const TI ni = nn[i];
     float mdist = eps;
     const int bs0 = int(izt[i]) + 1;
     const int be = bs0 + 1 < 256 ? bs0 + 1 : 256;
     const int bs = bs0 - 1 > 1 ? bs0 - 1 : 1;
     int32_t a = int32_t(i + 1);
-    for (uint32_t p = s_off[bs - 1]; p < s_off[be]; ++p) {
+    for (uint32_t p = S.off[bs - 1], pe = S.off[be]; p < pe; ++p) {
       const uint32_t j = B[p] - 1;
-      if (nn[j] < nn[i]) continue;
-      if (nn[j] == nn[i] && zt[j] >= zt[i]) continue;
-      const float dist = fabsf(__fsub_rn(zt[i], zt[j]));
+      const TI nj = nn[j];
+      if (nj < ni) continue;
+      const float zj = zt[j];
+      if (nj == ni && zj >= z) continue;
+      const float dist = fabsf(__fsub_rn(z, zj));
       if (dist > mdist) continue;
-      if (__fmul_rn(dist, dist) > __fmul_rn(chi2_max, __fadd_rn(ezt2[i], ezt2[j]))) continue;
+      if (__fmul_rn(dist, dist) > __fmul_rn(chi2_max, __fadd_rn(e2, ezt2[j]))) continue;
       mdist = dist;
       a = int32_t(j + 1);
     }
@@ -460,7 +516,7 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, int e, uint32_t n
     const bool root = i < nt && iv[i] == int32_t(i + 1);
     const bool seed = root && nn[i] >= 2;
     uint32_t tot;
-    const uint32_t ex = block_excl_scan(seed ? 1u : 0u, sh, &tot);
+    const uint32_t ex = block_excl_scan(seed ? 1u : 0u, S.sh, &tot);
     if (root) iv[i] = TI(seed ? -int32_t(found + ex + 1) : -9998);
     found += tot;
   }
@@ -470,126 +526,147 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, int e, uint32_t n
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) iv[i] = TI(-iv[i]);
   if (threadIdx.x == 0) {
-    if (found >= uint32_t(kMaxVtx)) { s_warn |= kWarnVertex; found = kMaxVtx - 1; }
-    s_nv = found;
-    s_nvi = found;
+    if (found >= uint32_t(kMaxVtx)) { S.warn |= kWarnVertex; found = kMaxVtx - 1; }
+    S.nv = found;
+    S.nvi = found;
   }
   __syncthreads();
   // per-vertex track lists in ascending track order (the order of the reference's loops over
   // all tracks); B (the z histogram) is free again. A vertex made by a split keeps its parent's
   // list and selects its own tracks by id, as the loops over all tracks do.
-  const uint32_t nv0 = s_nv;
-  for (uint32_t v = threadIdx.x; v < uint32_t(kMaxVtx); v += blockDim.x) { s_vcnt[v] = 0; s_parent[v] = uint16_t(v); }
+  const uint32_t nv0 = S.nv;
+  for (uint32_t v = threadIdx.x; v < uint32_t(kMaxVtx); v += blockDim.x) { S.vcnt[v] = 0; S.parent[v] = uint16_t(v); }
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x)
-    if (iv[i] >= 1 && uint32_t(iv[i]) <= nv0) atomicAdd(&s_vcnt[iv[i] - 1], 1u);
+    if (iv[i] >= 1 && uint32_t(iv[i]) <= nv0) atomicAdd(&S.vcnt[iv[i] - 1], 1u);
   __syncthreads();
   {
     uint32_t base = 0;
     for (uint32_t b = 0; b < nv0; b += blockDim.x) {
       const uint32_t v = b + threadIdx.x;
-      const uint32_t c = v < nv0 ? s_vcnt[v] : 0u;
+      const uint32_t c = v < nv0 ? S.vcnt[v] : 0u;
       uint32_t tot;
-      const uint32_t ex = block_excl_scan(c, sh, &tot);
-      if (v < nv0) { s_voff[v] = base + ex; s_vcnt[v] = base + ex; }
+      const uint32_t ex = block_excl_scan(c, S.sh, &tot);
+      if (v < nv0) { S.voff[v] = base + ex; S.vcnt[v] = base + ex; }
       base += tot;
     }
-    if (threadIdx.x == 0) s_voff[nv0] = base;
+    if (threadIdx.x == 0) S.voff[nv0] = base;
   }
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x)
-    if (iv[i] >= 1 && uint32_t(iv[i]) <= nv0) B[atomicAdd(&s_vcnt[iv[i] - 1], 1u)] = TB(i);
+    if (iv[i] >= 1 && uint32_t(iv[i]) <= nv0) C[atomicAdd(&S.vcnt[iv[i] - 1], 1u)] = TB(i);
   __syncthreads();
-  for (uint32_t v = threadIdx.x; v < nv0; v += blockDim.x) {
-    const uint32_t lo = s_voff[v], hi = s_voff[v + 1];
-    for (uint32_t p = lo + 1; p < hi; ++p) {
-      const uint32_t x = B[p];
-      uint32_t q = p;
-      while (q > lo && B[q - 1] > x) { B[q] = B[q - 1]; --q; }
-      B[q] = TB(x);
-    }
+  for (uint32_t p = threadIdx.x, n = S.voff[nv0]; p < n; p += blockDim.x) {
+    const uint32_t v = uint32_t(iv[C[p]]) - 1;
+    place_by_rank<false>(C, B, p, S.voff[v], S.voff[v + 1]);
   }
   __syncthreads();
-  // fit_vertices, :228-286 (one thread per vertex keeps the track order of the sums)
+  // fit_vertices, :228-286: a warp per vertex, its sums in track order
   auto fit = [&](double chi2max) {
-    const uint32_t nvf = s_nvi;
-    for (uint32_t v = threadIdx.x; v < nvf; v += blockDim.x) {
-      const uint32_t pv = s_parent[v], lo = s_voff[pv], hi = s_voff[pv + 1];
+    const uint32_t nvf = S.nvi;
+    for (uint32_t v = wid; v < nvf; v += nwarp) {
+      const uint32_t pv = S.parent[v], lo = S.voff[pv], hi = S.voff[pv + 1];
       float z = 0, w = 0;
-      for (uint32_t p = lo; p < hi; ++p) {
-        const uint32_t i = B[p];
-        if (iv[i] != int32_t(v + 1)) continue;
-        const float wi = __fdiv_rn(1.0f, ezt2[i]);
-        z = __fadd_rn(z, __fmul_rn(zt[i], wi));
-        w = __fadd_rn(w, wi);
+      for (uint32_t p0 = lo; p0 < hi; p0 += 32) {
+        float wi = 0.f, zw = 0.f;
+        if (p0 + lane < hi) {
+          const uint32_t i = B[p0 + lane];
+          if (iv[i] == int32_t(v + 1)) {
+            wi = __fdiv_rn(1.0f, ezt2[i]);
+            zw = __fmul_rn(zt[i], wi);
+          }
+        }
+        ordered_add2(zw, wi, hi - p0, z, w);
       }
-      if (!(w > 0)) atomicOr(&s_warn, kWarnVertex);
+      if (!(w > 0) && lane == 0) atomicOr(&S.warn, kWarnVertex);
       z = __fdiv_rn(z, w);
       float c2s = 0;
       int32_t cnt = -1;
-      for (uint32_t p = lo; p < hi; ++p) {
-        const uint32_t i = B[p];
-        if (iv[i] != int32_t(v + 1)) continue;
-        float c2 = __fsub_rn(z, zt[i]);
-        c2 = __fmul_rn(c2, __fdiv_rn(c2, ezt2[i]));
-        if (double(c2) > chi2max) { iv[i] = 9999; continue; }
-        c2s = __fadd_rn(c2s, c2);
-        cnt += 1;
+      for (uint32_t p0 = lo; p0 < hi; p0 += 32) {
+        float c2 = 0.f;
+        bool in = false;
+        if (p0 + lane < hi) {
+          const uint32_t i = B[p0 + lane];
+          if (iv[i] == int32_t(v + 1)) {
+            c2 = __fsub_rn(z, zt[i]);
+            c2 = __fmul_rn(c2, __fdiv_rn(c2, ezt2[i]));
+            in = !(double(c2) > chi2max);
+            if (!in) { iv[i] = 9999; c2 = 0.f; }
+          }
+        }
+        cnt += __popc(__ballot_sync(0xffffffffu, in));
+        c2s = ordered_add(c2, hi - p0, c2s);
       }
       if (cnt > 0) w = __fmul_rn(w, __fdiv_rn(float(cnt), c2s));
-      zv[v] = z; wv[v] = w; vchi2[v] = c2s; nn[v] = TI(cnt);
+      if (lane == 0) { zv[v] = z; wv[v] = w; vchi2[v] = c2s; nn[v] = TI(cnt); }
     }
     __syncthreads();
-    if (threadIdx.x == 0) s_nv = nvf;
+    if (threadIdx.x == 0) S.nv = nvf;
     __syncthreads();
   };
   fit(50.);
   // split_vertices, :288-371: each vertex decides alone; new ids follow the vertex order
   {
-    const uint32_t nvf = s_nv;
-    for (uint32_t b = 0; b < nvf; b += blockDim.x) {
-      const uint32_t kv = b + threadIdx.x;
+    const uint32_t nvf = S.nv;
+    for (uint32_t kv = wid; kv < nvf; kv += nwarp) {
       bool split = false;
-      float znew0 = 0, znew1 = 0;
-      const uint32_t lo = kv < nvf ? s_voff[kv] : 0u, hi = kv < nvf ? s_voff[kv + 1] : 0u;
-      if (kv < nvf && nn[kv] >= 4 && !(vchi2[kv] < __fmul_rn(9.0f, float(nn[kv])))) {
+      const uint32_t lo = S.voff[kv], hi = S.voff[kv + 1];
+      if (nn[kv] >= 4 && !(vchi2[kv] < __fmul_rn(9.0f, float(nn[kv])))) {
         if (nn[kv] >= 512) {
-          atomicOr(&s_warn, kWarnVertex);
+          if (lane == 0) atomicOr(&S.warn, kWarnVertex);
         } else {
-          // 2-means in the vertex's tracks (zz = zt - zv, weights 1/ezt2), at most 20 iterations
+          // 2-means in the vertex's tracks (zz = zt - zv, weights 1/ezt2), at most 20 iterations;
+          // first assignment: zz < 0 -> 1 else 2, kept per track in izt
           uint32_t nq = 0;
           const float zc = zv[kv];
-          for (uint32_t p = lo; p < hi; ++p) if (iv[B[p]] == int32_t(kv + 1)) ++nq;
-          if (nq != uint32_t(nn[kv] + 1)) atomicOr(&s_warn, kWarnVertex);
+          for (uint32_t p0 = lo; p0 < hi; p0 += 32) {
+            bool in = false;
+            if (p0 + lane < hi) {
+              const uint32_t i = B[p0 + lane];
+              in = iv[i] == int32_t(kv + 1);
+              if (in) izt[i] = __fsub_rn(zt[i], zc) < 0 ? 1 : 2;
+            }
+            nq += __popc(__ballot_sync(0xffffffffu, in));
+          }
+          if (nq != uint32_t(nn[kv] + 1) && lane == 0) atomicOr(&S.warn, kWarnVertex);
           bool more = true;
           int iter = 20;
-          // first assignment: zz < 0 -> 1 else 2, kept per track in izt
-          for (uint32_t p = lo; p < hi; ++p) {
-            const uint32_t i = B[p];
-            if (iv[i] == int32_t(kv + 1)) izt[i] = __fsub_rn(zt[i], zc) < 0 ? 1 : 2;
-          }
-          float w0 = 0, w1 = 0;
+          float znew0 = 0, znew1 = 0, w0 = 0, w1 = 0;
           while (more) {
-            more = false;
             znew0 = znew1 = 0; w0 = w1 = 0;
-            for (uint32_t p = lo; p < hi; ++p) {
-              const uint32_t i = B[p];
-              if (iv[i] != int32_t(kv + 1)) continue;
-              const float zz = __fsub_rn(zt[i], zc), ww = __fdiv_rn(1.0f, ezt2[i]);
-              if (izt[i] == 1) { znew0 = __fadd_rn(znew0, __fmul_rn(zz, ww)); w0 = __fadd_rn(w0, ww); }
-              else { znew1 = __fadd_rn(znew1, __fmul_rn(zz, ww)); w1 = __fadd_rn(w1, ww); }
+            for (uint32_t p0 = lo; p0 < hi; p0 += 32) {
+              float ww = 0.f, zw = 0.f;
+              bool first = false;
+              if (p0 + lane < hi) {
+                const uint32_t i = B[p0 + lane];
+                if (iv[i] == int32_t(kv + 1)) {
+                  ww = __fdiv_rn(1.0f, ezt2[i]);
+                  zw = __fmul_rn(__fsub_rn(zt[i], zc), ww);
+                  first = izt[i] == 1;
+                }
+              }
+              const uint32_t m1 = __ballot_sync(0xffffffffu, first);
+              const uint32_t n = hi - p0 < 32 ? hi - p0 : 32;
+#pragma unroll 4
+              for (uint32_t k = 0; k < n; ++k) {
+                const float a = __shfl_sync(0xffffffffu, zw, k), b = __shfl_sync(0xffffffffu, ww, k);
+                if ((m1 >> k) & 1u) { znew0 = __fadd_rn(znew0, a); w0 = __fadd_rn(w0, b); }
+                else { znew1 = __fadd_rn(znew1, a); w1 = __fadd_rn(w1, b); }
+              }
             }
             znew0 = __fdiv_rn(znew0, w0);
             znew1 = __fdiv_rn(znew1, w1);
-            for (uint32_t p = lo; p < hi; ++p) {
+            bool moved = false;
+            for (uint32_t p = lo + lane; p < hi; p += 32) {
               const uint32_t i = B[p];
               if (iv[i] != int32_t(kv + 1)) continue;
               const float zz = __fsub_rn(zt[i], zc);
               const float d0 = fabsf(__fsub_rn(znew0, zz)), d1 = fabsf(__fsub_rn(znew1, zz));
               const uint8_t newer = d0 < d1 ? 1 : 2;
-              more |= newer != izt[i];
+              moved |= newer != izt[i];
               izt[i] = newer;
             }
+            more = __any_sync(0xffffffffu, moved);
             if (--iter <= 0) more = false;
           }
           if (!(w0 == 0 || w1 == 0)) {
@@ -600,111 +677,176 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, int e, uint32_t n
           }
         }
       }
-      uint32_t tot;
-      const uint32_t ex = block_excl_scan(split ? 1u : 0u, sh, &tot);
-      if (split) {
-        const uint32_t slot = s_nvi + ex;  // 0-based id of the new vertex
-        const int32_t newv = int32_t(slot + 1);
-        if (slot < uint32_t(kMaxVtx)) s_parent[slot] = uint16_t(kv);
-        for (uint32_t p = lo; p < hi; ++p) {
-          const uint32_t i = B[p];
-          if (iv[i] == int32_t(kv + 1) && izt[i] == 2) iv[i] = TI(newv);
-        }
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) s_nvi += tot;
-      __syncthreads();
+      if (lane == 0) S.vcnt[kv] = split ? 1u : 0u;
     }
-    if (threadIdx.x == 0 && s_nvi >= uint32_t(kMaxVtx)) { s_warn |= kWarnVertex; s_nvi = kMaxVtx - 1; }
+    __syncthreads();
+    // ids of the new vertices (0xffffffff: not split)
+    uint32_t base = S.nvi;
+    for (uint32_t b = 0; b < nvf; b += blockDim.x) {
+      const uint32_t kv = b + threadIdx.x;
+      const bool split = kv < nvf && S.vcnt[kv] != 0;
+      uint32_t tot;
+      const uint32_t slot = base + block_excl_scan(split ? 1u : 0u, S.sh, &tot);
+      if (split && slot < uint32_t(kMaxVtx)) S.parent[slot] = uint16_t(kv);
+      if (kv < nvf) S.vcnt[kv] = split ? slot : 0xffffffffu;
+      base += tot;
+    }
+    __syncthreads();
+    for (uint32_t kv = wid; kv < nvf; kv += nwarp) {
+      const uint32_t slot = S.vcnt[kv];
+      if (slot == 0xffffffffu) continue;
+      for (uint32_t p = S.voff[kv] + lane; p < S.voff[kv + 1]; p += 32) {
+        const uint32_t i = B[p];
+        if (iv[i] == int32_t(kv + 1) && izt[i] == 2) iv[i] = TI(slot + 1);
+      }
+    }
+    if (threadIdx.x == 0) {
+      if (base >= uint32_t(kMaxVtx)) { atomicOr(&S.warn, kWarnVertex); base = kMaxVtx - 1; }
+      S.nvi = base;
+    }
     __syncthreads();
   }
   fit(5000.);
   // sort_by_pt2, :391-436 (the sorted order itself is dropped by the reference)
-  const uint32_t nvf = s_nv;
+  const uint32_t nvf = S.nv;
   if (nvf >= 1) {
     for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) d.idv[tb + itrk[i]] = int16_t(iv[i]);
-    for (uint32_t v = threadIdx.x; v < nvf; v += blockDim.x) {
-      const uint32_t pv = s_parent[v], lo = s_voff[pv], hi = s_voff[pv + 1];
+    for (uint32_t v = wid; v < nvf; v += nwarp) {
+      const uint32_t pv = S.parent[v], lo = S.voff[pv], hi = S.voff[pv + 1];
       float s = 0;
-      for (uint32_t p = lo; p < hi; ++p) {
-        const uint32_t i = B[p];
-        if (iv[i] == int32_t(v + 1)) s = __fadd_rn(s, ptt2[i]);
+      for (uint32_t p0 = lo; p0 < hi; p0 += 32) {
+        float x = 0.f;
+        if (p0 + lane < hi) {
+          const uint32_t i = B[p0 + lane];
+          if (iv[i] == int32_t(v + 1)) x = ptt2[i];
+        }
+        s = ordered_add(x, hi - p0, s);
       }
-      ptv2[v] = s;
+      if (lane == 0) ptv2[v] = s;
     }
     if (threadIdx.x == 0 && nvf == 1) sort_ind[0] = 1;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     E.n_vtx = nvf;
-    if (s_warn) E.warnings |= s_warn;
+    if (S.warn) E.warnings |= S.warn;
   }
 }
 
-__global__ void __launch_bounds__(kVtxThreads) k_vertices(Dev d) {
-  const int e = blockIdx.x;
-  EvInfo& E = d.ev[e];
+// zeroes the event's vertex products and selects its tracks (load_tracks, :51-82: >= 4 hits, loose,
+// pt >= 0.5, in tuple order); returns their number. A warp looks at 128 consecutive tuples per step,
+// its loads in flight together.
+__device__ __forceinline__ uint32_t vertex_tracks(const Dev& d, EvInfo& E, int e, uint32_t* sh) {
   const uint64_t tb = E.tuple_base;
   const uint32_t ntu = E.n_tuples;
-  float* zv = d.zv + size_t(e) * kMaxVtx;
-  float* wv = d.wv + size_t(e) * kMaxVtx;
-  float* vchi2 = d.vchi2 + size_t(e) * kMaxVtx;
-  float* ptv2 = d.ptv2 + size_t(e) * kMaxVtx;
-  uint16_t* sort_ind = d.sort_ind + size_t(e) * kMaxVtx;
   int32_t* nn = d.ndof + tb + size_t(e) * kMaxVtx;  // length n_tuples + 1024
-  float* zt = d.vws_zt + tb;
-  float* ezt2 = d.vws_ezt2 + tb;
-  float* ptt2 = d.vws_ptt2 + tb;
-  int32_t* iv = d.vws_iv + tb;     // 1-based values as the reference stores them
-  uint32_t* itrk = d.vws_itrk + tb;
-  uint8_t* izt = d.vws_izt + tb;
-  __shared__ VtxShared S;
-  __shared__ float s_zt[kVtxSmemTracks], s_ezt2[kVtxSmemTracks];
-  __shared__ int16_t s_iv[kVtxSmemTracks], s_nn[kVtxSmemTracks];
-  __shared__ uint16_t s_b[kVtxSmemTracks];
-  __shared__ uint8_t s_izt[kVtxSmemTracks];
-  uint32_t* sh = S.sh;
-  for (int v = threadIdx.x; v < kMaxVtx; v += blockDim.x) { zv[v] = 0; wv[v] = 0; vchi2[v] = 0; ptv2[v] = 0; sort_ind[v] = 0; }
+  for (uint32_t v = threadIdx.x; v < uint32_t(kMaxVtx); v += blockDim.x) {
+    const size_t g = size_t(e) * kMaxVtx + v;
+    d.zv[g] = 0; d.wv[g] = 0; d.vchi2[g] = 0; d.ptv2[g] = 0; d.sort_ind[g] = 0;
+  }
   for (uint32_t t = threadIdx.x; t < ntu + kMaxVtx; t += blockDim.x) nn[t] = 0;
   for (uint32_t t = threadIdx.x; t < ntu; t += blockDim.x) d.idv[tb + t] = -1;
-  if (threadIdx.x == 0) S.warn = 0;
-  // load_tracks (:51-82): >= 4 hits, loose, pt >= 0.5, in tuple order
+  constexpr int kStep = 4;
+  const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
   uint32_t nt = 0;
-  for (uint32_t b = 0; b < ntu; b += blockDim.x) {
-    const uint32_t t = b + threadIdx.x;
-    bool sel = false;
-    if (t < ntu) {
-      const uint64_t g = tb + t;
-      const uint32_t n = d.tuple_off[g + 1] - d.tuple_off[g];
-      sel = n >= 4 && d.quality[g] == 2 && !(d.t_pt[g] < 0.5f);
+  for (uint32_t b = 0; b < ntu; b += kStep * blockDim.x) {
+    const uint32_t t0 = b + wid * (32 * kStep) + lane;
+    uint32_t n[kStep];
+    uint8_t q[kStep];
+    float pt[kStep];
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      const uint32_t t = t0 + 32 * u;
+      n[u] = 0;
+      if (t < ntu) {
+        n[u] = d.tuple_off[tb + t + 1] - d.tuple_off[tb + t];
+        q[u] = d.quality[tb + t];
+        pt[u] = d.t_pt[tb + t];
+      }
+    }
+    uint32_t m[kStep], cnt = 0;
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      m[u] = __ballot_sync(0xffffffffu, n[u] >= 4 && q[u] == 2 && !(pt[u] < 0.5f));
+      cnt += __popc(m[u]);
     }
     uint32_t tot;
-    const uint32_t ex = block_excl_scan(sel ? 1u : 0u, sh, &tot);
-    if (sel) {
-      const uint64_t g = tb + t;
-      const uint32_t i = nt + ex;
-      const float pt = d.t_pt[g];
-      itrk[i] = t;
-      zt[i] = d.t_state[5 * g + 4];
-      ezt2[i] = d.t_cov[15 * g + 14];
-      ptt2[i] = __fmul_rn(pt, pt);
+    const uint32_t ex = block_excl_scan(lane == 0 ? cnt : 0u, sh, &tot);
+    uint32_t i0 = nt + __shfl_sync(0xffffffffu, ex, 0);
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) {
+      if ((m[u] >> lane) & 1u) {
+        const uint32_t t = t0 + 32 * u;
+        const uint64_t i = tb + i0 + __popc(m[u] & lt);
+        d.vws_itrk[i] = t;
+        d.vws_zt[i] = d.t_state[5 * (tb + t) + 4];
+        d.vws_ezt2[i] = d.t_cov[15 * (tb + t) + 14];
+        d.vws_ptt2[i] = __fmul_rn(pt[u], pt[u]);
+      }
+      i0 += __popc(m[u]);
     }
     nt += tot;
   }
   if (threadIdx.x == 0) E.n_vtx_tracks = nt;
   __syncthreads();
-  if (nt <= uint32_t(kVtxSmemTracks)) {
-    for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) { s_zt[i] = zt[i]; s_ezt2[i] = ezt2[i]; }
-    for (uint32_t i = threadIdx.x; i < uint32_t(kVtxSmemTracks); i += blockDim.x) s_nn[i] = 0;
+  return nt;
+}
+
+// Events e of the grid's stride. kSelect: the launch selects the tracks (else an earlier one did)
+// and takes the events of at most kCap tracks, and with kAll those above in global memory too;
+// without kSelect it takes the events above kVtxNarrowTracks.
+template <int kThreads, uint32_t kCap, bool kSelect, bool kAll>
+__global__ void __launch_bounds__(kThreads, 1) k_vertices(Dev d) {
+  extern __shared__ __align__(16) uint8_t s_vtx[];
+  VtxShared& S = *reinterpret_cast<VtxShared*>(s_vtx);
+  float* s_zt = reinterpret_cast<float*>(s_vtx + (sizeof(VtxShared) + 15) / 16 * 16);
+  float* s_ezt2 = s_zt + kCap;
+  int16_t* s_iv = reinterpret_cast<int16_t*>(s_ezt2 + kCap);
+  int16_t* s_nn = s_iv + kCap;
+  uint16_t* s_b = reinterpret_cast<uint16_t*>(s_nn + kCap);
+  uint16_t* s_c = s_b + kCap;
+  uint8_t* s_izt = reinterpret_cast<uint8_t*>(s_c + kCap);
+  for (int e = blockIdx.x; e < d.E; e += gridDim.x) {
+    EvInfo& E = d.ev[e];
+    const uint64_t tb = E.tuple_base;
+    uint32_t nt;
+    if (kSelect) {
+      nt = vertex_tracks(d, E, e, S.sh);
+      if (!kAll && nt > kCap) continue;
+    } else {
+      nt = E.n_vtx_tracks;
+      if (nt <= kVtxNarrowTracks) continue;
+    }
+    if (threadIdx.x == 0) S.warn = 0;
+    float* zv = d.zv + size_t(e) * kMaxVtx;
+    float* wv = d.wv + size_t(e) * kMaxVtx;
+    float* vchi2 = d.vchi2 + size_t(e) * kMaxVtx;
+    float* ptv2 = d.ptv2 + size_t(e) * kMaxVtx;
+    uint16_t* sort_ind = d.sort_ind + size_t(e) * kMaxVtx;
+    int32_t* nn = d.ndof + tb + size_t(e) * kMaxVtx;
+    const float* ptt2 = d.vws_ptt2 + tb;
+    const uint32_t* itrk = d.vws_itrk + tb;
+    if (nt <= kCap) {
+      for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
+        s_zt[i] = d.vws_zt[tb + i];
+        s_ezt2[i] = d.vws_ezt2[tb + i];
+      }
+      // neighbour counts of the tracks, then ndof of the vertices: the reference's nn array
+      const uint32_t nz = nt > uint32_t(kMaxVtx) ? nt : uint32_t(kMaxVtx);
+      for (uint32_t i = threadIdx.x; i < nz; i += blockDim.x) s_nn[i] = 0;
+      __syncthreads();
+      const VtxTracks<int16_t, uint16_t> A{s_zt, s_ezt2, s_iv, s_nn, s_b, s_c, s_izt};
+      vertex_core(d, E, nt, A, ptt2, itrk, zv, wv, vchi2, ptv2, sort_ind, S);
+      const uint32_t nw = nt > S.nv ? nt : S.nv;
+      for (uint32_t i = threadIdx.x; i < nw; i += blockDim.x) nn[i] = s_nn[i];
+    } else if (kAll) {
+      __syncthreads();
+      const VtxTracks<int32_t, uint32_t> A{d.vws_zt + tb, d.vws_ezt2 + tb, d.vws_iv + tb, nn, d.vws_bins + tb,
+                                           d.vws_list + tb, d.vws_izt + tb};
+      vertex_core(d, E, nt, A, ptt2, itrk, zv, wv, vchi2, ptv2, sort_ind, S);
+    }
     __syncthreads();
-    vertex_core<int16_t, uint16_t>(d, E, e, nt, s_zt, s_ezt2, ptt2, itrk, s_iv, s_nn, s_izt, s_b, zv, wv, vchi2, ptv2,
-                                   sort_ind, S);
-    // neighbour counts of the tracks, then ndof of the vertices: the reference's nn array
-    const uint32_t nw = nt > S.nv ? nt : S.nv;
-    for (uint32_t i = threadIdx.x; i < nw; i += blockDim.x) nn[i] = s_nn[i];
-  } else {
-    vertex_core<int32_t, uint32_t>(d, E, e, nt, zt, ezt2, ptt2, itrk, iv, nn, izt, d.vws_bins + tb, zv, wv, vchi2,
-                                   ptv2, sort_ind, S);
   }
 }
 
@@ -733,14 +875,28 @@ void launch_classify(const Dev& d, const Launch& L) {
 }
 
 int prepare_select_kernels() {
-  const cudaError_t err = cudaFuncSetAttribute(k_fast_dup_smem<kDupLargeTuples, kDupMaxTuples>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               int(dup_smem_bytes<kDupLargeTuples>()));
+  const int wide = int(vtx_smem_bytes(kVtxWideTracks));
+  cudaError_t err = cudaFuncSetAttribute(k_fast_dup_smem<kDupLargeTuples, kDupMaxTuples>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(dup_smem_bytes<kDupLargeTuples>()));
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(k_vertices<kVtxWideThreads, kVtxWideTracks, true, true>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, wide);
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(k_vertices<kVtxWideThreads, kVtxWideTracks, false, true>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, wide);
   return err == cudaSuccess ? 0 : -1;
 }
 
 void launch_vertices(const Dev& d, const Launch& L) {
-  k_vertices<<<d.E, kVtxThreads, 0, L.s>>>(d);
+  const size_t wide = vtx_smem_bytes(kVtxWideTracks), narrow = vtx_smem_bytes(kVtxNarrowTracks);
+  if (d.E <= 148) {  // at most one event per SM: the wide form for all
+    k_vertices<kVtxWideThreads, kVtxWideTracks, true, true><<<d.E, kVtxWideThreads, wide, L.s>>>(d);
+  } else {
+    k_vertices<kVtxNarrowThreads, kVtxNarrowTracks, true, false><<<d.E, kVtxNarrowThreads, narrow, L.s>>>(d);
+    if (d.tuples_per_event > kVtxNarrowTracks)
+      k_vertices<kVtxWideThreads, kVtxWideTracks, false, true><<<148, kVtxWideThreads, wide, L.s>>>(d);
+  }
   L.mark("vertices");
 }
 
