@@ -1143,7 +1143,6 @@ __global__ void k_tuple_bases(Dev d) {
     d.ev[e].tuple_base = uint32_t(v >> 32);
     d.ev[e].tuple_hit_base = uint32_t(v);
     // the pair list (cell, tuple) holds hits - tuples entries
-    d.ev[e].n_dup_cells = 0;
     return;
   }
   EvInfo& E = d.ev[e];
@@ -1160,8 +1159,6 @@ __global__ void k_tuple_bases(Dev d) {
     nt = 0;
   }
   E.n_tuples = nt;
-  E.n_dup_cells = 0;
-  E.dup_cell_base = 0;
 }
 
 // Tuple hit offsets end markers and the live sizes for the per-tuple loops. An event with more

@@ -4,9 +4,8 @@
 // kernel_triplet_cleaner) with the cuts of ca_hit_ntuplet_generator_kernels.jl:79-87,
 // and plugin-PixelVertexFinding/gpu_vertex_finder.jl:51-436.
 //
-// kernel_fast_duplicate_remover is order dependent (a cell sees the marks of the
-// cells before it), so it walks the cells in order within an event, one warp per
-// event, taking 32 cells at once when they share no track. The triplet cleaner only
+// kernel_fast_duplicate_remover is order dependent (a cell sees the marks of the cells before it);
+// it is solved as a fixed point over all cells at once. The triplet cleaner only
 // ever writes "dup" and tests "!= bad", so its hits run in parallel. Vertex sums keep
 // the reference's track order (a warp per vertex hands its tracks' terms over in order).
 #include <cstddef>
@@ -22,10 +21,13 @@ constexpr float kChi2Coeff[4] = {0.68177776f, 0.74609577f, -0.08035491f, 0.00315
 // kernel_classify_tracks
 __global__ void k_classify(Dev d) {
   const int e = blockIdx.y;
-  const EvInfo& E = d.ev[e];
+  EvInfo& E = d.ev[e];
   const uint64_t tb = E.tuple_base;
+  if (blockIdx.x == 0 && threadIdx.x == 0) { E.n_dup_cells = 0; E.n_dup_entries = 0; }  // filled by k_dup_cells
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < E.n_tuples; t += gridDim.x * blockDim.x) {
     const uint64_t g = tb + t;
+    d.dup_death0[g] = 0xffffffffu;
+    d.dup_death1[g] = 0xffffffffu;
     const uint32_t n = d.tuple_off[g + 1] - d.tuple_off[g];
     if (d.quality[g] == 1) continue;
     if (n < 3) continue;
@@ -45,238 +47,98 @@ __global__ void k_classify(Dev d) {
 }
 
 
-// kernel_fast_duplicate_remover: one warp per event, cells in order, qualities in global
-// memory; for the events above min_tuples tuples, which the shared-memory form cannot hold
-__global__ void k_fast_dup(Dev d, uint32_t min_tuples) {
-  const int e = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (e >= d.E) return;
-  const unsigned lane = threadIdx.x & 31u;
-  const EvInfo& E = d.ev[e];
-  if (E.n_cells == 0 || E.n_tuples <= min_tuples) return;
-  const uint64_t c_lo = E.cell_base, c_hi = c_lo + E.n_cells;
-  for (uint64_t wi = c_lo >> 5; wi <= (c_hi - 1) >> 5; ++wi) {
-   uint32_t bits = dup_word(d, wi, c_lo, c_hi);
-   while (bits) {
-    const uint32_t c = uint32_t(32 * wi) + uint32_t(__ffs(bits) - 1);
-    bits &= bits - 1;
-    const uint32_t l0 = d.ct_cnt[c];
-    uint32_t n = d.ct_cnt[c + 1] - l0;
-    if (n > uint32_t(kCellRows)) n = kCellRows;
-    // argmin |tip| over the loose tracks, first in list order on ties (strict <, mc = 10000)
-    float best = 10000.f;
-    uint32_t best_pos = 0xFFFFFFFFu;
-    for (uint32_t j = lane; j < n; j += 32) {
-      const uint32_t t = d.ct_list[l0 + j];
-      if (d.quality[t] == 2) {
-        const float s = fabsf(d.t_state[5 * size_t(t) + 1]);
-        if (s < best) { best = s; best_pos = j; }
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_down_sync(0xffffffffu, best, o);
-      const uint32_t op = __shfl_down_sync(0xffffffffu, best_pos, o);
-      if (ob < best || (ob == best && op < best_pos)) { best = ob; best_pos = op; }
-    }
-    best_pos = __shfl_sync(0xffffffffu, best_pos, 0);
-    const uint32_t im = best_pos == 0xFFFFFFFFu ? 0xFFFFFFFFu : d.ct_list[l0 + best_pos];
-    __syncwarp();
-    for (uint32_t j = lane; j < n; j += 32) {
-      const uint32_t t = d.ct_list[l0 + j];
-      if (d.quality[t] != 0 && t != im) d.quality[t] = 1;
-    }
-    __syncwarp();
-   }
-  }
-}
-
-// The same remover with the event's qualities in shared memory: one warp per event
-// stages the static part of 32 dup cells at a time (track lists and |tip|) into
-// shared memory, then walks the cells in order with shared-memory reads only. The
-// argmin takes the smallest |tip| bit pattern (|tip| >= 0 orders as its bits) and,
-// among equal ones, the first position: the reference's strict < in list order.
-constexpr int kDupMaxTuples = 32768;        // qualities of one event in shared memory (the reference's cap)
-constexpr int kDupLargeTuples = 256 * 1024;  // the same for extended-capacity events, 104 KB of shared memory
-constexpr int kDupStage = 1024;             // staged track entries per batch of cells
-
-template <int kMaxT>
-constexpr size_t dup_smem_bytes() { return 4 * (size_t(kMaxT) / 16 + size_t(kMaxT) / 32 + 2 * kDupStage + 33); }
-
-// qualities (0 bad, 1 dup, 2 loose) packed 2 bits per track, 16 per word
-__device__ __forceinline__ uint32_t q_get(const uint32_t* w, uint32_t t) { return (w[t >> 4] >> (2 * (t & 15))) & 3u; }
-__device__ __forceinline__ void q_set_dup(uint32_t* w, uint32_t t) {  // any non-bad quality -> dup
-  const uint32_t sh = 2 * (t & 15);
-  atomicAnd(&w[t >> 4], ~(2u << sh));
-  atomicOr(&w[t >> 4], 1u << sh);
-}
-
-// The inputs of the ordered walk, gathered with a whole CTA per event: the cells with two
-// or more tracks in cell order (from the bitmap), and for each its track entries (at most
-// kCellRows) as (event-local tuple id, |tip| bits), laid end to end with offsets.
-__global__ void __launch_bounds__(256) k_dup_prep(Dev d) {
-  const int e = blockIdx.x;
+// kernel_fast_duplicate_remover (…_impl.jl:244-280). The reference walks the cells in order: among
+// the loose tracks of a cell the one with the smallest |tip| stays (the first in the list on
+// ties) and the others become duplicates, which later cells no longer look at. So a track dies at
+// the first cell, in order, that also holds a still-loose track ahead of it in (|tip|, list order).
+// Whether that track is still loose there depends only on tracks ahead of it in turn, so the death
+// cells are the one fixed point of
+//   death(t) = min { c : t in c, a track u ahead of t in c has death(u) >= c },
+// reached from "nobody dies" in as many rounds as the longest such chain (three in events of pileup
+// 50 and 170). A round takes all cells at once. The walk in order, one warp per event, was a chain
+// of shared-memory latencies: 386 us for an event of pileup 50 and 1.92 ms for one of pileup 170.
+//
+// k_dup_cells gathers the cells with two or more loose tracks (614 of the 4160 cells with two or more
+// tracks at pileup 50): the tracks that are not loose can neither stay nor change. The cells carry
+// their index, so they are taken in any order.
+__global__ void __launch_bounds__(256) k_dup_cells(Dev d) {
+  const int e = blockIdx.y;
   EvInfo& E = d.ev[e];
-  __shared__ uint32_t sh[33];
-  if (E.n_cells == 0 || E.n_tuples > uint32_t(kDupLargeTuples)) {
-    if (threadIdx.x == 0) E.n_dup_cells = 0;
-    return;
-  }
+  if (E.n_cells == 0) return;
   const uint64_t tb = E.tuple_base;
   const uint64_t c_lo = E.cell_base, c_hi = c_lo + E.n_cells;
-  uint32_t* list = d.dup_list + c_lo;
-  // cells, in order
-  uint32_t ndup = 0;
-  for (uint64_t w0 = c_lo >> 5; w0 <= (c_hi - 1) >> 5; w0 += blockDim.x) {
-    const uint64_t wi = w0 + threadIdx.x;
-    uint32_t bits = wi <= (c_hi - 1) >> 5 ? dup_word(d, wi, c_lo, c_hi) : 0u;
-    uint32_t tot;
-    uint32_t pos = ndup + block_excl_scan(__popc(bits), sh, &tot);
-    for (; bits; bits &= bits - 1) list[pos++] = uint32_t(32 * wi) + uint32_t(__ffs(bits) - 1);
-    ndup += tot;
-  }
-  __syncthreads();
-  // entries
-  uint32_t* eoff = d.dup_eoff + c_lo + e;
   uint32_t* et = d.dup_et + E.tuple_hit_base;
   uint32_t* ek = d.dup_ek + E.tuple_hit_base;
-  uint32_t base = 0;
-  for (uint32_t q0 = 0; q0 < ndup; q0 += blockDim.x) {
-    const uint32_t q = q0 + threadIdx.x;
-    uint32_t n = 0, l0 = 0;
-    if (q < ndup) {
-      const uint32_t c = list[q];
-      l0 = d.ct_cnt[c];
-      n = d.ct_cnt[c + 1] - l0;
+  for (uint64_t wi = (c_lo >> 5) + blockIdx.x * blockDim.x + threadIdx.x; wi <= (c_hi - 1) >> 5;
+       wi += uint64_t(gridDim.x) * blockDim.x) {
+    for (uint32_t bits = dup_word(d, wi, c_lo, c_hi); bits; bits &= bits - 1) {
+      const uint64_t c = 32 * wi + uint32_t(__ffs(bits) - 1);
+      const uint32_t l0 = d.ct_cnt[c];
+      uint32_t n = d.ct_cnt[c + 1] - l0;
       if (n > uint32_t(kCellRows)) n = kCellRows;
-    }
-    uint32_t tot;
-    const uint32_t o = base + block_excl_scan(n, sh, &tot);
-    if (q < ndup) {
-      eoff[q] = o;
-      for (uint32_t j = 0; j < n; ++j) {
-        const uint32_t t = d.ct_list[l0 + j];
-        et[o + j] = uint32_t(t - tb);
-        ek[o + j] = __float_as_uint(fabsf(d.t_state[5 * size_t(t) + 1]));
+      uint64_t loose = 0;
+      for (uint32_t j = 0; j < n; ++j) loose |= uint64_t(d.quality[d.ct_list[l0 + j]] == 2) << j;
+      const uint32_t m = __popcll(loose);
+      if (m < 2) continue;
+      const uint32_t slot = atomicAdd(&E.n_dup_cells, 1u);
+      uint32_t o = atomicAdd(&E.n_dup_entries, m);
+      d.dup_cell[c_lo + slot] = uint32_t(c - c_lo);
+      d.dup_rng[c_lo + slot] = make_uint2(o, m);
+      for (; loose; loose &= loose - 1, ++o) {
+        const uint32_t t = d.ct_list[l0 + uint32_t(__ffsll(loose) - 1)];
+        et[o] = uint32_t(t - tb);
+        ek[o] = __float_as_uint(fabsf(d.t_state[5 * size_t(t) + 1]));  // |tip| >= 0 orders as its bits
       }
     }
-    base += tot;
-  }
-  if (threadIdx.x == 0) {
-    eoff[ndup] = base;
-    E.n_dup_cells = ndup;
   }
 }
+static_assert(kCellRows <= 64, "loose tracks of a cell as a 64-bit mask");
 
-// Events of kMinT < n_tuples <= kMaxT tuples (dynamic shared memory of dup_smem_bytes<kMaxT>()).
-template <int kMaxT, int kMinT>
-__global__ void __launch_bounds__(32) k_fast_dup_smem(Dev d) {
-  extern __shared__ uint32_t s_dup[];
-  uint32_t* s_q = s_dup;                          // [kMaxT / 16]
-  uint32_t* s_seen = s_q + kMaxT / 16;            // [kMaxT / 32]
-  uint32_t* s_t = s_seen + kMaxT / 32;            // [kDupStage]
-  uint32_t* s_tip = s_t + kDupStage;              // [kDupStage]
-  uint32_t* s_off = s_tip + kDupStage;            // [33]
-  const int e = blockIdx.x;
-  const unsigned lane = threadIdx.x;
-  const EvInfo& E = d.ev[e];
+// The rounds, one CTA per event; the death cells (event-local, 0xffffffff: none) start at none
+// (k_classify) and sit in global memory, of which an event uses a few KB.
+__global__ void k_dup_resolve(Dev d) {
+  const EvInfo& E = d.ev[blockIdx.x];
+  const uint32_t nc = E.n_dup_cells, ne = E.n_dup_entries;
+  if (nc == 0) return;
   const uint64_t tb = E.tuple_base;
-  const uint32_t nt = E.n_tuples;
-  if (nt > uint32_t(kMaxT) || nt <= uint32_t(kMinT)) return;  // another form handles such events
-  if (E.n_dup_cells == 0) return;
-  const uint32_t nw = (nt + 15) / 16;
-  for (uint32_t w = lane; w < nw; w += 32) {
-    uint32_t v = 0;
-    for (uint32_t k = 0; k < 16; ++k) {
-      const uint32_t t = 16 * w + k;
-      if (t < nt) v |= uint32_t(d.quality[tb + t] & 3u) << (2 * k);
-    }
-    s_q[w] = v;
-  }
-  for (uint32_t w = lane; w < uint32_t(kMaxT / 32); w += 32) s_seen[w] = 0;
-  __syncwarp();
-  // the event's cells with two or more tracks, in order, and their track entries as
-  // k_dup_prep laid them out: offsets (ndup + 1) and (tuple, |tip| bits) per entry
-  const uint32_t ndup = E.n_dup_cells;
-  const uint32_t* eoff = d.dup_eoff + E.cell_base + e;
+  const uint32_t* cell = d.dup_cell + E.cell_base;
+  const uint2* rng = d.dup_rng + E.cell_base;
   const uint32_t* et = d.dup_et + E.tuple_hit_base;
   const uint32_t* ek = d.dup_ek + E.tuple_hit_base;
-  for (uint32_t q0 = 0; q0 < ndup;) {
-    // stage up to 32 cells whose entries fit kDupStage
-    const uint32_t q = q0 + lane;
-    const uint32_t o_lo = eoff[q0];
-    const uint32_t o = q <= ndup ? eoff[q] : 0xffffffffu;
-    const uint32_t o_next = __shfl_down_sync(0xffffffffu, o, 1);
-    const uint32_t o_last = q0 + 32 <= ndup ? eoff[q0 + 32] : 0xffffffffu;
-    const uint32_t end = lane == 31 ? o_last : o_next;  // end of cell q's entries
-    const bool fits = q < ndup && end - o_lo <= uint32_t(kDupStage);
-    const uint32_t ncell = __popc(__ballot_sync(0xffffffffu, fits));
-    const uint32_t total = __shfl_sync(0xffffffffu, end, ncell - 1) - o_lo;
-    if (lane < ncell) s_off[lane] = o - o_lo;
-    if (lane == 0) s_off[ncell] = total;
-    for (uint32_t x = lane; x < total; x += 32) {
-      s_t[x] = et[o_lo + x];
-      s_tip[x] = ek[o_lo + x];
-    }
-    __syncwarp();
-    // cells that share no track are independent: when no track is listed twice in the
-    // stage, each lane takes one cell (same result as the ordered walk)
-    bool twice = false;
-    for (uint32_t x = lane; x < total; x += 32) {
-      const uint32_t t = s_t[x], bit = 1u << (t & 31);
-      twice |= (atomicOr(&s_seen[t >> 5], bit) & bit) != 0;
-    }
-    __syncwarp();
-    for (uint32_t x = lane; x < total; x += 32) s_seen[s_t[x] >> 5] = 0;
-    __syncwarp();
-    // |tip| < 10000 as the reference's initial best (mc = 10000, strict <)
-    const uint32_t lim = __float_as_uint(10000.f);
-    if (!__any_sync(0xffffffffu, twice)) {
-      if (lane < ncell) {
-        const uint32_t o = s_off[lane], nk = s_off[lane + 1] - o;
-        uint32_t best = lim, im = 0xffffffffu;
-        for (uint32_t j = 0; j < nk; ++j) {
-          const uint32_t t = s_t[o + j];
-          const uint32_t key = s_tip[o + j];
-          if (key < best && q_get(s_q, t) == 2) { best = key; im = t; }
-        }
-        for (uint32_t j = 0; j < nk; ++j) {
-          const uint32_t t = s_t[o + j];
-          if (t != im && q_get(s_q, t) != 0) q_set_dup(s_q, t);
-        }
+  uint32_t* cur = d.dup_death0 + tb;
+  uint32_t* nxt = d.dup_death1 + tb;
+  for (uint32_t round = 0; round <= ne; ++round) {  // every round settles at least one more track
+    for (uint32_t i = threadIdx.x; i < nc; i += blockDim.x) {
+      const uint32_t c = cell[i];
+      const uint2 r = rng[i];
+      uint32_t best = 0xffffffffu, pos = 0;
+      for (uint32_t x = r.x; x < r.x + r.y; ++x) {
+        const uint32_t key = ek[x];
+        if (__ldcg(&cur[et[x]]) >= c && key < best) { best = key; pos = x; }
       }
-      __syncwarp();
-      q0 += ncell;
-      continue;
+      if (best == 0xffffffffu) continue;
+      for (uint32_t x = r.x; x < r.x + r.y; ++x) {
+        const uint32_t key = ek[x];
+        if (key > best || (key == best && x > pos)) atomicMin(&nxt[et[x]], c);
+      }
     }
-    for (uint32_t k = 0; k < ncell; ++k) {
-      const uint32_t o = s_off[k], nk = s_off[k + 1] - o;
-      uint32_t key0 = 0xffffffffu, key1 = 0xffffffffu, q0v = 0, q1v = 0;
-      uint32_t t0 = 0, t1 = 0;
-      if (lane < nk) {
-        t0 = s_t[o + lane];
-        q0v = q_get(s_q, t0);
-        if (q0v == 2) key0 = s_tip[o + lane];
-      }
-      if (lane + 32 < nk) {
-        t1 = s_t[o + lane + 32];
-        q1v = q_get(s_q, t1);
-        if (q1v == 2) key1 = s_tip[o + lane + 32];
-      }
-      if (key0 >= lim) key0 = 0xffffffffu;
-      if (key1 >= lim) key1 = 0xffffffffu;
-      const uint32_t kmin = __reduce_min_sync(0xffffffffu, key0 < key1 ? key0 : key1);
-      uint32_t im = 0xffffffffu;
-      if (kmin != 0xffffffffu) {
-        const uint32_t pos = __reduce_min_sync(0xffffffffu, key0 == kmin ? lane : (key1 == kmin ? lane + 32 : 0xffffffffu));
-        im = s_t[o + pos];
-      }
-      if (lane < nk && q0v != 0 && t0 != im) q_set_dup(s_q, t0);
-      if (lane + 32 < nk && q1v != 0 && t1 != im) q_set_dup(s_q, t1);
-      __syncwarp();
+    __syncthreads();
+    bool moved = false;
+    for (uint32_t x = threadIdx.x; x < ne; x += blockDim.x) {
+      const uint32_t t = et[x];
+      moved |= __ldcg(&cur[t]) != __ldcg(&nxt[t]);
     }
-    q0 += ncell;
+    if (!__syncthreads_or(moved)) break;
+    for (uint32_t x = threadIdx.x; x < ne; x += blockDim.x) cur[et[x]] = 0xffffffffu;
+    __syncthreads();
+    uint32_t* t = cur;
+    cur = nxt;
+    nxt = t;
   }
-  __syncwarp();
-  for (uint32_t t = lane; t < nt; t += 32) d.quality[tb + t] = uint8_t(q_get(s_q, t));
+  for (uint32_t x = threadIdx.x; x < ne; x += blockDim.x) {
+    const uint32_t t = et[x];
+    if (__ldcg(&cur[t]) != 0xffffffffu) d.quality[tb + t] = 1;
+  }
 }
 
 // hit -> loose tuple lists
@@ -856,14 +718,9 @@ void launch_classify(const Dev& d, const Launch& L) {
   auto g = [&](int seg) { return dim3(L.bpe_of(seg), d.E); };
   k_classify<<<g(kTuneClassify), 256, 0, L.s>>>(d);
   L.mark("classify");
-  // events by tuple count: shared-memory qualities up to 32K tuples (every event at the
-  // reference's capacities), a 104 KB form up to 256K, global memory above
-  k_dup_prep<<<d.E, 256, 0, L.s>>>(d);
-  k_fast_dup_smem<kDupMaxTuples, 0><<<d.E, 32, dup_smem_bytes<kDupMaxTuples>(), L.s>>>(d);
-  if (d.tuples_per_event > uint32_t(kDupMaxTuples)) {
-    k_fast_dup_smem<kDupLargeTuples, kDupMaxTuples><<<d.E, 32, dup_smem_bytes<kDupLargeTuples>(), L.s>>>(d);
-  }
-  if (d.tuples_per_event > uint32_t(kDupLargeTuples)) k_fast_dup<<<div_up(d.E, 4), 128, 0, L.s>>>(d, kDupLargeTuples);
+  k_dup_cells<<<g(kTuneClassify), 256, 0, L.s>>>(d);
+  // a CTA per event: many threads where an SM has one event to itself, several events per SM else
+  k_dup_resolve<<<d.E, d.E <= 148 ? 1024 : 256, 0, L.s>>>(d);
   L.mark("fast_duplicate_remover");
   cudaMemsetAsync(d.htt_cur, 0, size_t(d.cap_hits) * sizeof(uint32_t), L.s);
   k_hit_to_tuple<0><<<g(kTuneHitToTuple), 256, 0, L.s>>>(d);
@@ -876,12 +733,8 @@ void launch_classify(const Dev& d, const Launch& L) {
 
 int prepare_select_kernels() {
   const int wide = int(vtx_smem_bytes(kVtxWideTracks));
-  cudaError_t err = cudaFuncSetAttribute(k_fast_dup_smem<kDupLargeTuples, kDupMaxTuples>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(dup_smem_bytes<kDupLargeTuples>()));
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_vertices<kVtxWideThreads, kVtxWideTracks, true, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, wide);
+  cudaError_t err = cudaFuncSetAttribute(k_vertices<kVtxWideThreads, kVtxWideTracks, true, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, wide);
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(k_vertices<kVtxWideThreads, kVtxWideTracks, false, true>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, wide);

@@ -91,7 +91,7 @@ struct EvInfo {
   uint32_t n_errors, error_base;
   uint32_t warnings;
   uint32_t tm_off[9];               // tuple multiplicity offsets (bins 1..8, reference layout)
-  uint32_t n_dup_cells, dup_cell_base;
+  uint32_t n_dup_cells, n_dup_entries;  // cells with two or more loose tracks, and their entries
   uint32_t n_cols_nb, n_cols_tr;    // non-empty neighbour / track lists (column store use)
   uint32_t n_fit3, n_fit4;          // tuples fitted with 3 and with 4 hits (fit5as4 included)
   uint32_t n_refit3, n_refit4;      // of those, mixed-precision fits redone in FP64
@@ -214,12 +214,14 @@ struct Dev {
   uint32_t* htt_cnt;       // [cap_hits + 1]
   uint32_t* htt_cur;
   uint32_t* htt_list;      // [cap_tuple_hits]
-  // cells with >= 2 tracks, compacted per event
+  // duplicate removal, packed per event
   uint32_t* dup_bits;      // [cap_cells / 32 + 2] cells with two or more tracks, one bit each
-  uint32_t* dup_list;      // [cap_cells] those cells in order, at the event's cell base
-  uint32_t* dup_eoff;      // [cap_cells + E + 1] their entry offsets, at cell base + event index
+  uint32_t* dup_cell;      // [cap_cells] event-local index of the cells with two or more loose tracks, at the cell base
+  uint2* dup_rng;          // [cap_cells] first entry and number of entries of each of them
   uint32_t* dup_et;        // [cap_tuple_hits] entries: event-local tuple id, at the tuple-hit base
   uint32_t* dup_ek;        // [cap_tuple_hits] entries: |tip| bits
+  uint32_t* dup_death0;    // [cap_tuples] cell at which the duplicate remover drops the track (two rounds' values)
+  uint32_t* dup_death1;
   // vertices, per event
   int16_t* idv;            // [cap_tuples] per tuple (global tuple index), -1 when unused
   float* vws_zt; float* vws_ezt2; float* vws_ptt2;  // [cap_tuples] vertex-finder workspace per selected track
