@@ -20,6 +20,13 @@
 //    |r0| so that the linearisation circle passes exactly through hit 0.
 //    The line fit works on (S, Z) relative to hit 0 and moves the intercept
 //    back in FP64.
+//  * Few divisions and transcendental calls. A fit is one thread's chain of FP64
+//    operations: its time is the length of that chain and of its code, which
+//    must stream through the instruction cache (a quarter of the stalls). So
+//    every divisor is inverted once and shared (segment lengths, scattering
+//    variances, pivots, hit radii), a segment's scattering variance is computed
+//    once for its two kinks, and the Karimaki translations carry the direction
+//    as a unit vector, so that an angle is taken only at the end.
 // T is the working type of the hit geometry, the weights, the multiple-
 // scattering variances, the band-matrix entries and the chi2: T = double is the
 // FP64 fit, T = float the mixed-precision fit.
@@ -42,6 +49,29 @@ template <> BL_HD float s_atan<float>(float x) { return atanf(x); }
 template <class T> BL_HD T s_log(T x);
 template <> BL_HD double s_log<double>(double x) { return log(x); }
 template <> BL_HD float s_log<float>(float x) { return logf(x); }
+// 1 / sqrt(x) (host: two operations)
+template <class T> BL_HD T s_rsqrt(T x) {
+#ifdef __CUDA_ARCH__
+  return rsqrt(x);
+#else
+  return T(1) / s_sqrt<T>(x);
+#endif
+}
+// a b, rounded (not contracted into a following sum)
+BL_HD double s_mul(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+BL_HD float s_mul(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
 template <class T> BL_HD T s_abs(T x) { return x < T(0) ? -x : x; }
 
 constexpr double kPi = 3.141592653589793;
@@ -56,24 +86,23 @@ BL_HD T bl_atan2(T y, T x) {
   return T(NAN);
 }
 
-// multiple-scattering variance of one segment (broken_line.jl:46-57)
+// multiple-scattering variance of one segment (broken_line.jl:46-57), without the factor
+// mult_scatt_scale that the segments of a track share
 template <class T>
-BL_HD T mult_scatt(T length, T B, T R, T slope) {
-  T pt2 = B * R;
-  pt2 = pt2 < T(20.0) ? pt2 : T(20.0);
-  pt2 = pt2 * pt2;
+BL_HD T mult_scatt_len(T length, T& lt) {
   const T XXI_0 = T(0.06 / 16.0);
-  const T fact = T(0.7 * ((13.6 / 1000) * (13.6 / 1000)));
   const T abs_len = s_abs(length) * XXI_0;
-  const T lt = T(1) + T(0.038) * s_log<T>(abs_len);
-  return fact / (pt2 * (T(1) + slope * slope)) * abs_len * (lt * lt);
+  lt = T(1) + T(0.038) * s_log<T>(abs_len);
+  return abs_len * (lt * lt);
 }
 
 template <class T>
-BL_HD void rotation_matrix(T slope, T R[2][2]) {
-  const T a = T(1) / s_sqrt<T>(T(1) + slope * slope);
-  const T b = slope * a;
-  R[0][0] = a; R[0][1] = b; R[1][0] = -b; R[1][1] = a;
+BL_HD T mult_scatt_scale(T B, T R, T slope) {
+  T pt2 = B * R;
+  pt2 = pt2 < T(20.0) ? pt2 : T(20.0);
+  pt2 = pt2 * pt2;
+  const T fact = T(0.7 * ((13.6 / 1000) * (13.6 / 1000)));
+  return fact / (pt2 * (T(1) + slope * slope));
 }
 
 // Power of the point p with respect to the circle through the local origin whose
@@ -120,40 +149,44 @@ BL_HD T diff_of_products(T a, T d, T b, T c) {
 template <int N, bool Border>
 struct Band {
   static constexpr int M = N + (Border ? 1 : 0);
-  double D[M];   // pivots
+  double iD[M];  // 1 / pivots
   double l1[N];  // L[k][k-1]
   double l2[N];  // L[k][k-2]
   double g[N];   // L[border][k]
 };
 
-// d: diagonal, e1[k]: entry (k, k+1), e2[k]: entry (k, k+2), b[k]: (border, k), c: (border, border)
+// d: diagonal, e1[k]: entry (k, k+1), e2[k]: entry (k, k+2), b[k]: (border, k), c: (border, border).
+// t1 and tg are the entries of row k before the division by the pivot (L D).
 template <int N, bool Border>
 BL_HD void band_factor(const double d[N], const double e1[N], const double e2[N],
                                             const double b[N], double c, Band<N, Border>& f) {
+  double dn = c;
+  double tg[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    double l2 = 0.0, l1 = 0.0;
-    if (k >= 2) l2 = e2[k - 2] / f.D[k - 2];
-    if (k >= 1) l1 = (e1[k - 1] - (k >= 2 ? l2 * f.D[k - 2] * f.l1[k - 1] : 0.0)) / f.D[k - 1];
+    double l2 = 0.0, l1 = 0.0, t1 = 0.0;
+    if (k >= 2) l2 = e2[k - 2] * f.iD[k - 2];
+    if (k >= 1) {
+      t1 = e1[k - 1];
+      if (k >= 2) t1 -= e2[k - 2] * f.l1[k - 1];
+      l1 = t1 * f.iD[k - 1];
+    }
     f.l1[k] = l1;
     f.l2[k] = l2;
     double dk = d[k];
-    if (k >= 1) dk -= l1 * l1 * f.D[k - 1];
-    if (k >= 2) dk -= l2 * l2 * f.D[k - 2];
-    f.D[k] = dk;
+    if (k >= 1) dk -= l1 * t1;
+    if (k >= 2) dk -= l2 * e2[k - 2];
+    f.iD[k] = 1.0 / dk;
     if constexpr (Border) {
       double gk = b[k];
-      if (k >= 1) gk -= f.g[k - 1] * f.D[k - 1] * l1;
-      if (k >= 2) gk -= f.g[k - 2] * f.D[k - 2] * l2;
-      f.g[k] = gk / dk;
+      if (k >= 1) gk -= tg[k - 1] * l1;
+      if (k >= 2) gk -= tg[k - 2] * l2;
+      tg[k] = gk;
+      f.g[k] = gk * f.iD[k];
+      dn -= f.g[k] * gk;
     }
   }
-  if constexpr (Border) {
-    double dn = c;
-#pragma unroll
-    for (int k = 0; k < N; ++k) dn -= f.g[k] * f.g[k] * f.D[k];
-    f.D[N] = dn;
-  }
+  if constexpr (Border) f.iD[N] = 1.0 / dn;
 }
 
 // solves the system for a right-hand side that is zero on the border; x[M]
@@ -175,7 +208,7 @@ BL_HD void band_solve(const Band<N, Border>& f, const double r[N], double x[Band
     y[N] = v;
   }
 #pragma unroll
-  for (int k = 0; k < M; ++k) y[k] /= f.D[k];
+  for (int k = 0; k < M; ++k) y[k] *= f.iD[k];
   if constexpr (Border) x[N] = y[N];
 #pragma unroll
   for (int k = N - 1; k >= 0; --k) {
@@ -198,10 +231,10 @@ BL_HD void band_trailing_inverse(const Band<N, Border>& f, double inv[3][3]) {
   if constexpr (Border) {
     gb = f.g[N - 2];
     gc = f.g[N - 1];
-    idn = 1.0 / f.D[N];
+    idn = f.iD[N];
   }
   const double Mi[3][3] = {{1.0, 0.0, 0.0}, {-a, 1.0, 0.0}, {a * gc - gb, -gc, 1.0}};
-  const double iD[3] = {1.0 / f.D[N - 2], 1.0 / f.D[N - 1], idn};
+  const double iD[3] = {f.iD[N - 2], f.iD[N - 1], idn};
   double blk[3][3];
 #pragma unroll
   for (int p = 0; p < 3; ++p)
@@ -220,38 +253,39 @@ BL_HD void band_trailing_inverse(const Band<N, Border>& f, double inv[3][3]) {
     for (int q = 0; q < 3; ++q) inv[p][q] = blk[o[p]][o[q]];
 }
 
-// band entries of matrixc_u (broken_line.jl:217-250) for weights w, abscissae S and
-// scattering variances VB, in elimination order (k = hit N-1-k)
+// inverse segment lengths h[i] = 1 / (S[i+1] - S[i])
 template <int N, class T>
-BL_HD void band_entries(const T w[N], const T S[N], const T VB[N], double d[N], double e1[N],
-                                             double e2[N]) {
-  T dS[N];  // dS[i] = S[i+1] - S[i]
+BL_HD void inverse_segments(const T S[N], double h[N - 1]) {
 #pragma unroll
-  for (int i = 0; i + 1 < N; ++i) dS[i] = S[i + 1] - S[i];
-  dS[N - 1] = T(1);
-  T iv[N];  // 1 / VB at the interior hits
-#pragma unroll
-  for (int i = 0; i < N; ++i) iv[i] = (i > 0 && i < N - 1) ? T(1) / VB[i] : T(0);
+  for (int i = 0; i + 1 < N; ++i) h[i] = 1.0 / (double(S[i + 1]) - double(S[i]));
+}
+
+// band entries of matrixc_u (broken_line.jl:217-250) for weights w, inverse segment lengths h and
+// inverse scattering variances iv (interior hits), in elimination order (k = hit N-1-k). The
+// kink at hit i is h[i-1] u[i-1] - (h[i-1] + h[i]) u[i] + h[i] u[i+1].
+template <int N>
+BL_HD void band_entries(const double w[N], const double h[N - 1], const double iv[N], double d[N], double e1[N],
+                        double e2[N]) {
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    T dg = w[i];
-    if (i > 1) dg += iv[i - 1] / (dS[i - 1] * dS[i - 1]);
+    double dg = w[i];
+    if (i > 1) dg += iv[i - 1] * (h[i - 1] * h[i - 1]);
     if (i > 0 && i < N - 1) {
-      const T q = (dS[i] + dS[i - 1]) / (dS[i] * dS[i - 1]);
+      const double q = h[i] + h[i - 1];
       dg += iv[i] * (q * q);
     }
-    if (i < N - 2) dg += iv[i + 1] / (dS[i] * dS[i]);
-    T o1 = T(0), o2 = T(0);
-    if (i > 0 && i < N - 1) o1 = -iv[i] / dS[i] * ((dS[i] + dS[i - 1]) / (dS[i] * dS[i - 1]));
+    if (i < N - 2) dg += iv[i + 1] * (h[i] * h[i]);
+    double o1 = 0.0, o2 = 0.0;
+    if (i > 0 && i < N - 1) o1 = -iv[i] * (h[i] * (h[i] + h[i - 1]));
     if (i < N - 2) {
-      o1 += -iv[i + 1] / dS[i] * ((dS[i + 1] + dS[i]) / (dS[i + 1] * dS[i]));
-      o2 = iv[i + 1] / (dS[i + 1] * dS[i]);
+      o1 -= iv[i + 1] * (h[i] * (h[i + 1] + h[i]));
+      o2 = iv[i + 1] * (h[i + 1] * h[i]);
     }
     const int k = N - 1 - i;
-    d[k] = double(dg);
+    d[k] = dg;
     // entry (i, i+1) is (k-1, k) in elimination order, (i, i+2) is (k-2, k)
-    if (i + 1 < N) e1[k - 1] = double(o1);
-    if (i + 2 < N) e2[k - 2] = double(o2);
+    if (i + 1 < N) e1[k - 1] = o1;
+    if (i + 2 < N) e2[k - 2] = o2;
   }
   e1[N - 1] = 0.0;
   e2[N - 2] = 0.0;
@@ -270,11 +304,16 @@ struct Prep {
   int q;
   T R, f3, slope;
   T cx, cy;       // fast-fit centre relative to hit 0
+  T alpha;        // angle at the centre from hit 0 to the last hit
   T rx[N], ry[N]; // hit - centre
+  T irn[N];       // 1 / their lengths
   T s[N];         // arc length relative to hit 0
   double s0;      // arc length of hit 0
   T S[N], Z[N];   // line-fit coordinates relative to hit 0
-  T VB[N];
+  T VB[N];        // scattering variances of the kinks (interior hits)
+  T ms0;          // that of the first segment
+  T scale;        // mult_scatt_scale
+  T lt[N];        // the segments' 1 + 0.038 log (radiation lengths)
   T Rl[2][2];     // line-fit rotation
 };
 
@@ -295,7 +334,8 @@ BL_HD void fast_fit(const Geo<N, T>& G, Prep<N, T>& P) {
   const T d1 = -P.cx, d2 = -P.cy;
   const T de = d1 * G.p[1][N - 1] - d2 * G.p[0][N - 1];
   const T dotde = d1 * d1 + d2 * d2 + d1 * G.p[0][N - 1] + d2 * G.p[1][N - 1];
-  P.f3 = P.R * bl_atan2<T>(de, dotde) / G.p[2][N - 1];
+  P.alpha = bl_atan2<T>(de, dotde);
+  P.f3 = P.R * P.alpha / G.p[2][N - 1];
 }
 
 // prepare_broken_line_data (broken_line.jl:150-207)
@@ -303,11 +343,19 @@ template <int N, class T>
 BL_HD void prepare(const Geo<N, T>& G, T B, Prep<N, T>& P) {
   const T x1 = G.p[0][1], y1 = G.p[1][1];
   const T xn = G.p[0][N - 1] - G.p[0][N - 2], yn = G.p[1][N - 1] - G.p[1][N - 2];
-  P.q = (x1 * yn - y1 * xn) > T(0) ? -1 : 1;
+  P.q = s_mul(x1, yn) - s_mul(y1, xn) > T(0) ? -1 : 1;  // collinear hits: exactly 0
   P.slope = -T(P.q) / P.f3;
-  rotation_matrix<T>(P.slope, P.Rl);
+  {
+    const T a = s_rsqrt<T>(T(1) + P.slope * P.slope);
+    const T b = P.slope * a;
+    P.Rl[0][0] = a; P.Rl[0][1] = b; P.Rl[1][0] = -b; P.Rl[1][1] = a;
+  }
 #pragma unroll
-  for (int i = 0; i < N; ++i) { P.rx[i] = G.p[0][i] - P.cx; P.ry[i] = G.p[1][i] - P.cy; }
+  for (int i = 0; i < N; ++i) {
+    P.rx[i] = G.p[0][i] - P.cx;
+    P.ry[i] = G.p[1][i] - P.cy;
+    P.irn[i] = s_rsqrt<T>(P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i]);
+  }
   const T ux = -P.cx, uy = -P.cy, uu = ux * ux + uy * uy;
   const T fac = T(P.q) * P.R;
   // the reference measures s from the direction centre -> origin: e ~ u - hit0
@@ -315,8 +363,9 @@ BL_HD void prepare(const Geo<N, T>& G, T B, Prep<N, T>& P) {
   P.s0 = double(fac * bl_atan2<T>(-(ux * hy - uy * hx), uu - (ux * hx + uy * hy)));
   P.s[0] = T(0);
 #pragma unroll
-  for (int i = 1; i < N; ++i)
+  for (int i = 1; i + 1 < N; ++i)
     P.s[i] = -fac * bl_atan2<T>(ux * G.p[1][i] - uy * G.p[0][i], uu + ux * G.p[0][i] + uy * G.p[1][i]);
+  P.s[N - 1] = -fac * P.alpha;  // the fast fit's angle
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     P.S[i] = P.Rl[0][0] * P.s[i] + P.Rl[0][1] * G.p[2][i];
@@ -324,9 +373,15 @@ BL_HD void prepare(const Geo<N, T>& G, T B, Prep<N, T>& P) {
   }
   P.VB[0] = T(0);
   P.VB[N - 1] = T(0);
+  P.scale = mult_scatt_scale<T>(B, P.R, P.slope);
+  T before = P.scale * mult_scatt_len<T>(P.S[1] - P.S[0], P.lt[0]);
+  P.ms0 = before;
 #pragma unroll
-  for (int i = 1; i < N - 1; ++i)
-    P.VB[i] = mult_scatt<T>(P.S[i + 1] - P.S[i], B, P.R, P.slope) + mult_scatt<T>(P.S[i] - P.S[i - 1], B, P.R, P.slope);
+  for (int i = 1; i < N - 1; ++i) {
+    const T after = P.scale * mult_scatt_len<T>(P.S[i + 1] - P.S[i], P.lt[i]);
+    P.VB[i] = after + before;
+    before = after;
+  }
 }
 
 BL_HD void sandwich2(const double J[2][2], double C[2][2]) {
@@ -355,7 +410,7 @@ BL_HD void line_weights(const float ge[6][N], const Prep<N, T>& P, T w[N]) {
     auto z = [&](float v) { return fabs(double(v)) < tol ? T(0) : T(v); };
     const T V[3][3] = {{T(ge[0][i]), z(ge[1][i]), z(ge[3][i])}, {z(ge[1][i]), T(ge[2][i]), z(ge[4][i])},
                        {z(ge[3][i]), z(ge[4][i]), T(ge[5][i])}};
-    const T tmp = T(1) / s_sqrt<T>(P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i]);
+    const T tmp = P.irn[i];
     const T J[2][3] = {{P.ry[i] * tmp, -P.rx[i] * tmp, T(0)}, {T(0), T(0), T(1)}};
     // second row of R J V J^T R^T
     T rj[3];
@@ -373,16 +428,18 @@ BL_HD void line_weights(const float ge[6][N], const Prep<N, T>& P, T w[N]) {
   }
 }
 
-// line-fit system: weights, band factorisation and solution u (hit order)
+// line-fit system: weights, inverse segments, band factorisation and solution u (hit order)
 template <int N, class T>
-BL_HD void line_system(const float ge[6][N], const Prep<N, T>& P, T w[N], Band<N, false>& f, double u[N]) {
+BL_HD void line_system(const float ge[6][N], const Prep<N, T>& P, const double iv[N], T w[N], double h[N - 1],
+                       Band<N, false>& f, double u[N]) {
   line_weights<N, T>(ge, P, w);
   // assembled in FP64, as the circle system (circle_system)
-  double wd[N], Sd[N], VBd[N];
+  double wd[N];
 #pragma unroll
-  for (int i = 0; i < N; ++i) { wd[i] = double(w[i]); Sd[i] = double(P.S[i]); VBd[i] = double(P.VB[i]); }
+  for (int i = 0; i < N; ++i) wd[i] = double(w[i]);
+  inverse_segments<N, T>(P.S, h);
   double d[N], e1[N], e2[N], r[N];
-  band_entries<N, double>(wd, Sd, VBd, d, e1, e2);
+  band_entries<N>(wd, h, iv, d, e1, e2);
 #pragma unroll
   for (int i = 0; i < N; ++i) r[N - 1 - i] = wd[i] * double(P.Z[i]);
   band_factor<N, false>(d, e1, e2, nullptr, 0.0, f);
@@ -392,25 +449,29 @@ BL_HD void line_system(const float ge[6][N], const Prep<N, T>& P, T w[N], Band<N
   for (int i = 0; i < N; ++i) u[i] = ue[N - 1 - i];
 }
 
+// inverse scattering variances of the line's kinks (interior hits)
+template <int N, class T>
+BL_HD void inverse_variances(const Prep<N, T>& P, double iv[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) iv[i] = (i > 0 && i < N - 1) ? 1.0 / double(P.VB[i]) : 0.0;
+}
+
 // BL_Line_fit (broken_line.jl:546-696)
 template <int N, class T>
-BL_HD void line_fit(const float ge[6][N], const Geo<N, T>& G, T B, const Prep<N, T>& P, LineOut& L) {
+BL_HD void line_fit(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>& P, const double iv[N], LineOut& L) {
   T w[N];
   Band<N, false> f;
-  double u[N];
-  line_system<N, T>(ge, P, w, f, u);
+  double u[N], h[N - 1];
+  line_system<N, T>(ge, P, iv, w, h, f, u);
   double I[3][3];
   band_trailing_inverse<N, false>(f, I);
   // absolute position of hit 0 in the rotated (S, Z) frame
   const double Sc = double(P.Rl[0][0]) * P.s0 + double(P.Rl[0][1]) * G.h0[2];
   const double Zc = double(P.Rl[1][0]) * P.s0 + double(P.Rl[1][1]) * G.h0[2];
-  const double dS0 = double(P.S[1]) - double(P.S[0]);
-  double par0 = (u[1] - u[0]) / dS0;
+  const double idiff = h[0];
+  double par0 = (u[1] - u[0]) * idiff;
   double par1 = (u[0] + Zc) - par0 * (double(P.S[0]) + Sc);
-  const double idiff = 1.0 / dS0;
-  double cov[2][2] = {{(I[0][0] - 2 * I[0][1] + I[1][1]) * (idiff * idiff) +
-                           double(mult_scatt<T>(P.S[1] - P.S[0], B, P.R, P.slope)),
-                       (I[0][1] - I[0][0]) * idiff},
+  double cov[2][2] = {{(I[0][0] - 2 * I[0][1] + I[1][1]) * (idiff * idiff) + double(P.ms0), (I[0][1] - I[0][0]) * idiff},
                       {(I[0][1] - I[0][0]) * idiff, I[0][0]}};
   double jac[2][2] = {{1, 0}, {-(double(P.S[0]) + Sc), 1}};
   sandwich2(jac, cov);
@@ -426,97 +487,95 @@ BL_HD void line_fit(const float ge[6][N], const Geo<N, T>& G, T B, const Prep<N,
   L.par[0] = par0;
   L.par[1] = par1;
   for (int a = 0; a < 2; ++a) for (int b = 0; b < 2; ++b) L.cov[a][b] = cov[a][b];
-  T chi2 = 0;
+  double chi2 = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const T diff = P.Z[i] - T(u[i]);
-    chi2 += w[i] * (diff * diff);
+    const double diff = double(P.Z[i]) - u[i];
+    chi2 += double(w[i]) * (diff * diff);
     if (i > 0 && i < N - 1) {
-      const T d1 = P.S[i] - P.S[i - 1], d2 = P.S[i + 1] - P.S[i];
-      const T t = T(u[i - 1]) / d1 - T(u[i]) * ((d1 + d2) / (d2 * d1)) + T(u[i + 1]) / d2;
-      chi2 += (t * t) / P.VB[i];
+      const double t = (u[i - 1] - u[i]) * h[i - 1] + (u[i + 1] - u[i]) * h[i];
+      chi2 += (t * t) * iv[i];
     }
   }
-  L.chi2 = double(chi2);
+  L.chi2 = chi2;
 }
 
-// Karimaki translation of (phi, d, rho) and its covariance to a point (x0, y0) (broken_line.jl:85-127).
-// With rot, the fit ran in a frame rotated by -theta (cos, sin = cr, sr): the direction vector
-// (C, BB) is turned back by theta before phi is taken, so phi comes out in the global frame and
-// on the reference's atan2 branch; d, rho and the covariance do not depend on the frame.
-BL_HD void translate_karimaki(CircleOut& c, double x0, double y0, bool rot = false, double cr = 1.0,
-                              double sr = 0.0) {
-  const double p1 = c.par[0], p2 = c.par[1], p3 = c.par[2];
-  double sn, cs;
-  sincos(p1, &sn, &cs);
+// Karimaki translation of (phi, d, rho) and its covariance to a point (x0, y0) (broken_line.jl:85-127);
+// the direction phi is carried as (cos, sin) = (cs, sn).
+BL_HD void translate_karimaki(double& cs, double& sn, CircleOut& c, double x0, double y0) {
+  const double p2 = c.par[1], p3 = c.par[2];
   const double DP = x0 * cs + y0 * sn;
   const double DO = x0 * sn - y0 * cs + p2;
   const double uu = 1.0 + p3 * p2;
   const double C = -p3 * y0 + uu * cs;
   const double BB = p3 * x0 + uu * sn;
-  const double A = 2.0 * DO + p3 * (DO * DO + DP * DP);
-  const double U = sqrt(1.0 + p3 * A);
-  const double xi = 1.0 / (BB * BB + C * C);
-  const double v = 1.0 + p3 * DO;
-  const double lambda = (0.5 * A) / (U * ((1.0 + U) * (1.0 + U)));
-  const double mu = 1.0 / (U * (1.0 + U)) + p3 * lambda;
   const double zeta = DO * DO + DP * DP;
+  const double A = 2.0 * DO + p3 * zeta;
+  const double U = sqrt(1.0 + p3 * A);
+  const double ixi = s_rsqrt<double>(BB * BB + C * C);
+  const double xi = ixi * ixi;
+  const double v = 1.0 + p3 * DO;
+  const double iu = 1.0 / (U * (1.0 + U));  // 1 / (1 + U) = U iu
+  const double au = A * (U * iu);           // A / (1 + U)
+  const double lambda = 0.5 * au * iu;
+  const double mu = iu + p3 * lambda;
   const double J[3][3] = {{xi * uu * v, -xi * (p3 * p3) * DP, xi * DP},
                           {2.0 * mu * uu * DP, 2.0 * mu * v, mu * zeta - lambda * A},
                           {0.0, 0.0, 1.0}};
-  if (rot) c.par[0] = bl_atan2<double>(C * sr + BB * cr, C * cr - BB * sr);
-  else c.par[0] = bl_atan2<double>(BB, C);
-  c.par[1] = A / (1.0 + U);
+  cs = C * ixi;
+  sn = BB * ixi;
+  c.par[1] = au;
   sandwich3(J, c.cov);
 }
 
-// circle-fit system: scaled scattering variances, radial residuals, weights, band
-// factorisation (border = curvature correction) and solution u[N+1] (hit order)
+// circle-fit system: inverse scaled scattering variances, radial residuals, weights, inverse
+// segments, band factorisation (border = curvature correction) and solution u[N+1] (hit order).
+// iv: inverse scattering variances of the line.
 template <int N, class T>
-BL_HD void circle_system(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>& P, T VB[N], T Z[N], T rn[N],
-                         T w[N], Band<N, true>& f, double u[N + 1]) {
-  const T ms_scale = T(1.0) + P.slope * P.slope;
-#pragma unroll
-  for (int i = 0; i < N; ++i) VB[i] = P.VB[i] * ms_scale;
+BL_HD void circle_system(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>& P, const double iv[N],
+                         double ivc[N], T Z[N], T w[N], double h[N - 1], Band<N, true>& f, double u[N + 1]) {
   // radial residuals of the hits to the fast-fit circle, which passes through hit 0
   const T ux = -P.cx, uy = -P.cy;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    rn[i] = s_sqrt<T>(P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i]);
     const T px = G.p[0][i], py = G.p[1][i];
-    Z[i] = power_of_point<T>(ux, uy, px, py) / (rn[i] + P.R);
+    const T rn = (P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i]) * P.irn[i];
+    Z[i] = power_of_point<T>(ux, uy, px, py) / (rn + P.R);
   }
   const double tol = 1e-12;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     auto z = [&](float v) { return fabs(double(v)) < tol ? T(0) : T(v); };
-    const T V[2][2] = {{z(ge[0][i]), z(ge[1][i])}, {z(ge[1][i]), z(ge[2][i])}};
-    T RR[2][2];
-    rotation_matrix<T>(-P.rx[i] / P.ry[i], RR);
-    const T t0 = RR[1][0] * V[0][0] + RR[1][1] * V[1][0];
-    const T t1 = RR[1][0] * V[0][1] + RR[1][1] * V[1][1];
-    w[i] = T(1.0) / (t0 * RR[1][0] + t1 * RR[1][1]);
+    // variance along the radius: the direction is the second row of the reference's rotation
+    const T hx = P.rx[i] * P.irn[i], hy = P.ry[i] * P.irn[i];
+    const T vxy = z(ge[1][i]);
+    w[i] = T(1.0) / ((hx * z(ge[0][i]) + hy * vxy) * hx + (hx * vxy + hy * z(ge[2][i])) * hy);
   }
   // The system is assembled in FP64 from the FP32 weights, arc lengths, scattering variances
   // and residuals: for a stiff track the scattering terms are large and nearly cancel against
   // each other in the elimination, and FP32 entries would cost the curvature correction digits
   // (which the fast-fit curvature then cancels further when the fast fit is far off).
-  double wd[N], sd[N], VBd[N];
+  double wd[N], D[N];  // D[i] = s[i+1] - s[i-1]
+  const double is = 1.0 / (1.0 + double(P.slope) * double(P.slope));
 #pragma unroll
-  for (int i = 0; i < N; ++i) { wd[i] = double(w[i]); sd[i] = double(P.s[i]); VBd[i] = double(VB[i]); }
+  for (int i = 0; i < N; ++i) {
+    wd[i] = double(w[i]);
+    ivc[i] = iv[i] * is;
+    D[i] = (i > 0 && i < N - 1) ? double(P.s[i + 1]) - double(P.s[i - 1]) : 0.0;
+  }
+  inverse_segments<N, T>(P.s, h);
   double d[N], e1[N], e2[N], b[N], r[N];
-  band_entries<N, double>(wd, sd, VBd, d, e1, e2);
-  const double* s = sd;
+  band_entries<N>(wd, h, ivc, d, e1, e2);
   double cnn = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     double v = 0;
-    if (i > 0 && i < N - 1) v += -(s[i + 1] - s[i - 1]) * (s[i + 1] - s[i - 1]) / (2.0 * VBd[i] * (s[i + 1] - s[i]) * (s[i] - s[i - 1]));
-    if (i > 1) v += (s[i] - s[i - 2]) / (2.0 * VBd[i - 1] * (s[i] - s[i - 1]));
-    if (i < N - 2) v += (s[i + 2] - s[i]) / (2.0 * VBd[i + 1] * (s[i + 1] - s[i]));
-    b[N - 1 - i] = v;
+    if (i > 0 && i < N - 1) v -= (ivc[i] * D[i]) * (h[i] + h[i - 1]);
+    if (i > 1) v += (ivc[i - 1] * D[i - 1]) * h[i - 1];
+    if (i < N - 2) v += (ivc[i + 1] * D[i + 1]) * h[i];
+    b[N - 1 - i] = 0.5 * v;
     r[N - 1 - i] = wd[i] * double(Z[i]);
-    if (i > 0 && i < N - 1) cnn += ((s[i + 1] - s[i - 1]) * (s[i + 1] - s[i - 1])) / (4.0 * VBd[i]);
+    if (i > 0 && i < N - 1) cnn += (D[i] * D[i]) * (0.25 * ivc[i]);
   }
   band_factor<N, true>(d, e1, e2, b, cnn, f);
   double ue[N + 1];
@@ -526,63 +585,65 @@ BL_HD void circle_system(const float ge[6][N], const Geo<N, T>& G, const Prep<N,
   u[N] = ue[N];
 }
 
-// BL_Circle_fit (broken_line.jl:330-528); returns false where the reference raises. rot, cr,
-// sr: the frame rotation of the hits (fit_track), undone on phi.
+// BL_Circle_fit (broken_line.jl:330-528); returns false where the reference raises. rot, cr, sr:
+// the fit ran in a frame rotated by -theta (cos, sin = cr, sr); the final direction is turned back by
+// theta before phi is taken, so phi comes out in the global frame and on the reference's atan2
+// branch; d, rho and the covariance do not depend on the frame.
 template <int N, class T>
-BL_HD bool circle_fit(const float ge[6][N], const Geo<N, T>& G, T B, const Prep<N, T>& P,
+BL_HD bool circle_fit(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>& P, const double iv[N],
                                            CircleOut& c, bool rot = false, double cr = 1.0, double sr = 0.0) {
   bool ok = true;
   c.q = P.q;
-  const T ms_scale = T(1.0) + P.slope * P.slope;
-  T VB[N], Z[N], rn[N], w[N];
+  T Z[N], w[N];
   Band<N, true> f;
-  double u[N + 1];
-  circle_system<N, T>(ge, G, P, VB, Z, rn, w, f, u);
-  const T* s = P.s;
+  double u[N + 1], ivc[N], h[N - 1];
+  circle_system<N, T>(ge, G, P, iv, ivc, Z, w, h, f, u);
   double I[3][3];
   band_trailing_inverse<N, true>(f, I);
   // fitted points 0 and 1 (hit-0 frame), FP64 from here on
-  const double R = double(P.R);
-  const double n0 = double(rn[0]), n1 = double(rn[1]);
-  const double r0x = double(P.rx[0]) / n0, r0y = double(P.ry[0]) / n0;
-  const double r1x = double(P.rx[1]) / n1, r1y = double(P.ry[1]) / n1;
+  const double R = double(P.R), q = double(c.q);
+  const double n0 = double(P.irn[0]), n1 = double(P.irn[1]);
+  const double r0x = double(P.rx[0]) * n0, r0y = double(P.ry[0]) * n0;
+  const double r1x = double(P.rx[1]) * n1, r1y = double(P.ry[1]) * n1;
   const double tmp1 = u[0] - double(Z[0]);
   const double dv0 = tmp1 * r0x, dv1 = tmp1 * r0y;
   const double tmp2 = u[1] - double(Z[1]);
   const double ev0 = double(G.p[0][1]) + tmp2 * r1x, ev1 = double(G.p[1][1]) + tmp2 * r1y;
   const double emd0 = ev0 - dv0, emd1 = ev1 - dv1;
   const double t1 = emd0 * emd0 + emd1 * emd1;
-  c.par[0] = bl_atan2<double>(emd1, emd0);
+  const double il = s_rsqrt<double>(t1), it1 = il * il;
+  double cs = emd0 * il, sn = emd1 * il;
   const double inner = R * R - 0.25 * t1;
   if (inner < 0) ok = false;
-  c.par[1] = -double(c.q) * (0.25 * t1) / (R + sqrt(inner));
-  c.par[2] = double(c.q) * (1.0 / R + u[N]);
-  if (!(double(c.q) * c.par[1] <= 0)) ok = false;
-  const double fl = floor(double(c.q) / 2);
-  const double den = sqrt((2 * R) * (2 * R) - t1);
+  const double half_den = sqrt(inner);  // sqrt((2 R)^2 - t1) = 2 sqrt(inner)
+  c.par[1] = -q * (0.25 * t1) / (R + half_den);
+  c.par[2] = q * (1.0 / R + u[N]);
+  if (!(q * c.par[1] <= 0)) ok = false;
+  const double fl = c.q < 0 ? -0.5 / half_den : 0.0 * half_den;  // floor(q / 2) / den
   const double J[3][3] = {
-      {(r0y * emd0 - emd1 * r0x) / t1, (r1y * emd0 - emd1 * r1x) / t1, 0},
-      {fl * (emd0 * r0x + emd1 * r0y) / den, fl * (emd0 * r1x + emd1 * r1y) / den, 0},
-      {0, 0, double(c.q)}};
+      {(r0y * emd0 - emd1 * r0x) * it1, (r1y * emd0 - emd1 * r1x) * it1, 0},
+      {fl * (emd0 * r0x + emd1 * r0y), fl * (emd0 * r1x + emd1 * r1y), 0},
+      {0, 0, q}};
   c.cov[0][0] = I[0][0]; c.cov[0][1] = I[0][1]; c.cov[0][2] = I[0][2];
   c.cov[1][0] = I[1][0]; c.cov[1][1] = I[1][1]; c.cov[1][2] = I[1][2];
   c.cov[2][0] = I[2][0]; c.cov[2][1] = I[2][1]; c.cov[2][2] = I[2][2];
   sandwich3(J, c.cov);
-  translate_karimaki(c, 0.5 * emd0, 0.5 * emd1);
-  c.cov[0][0] += double(ms_scale * mult_scatt<T>(P.S[1] - P.S[0], B, P.R, P.slope));
-  translate_karimaki(c, G.h0[0] + dv0, G.h0[1] + dv1, rot, cr, sr);
-  T chi2 = 0;
+  translate_karimaki(cs, sn, c, 0.5 * emd0, 0.5 * emd1);
+  c.cov[0][0] += double((T(1.0) + P.slope * P.slope) * P.ms0);
+  translate_karimaki(cs, sn, c, G.h0[0] + dv0, G.h0[1] + dv1);
+  c.par[0] = rot ? bl_atan2<double>(cs * sr + sn * cr, cs * cr - sn * sr) : bl_atan2<double>(sn, cs);
+  double chi2 = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const T diff = Z[i] - T(u[i]);
-    chi2 += w[i] * (diff * diff);
+    const double diff = double(Z[i]) - u[i];
+    chi2 += double(w[i]) * (diff * diff);
     if (i > 0 && i < N - 1) {
-      const T d1 = s[i] - s[i - 1], d2 = s[i + 1] - s[i], d3 = s[i + 1] - s[i - 1];
-      const T t = T(u[i - 1]) / d1 - (T(u[i]) * d3) / (d1 * d2) + T(u[i + 1]) / d2 + (d3 * T(u[N])) / T(2.0);
-      chi2 += (t * t) / VB[i];
+      const double d3 = double(P.s[i + 1]) - double(P.s[i - 1]);
+      const double t = (u[i - 1] - u[i]) * h[i - 1] + (u[i + 1] - u[i]) * h[i] + 0.5 * (d3 * u[N]);
+      chi2 += (t * t) * ivc[i];
     }
   }
-  c.chi2 = double(chi2);
+  c.chi2 = chi2;
   return ok;
 }
 
@@ -661,10 +722,12 @@ BL_HD bool fit_track(const double hits[3][N], const float ge_in[6][N], double Bd
   Prep<N, T> P;
   fast_fit<N, T>(G, P);
   prepare<N, T>(G, B, P);
+  double iv[N];
+  inverse_variances<N, T>(P, iv);
   LineOut L;
-  line_fit<N, T>(ge, G, B, P, L);
+  line_fit<N, T>(ge, G, P, iv, L);
   CircleOut C;
-  const bool ok = circle_fit<N, T>(ge, G, B, P, C, rot, cr, sr);
+  const bool ok = circle_fit<N, T>(ge, G, P, iv, C, rot, cr, sr);
   const double b = 1.0 / Bd;
   o.state[0] = C.par[0]; o.state[1] = C.par[1]; o.state[2] = C.par[2] * b; o.state[3] = L.par[0]; o.state[4] = L.par[1];
   const double cv[15] = {C.cov[0][0], C.cov[0][1], b * C.cov[0][2], 0.0, 0.0, C.cov[1][1], b * C.cov[1][2], 0.0, 0.0,

@@ -28,14 +28,14 @@ using bl::bl_atan2;
 // inverse of a symmetric positive-definite N x N matrix via Cholesky (A = L L^T)
 template <int N>
 BL_HD void chol_inverse(const double A[N][N], double Inv[N][N]) {
-  double L[N][N];
+  double L[N][N], iL[N];  // iL: 1 / the diagonal
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     double d = A[j][j];
 #pragma unroll
     for (int k = 0; k < j; ++k) d -= L[j][k] * L[j][k];
-    const double ljj = sqrt(d), il = 1.0 / ljj;
-    L[j][j] = ljj;
+    const double il = bl::s_rsqrt<double>(d);
+    iL[j] = il;
 #pragma unroll
     for (int i = j + 1; i < N; ++i) {
       double v = A[i][j];
@@ -48,7 +48,7 @@ BL_HD void chol_inverse(const double A[N][N], double Inv[N][N]) {
   double M[N][N];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    M[i][i] = 1.0 / L[i][i];
+    M[i][i] = iL[i];
 #pragma unroll
     for (int j = 0; j < i; ++j) {
       double v = 0.0;
@@ -82,7 +82,7 @@ BL_HD void min_eigen3(const double Ain[3][3], double v[3], double& lambda) {
         if (A[p][q] == 0.0) continue;
         const double th = (A[q][q] - A[p][p]) / (2.0 * A[p][q]);
         const double t = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-        const double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
+        const double c = bl::s_rsqrt<double>(t * t + 1.0), s = t * c;
         for (int k = 0; k < 3; ++k) {
           const double akp = A[k][p], akq = A[k][q];
           A[k][p] = c * akp - s * akq;
