@@ -38,6 +38,8 @@ BL_HD double chi2_adjoint(const double hits[3][N], const float ge[6][N], double 
     for (int i = 0; i < N; ++i) G.p[a][i] = hits[a][i] - hits[a][0];
   }
   // ---------------------------------------------------------------- forward (recomputed)
+  // The line system's partials are taken before the circle system is built, so that the two
+  // systems' arrays are not live together.
   Prep<N, T> P;
   fast_fit<N, T>(G, P);
   prepare<N, T>(G, B, P);
@@ -46,10 +48,6 @@ BL_HD double chi2_adjoint(const double hits[3][N], const float ge[6][N], double 
   double ul[N];
   inverse_variances<N, T>(P, iv);
   line_system<N, T>(ge, P, iv, wl, hl, fl, ul);
-  T ivc[N], Zc[N], wc[N], hc[N - 1];
-  Band<N, true> fc;
-  double uc[N + 1];
-  circle_system<N, T>(ge, G, P, iv, ivc, Zc, wc, hc, fc, uc);
   const T m = P.slope, a = P.Rl[0][0], b = P.Rl[0][1];
   const T sig = 1.0 + m * m;
   const T* s = P.s;
@@ -80,6 +78,34 @@ BL_HD double chi2_adjoint(const double hits[3][N], const float ge[6][N], double 
       gS[i + 1] += gbeta * dd2;
     }
   }
+  // ---------------------------------------------------------------- line weights
+  {
+    const double tol = 1e-12;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      auto z = [&](float v) { return fabs(double(v)) < tol ? 0.0 : double(v); };
+      const double V[3][3] = {{double(ge[0][i]), z(ge[1][i]), z(ge[3][i])}, {z(ge[1][i]), double(ge[2][i]), z(ge[4][i])},
+                              {z(ge[3][i]), z(ge[4][i]), double(ge[5][i])}};
+      const double in = P.irn[i], hx = P.rx[i] * in, hy = P.ry[i] * in;
+      const double rj[3] = {-b * hy, b * hx, a};
+      // w = 1 / (rj^T V rj): g_rj = -w^2 * 2 V rj * g_w
+      const double gm22 = -gwl[i] * wl[i] * wl[i];
+      double grj[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) grj[k] = 2.0 * gm22 * (V[k][0] * rj[0] + V[k][1] * rj[1] + V[k][2] * rj[2]);
+      gb += grj[1] * hx - grj[0] * hy;
+      ga += grj[2];
+      const double bi = b * in;
+      const double gn = bi * (grj[0] * hy - grj[1] * hx);
+      grx[i] += grj[1] * bi + gn * hx;
+      gry[i] += gn * hy - grj[0] * bi;
+    }
+  }
+  // ---------------------------------------------------------------- circle system
+  T ivc[N], Zc[N], wc[N], hc[N - 1];
+  Band<N, true> fc;
+  double uc[N + 1];
+  circle_system<N, T>(ge, G, P, iv, ivc, Zc, wc, hc, fc, uc);
   // ---------------------------------------------------------------- circle chi2 partials
   double gsig = 0.0;
 #pragma unroll
@@ -133,29 +159,6 @@ BL_HD double chi2_adjoint(const double hits[3][N], const float ge[6][N], double 
     }
     if (B * P.R < 20.0) gR -= 2.0 * gms * iR;
     gm -= 2.0 * gms * m * (a * a);
-  }
-  // ---------------------------------------------------------------- line weights
-  {
-    const double tol = 1e-12;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      auto z = [&](float v) { return fabs(double(v)) < tol ? 0.0 : double(v); };
-      const double V[3][3] = {{double(ge[0][i]), z(ge[1][i]), z(ge[3][i])}, {z(ge[1][i]), double(ge[2][i]), z(ge[4][i])},
-                              {z(ge[3][i]), z(ge[4][i]), double(ge[5][i])}};
-      const double in = P.irn[i], hx = P.rx[i] * in, hy = P.ry[i] * in;
-      const double rj[3] = {-b * hy, b * hx, a};
-      // w = 1 / (rj^T V rj): g_rj = -w^2 * 2 V rj * g_w
-      const double gm22 = -gwl[i] * wl[i] * wl[i];
-      double grj[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) grj[k] = 2.0 * gm22 * (V[k][0] * rj[0] + V[k][1] * rj[1] + V[k][2] * rj[2]);
-      gb += grj[1] * hx - grj[0] * hy;
-      ga += grj[2];
-      const double bi = b * in;
-      const double gn = bi * (grj[0] * hy - grj[1] * hx);
-      grx[i] += grj[1] * bi + gn * hx;
-      gry[i] += gn * hy - grj[0] * bi;
-    }
   }
   // ---------------------------------------------------------------- rotation (S, Z) = R(m) (s, z)
 #pragma unroll

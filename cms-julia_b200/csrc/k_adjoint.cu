@@ -33,59 +33,58 @@ struct AdjArgs {
 };
 
 template <int N>
-__global__ void __launch_bounds__(128) k_bl_adjoint(AdjArgs A) {
-  const uint32_t cnt = A.plan->count[N];
-  const int32_t* list = A.plan->list + A.plan->base_of(N);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-    const int32_t t = list[i];
-    const int32_t first = A.offs[t];
-    double h[3][N];
-    float ge[6][N];
-    int mod[N];
+__device__ __forceinline__ void adjoint_track(const AdjArgs& A, int32_t t) {
+  const int32_t first = A.offs[t];
+  double h[3][N];
+  float ge[6][N];
+  int mod[N];
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      const size_t j = size_t(first) + k;
-      double x = A.hits[3 * j], y = A.hits[3 * j + 1], z = A.hits[3 * j + 2];
-      mod[k] = A.hit_module ? int(A.hit_module[j]) : -1;
-      if (mod[k] >= A.n_modules) mod[k] = -1;
-      if (A.align && mod[k] >= 0) {
-        const float* al = A.align + 6 * mod[k];
-        const double* c = A.module_pos + 3 * mod[k];
-        const double rx = x - c[0], ry = y - c[1], rz = z - c[2];
-        const double wx = al[3], wy = al[4], wz = al[5];
-        x += al[0] + (wy * rz - wz * ry);
-        y += al[1] + (wz * rx - wx * rz);
-        z += al[2] + (wx * ry - wy * rx);
-      }
-      h[0][k] = x; h[1][k] = y; h[2][k] = z;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) ge[q][k] = A.ge[6 * j + q];
+  for (int k = 0; k < N; ++k) {
+    const size_t j = size_t(first) + k;
+    double x = A.hits[3 * j], y = A.hits[3 * j + 1], z = A.hits[3 * j + 2];
+    mod[k] = A.hit_module ? int(A.hit_module[j]) : -1;
+    if (mod[k] >= A.n_modules) mod[k] = -1;
+    if (A.align && mod[k] >= 0) {
+      const float* al = A.align + 6 * mod[k];
+      const double* c = A.module_pos + 3 * mod[k];
+      const double rx = x - c[0], ry = y - c[1], rz = z - c[2];
+      const double wx = al[3], wy = al[4], wz = al[5];
+      x += al[0] + (wy * rz - wz * ry);
+      y += al[1] + (wz * rx - wx * rz);
+      z += al[2] + (wx * ry - wy * rx);
     }
-    double g[3][N];
-    const double c2 = bl::chi2_adjoint<N>(h, ge, A.B, g);
-    if (A.chi2) A.chi2[t] = float(c2);
+    h[0][k] = x; h[1][k] = y; h[2][k] = z;
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      const size_t j = size_t(first) + k;
-      if (A.grad_hits) {
-        A.grad_hits[3 * j] = float(g[0][k]);
-        A.grad_hits[3 * j + 1] = float(g[1][k]);
-        A.grad_hits[3 * j + 2] = float(g[2][k]);
-      }
-      if (A.acc && mod[k] >= 0) {
-        // lever arm of the nominal hit about the module centre
-        const double* c = A.module_pos + 3 * mod[k];
-        const double rx = A.hits[3 * j] - c[0], ry = A.hits[3 * j + 1] - c[1], rz = A.hits[3 * j + 2] - c[2];
-        double* a = A.acc + 6 * mod[k];
-        atomicAdd(a + 0, g[0][k]);
-        atomicAdd(a + 1, g[1][k]);
-        atomicAdd(a + 2, g[2][k]);
-        atomicAdd(a + 3, ry * g[2][k] - rz * g[1][k]);
-        atomicAdd(a + 4, rz * g[0][k] - rx * g[2][k]);
-        atomicAdd(a + 5, rx * g[1][k] - ry * g[0][k]);
-      }
+    for (int q = 0; q < 6; ++q) ge[q][k] = A.ge[6 * j + q];
+  }
+  double g[3][N];
+  const double c2 = bl::chi2_adjoint<N>(h, ge, A.B, g);
+  if (A.chi2) A.chi2[t] = float(c2);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const size_t j = size_t(first) + k;
+    if (A.grad_hits) {
+      A.grad_hits[3 * j] = float(g[0][k]);
+      A.grad_hits[3 * j + 1] = float(g[1][k]);
+      A.grad_hits[3 * j + 2] = float(g[2][k]);
+    }
+    if (A.acc && mod[k] >= 0) {
+      // lever arm of the nominal hit about the module centre
+      const double* c = A.module_pos + 3 * mod[k];
+      const double rx = A.hits[3 * j] - c[0], ry = A.hits[3 * j + 1] - c[1], rz = A.hits[3 * j + 2] - c[2];
+      double* a = A.acc + 6 * mod[k];
+      atomicAdd(a + 0, g[0][k]);
+      atomicAdd(a + 1, g[1][k]);
+      atomicAdd(a + 2, g[2][k]);
+      atomicAdd(a + 3, ry * g[2][k] - rz * g[1][k]);
+      atomicAdd(a + 4, rz * g[0][k] - rx * g[2][k]);
+      atomicAdd(a + 5, rx * g[1][k] - ry * g[0][k]);
     }
   }
+}
+
+__global__ void __launch_bounds__(kFitThreads, 3) k_bl_adjoint(AdjArgs A) {
+  for_bucket_track(*A.plan, [&](auto n, int32_t t) { adjoint_track<decltype(n)::value>(A, t); });
 }
 
 __global__ void k_align_out(const double* acc, int32_t n, float* out32, double* out64) {
@@ -123,18 +122,7 @@ extern "C" int32_t pxl_bl_fit_adjoint(const double* hits, const float* hits_ge, 
     if (rc) return rc;
     AdjArgs A{hits, hits_ge, offs, plan, b_field, hit_module, module_pos, align, n_modules, chi2, grad_hits,
               want_align ? acc : nullptr};
-    const int g = 148 * 4;
-    rc = fan_out(s, 6, [&](int k, cudaStream_t st) {
-      switch (k) {
-        case 0: k_bl_adjoint<3><<<g, 128, 0, st>>>(A); break;
-        case 1: k_bl_adjoint<4><<<g, 128, 0, st>>>(A); break;
-        case 2: k_bl_adjoint<5><<<g, 128, 0, st>>>(A); break;
-        case 3: k_bl_adjoint<6><<<g, 128, 0, st>>>(A); break;
-        case 4: k_bl_adjoint<7><<<g, 128, 0, st>>>(A); break;
-        default: k_bl_adjoint<8><<<g, 128, 0, st>>>(A); break;
-      }
-    });
-    if (rc) return PXL_ERR_CUDA;
+    k_bl_adjoint<<<fit_blocks(n), kFitThreads, 0, s>>>(A);
   }
   if (want_align) k_align_out<<<std::max(1, (6 * n_modules + 255) / 256), 256, 0, s>>>(acc, 6 * n_modules, grad_align, grad_align64);
   return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;

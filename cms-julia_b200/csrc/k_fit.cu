@@ -3,7 +3,6 @@
 // with their first 4 hits, at most 24576 per multiplicity) and the stand-alone
 // fit entry point pxl_bl_fit (3..8 hits, FP64 or mixed precision).
 #include <algorithm>
-#include <mutex>
 
 #include "../../include/pxl.h"
 #include "bl_fit.cuh"
@@ -277,32 +276,26 @@ __global__ void __launch_bounds__(1024) k_fit_plan_one(const int32_t* __restrict
 
 namespace {
 
-template <int N, class T>
-__global__ void __launch_bounds__(128, 4) k_fit_bucket(const double* __restrict__ hits, const float* __restrict__ ge,
-                                                    const int32_t* __restrict__ offs, const FitPlan* __restrict__ plan,
-                                                    double B, float* state, float* cov, float* chi2, float* pt,
-                                                    float* eta, int32_t* status) {
-  const uint32_t cnt = plan->count[N];
-  const int32_t* list = plan->list + plan->base_of(N);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-    const int32_t t = list[i];
-    standalone_fit<N, T>(hits, ge, offs[t], B, state, cov, chi2, pt, eta, status, t);
-  }
+// One launch for all hit counts, where six launches on three streams, forked and joined by events,
+// left each kernel's tail and the event waits (1237 mixed fits 43 us, now 27; 99991 FP64 fits 98 us,
+// now 81).
+constexpr int kFitResident = 4;  // blocks per SM: 128 registers a thread
+
+// A block per 128 tracks, long fits first, so that the blocks even out; from four waves on one wave
+// of blocks that go on to further tracks saves the blocks' starts (2^20 mixed fits 374 us instead
+// of 416), which at 1.3 waves costs more in balance than it saves (99991 FP64 fits 92 us instead of 81).
+inline int bl_fit_blocks(int32_t n) {
+  const int all = fit_blocks(n), wave = 148 * kFitResident;
+  return all < 4 * wave ? all : wave;
 }
 
 template <class T>
-int launch_bucket_fits(const double* hits, const float* ge, const int32_t* offs, const FitPlan* plan, double B,
-                       float* state, float* cov, float* chi2, float* pt, float* eta, int32_t* status, cudaStream_t s) {
-  const int g = 148 * 4;
-  return fan_out(s, 6, [&](int k, cudaStream_t st) {
-    switch (k) {
-      case 0: k_fit_bucket<3, T><<<g, 128, 0, st>>>(hits, ge, offs, plan, B, state, cov, chi2, pt, eta, status); break;
-      case 1: k_fit_bucket<4, T><<<g, 128, 0, st>>>(hits, ge, offs, plan, B, state, cov, chi2, pt, eta, status); break;
-      case 2: k_fit_bucket<5, T><<<g, 128, 0, st>>>(hits, ge, offs, plan, B, state, cov, chi2, pt, eta, status); break;
-      case 3: k_fit_bucket<6, T><<<g, 128, 0, st>>>(hits, ge, offs, plan, B, state, cov, chi2, pt, eta, status); break;
-      case 4: k_fit_bucket<7, T><<<g, 128, 0, st>>>(hits, ge, offs, plan, B, state, cov, chi2, pt, eta, status); break;
-      default: k_fit_bucket<8, T><<<g, 128, 0, st>>>(hits, ge, offs, plan, B, state, cov, chi2, pt, eta, status); break;
-    }
+__global__ void __launch_bounds__(kFitThreads, kFitResident) k_fit_buckets(const double* __restrict__ hits, const float* __restrict__ ge,
+                                                    const int32_t* __restrict__ offs, const FitPlan* __restrict__ plan,
+                                                    double B, float* state, float* cov, float* chi2, float* pt,
+                                                    float* eta, int32_t* status) {
+  for_bucket_track(*plan, [&](auto n, int32_t t) {
+    standalone_fit<decltype(n)::value, T>(hits, ge, offs[t], B, state, cov, chi2, pt, eta, status, t);
   });
 }
 
@@ -336,37 +329,6 @@ int64_t fit_plan_bytes(int32_t n_tracks) {
   return (int64_t(sizeof(FitPlan)) + 4 * int64_t(n_tracks > 0 ? n_tracks : 0) + 255) / 256 * 256;
 }
 
-namespace {
-constexpr int kMaxDevices = 64;
-std::mutex g_side_mu;
-SideStreams g_side[kMaxDevices];
-bool g_side_made[kMaxDevices];
-}  // namespace
-
-SideStreams* side_streams_lock() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-  g_side_mu.lock();
-  if (!g_side_made[dev]) {
-    SideStreams& ss = g_side[dev];
-    bool ok = true;
-    for (int j = 0; j < 2; ++j) {
-      ok = ok && cudaStreamCreateWithFlags(&ss.st[j], cudaStreamNonBlocking) == cudaSuccess;
-      ok = ok && cudaEventCreateWithFlags(&ss.join[j], cudaEventDisableTiming) == cudaSuccess;
-    }
-    ok = ok && cudaEventCreateWithFlags(&ss.fork, cudaEventDisableTiming) == cudaSuccess;
-    if (!ok) {
-      cudaGetLastError();
-      g_side_mu.unlock();
-      return nullptr;
-    }
-    g_side_made[dev] = true;
-  }
-  return &g_side[dev];
-}
-
-void side_streams_unlock() { g_side_mu.unlock(); }
-
 int fit_plan_build(const int32_t* offs, int32_t n, FitPlan* plan, int32_t* status, cudaStream_t s) {
   if (n <= kPlanOneCta) {
     // one launch instead of a clear, a count and a fill; above, one CTA takes longer than they do
@@ -396,8 +358,10 @@ extern "C" int32_t pxl_bl_fit(const double* hits, const float* hits_ge, const in
   auto* plan = static_cast<pxl::FitPlan*>(workspace);
   int rc = pxl::fit_plan_build(offs, n, plan, status, s);
   if (rc) return rc;
-  rc = precision == 0
-           ? pxl::launch_bucket_fits<double>(hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status, s)
-           : pxl::launch_bucket_fits<float>(hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status, s);
-  return rc == 0 ? 0 : PXL_ERR_CUDA;
+  const int g = pxl::bl_fit_blocks(n);
+  if (precision == 0)
+    pxl::k_fit_buckets<double><<<g, pxl::kFitThreads, 0, s>>>(hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
+  else
+    pxl::k_fit_buckets<float><<<g, pxl::kFitThreads, 0, s>>>(hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
+  return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;
 }

@@ -1,5 +1,5 @@
 // Stand-alone Riemann fits (C ABI pxl_riemann_fit): tracks grouped by hit count
-// with the same workspace plan as pxl_bl_fit, one kernel per hit count.
+// with the same workspace plan as pxl_bl_fit.
 #include <algorithm>
 
 #include "../../include/pxl.h"
@@ -23,45 +23,30 @@ struct RmArgs {
 };
 
 template <int N, class T>
-__global__ void __launch_bounds__(128) k_riemann(RmArgs A) {
-  const uint32_t cnt = A.plan->count[N];
-  const int32_t* list = A.plan->list + A.plan->base_of(N);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-    const int32_t t = list[i];
-    const int32_t first = A.offs[t];
-    double h[3][N];
-    float ge[6][N];
+__device__ __forceinline__ void riemann_track(const RmArgs& A, int32_t t) {
+  const int32_t first = A.offs[t];
+  double h[3][N];
+  float ge[6][N];
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
+  for (int k = 0; k < N; ++k) {
 #pragma unroll
-      for (int a = 0; a < 3; ++a) h[a][k] = A.hits[3 * size_t(first + k) + a];
+    for (int a = 0; a < 3; ++a) h[a][k] = A.hits[3 * size_t(first + k) + a];
 #pragma unroll
-      for (int q = 0; q < 6; ++q) ge[q][k] = A.ge[6 * size_t(first + k) + q];
-    }
-    rm::RiemannOut o;
-    const bool ok = rm::riemann_fit<N, T>(h, ge, A.B, o);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) A.state[5 * size_t(t) + k] = float(o.state[k]);
-    A.chi2[2 * size_t(t)] = float(o.chi2_circle);
-    A.chi2[2 * size_t(t) + 1] = float(o.chi2_line);
-    A.pt[t] = float(o.pt);
-    A.status[t] = ok ? 0 : 1;
+    for (int q = 0; q < 6; ++q) ge[q][k] = A.ge[6 * size_t(first + k) + q];
   }
+  rm::RiemannOut o;
+  const bool ok = rm::riemann_fit<N, T>(h, ge, A.B, o);
+#pragma unroll
+  for (int k = 0; k < 5; ++k) A.state[5 * size_t(t) + k] = float(o.state[k]);
+  A.chi2[2 * size_t(t)] = float(o.chi2_circle);
+  A.chi2[2 * size_t(t) + 1] = float(o.chi2_line);
+  A.pt[t] = float(o.pt);
+  A.status[t] = ok ? 0 : 1;
 }
 
 template <class T>
-int launch_riemann(const RmArgs& A, cudaStream_t s) {
-  const int g = 148 * 4;
-  return fan_out(s, 6, [&](int k, cudaStream_t st) {
-    switch (k) {
-      case 0: k_riemann<3, T><<<g, 128, 0, st>>>(A); break;
-      case 1: k_riemann<4, T><<<g, 128, 0, st>>>(A); break;
-      case 2: k_riemann<5, T><<<g, 128, 0, st>>>(A); break;
-      case 3: k_riemann<6, T><<<g, 128, 0, st>>>(A); break;
-      case 4: k_riemann<7, T><<<g, 128, 0, st>>>(A); break;
-      default: k_riemann<8, T><<<g, 128, 0, st>>>(A); break;
-    }
-  });
+__global__ void __launch_bounds__(kFitThreads, 3) k_riemann(RmArgs A) {
+  for_bucket_track(*A.plan, [&](auto n, int32_t t) { riemann_track<decltype(n)::value, T>(A, t); });
 }
 
 }  // namespace
@@ -81,6 +66,7 @@ extern "C" int32_t pxl_riemann_fit(const double* hits, const float* hits_ge, con
   int rc = fit_plan_build(offs, n, plan, status, s);
   if (rc) return rc;
   RmArgs A{hits, hits_ge, offs, plan, b_field, state, chi2, pt, status};
-  rc = precision == 0 ? launch_riemann<double>(A, s) : launch_riemann<float>(A, s);
-  return rc == 0 ? 0 : PXL_ERR_CUDA;
+  if (precision == 0) k_riemann<double><<<fit_blocks(n), kFitThreads, 0, s>>>(A);
+  else k_riemann<float><<<fit_blocks(n), kFitThreads, 0, s>>>(A);
+  return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;
 }

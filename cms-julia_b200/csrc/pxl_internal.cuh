@@ -12,6 +12,7 @@
 // integer products match the reference element by element.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 namespace pxl {
@@ -310,33 +311,32 @@ struct FitPlan {
 int64_t fit_plan_bytes(int32_t n_tracks);
 int fit_plan_build(const int32_t* offs, int32_t n, FitPlan* plan, int32_t* status, cudaStream_t s);
 
-// Two side streams of the current device with a fork event and two join events, created on
-// first use; side_streams_lock returns them held by the caller until side_streams_unlock
-// (nullptr, and nothing held, when they could not be created).
-struct SideStreams {
-  cudaStream_t st[2];
-  cudaEvent_t fork, join[2];
-};
-SideStreams* side_streams_lock();
-void side_streams_unlock();
+// The per-hit-count fits run in one launch: a block takes kFitThreads tracks of one list at a
+// time, the lists of long tracks first, so that the last blocks are short ones.
+// for_bucket_track calls f(hit count as an integral constant, track) for each track of the thread.
+constexpr int kFitThreads = 128;
+inline int fit_blocks(int32_t n) { return n / kFitThreads + (kFitMaxN - 2); }
 
-// Enqueues launch(k, stream) for k = 0 .. n-1 round robin on s and the two side streams,
-// forked from s and joined back into it: the per-hit-count fit kernels then overlap where an
-// earlier one's last blocks leave SMs idle. Without side streams every launch goes on s.
-template <class F>
-int fan_out(cudaStream_t s, int n, F&& launch) {
-  SideStreams* ss = side_streams_lock();
-  if (!ss) {
-    for (int k = 0; k < n; ++k) launch(k, s);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+template <int N, class F>
+__device__ __forceinline__ void for_bucket_track_n(const int32_t* list, const uint32_t* cnt, uint32_t base_end, uint32_t b,
+                                                   F&& f) {
+  if constexpr (N >= 3) {
+    const uint32_t c = cnt[N], nb = (c + kFitThreads - 1) / kFitThreads;
+    for (; b < nb; b += gridDim.x) {
+      const uint32_t i = b * kFitThreads + threadIdx.x;
+      if (i < c) f(std::integral_constant<int, N>{}, list[base_end - c + i]);
+    }
+    for_bucket_track_n<N - 1>(list, cnt, base_end - c, b - nb, f);
   }
-  bool ok = cudaEventRecord(ss->fork, s) == cudaSuccess && cudaStreamWaitEvent(ss->st[0], ss->fork, 0) == cudaSuccess &&
-            cudaStreamWaitEvent(ss->st[1], ss->fork, 0) == cudaSuccess;
-  for (int k = 0; ok && k < n; ++k) launch(k, k % 3 == 0 ? s : ss->st[k % 3 - 1]);
-  for (int j = 0; ok && j < 2; ++j)
-    ok = cudaEventRecord(ss->join[j], ss->st[j]) == cudaSuccess && cudaStreamWaitEvent(s, ss->join[j], 0) == cudaSuccess;
-  side_streams_unlock();
-  return ok && cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+template <class F>
+__device__ __forceinline__ void for_bucket_track(const FitPlan& plan, F&& f) {
+  uint32_t cnt[kFitMaxN + 1], end = 0;  // read at once: the block waits for one latency
+#pragma unroll
+  for (int n = 3; n <= kFitMaxN; ++n) cnt[n] = plan.count[n];
+#pragma unroll
+  for (int n = 3; n <= kFitMaxN; ++n) end += cnt[n];
+  for_bucket_track_n<kFitMaxN>(plan.list, cnt, end, blockIdx.x, f);
 }
 
 // ---------------------------------------------------------------- helpers
