@@ -83,6 +83,10 @@ __device__ __forceinline__ void adjoint_track(const AdjArgs& A, int32_t t) {
   }
 }
 
+// Bound by the latency of one thread's FP64 chain at few warps per SM (and by its instruction
+// fetch). Three blocks per SM (168 registers) against two: 2^19 tracks with alignment 456 us and 470 us,
+// 502 and 575 us when the call is waited for; four: 477 us. Before the shared reciprocals and
+// with a launch per hit count it was 966 us.
 __global__ void __launch_bounds__(kFitThreads, 3) k_bl_adjoint(AdjArgs A) {
   for_bucket_track(*A.plan, [&](auto n, int32_t t) { adjoint_track<decltype(n)::value>(A, t); });
 }

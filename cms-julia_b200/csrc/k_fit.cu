@@ -3,6 +3,7 @@
 // with their first 4 hits, at most 24576 per multiplicity) and the stand-alone
 // fit entry point pxl_bl_fit (3..8 hits, FP64 or mixed precision).
 #include <algorithm>
+#include <cstddef>
 
 #include "../../include/pxl.h"
 #include "bl_fit.cuh"
@@ -54,25 +55,25 @@ __device__ bool fit_tuple(const Dev& d, uint64_t g, uint32_t hb, const uint32_t*
 // Which tuples are fitted, and with how many hits: 3-hit tuples with 3, 4- and
 // 5-hit tuples with 4 (fit5as4), none flagged duplicate, at most fits_per_mult
 // per multiplicity (the bin is read in decreasing id, so the largest ids win).
-// One block per event: the fitted tuples go to the event's region of fit_list
-// (3-hit from the front, 4-hit from the back) so that every warp of the fit
-// kernel runs one hit count; the others get zero outputs here. The first pass
-// sets t_fitted for every tuple (the fit kernel writes it again) and takes list
-// slots one atomic per warp; the second zeroes the state and covariance words of
-// the tuples left out, walking the packed arrays word by word so that the stores
-// coalesce.
+// The fitted tuples go to the event's region of fit_list (3-hit from the front, 4-hit from the
+// back) so that every warp of the fit kernel runs one hit count; the others get zero outputs here.
+// A block takes 256 tuples at a time: their list slots with one atomic per hit count, then the
+// state and covariance words of the tuples left out, in word order so that the stores coalesce. An
+// event has blocks as event_blocks gives them (one block took 580 us for the 51 k tuples of an event
+// of pileup 170); its counters are cleared before the launch.
 __global__ void __launch_bounds__(256) k_fit_list(Dev d) {
-  const int e = blockIdx.x;
+  const int e = blockIdx.y;
   EvInfo& E = d.ev[e];
-  __shared__ uint32_t s_n3, s_n4;
-  if (threadIdx.x == 0) { s_n3 = 0; s_n4 = 0; }
-  __syncthreads();
+  __shared__ uint32_t s_n[2], s_base[2];
+  __shared__ uint8_t s_fit[256];
   const uint64_t tb = E.tuple_base;
   const uint32_t nt = E.n_tuples;
-  const unsigned lane = threadIdx.x & 31u;
-  const uint32_t nt_pad = (nt + 31u) & ~31u;
-  for (uint32_t t = threadIdx.x; t < nt_pad; t += blockDim.x) {
+  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  for (uint32_t t0 = blockIdx.x * 256u; t0 < nt; t0 += gridDim.x * 256u) {
+    const uint32_t t = t0 + threadIdx.x;
     const uint64_t g = tb + t;
+    if (threadIdx.x < 2) s_n[threadIdx.x] = 0;
+    __syncthreads();
     bool fit = false;
     uint32_t n = 0;
     if (t < nt) {
@@ -89,32 +90,33 @@ __global__ void __launch_bounds__(256) k_fit_list(Dev d) {
           fit = larger < d.fits_per_mult;
         }
       }
+      d.t_fitted[g] = fit ? 1 : 0;
+      if (!fit) { d.t_pt[g] = 0.f; d.t_eta[g] = 0.f; d.t_chi2[g] = 0.f; }
     }
+    s_fit[threadIdx.x] = fit ? 1 : 0;
     const unsigned m3 = __ballot_sync(0xffffffffu, fit && n == 3);
     const unsigned m4 = __ballot_sync(0xffffffffu, fit && n != 3);
-    uint32_t b3 = 0, b4 = 0;
+    uint32_t w3 = 0, w4 = 0;
     if (lane == 0) {
-      if (m3) b3 = atomicAdd(&s_n3, uint32_t(__popc(m3)));
-      if (m4) b4 = atomicAdd(&s_n4, uint32_t(__popc(m4)));
+      if (m3) w3 = atomicAdd(&s_n[0], uint32_t(__popc(m3)));
+      if (m4) w4 = atomicAdd(&s_n[1], uint32_t(__popc(m4)));
     }
-    b3 = __shfl_sync(0xffffffffu, b3, 0);
-    b4 = __shfl_sync(0xffffffffu, b4, 0);
-    const unsigned below = (1u << lane) - 1u;
-    if (t >= nt) continue;
-    d.t_fitted[g] = fit ? 1 : 0;
+    w3 = __shfl_sync(0xffffffffu, w3, 0);
+    w4 = __shfl_sync(0xffffffffu, w4, 0);
+    __syncthreads();
+    if (threadIdx.x < 2 && s_n[threadIdx.x]) s_base[threadIdx.x] = atomicAdd(threadIdx.x ? &E.n_fit4 : &E.n_fit3, s_n[threadIdx.x]);
+    __syncthreads();
     if (fit) {
-      if (n == 3) d.fit_list[tb + b3 + __popc(m3 & below)] = t;
-      else d.fit_list[tb + nt - 1 - (b4 + __popc(m4 & below))] = t;
-      continue;
+      if (n == 3) d.fit_list[tb + s_base[0] + w3 + __popc(m3 & below)] = t;
+      else d.fit_list[tb + nt - 1 - (s_base[1] + w4 + __popc(m4 & below))] = t;
     }
-    d.t_pt[g] = 0.f; d.t_eta[g] = 0.f; d.t_chi2[g] = 0.f;
+    const uint32_t m = nt - t0 < 256u ? nt - t0 : 256u;
+    for (uint32_t w = threadIdx.x; w < 5 * m; w += 256u)
+      if (!s_fit[w / 5]) d.t_state[5 * (tb + t0) + w] = 0.f;
+    for (uint32_t w = threadIdx.x; w < 15 * m; w += 256u)
+      if (!s_fit[w / 15]) d.t_cov[15 * (tb + t0) + w] = 0.f;
+    __syncthreads();
   }
-  __syncthreads();
-  for (uint32_t w = threadIdx.x; w < 5 * nt; w += blockDim.x)
-    if (!d.t_fitted[tb + w / 5]) d.t_state[5 * tb + w] = 0.f;
-  for (uint32_t w = threadIdx.x; w < 15 * nt; w += blockDim.x)
-    if (!d.t_fitted[tb + w / 15]) d.t_cov[15 * tb + w] = 0.f;
-  if (threadIdx.x == 0) { E.n_fit3 = s_n3; E.n_fit4 = s_n4; E.n_refit3 = 0; E.n_refit4 = 0; }
 }
 
 // one hit count per launch, so that each instantiation keeps only its own registers.
@@ -301,8 +303,12 @@ __global__ void __launch_bounds__(kFitThreads, kFitResident) k_fit_buckets(const
 
 }  // namespace
 
+static_assert(offsetof(EvInfo, n_refit4) == offsetof(EvInfo, n_fit3) + 3 * sizeof(uint32_t), "cleared together");
+
 void launch_fit(const Dev& d, const Launch& L) {
-  k_fit_list<<<d.E, 256, 0, L.s>>>(d);
+  // the events' n_fit3, n_fit4, n_refit3, n_refit4
+  cudaMemset2DAsync(&d.ev[0].n_fit3, sizeof(EvInfo), 0, 4 * sizeof(uint32_t), size_t(d.E), L.s);
+  k_fit_list<<<dim3(event_blocks(d.E, 148 * 4, 64), d.E), 256, 0, L.s>>>(d);
   L.mark("fit_list");
   // about 7000 fits per PU50 event: enough CTAs for every SM with few events
   const int bx = (L.tune && L.tune[kTuneFitTuples] > 0) ? L.tune[kTuneFitTuples]
@@ -313,9 +319,11 @@ void launch_fit(const Dev& d, const Launch& L) {
     L.mark("broken_line_fit_3");
     k_fit_tuples<4, float><<<dim3(bx, d.E), 128, 0, L.s>>>(d);
     L.mark("broken_line_fit_4");
-    // about 1 % of the fits: one block per event and hit count
-    k_refit_tuples<3><<<dim3(1, d.E), 128, 0, L.s>>>(d);
-    k_refit_tuples<4><<<dim3(1, d.E), 128, 0, L.s>>>(d);
+    // about 1 % of the fits: one block per event and hit count, more where an event has the GPU
+    // to itself (a block's fits follow one another)
+    const dim3 gr(event_blocks(d.E, 148, 16), d.E);
+    k_refit_tuples<3><<<gr, 128, 0, L.s>>>(d);
+    k_refit_tuples<4><<<gr, 128, 0, L.s>>>(d);
     L.mark("broken_line_refit_fp64");
   } else {
     k_fit_tuples<3, double><<<dim3(bx, d.E), 128, 0, L.s>>>(d);

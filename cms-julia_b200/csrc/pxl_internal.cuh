@@ -92,6 +92,7 @@ struct EvInfo {
   uint32_t n_errors, error_base;
   uint32_t warnings;
   uint32_t tm_off[9];               // tuple multiplicity offsets (bins 1..8, reference layout)
+  uint32_t tm_cnt[9], tm_done;      // k_multiplicity: counts so far, blocks that added theirs
   uint32_t n_dup_cells, n_dup_entries;  // cells with two or more loose tracks, and their entries
   uint32_t n_cols_nb, n_cols_tr;    // non-empty neighbour / track lists (column store use)
   uint32_t n_fit3, n_fit4;          // tuples fitted with 3 and with 4 hits (fit5as4 included)
@@ -254,6 +255,7 @@ struct ExportSet {
   float* state = nullptr; float* cov = nullptr; float* pt = nullptr; float* eta = nullptr; float* chi2 = nullptr;
   uint8_t* n_hits = nullptr; int16_t* vertex = nullptr; uint32_t* tuple = nullptr;
   float* zv = nullptr; float* wv = nullptr; float* vchi2 = nullptr; float* ptv2 = nullptr; int32_t* ndof = nullptr;
+  uint32_t* block = nullptr;  // loose tracks per block of the event, then the first track of each
   uint32_t cap_tracks = 0, cap_vertices = 0;
   cudaEvent_t ready = nullptr, copied = nullptr;  // kernels done (compute stream), copies done (copy stream)
 };
@@ -414,6 +416,13 @@ __device__ __forceinline__ uint32_t dup_word(const Dev& d, uint64_t wi, uint64_t
 }
 
 inline int div_up(int64_t a, int64_t b) { return int((a + b - 1) / b); }
+
+// Blocks per event of a kernel whose work one block per event would do one after the other: enough
+// to put `target` blocks on the GPU, at most `most`, one for large batches.
+inline int event_blocks(int E, int target, int most) {
+  const int b = target / (E > 0 ? E : 1);
+  return b < 1 ? 1 : (b < most ? b : most);
+}
 
 // ---------------------------------------------------------------- launchers (per stage file)
 // Optional per-kernel timing: when enabled, the launchers record a CUDA event after
