@@ -44,45 +44,86 @@ __device__ __forceinline__ int32_t ld_i32(const uint8_t* p) {
 // One block per event: FedRawDataCollection directory (bin/ReadRAW.jl:23-31), then the
 // payload word counts in fedIds order (SiPixelRawToClusterCUDA.jl:75-131: skip FED 40,
 // skip empty FEDs, payload = bytes [8, size-8)). The directory is a chain of records whose
-// positions depend on every earlier size, so one thread follows it; the FED header and
-// trailer checks then run one FED per thread.
-__global__ void k_fed_table(Dev d, const int16_t* __restrict__ fed_slot_of) {
+// positions depend on every earlier size, so one thread follows it, a window of the event at a
+// time that the whole block has just read (the chain's loads then come from L1; from L2 and with
+// the slot lookup between two hops a single event's table took 44 us). The slots of the records, a
+// repeated FED id's last record winning, and the FED header and trailer checks then run in parallel.
+constexpr uint32_t kFedWindow = 96 * 1024;  // bytes per window
+constexpr int kFedHops = 256;               // records per window
+
+__global__ void __launch_bounds__(256) k_fed_table(Dev d, const int16_t* __restrict__ fed_slot_of) {
   const int e = blockIdx.x;
   const int NF = d.n_fed_slots;
   __shared__ uint64_t s_src[kMaxFedSlots];
   __shared__ uint32_t s_nw[kMaxFedSlots];
   __shared__ int32_t s_len[kMaxFedSlots];
+  __shared__ uint32_t s_last[kMaxFedSlots];  // 1 + the slot's last record so far
+  __shared__ uint64_t s_pos[kFedHops];
+  __shared__ int32_t s_fid[kFedHops], s_size[kFedHops];
+  __shared__ uint64_t s_p;       // position of the next record
+  __shared__ int32_t s_hop;      // its number
+  __shared__ int s_n;            // records of the window
   __shared__ uint32_t sh[33];
   __shared__ uint32_t s_warn;
-  for (int f = threadIdx.x; f < NF; f += blockDim.x) { s_nw[f] = 0; s_src[f] = 0; s_len[f] = 0; }
-  if (threadIdx.x == 0) s_warn = 0;
+  for (int f = threadIdx.x; f < NF; f += blockDim.x) { s_nw[f] = 0; s_src[f] = 0; s_len[f] = 0; s_last[f] = 0; }
+  if (threadIdx.x == 0) { s_warn = 0; s_p = 4; s_hop = 0; }
   __syncthreads();
   const uint64_t off0 = d.ev_off[e], off1 = d.ev_off[e + 1];
   const uint8_t* ev = d.raw + off0;
   const uint64_t nbytes = off1 - off0;
-  if (threadIdx.x == 0) {
-    if (nbytes >= 4) {
-      int32_t nfeds = ld_i32(ev);
-      uint64_t p = 4;
-      for (int32_t k = 0; k < nfeds; ++k) {
-        if (p + 8 > nbytes) { s_warn |= kWarnBuffer; break; }
-        int32_t fid = ld_i32(ev + p), size = ld_i32(ev + p + 4);
-        if (size < 0 || p + 8 + uint64_t(size) > nbytes) { s_warn |= kWarnBuffer; break; }
-        if (fid >= 0 && fid < 4096) {
-          int slot = fed_slot_of[fid];
-          if (slot >= 0) {
-            uint32_t nw64 = uint32_t(size) / 8;
-            uint32_t nw32 = nw64 == 0 ? 0u : (size >= 16 ? uint32_t(size - 16) / 4 : 0u);
-            s_nw[slot] = nw32;
-            s_src[slot] = off0 + p + 8 + 8;
-            s_len[slot] = size;
-          }
+  const bool words = (reinterpret_cast<uintptr_t>(ev) & 3u) == 0;
+  const int32_t nfeds = nbytes >= 4 ? ld_i32(ev) : 0;
+  while (s_hop < nfeds) {  // the same for all threads
+    const uint64_t w0 = s_p, w1 = w0 + kFedWindow < nbytes ? w0 + kFedWindow : nbytes;
+    for (uint64_t q = w0 + 128u * threadIdx.x; q < w1; q += 128u * blockDim.x) {
+      uint32_t v;
+      asm volatile("ld.global.ca.u8 %0, [%1];" : "=r"(v) : "l"(ev + q));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint64_t p = w0;
+      int32_t k = s_hop;
+      int n = 0;
+      while (k < nfeds && n < kFedHops && (p < w1 || n == 0)) {
+        if (p + 8 > nbytes) { s_warn |= kWarnBuffer; k = nfeds; break; }
+        int32_t fid, size;
+        if (words && (p & 3u) == 0) {
+          fid = *reinterpret_cast<const int32_t*>(ev + p);
+          size = *reinterpret_cast<const int32_t*>(ev + p + 4);
+        } else {
+          fid = ld_i32(ev + p);
+          size = ld_i32(ev + p + 4);
         }
+        if (size < 0 || p + 8 + uint64_t(size) > nbytes) { s_warn |= kWarnBuffer; k = nfeds; break; }
+        s_pos[n] = p;
+        s_fid[n] = fid;
+        s_size[n] = size;
+        ++n;
+        ++k;
         p += 8 + uint64_t(size);
       }
+      s_p = p;
+      s_n = n;
+      s_hop = k;
     }
+    __syncthreads();
+    const int r = threadIdx.x;  // kFedHops records at most, one per thread
+    const int fid = r < s_n ? s_fid[r] : -1;
+    const int slot = fid >= 0 && fid < 4096 ? fed_slot_of[fid] : -1;
+    if (slot >= 0) atomicMax(&s_last[slot], uint32_t(r) + 1u);
+    __syncthreads();
+    if (slot >= 0 && s_last[slot] == uint32_t(r) + 1u) {
+      const int32_t size = s_size[r];
+      const uint32_t nw64 = uint32_t(size) / 8;
+      s_nw[slot] = nw64 == 0 ? 0u : (size >= 16 ? uint32_t(size - 16) / 4 : 0u);
+      s_src[slot] = off0 + s_pos[r] + 8 + 8;
+      s_len[slot] = size;
+    }
+    __syncthreads();
+    if (slot >= 0) s_last[slot] = 0;
+    __syncthreads();
   }
-  __syncthreads();
+  static_assert(kFedHops == 256, "one record per thread");
   // Header and trailer checks (SiPixelRawToClusterCUDA.jl:90-128, ErrorChecker.jl:82-137). The
   // reference's checker stores no error record (_includeErrors = false, ErrorChecker.jl:30-35):
   // a header failing check() ends its loop silently and a foreign source id only prints. A header
@@ -252,17 +293,19 @@ __device__ __forceinline__ void unpack_word(const Dev& d, int e, uint32_t local,
   d.xx[g] = xx; d.yy[g] = yy; d.adc[g] = adc; d.mid[g] = mid; d.pdigi[g] = pdigi; d.rawid[g] = rawid;
 }
 
-// raw_to_digi_kernal + calib_digis for the words of one FED slot per warp (kUnpackWarps slots
-// per block: a FED holds a few hundred words, which one warp decodes in a few steps). The payload
+// raw_to_digi_kernal + calib_digis for the words of one FED slot per `parts` warps (a FED holds a
+// few hundred words, which one warp decodes in a few steps; in a small batch, where the slots do not
+// fill the GPU, its steps go to several warps: 78 us for one event of pileup 50 with one). The payload
 // is read with 128-bit loads where it sits on 4-byte boundaries (always, for FED sizes in whole
 // 64-bit words): the words before the first 16-byte boundary and after the last one are read
 // singly, the rest as 16-byte vectors.
 constexpr int kUnpackWarps = 8;
 
-__global__ void __launch_bounds__(32 * kUnpackWarps) k_unpack(Dev d) {
+__global__ void __launch_bounds__(32 * kUnpackWarps) k_unpack(Dev d, uint32_t parts) {
   __shared__ __align__(16) uint32_t s_words[kUnpackWarps][128];
   const unsigned lane = threadIdx.x & 31u, wq = threadIdx.x >> 5;
-  const int f = blockIdx.x * kUnpackWarps + int(wq), e = blockIdx.y;
+  const uint32_t wid = blockIdx.x * kUnpackWarps + wq, part = wid % parts;
+  const int f = int(wid / parts), e = blockIdx.y;
   const int NF = d.n_fed_slots;
   if (f >= NF) return;
   const size_t fs = size_t(e) * NF + f;
@@ -294,14 +337,14 @@ __global__ void __launch_bounds__(32 * kUnpackWarps) k_unpack(Dev d) {
     const uint32_t* src32 = reinterpret_cast<const uint32_t*>(src);
     uint32_t head = uint32_t((16u - (reinterpret_cast<uintptr_t>(src) & 15u)) & 15u) >> 2;
     head = head < nw ? head : nw;
-    if (lane < head) word(lane, __ldg(src32 + lane));
+    if (part == 0 && lane < head) word(lane, __ldg(src32 + lane));
     const uint32_t nvec = (nw - head) >> 2;
     const uint4* v = reinterpret_cast<const uint4*>(src32 + head);
     // the warp loads 32 aligned 16-byte vectors (128 words) and decodes them word by word through
     // shared memory, lane l taking words l, l + 32, l + 64, l + 96, so that the per-digi stores
     // of consecutive lanes stay consecutive
     uint32_t* sw = s_words[wq];
-    for (uint32_t j0 = 0; j0 < nvec; j0 += 32) {
+    for (uint32_t j0 = 32 * part; j0 < nvec; j0 += 32 * parts) {
       if (j0 + lane < nvec) reinterpret_cast<uint4*>(sw)[lane] = __ldg(v + j0 + lane);
       __syncwarp();
       const uint32_t nwords = 4u * min(32u, nvec - j0);
@@ -312,9 +355,10 @@ __global__ void __launch_bounds__(32 * kUnpackWarps) k_unpack(Dev d) {
       }
       __syncwarp();
     }
-    for (uint32_t k = head + 4 * nvec + lane; k < nw; k += 32) word(k, __ldg(src32 + k));
+    if (part == 0)
+      for (uint32_t k = head + 4 * nvec + lane; k < nw; k += 32) word(k, __ldg(src32 + k));
   } else {
-    for (uint32_t k = lane; k < nw; k += 32) {
+    for (uint32_t k = 32 * part + lane; k < nw; k += 32 * parts) {
       uint32_t ww;
       memcpy(&ww, src + 4ull * k, 4);
       word(k, ww);
@@ -331,31 +375,38 @@ __device__ __forceinline__ bool module_start_flag(const Dev& d, uint64_t ebase, 
   return j < 0 || d.mid[ebase + j] != id;
 }
 
-// Module starts per FED slot, one warp per slot (kModWarps slots per block): the flags of 32
-// words per step, counted with a ballot.
+// Module starts per FED slot, `parts` warps per slot, each a range of its words (one warp where
+// the batch's slots fill the GPU): the flags of 32 words per step, counted with a ballot.
 constexpr int kModWarps = 8;
 
-__global__ void __launch_bounds__(32 * kModWarps) k_modstart_count(Dev d) {
-  const int f = blockIdx.x * kModWarps + int(threadIdx.x >> 5), e = blockIdx.y;
+__device__ __forceinline__ uint2 part_words(uint32_t nw, uint32_t part, uint32_t parts) {
+  const uint32_t len = ((nw + parts - 1) / parts + 31u) & ~31u;
+  return make_uint2(min(nw, part * len), min(nw, (part + 1) * len));
+}
+
+__global__ void __launch_bounds__(32 * kModWarps) k_modstart_count(Dev d, uint32_t parts) {
+  const uint32_t wid = blockIdx.x * kModWarps + (threadIdx.x >> 5);
+  const int f = int(wid / parts), e = blockIdx.y;
   const int NF = d.n_fed_slots;
   if (f >= NF) return;
   const unsigned lane = threadIdx.x & 31u;
   const size_t fs = size_t(e) * NF + f;
   const uint32_t nw = d.fed_nw[fs], wo = d.fed_wo[fs];
+  const uint2 r = part_words(nw, wid % parts, parts);
   uint32_t cnt = 0;
   const uint64_t ebase = d.ev[e].word_base;
   if (ebase + wo + nw <= uint64_t(d.cap_words))
-    for (uint32_t k0 = 0; k0 < nw; k0 += 32) {
+    for (uint32_t k0 = r.x; k0 < r.y; k0 += 32) {
       const uint32_t k = k0 + lane;
-      cnt += __popc(__ballot_sync(0xffffffffu, k < nw && module_start_flag(d, ebase, wo + k)));
+      cnt += __popc(__ballot_sync(0xffffffffu, k < r.y && module_start_flag(d, ebase, wo + k)));
     }
-  if (lane == 0) d.fed_nmod[fs] = cnt;
+  if (lane == 0) d.fed_nmod[fs * parts + wid % parts] = cnt;
 }
 
-// per event: module-start offsets per FED slot, n_modules; zero the cluster counters
-__global__ void k_modstart_scan(Dev d) {
+// per event: module-start offsets per part of a FED slot, n_modules; zero the cluster counters
+__global__ void k_modstart_scan(Dev d, uint32_t parts) {
   const int e = blockIdx.x;
-  const int NF = d.n_fed_slots;
+  const int NF = d.n_fed_slots * int(parts);
   __shared__ uint32_t sh[33];
   uint32_t carry = 0;
   for (int b = 0; b < NF; b += blockDim.x) {
@@ -380,10 +431,11 @@ __global__ void k_modstart_scan(Dev d) {
   }
 }
 
-// The module starts of each FED slot at the slot's offset, one warp per slot, in word order
-// (rank of a flag = flags of the earlier lanes plus those of the earlier steps).
-__global__ void __launch_bounds__(32 * kModWarps) k_modstart_fill(Dev d) {
-  const int f = blockIdx.x * kModWarps + int(threadIdx.x >> 5), e = blockIdx.y;
+// The module starts of each part of a FED slot at the part's offset, one warp per part, in word
+// order (rank of a flag = flags of the earlier lanes plus those of the earlier steps).
+__global__ void __launch_bounds__(32 * kModWarps) k_modstart_fill(Dev d, uint32_t parts) {
+  const uint32_t wid = blockIdx.x * kModWarps + (threadIdx.x >> 5);
+  const int f = int(wid / parts), e = blockIdx.y;
   const int NF = d.n_fed_slots;
   if (f >= NF) return;
   const unsigned lane = threadIdx.x & 31u;
@@ -392,11 +444,12 @@ __global__ void __launch_bounds__(32 * kModWarps) k_modstart_fill(Dev d) {
   const uint32_t nw = d.fed_nw[fs], wo = d.fed_wo[fs];
   const uint64_t ebase = d.ev[e].word_base;
   if (ebase + wo + nw > uint64_t(d.cap_words)) return;
-  uint32_t carry = d.fed_nmod[fs];
+  const uint2 range = part_words(nw, wid % parts, parts);
+  uint32_t carry = d.fed_nmod[fs * parts + wid % parts];
   uint32_t* ms = d.module_start + size_t(e) * (kMaxNumModules + 1);
-  for (uint32_t k0 = 0; k0 < nw; k0 += 32) {
+  for (uint32_t k0 = range.x; k0 < range.y; k0 += 32) {
     const uint32_t k = k0 + lane;
-    const bool fl = k < nw && module_start_flag(d, ebase, wo + k);
+    const bool fl = k < range.y && module_start_flag(d, ebase, wo + k);
     const uint32_t bal = __ballot_sync(0xffffffffu, fl);
     if (fl) {
       const uint32_t r = carry + __popc(bal & lt);
@@ -423,20 +476,19 @@ void launch_raw(const Dev& d, const Launch& L, const int16_t* fed_slot_of) {
   k_ev_scan<<<1, 1024, 0, L.s>>>(d.ev, d.E, int(offsetof(EvInfo, n_words)), int(offsetof(EvInfo, word_base)));
   launch_ev_clamp(d, L.s, int(offsetof(EvInfo, n_words)), int(offsetof(EvInfo, word_base)), d.cap_words);
   L.mark("fed_table");
-  k_unpack<<<dim3(div_up(NF, kUnpackWarps), d.E), 32 * kUnpackWarps, 0, L.s>>>(d);
+  // warps per FED slot: one, more in a batch whose slots give an SM less than a wave of warps
+  const int parts = event_blocks(d.E * NF, kFedParts, 16);
+  k_unpack<<<dim3(div_up(int64_t(NF) * parts, kUnpackWarps), d.E), 32 * kUnpackWarps, 0, L.s>>>(d, uint32_t(parts));
   L.mark("unpack_calib");
-  const dim3 gm(div_up(NF, kModWarps), d.E);
-  k_modstart_count<<<gm, 32 * kModWarps, 0, L.s>>>(d);
-  k_modstart_scan<<<d.E, 256, 0, L.s>>>(d);
-  k_modstart_fill<<<gm, 32 * kModWarps, 0, L.s>>>(d);
+  launch_modstart(d, L, parts);
   L.mark("module_starts");
 }
 
-void launch_modstart(const Dev& d, const Launch& L) {
-  const dim3 gm(div_up(d.n_fed_slots, kModWarps), d.E);
-  k_modstart_count<<<gm, 32 * kModWarps, 0, L.s>>>(d);
-  k_modstart_scan<<<d.E, 256, 0, L.s>>>(d);
-  k_modstart_fill<<<gm, 32 * kModWarps, 0, L.s>>>(d);
+void launch_modstart(const Dev& d, const Launch& L, int parts) {
+  const dim3 gm(div_up(int64_t(d.n_fed_slots) * parts, kModWarps), d.E);
+  k_modstart_count<<<gm, 32 * kModWarps, 0, L.s>>>(d, uint32_t(parts));
+  k_modstart_scan<<<d.E, 256, 0, L.s>>>(d, uint32_t(parts));
+  k_modstart_fill<<<gm, 32 * kModWarps, 0, L.s>>>(d, uint32_t(parts));
 }
 
 void launch_ev_scan(const Dev& d, cudaStream_t s, int count_off, int base_off) {

@@ -140,7 +140,7 @@ extern "C" int32_t pxl_clusterize_digis_noalloc(const uint16_t* id, const int16_
   d.cap_big = kMaxNumModules;
   d.bpe = 148 * 4;
   Launch L{st, d.bpe, 256};
-  launch_modstart(d, L);
+  launch_modstart(d, L, 1);
   launch_cluster(d, L);
   return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;
 }

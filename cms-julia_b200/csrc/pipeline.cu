@@ -217,7 +217,7 @@ int alloc_batch(PxlCtx* ctx) {
   int rc = 0;
 #define A(ptr, n) do { rc = dalloc(ctx, &d.ptr, (n)); if (rc) return rc; } while (0)
   A(ev, E + 1);
-  A(fed_src, E * NF); A(fed_nw, E * NF); A(fed_wo, E * NF); A(fed_nmod, E * NF);
+  A(fed_src, E * NF); A(fed_nw, E * NF); A(fed_wo, E * NF); A(fed_nmod, E * NF + kFedParts);
   A(xx, d.cap_words); A(yy, d.cap_words); A(adc, d.cap_words); A(mid, d.cap_words); A(clus, d.cap_words);
   A(pdigi, d.cap_words); A(rawid, d.cap_words);
   A(err, 5 * d.cap_words); A(err_count, 1); A(id_seen, E * 64);
@@ -855,7 +855,7 @@ int32_t pxl_clusterize_digis(PxlCtx* ctx, const uint16_t* id, const int16_t* x, 
   CK(cudaMemcpyAsync(d.fed_nw, &nw, 4, cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d.fed_wo, &zero, 4, cudaMemcpyHostToDevice, s));
   Launch L{s, d.bpe, 256};
-  launch_modstart(d, L);
+  launch_modstart(d, L, 256);  // one slot, so 256 warps
   launch_cluster(d, L);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(module_start, d.module_start, (kMaxNumModules + 1) * 4, cudaMemcpyDeviceToHost, s));

@@ -35,6 +35,7 @@ constexpr int kMaxActiveColumns = 512 * 1024 / 8;  // MAX_NUM_OF_ACTIVE_DOUBLETS
 constexpr uint32_t kHitIdBits = 21;                // event-local hit ids are below 2^21
 constexpr uint32_t kMaxHitsPerEvent = 1u << kHitIdBits;
 constexpr int kMaxFedSlots = 160;
+constexpr int kFedParts = 148 * 32;  // warps over the FED slots of a small batch
 constexpr int kWarpModulePix = 256;  // modules up to this many digis are clustered by one warp
 
 // per-event warning bits (same values as PXL_WARN_* in include/pxl.h)
@@ -141,7 +142,7 @@ struct Dev {
   uint64_t* fed_src;
   uint32_t* fed_nw;
   uint32_t* fed_wo;
-  uint32_t* fed_nmod;  // module starts found per FED slot
+  uint32_t* fed_nmod;  // module starts found per part of a FED slot
   // digis [cap_words]
   int16_t* xx; int16_t* yy; int32_t* adc; int16_t* mid; int32_t* clus; uint32_t* pdigi; uint32_t* rawid;
   // FED error records [cap_words]: raw_id, word, type | fed << 8
@@ -473,7 +474,8 @@ void launch_wq_order(const Dev& d, cudaStream_t s);
 WorkQueue launch_wq_plan(const Dev& d, const Launch& L, int count_off, uint32_t units_per_block);
 
 void launch_raw(const Dev& d, const Launch& L, const int16_t* fed_slot_of);  // a1-a4
-void launch_modstart(const Dev& d, const Launch& L);  // a4 only (digis already in place)
+// a4 only (digis already in place); parts: warps per FED slot, fed_nmod holds parts counts per slot
+void launch_modstart(const Dev& d, const Launch& L, int parts);
 void launch_ev_scan(const Dev& d, cudaStream_t s, int count_off, int base_off);
 void launch_ev_clamp(const Dev& d, cudaStream_t s, int count_off, int base_off, int64_t cap);
 void launch_cluster(const Dev& d, const Launch& L);   // a5-a7
