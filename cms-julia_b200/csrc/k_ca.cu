@@ -1218,15 +1218,27 @@ __global__ void k_early_dup(Dev d) {
       const uint32_t lo = d.ct_cnt[c];
       uint32_t n = d.ct_cnt[c + 1] - lo;
       if (n > uint32_t(kCellRows)) n = kCellRows;
+      // kListBatch entries at a time, their loads independent of one another: a cell of 64 tracks
+      // otherwise waits for 128 latencies one after the other (42 us for an event of 100 tracks)
       uint32_t maxn = 0;
-      for (uint32_t j = 0; j < n; ++j) {
-        const uint32_t t = d.ct_list[lo + j];
-        const uint32_t s = d.tuple_off[t + 1] - d.tuple_off[t];
-        maxn = s > maxn ? s : maxn;
+      for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
+        uint32_t t[kListBatch], s[kListBatch];
+#pragma unroll
+        for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[lo + min(j0 + u, n - 1)];
+#pragma unroll
+        for (int u = 0; u < kListBatch; ++u) s[u] = d.tuple_off[t[u] + 1] - d.tuple_off[t[u]];
+#pragma unroll
+        for (int u = 0; u < kListBatch; ++u) maxn = s[u] > maxn ? s[u] : maxn;
       }
-      for (uint32_t j = 0; j < n; ++j) {
-        const uint32_t t = d.ct_list[lo + j];
-        if (d.tuple_off[t + 1] - d.tuple_off[t] != maxn) d.quality[t] = 1;
+      for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
+        uint32_t t[kListBatch], s[kListBatch];
+#pragma unroll
+        for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[lo + min(j0 + u, n - 1)];
+#pragma unroll
+        for (int u = 0; u < kListBatch; ++u) s[u] = d.tuple_off[t[u] + 1] - d.tuple_off[t[u]];
+#pragma unroll
+        for (int u = 0; u < kListBatch; ++u)
+          if (s[u] != maxn) d.quality[t[u]] = 1;
       }
     }
   }

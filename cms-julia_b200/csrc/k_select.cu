@@ -77,7 +77,15 @@ __global__ void __launch_bounds__(256) k_dup_cells(Dev d) {
       uint32_t n = d.ct_cnt[c + 1] - l0;
       if (n > uint32_t(kCellRows)) n = kCellRows;
       uint64_t loose = 0;
-      for (uint32_t j = 0; j < n; ++j) loose |= uint64_t(d.quality[d.ct_list[l0 + j]] == 2) << j;
+      for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
+        uint32_t t[kListBatch];
+#pragma unroll
+        for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[l0 + min(j0 + u, n - 1)];
+        uint32_t m = 0;
+#pragma unroll
+        for (int u = 0; u < kListBatch; ++u) m |= uint32_t(j0 + u < n && d.quality[t[u]] == 2) << u;
+        loose |= uint64_t(m) << j0;
+      }
       const uint32_t m = __popcll(loose);
       if (m < 2) continue;
       const uint32_t slot = atomicAdd(&E.n_dup_cells, 1u);
@@ -111,15 +119,32 @@ __global__ void k_dup_resolve(Dev d) {
     for (uint32_t i = threadIdx.x; i < nc; i += blockDim.x) {
       const uint32_t c = cell[i];
       const uint2 r = rng[i];
-      uint32_t best = 0xffffffffu, pos = 0;
-      for (uint32_t x = r.x; x < r.x + r.y; ++x) {
-        const uint32_t key = ek[x];
-        if (__ldcg(&cur[et[x]]) >= c && key < best) { best = key; pos = x; }
+      // nearly all cells have up to four loose tracks: their loads in flight together
+      constexpr uint32_t kN = 4;
+      uint32_t t[kN], key[kN], best = 0xffffffffu, pos = 0;
+      bool alive[kN];
+#pragma unroll
+      for (uint32_t u = 0; u < kN; ++u) {
+        const uint32_t x = r.x + min(u, r.y - 1);
+        t[u] = et[x];
+        key[u] = ek[x];
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kN; ++u) alive[u] = u < r.y && __ldcg(&cur[t[u]]) >= c;
+#pragma unroll
+      for (uint32_t u = 0; u < kN; ++u)
+        if (alive[u] && key[u] < best) { best = key[u]; pos = u; }
+      for (uint32_t u = kN; u < r.y; ++u) {
+        const uint32_t k = ek[r.x + u];
+        if (__ldcg(&cur[et[r.x + u]]) >= c && k < best) { best = k; pos = u; }
       }
       if (best == 0xffffffffu) continue;
-      for (uint32_t x = r.x; x < r.x + r.y; ++x) {
-        const uint32_t key = ek[x];
-        if (key > best || (key == best && x > pos)) atomicMin(&nxt[et[x]], c);
+#pragma unroll
+      for (uint32_t u = 0; u < kN; ++u)
+        if (u < r.y && (key[u] > best || (key[u] == best && u > pos))) atomicMin(&nxt[t[u]], c);
+      for (uint32_t u = kN; u < r.y; ++u) {
+        const uint32_t k = ek[r.x + u];
+        if (k > best || (k == best && u > pos)) atomicMin(&nxt[et[r.x + u]], c);
       }
     }
     __syncthreads();
