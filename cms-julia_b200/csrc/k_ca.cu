@@ -578,7 +578,6 @@ __device__ __forceinline__ void sort_list(uint32_t* a, uint32_t n) {
   }
 }
 
-// per-hit lists (kind 0: cells ending on the hit; 2: tuples through the hit, descending)
 // lists above the short-sort limit, sorted afterwards by k_sort_long (a list of n entries
 // needs n > 8, so the buffer of cap_long = entries / 9 entries cannot overflow)
 __device__ __forceinline__ void push_long_list(const Dev& d, uint32_t lo, uint32_t n) {
@@ -596,17 +595,47 @@ __global__ void __launch_bounds__(256) k_sort_long(Dev d, uint32_t* list) {
   }
 }
 
-template <int kKind>
+// Sorts a list of 33..128 entries with a whole warp: each lane holds four entries and counts, for
+// each, the entries below it as they go round by shuffles (entries differ).
+__device__ __forceinline__ void sort_list_warp(uint32_t* a, uint32_t n) {
+  const unsigned lane = threadIdx.x & 31u;
+  uint32_t v[4], r[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int u = 0; u < 4; ++u) v[u] = lane + 32u * u < n ? a[lane + 32u * u] : 0xffffffffu;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    for (uint32_t k = 0; k < 32 && 32u * q + k < n; ++k) {
+      const uint32_t x = __shfl_sync(0xffffffffu, v[q], int(k));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) r[u] += x < v[u];
+    }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (lane + 32u * u < n) a[r[u]] = v[u];
+}
+
+// A thread per hit sorts the lists of up to 32 entries in registers; the warp then takes its hits'
+// longer ones together (an insertion sort by one thread, kept above 128 entries, made the kernel
+// 248 us for one event of pileup 170).
 __global__ void k_sort_hit_lists(Dev d) {
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
-  const uint32_t hb = E.hit_base;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < E.n_hits; k += gridDim.x * blockDim.x) {
-    const uint32_t h = hb + k;
-    if (kKind == 0) {
-      const uint32_t lo = d.ohc_cnt[h], hi = d.ohc_cnt[h + 1];
-      sort_list(d.ohc_list + lo, hi - lo);
-      if (hi - lo > uint32_t(kMaxCellsPerHit)) atomic_or_warn(&d.ev[e], kWarnLists);
+  const uint32_t hb = E.hit_base, nh = E.n_hits;
+  const unsigned lane = threadIdx.x & 31u;
+  for (uint32_t k0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); k0 < nh; k0 += gridDim.x * blockDim.x) {
+    const uint32_t k = k0 + lane;
+    uint32_t lo = 0, n = 0;
+    if (k < nh) {
+      lo = d.ohc_cnt[hb + k];
+      n = d.ohc_cnt[hb + k + 1] - lo;
+      if (n > uint32_t(kMaxCellsPerHit)) atomic_or_warn(&d.ev[e], kWarnLists);
+    }
+    const bool together = n > 32 && n <= 128;
+    if (!together) sort_list(d.ohc_list + lo, n);
+    for (uint32_t m = __ballot_sync(0xffffffffu, together); m; m &= m - 1) {
+      const int src = __ffs(m) - 1;
+      sort_list_warp(d.ohc_list + __shfl_sync(0xffffffffu, lo, src), __shfl_sync(0xffffffffu, n, src));
     }
   }
 }
@@ -1354,7 +1383,7 @@ void launch_ca(const Dev& d, const Launch& L) {
   // cells ending on each hit (counted by the doublet fill)
   excl_scan_shift_u32(d.ohc_cur, d.ohc_cnt, d.cap_hits, &d.ev[d.E].n_hits, d.scan_tmp, L.s);
   k_ohc_fill<<<g(kTuneHitLists), 256, 0, L.s>>>(d);
-  k_sort_hit_lists<0><<<g(kTuneHitLists), 256, 0, L.s>>>(d);
+  k_sort_hit_lists<<<g(kTuneHitLists), 256, 0, L.s>>>(d);
   k_ohc_records<<<g(kTuneHitLists), 256, 0, L.s>>>(d);
   L.mark("outer_hit_lists");
   // connection and neighbour lists

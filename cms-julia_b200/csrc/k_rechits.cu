@@ -348,6 +348,14 @@ __global__ void __launch_bounds__(256) k_get_hits_block(Dev d) {
   }
 }
 
+// 1-based phi bin of hit i (0-based) with azimuth t: 128 bins per layer
+__device__ __forceinline__ uint32_t phi_bin_of(int16_t t, uint32_t i, const uint32_t* hls) {
+  int k = 0;
+  while (k < 11 && hls[k] < i) ++k;  // searchsortedfirst
+  const int layer = (k < 11 && hls[k] == i) ? k : k - 1;
+  return ((uint32_t(int32_t(t >> 9)) & 127u) + 1u) + 128u * uint32_t(layer);
+}
+
 // setHitsLayerStart + fill_many_from_vector for the 10x128 phi histogram, one block per event.
 // Bins end up holding hit ids in decreasing order (the reference fill decrements the bin cursor).
 __global__ void __launch_bounds__(1024) k_phi_binner(Dev d) {
@@ -372,15 +380,7 @@ __global__ void __launch_bounds__(1024) k_phi_binner(Dev d) {
     return;
   }
   const uint32_t ntot = s_hls[10];
-  auto layer_of = [&](uint32_t i) -> int {
-    int k = 0;
-    while (k < 11 && s_hls[k] < i) ++k;  // searchsortedfirst
-    return (k < 11 && s_hls[k] == i) ? k : k - 1;
-  };
-  auto bin_of = [&](uint32_t i) -> uint32_t {
-    const int16_t t = d.iphi[hb + i];
-    return ((uint32_t(int32_t(t >> 9)) & 127u) + 1u) + 128u * uint32_t(layer_of(i));
-  };
+  auto bin_of = [&](uint32_t i) -> uint32_t { return phi_bin_of(d.iphi[hb + i], i, s_hls); };
   for (uint32_t i = threadIdx.x; i < ntot; i += blockDim.x) atomicAdd(&s_off[bin_of(i) - 1], 1u);
   __syncthreads();
   // inclusive scan of 1281 counters
@@ -396,32 +396,56 @@ __global__ void __launch_bounds__(1024) k_phi_binner(Dev d) {
     }
   }
   __syncthreads();
-  uint32_t* bins = d.phi_bins + hb;
+  uint32_t* bins = d.phi_fill + hb;  // in any order; k_phi_place puts them in order
   for (uint32_t i = threadIdx.x; i < ntot; i += blockDim.x) {
     uint32_t w = atomicSub(&s_off[bin_of(i) - 1], 1u);
     bins[w - 1] = i + 1;
   }
   __syncthreads();
   for (int b = threadIdx.x; b < kPhiTotBins; b += blockDim.x) poff[b] = s_off[b];
-  // Each binned hit's place in two orders of its bin, by its rank among the bin's hits (a
-  // bin holds a few tens of hits): decreasing hit id, the reference's order (its fill
-  // decrements the bin cursor), for the doublet records and the bins; and increasing iphi
-  // (as uint16, ties by decreasing id) for the records of the doublet search's exact phi
-  // windows.
+}
+
+// Each binned hit's place in two orders of its bin, by its rank among the bin's hits (a
+// bin holds a few tens of hits): decreasing hit id, the reference's order (its fill
+// decrements the bin cursor), for the doublet records and the bins; and increasing iphi
+// (as uint16, ties by decreasing id) for the records of the doublet search's exact phi
+// windows. A thread per hit over all the event's blocks (within k_phi_binner's one block per
+// event, 85 us of one event of pileup 170 went here).
+__global__ void __launch_bounds__(256) k_phi_place(Dev d) {
+  const int e = blockIdx.y;
+  const EvInfo& E = d.ev[e];
+  const uint32_t hb = E.hit_base;
+  const uint32_t nh = E.n_hits;
+  if (nh == 0 || uint64_t(hb) + nh > uint64_t(d.cap_hits)) return;
+  __shared__ uint32_t s_hls[11];
+  if (threadIdx.x < 11) s_hls[threadIdx.x] = d.hits_layer_start[size_t(e) * 11 + threadIdx.x];
+  __syncthreads();
+  const uint32_t ntot = s_hls[10];
+  const uint32_t* poff = d.phi_off + size_t(e) * kPhiTotBins;
+  const uint32_t* from = d.phi_fill + hb;
   HitRec* rec = d.hit_rec + hb;
   HitRec* rs = d.hit_rec_s + hb;
   uint16_t* us = d.hit_u_s + hb;
-  for (uint32_t p = threadIdx.x; p < ntot; p += blockDim.x) {
-    const uint32_t v = bins[p], i = v - 1u;
-    const uint32_t b = bin_of(i) - 1u;
-    const uint32_t lo = s_off[b], hi = s_off[b + 1];
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < ntot; p += gridDim.x * blockDim.x) {
+    const uint32_t v = from[p], i = v - 1u;
     const uint16_t u = uint16_t(d.iphi[hb + i]);
+    const uint32_t b = phi_bin_of(int16_t(u), i, s_hls) - 1u;
+    const uint32_t lo = poff[b], hi = poff[b + 1];
     uint32_t rid = 0, ru = 0;
-    for (uint32_t q = lo; q < hi; ++q) {
-      const uint32_t w = bins[q];
-      const uint16_t uq = uint16_t(d.iphi[hb + w - 1u]);
-      rid += w > v;
-      ru += uq < u || (uq == u && w > v);
+    constexpr int kB = 4;  // entries whose loads are in flight together
+    for (uint32_t q = lo; q < hi; q += kB) {
+      uint32_t w[kB];
+      uint16_t uq[kB];
+#pragma unroll
+      for (int k = 0; k < kB; ++k) w[k] = from[min(q + k, hi - 1)];
+#pragma unroll
+      for (int k = 0; k < kB; ++k) uq[k] = uint16_t(d.iphi[hb + w[k] - 1u]);
+#pragma unroll
+      for (int k = 0; k < kB; ++k) {
+        const bool in = q + k < hi;
+        rid += in && w[k] > v;
+        ru += in && (uq[k] < u || (uq[k] == u && w[k] > v));
+      }
     }
     HitRec r;
     r.z = d.zg[hb + i];
@@ -433,9 +457,8 @@ __global__ void __launch_bounds__(1024) k_phi_binner(Dev d) {
     rec[lo + rid] = r;
     rs[lo + ru] = r;
     us[lo + ru] = u;
+    d.phi_bins[hb + lo + rid] = v;
   }
-  __syncthreads();
-  for (uint32_t p = threadIdx.x; p < ntot; p += blockDim.x) bins[p] = (rec[p].det_id & (kMaxHitsPerEvent - 1u)) + 1u;
 }
 
 }  // namespace
@@ -453,6 +476,7 @@ void launch_rechits(const Dev& d, const Launch& L) {
   k_get_hits_block<<<148 * 2, 256, 0, L.s>>>(d);
   L.mark("get_hits_block");
   k_phi_binner<<<d.E, 1024, 0, L.s>>>(d);
+  k_phi_place<<<dim3(event_blocks(d.E, 148 * 32, 128), d.E), 256, 0, L.s>>>(d);
   L.mark("phi_binner");
 }
 

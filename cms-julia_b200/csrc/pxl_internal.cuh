@@ -161,6 +161,7 @@ struct Dev {
   uint32_t* hits_layer_start;  // [E][11]
   uint32_t* phi_off;           // [E][1281]
   uint32_t* phi_bins;          // [cap_hits], 1-based hit ids
+  uint32_t* phi_fill;          // [cap_hits] the same, in any order within a bin
   struct HitRec* hit_rec;      // [cap_hits] the binned hits' doublet fields, in bin order
   struct HitRec* hit_rec_s;    // [cap_hits] the same, sorted by iphi (as uint16) within each bin
   uint16_t* hit_u_s;           // [cap_hits] their iphi (as uint16), for the phi-window searches
