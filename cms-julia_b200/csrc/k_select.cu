@@ -236,10 +236,11 @@ __global__ void k_triplet_cleaner(Dev d) {
 // and one of pileup 50 326 us.
 constexpr int kMaxVtx = 1024;
 constexpr int kVtxWideThreads = 1024, kVtxNarrowThreads = 256;
-// Selected tracks whose arrays fit shared memory. The narrow form (46 KB, four or five CTAs per SM)
-// serves batches that fill the SMs with one CTA per event; the wide form (one CTA per SM) serves
-// small batches and the few events above the narrow capacity; above both, global memory.
-constexpr uint32_t kVtxWideTracks = 12288, kVtxNarrowTracks = 2048;
+// Selected tracks whose arrays fit shared memory. The narrow form (54 KB, four CTAs per SM) serves
+// batches that fill the SMs with one CTA per event; the wide form (one CTA per SM) serves small
+// batches and the few events above the narrow capacity; above both, global memory.
+constexpr uint32_t kVtxWideTracks = 11264, kVtxNarrowTracks = 2048;
+constexpr int kVtxParts = 64;  // most blocks that select an event's tracks
 
 struct VtxShared {
   uint32_t sh[33];
@@ -247,32 +248,24 @@ struct VtxShared {
   uint32_t cur[256];
   uint32_t nv, nvi, warn;
   uint32_t vcnt[kMaxVtx], voff[kMaxVtx + 1];
+  int32_t vnd[kMaxVtx];  // the vertices' ndof
   uint16_t parent[kMaxVtx];
 };
 
-// per-track arrays of one event, in shared or global memory
+// per-track arrays of one event, in shared or global memory, by position in z order
 template <typename TI, typename TB>
 struct VtxTracks {
-  const float* zt;
-  const float* ezt2;
-  TI* iv;        // 1-based values as the reference stores them
+  float* zt;
+  float* ezt2;
+  TI* iv;        // 1-based values as the reference stores them; positions until the vertices are numbered
   TI* nn;
-  TB* B;         // z histogram, then the vertices' track lists
-  TB* C;         // unordered form of B
-  uint8_t* izt;
+  TB* ord;       // the track (in tuple order) at a position
+  TB* B;         // the vertices' track lists (positions)
+  TB* C;         // scratch
+  uint8_t* izt;  // z bins by track; then the 2-means sides by position
 };
 
-constexpr size_t vtx_smem_bytes(uint32_t tracks) { return (sizeof(VtxShared) + 15) / 16 * 16 + size_t(tracks) * 17; }
-
-// entries [lo, hi) of C put in order into B: ascending, or descending with kDown. Each entry counts
-// the ones before it; the runs are short (a z bin, a vertex) and all entries count at once.
-template <bool kDown, typename TB>
-__device__ __forceinline__ void place_by_rank(const TB* C, TB* B, uint32_t p, uint32_t lo, uint32_t hi) {
-  const TB x = C[p];
-  uint32_t r = lo;
-  for (uint32_t q = lo; q < hi; ++q) r += kDown ? C[q] > x : C[q] < x;
-  B[r] = x;
-}
+constexpr size_t vtx_smem_bytes(uint32_t tracks) { return (sizeof(VtxShared) + 15) / 16 * 16 + size_t(tracks) * 19; }
 
 // acc0 + a[0] + a[1] + ... and acc1 + b[0] + ... over the lanes of a warp in lane order (lanes that
 // take no part hold +0, which leaves a sum that is never -0 as it is); every lane gets the sums
@@ -304,16 +297,19 @@ __device__ __forceinline__ float ordered_add(float a, uint32_t n, float acc) {
 }
 
 // cluster_tracks_by_density, fit_vertices, split_vertices and sort_by_pt2 on the nt selected
-// tracks of one event (one CTA).
+// tracks of one event (one CTA); gz, ge, ptt2 and itrk are theirs in tuple order, nn_out receives the
+// reference's nn array (neighbour counts of the tracks, then ndof of the vertices).
 template <typename TI, typename TB>
 __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, const VtxTracks<TI, TB>& A,
-                                            const float* ptt2, const uint32_t* itrk, float* zv, float* wv,
-                                            float* vchi2, float* ptv2, uint16_t* sort_ind, VtxShared& S) {
+                                            const float* gz, const float* ge, const float* ptt2, const uint32_t* itrk,
+                                            float* zv, float* wv, float* vchi2, float* ptv2, uint16_t* sort_ind,
+                                            int32_t* nn_out, VtxShared& S) {
   const uint64_t tb = E.tuple_base;
-  const float* zt = A.zt;
-  const float* ezt2 = A.ezt2;
+  float* zt = A.zt;
+  float* ezt2 = A.ezt2;
   TI* iv = A.iv;
   TI* nn = A.nn;
+  TB* ord = A.ord;
   TB* B = A.B;
   TB* C = A.C;
   uint8_t* izt = A.izt;
@@ -321,12 +317,14 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
   // cluster_tracks_by_density (:84-206), HisToContainer{UInt8,256,16000,8,UInt16}
   for (uint32_t b = threadIdx.x; b < 257; b += blockDim.x) S.off[b] = 0;
   __syncthreads();
+  float* z0 = ezt2;  // z in tuple order, until the positions are known
   for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
-    int32_t iz = int32_t(trunc(__dmul_rn(double(zt[i]), 10.)));
+    const float z = gz[i];
+    int32_t iz = int32_t(trunc(__dmul_rn(double(z), 10.)));
     iz = iz < -128 ? -128 : (iz > 127 ? 127 : iz);
+    z0[i] = z;
     izt[i] = uint8_t(iz + 128);
-    atomicAdd(&S.off[izt[i]], 1u);
-    iv[i] = TI(i + 1);
+    atomicAdd(&S.off[iz + 128], 1u);
   }
   __syncthreads();
   {  // exclusive starts of the 256 bins
@@ -337,81 +335,96 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
     if (threadIdx.x == 0) S.off[256] = tot;
   }
   __syncthreads();
-  // histogram contents (1-based track indices), decreasing track index within a bin
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) C[atomicAdd(&S.cur[izt[i]], 1u)] = TB(i + 1);
+  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) C[atomicAdd(&S.cur[izt[i]], 1u)] = TB(i);
   __syncthreads();
-  for (uint32_t p = threadIdx.x; p < nt; p += blockDim.x) {
-    const uint32_t b = izt[C[p] - 1];
-    place_by_rank<true>(C, B, p, S.off[b], S.off[b + 1]);
+  // Positions in z order (the bins are z ranges; equal z by decreasing track, the reference's order
+  // in a bin). The reference scans a track's bin and the two next to it, 1 mm each; in z order the
+  // tracks within eps = 0.7 mm are one run around it, which two short walks find: half the pairs,
+  // and the arrays read in order (370 k of 600 k cycles of an event of 4.3 k tracks were these scans).
+  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
+    const uint32_t b = izt[i], hi = S.off[b + 1];
+    const float z = z0[i];
+    uint32_t r = S.off[b];
+    for (uint32_t q = r; q < hi; ++q) {
+      const uint32_t j = C[q];
+      const float zj = z0[j];
+      r += zj < z || (zj == z && j > i);
+    }
+    ord[r] = TB(i);
   }
   __syncthreads();
-  // the density loops go over the tracks in histogram order: the lanes of a warp then scan the
-  // same few bins
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) zt[s] = z0[ord[s]];
+  __syncthreads();
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) ezt2[s] = ge[ord[s]];
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) C[ord[s]] = TB(s);
+  __syncthreads();
   const float eps = 0.07f, err2_max = __fmul_rn(0.01f, 0.01f), chi2_max = 9.0f;
   for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) {
-    const uint32_t i = B[s] - 1;
-    const float e2 = ezt2[i], z = zt[i];
-    if (e2 > err2_max) continue;
-    const int bs0 = int(izt[i]) + 1;
-    const int be = bs0 + 1 < 256 ? bs0 + 1 : 256;
-    const int bs = bs0 - 1 > 1 ? bs0 - 1 : 1;
+    const float e2 = ezt2[s], z = zt[s];
     int32_t cnt = 0;
-    for (uint32_t p = S.off[bs - 1], pe = S.off[be]; p < pe; ++p) {
-      const uint32_t j = B[p] - 1;
-      if (j == i) continue;
-      const float dist = fabsf(__fsub_rn(z, zt[j]));
-      if (dist > eps) continue;
-      if (__fmul_rn(dist, dist) > __fmul_rn(chi2_max, __fadd_rn(e2, ezt2[j]))) continue;
-      ++cnt;
+    if (!(e2 > err2_max)) {
+      auto step = [&](uint32_t p) {
+        const float dist = fabsf(__fsub_rn(z, zt[p]));
+        if (dist > eps) return false;
+        if (!(__fmul_rn(dist, dist) > __fmul_rn(chi2_max, __fadd_rn(e2, ezt2[p])))) ++cnt;
+        return true;
+      };
+      for (uint32_t p = s + 1; p < nt && step(p); ++p) {}
+      for (uint32_t p = s; p > 0 && step(p - 1); --p) {}
     }
-    nn[i] = TI(cnt);
+    nn[s] = TI(cnt);
+  }
+  __syncthreads();
+  // the nearest track of more neighbours (of as many, at smaller z); among equally near ones the
+  // last in the reference's order (bins up, tracks down within a bin)
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) {
+    const float e2 = ezt2[s], z = zt[s];
+    const TI ni = nn[s];
+    float mdist = eps;
+    uint32_t a = s;
+    auto step = [&](uint32_t p) {
+      const float zp = zt[p];
+      const float dist = fabsf(__fsub_rn(z, zp));
+      if (dist > mdist) return false;  // and so are the tracks beyond
+      const TI np = nn[p];
+      if (np < ni || (np == ni && zp >= z)) return true;
+      if (__fmul_rn(dist, dist) > __fmul_rn(chi2_max, __fadd_rn(e2, ezt2[p]))) return true;
+      if (dist == mdist && a != s) {
+        const uint32_t ip = ord[p], ia = ord[a];
+        const uint8_t bp = izt[ip], ba = izt[ia];
+        if (bp != ba ? bp < ba : ip > ia) return true;
+      }
+      mdist = dist;
+      a = p;
+      return true;
+    };
+    for (uint32_t p = s + 1; p < nt && step(p); ++p) {}
+    for (uint32_t p = s; p > 0 && step(p - 1); --p) {}
+    iv[s] = TI(a + 1);
   }
   __syncthreads();
   for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) {
-    const uint32_t i = B[s] - 1;
-    const float e2 = ezt2[i], z = zt[i];
-    const TI ni = nn[i];
-    float mdist = eps;
-    const int bs0 = int(izt[i]) + 1;
-    const int be = bs0 + 1 < 256 ? bs0 + 1 : 256;
-    const int bs = bs0 - 1 > 1 ? bs0 - 1 : 1;
-    int32_t a = int32_t(i + 1);
-    for (uint32_t p = S.off[bs - 1], pe = S.off[be]; p < pe; ++p) {
-      const uint32_t j = B[p] - 1;
-      const TI nj = nn[j];
-      if (nj < ni) continue;
-      const float zj = zt[j];
-      if (nj == ni && zj >= z) continue;
-      const float dist = fabsf(__fsub_rn(z, zj));
-      if (dist > mdist) continue;
-      if (__fmul_rn(dist, dist) > __fmul_rn(chi2_max, __fadd_rn(e2, ezt2[j]))) continue;
-      mdist = dist;
-      a = int32_t(j + 1);
-    }
-    iv[i] = TI(a);
-  }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
-    int32_t m = iv[i];
+    int32_t m = iv[s];
     while (m != int32_t(iv[m - 1])) m = iv[m - 1];
-    iv[i] = TI(m);
+    iv[s] = TI(m);
   }
   __syncthreads();
-  uint32_t found = 0;
+  uint32_t found = 0;  // vertices are numbered in tuple order
   for (uint32_t b = 0; b < nt; b += blockDim.x) {
     const uint32_t i = b + threadIdx.x;
-    const bool root = i < nt && iv[i] == int32_t(i + 1);
-    const bool seed = root && nn[i] >= 2;
+    const uint32_t s = i < nt ? C[i] : 0u;
+    const bool root = i < nt && iv[s] == TI(s + 1);
+    const bool seed = root && nn[s] >= 2;
     uint32_t tot;
     const uint32_t ex = block_excl_scan(seed ? 1u : 0u, S.sh, &tot);
-    if (root) iv[i] = TI(seed ? -int32_t(found + ex + 1) : -9998);
+    if (root) iv[s] = TI(seed ? -int32_t(found + ex + 1) : -9998);
     found += tot;
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x)
-    if (iv[i] >= 0) iv[i] = iv[iv[i] - 1];
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x)
+    if (iv[s] >= 0) iv[s] = iv[iv[s] - 1];
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) iv[i] = TI(-iv[i]);
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) iv[s] = TI(-iv[s]);
   if (threadIdx.x == 0) {
     if (found >= uint32_t(kMaxVtx)) { S.warn |= kWarnVertex; found = kMaxVtx - 1; }
     S.nv = found;
@@ -419,13 +432,13 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
   }
   __syncthreads();
   // per-vertex track lists in ascending track order (the order of the reference's loops over
-  // all tracks); B (the z histogram) is free again. A vertex made by a split keeps its parent's
+  // all tracks). A vertex made by a split keeps its parent's
   // list and selects its own tracks by id, as the loops over all tracks do.
   const uint32_t nv0 = S.nv;
   for (uint32_t v = threadIdx.x; v < uint32_t(kMaxVtx); v += blockDim.x) { S.vcnt[v] = 0; S.parent[v] = uint16_t(v); }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x)
-    if (iv[i] >= 1 && uint32_t(iv[i]) <= nv0) atomicAdd(&S.vcnt[iv[i] - 1], 1u);
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x)
+    if (iv[s] >= 1 && uint32_t(iv[s]) <= nv0) atomicAdd(&S.vcnt[iv[s] - 1], 1u);
   __syncthreads();
   {
     uint32_t base = 0;
@@ -440,13 +453,16 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
     if (threadIdx.x == 0) S.voff[nv0] = base;
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x)
-    if (iv[i] >= 1 && uint32_t(iv[i]) <= nv0) C[atomicAdd(&S.vcnt[iv[i] - 1], 1u)] = TB(i);
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x)
+    if (iv[s] >= 1 && uint32_t(iv[s]) <= nv0) C[atomicAdd(&S.vcnt[iv[s] - 1], 1u)] = ord[s];
   __syncthreads();
-  for (uint32_t p = threadIdx.x, n = S.voff[nv0]; p < n; p += blockDim.x) {
-    const uint32_t v = uint32_t(iv[C[p]]) - 1;
-    place_by_rank<false>(C, B, p, S.voff[v], S.voff[v + 1]);
-  }
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x)
+    if (iv[s] >= 1 && uint32_t(iv[s]) <= nv0) {  // its rank among the vertex's tracks
+      const TB i = ord[s];
+      uint32_t r = S.voff[iv[s] - 1];
+      for (uint32_t q = r, hi = S.voff[iv[s]]; q < hi; ++q) r += C[q] < i;
+      B[r] = TB(s);
+    }
   __syncthreads();
   // fit_vertices, :228-286: a warp per vertex, its sums in track order
   auto fit = [&](double chi2max) {
@@ -485,7 +501,7 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
         c2s = ordered_add(c2, hi - p0, c2s);
       }
       if (cnt > 0) w = __fmul_rn(w, __fdiv_rn(float(cnt), c2s));
-      if (lane == 0) { zv[v] = z; wv[v] = w; vchi2[v] = c2s; nn[v] = TI(cnt); }
+      if (lane == 0) { zv[v] = z; wv[v] = w; vchi2[v] = c2s; S.vnd[v] = cnt; }
     }
     __syncthreads();
     if (threadIdx.x == 0) S.nv = nvf;
@@ -498,8 +514,8 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
     for (uint32_t kv = wid; kv < nvf; kv += nwarp) {
       bool split = false;
       const uint32_t lo = S.voff[kv], hi = S.voff[kv + 1];
-      if (nn[kv] >= 4 && !(vchi2[kv] < __fmul_rn(9.0f, float(nn[kv])))) {
-        if (nn[kv] >= 512) {
+      if (S.vnd[kv] >= 4 && !(vchi2[kv] < __fmul_rn(9.0f, float(S.vnd[kv])))) {
+        if (S.vnd[kv] >= 512) {
           if (lane == 0) atomicOr(&S.warn, kWarnVertex);
         } else {
           // 2-means in the vertex's tracks (zz = zt - zv, weights 1/ezt2), at most 20 iterations;
@@ -515,7 +531,7 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
             }
             nq += __popc(__ballot_sync(0xffffffffu, in));
           }
-          if (nq != uint32_t(nn[kv] + 1) && lane == 0) atomicOr(&S.warn, kWarnVertex);
+          if (nq != uint32_t(S.vnd[kv] + 1) && lane == 0) atomicOr(&S.warn, kWarnVertex);
           bool more = true;
           int iter = 20;
           float znew0 = 0, znew1 = 0, w0 = 0, w1 = 0;
@@ -597,7 +613,7 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
   // sort_by_pt2, :391-436 (the sorted order itself is dropped by the reference)
   const uint32_t nvf = S.nv;
   if (nvf >= 1) {
-    for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) d.idv[tb + itrk[i]] = int16_t(iv[i]);
+    for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x) d.idv[tb + itrk[ord[s]]] = int16_t(iv[s]);
     for (uint32_t v = wid; v < nvf; v += nwarp) {
       const uint32_t pv = S.parent[v], lo = S.voff[pv], hi = S.voff[pv + 1];
       float s = 0;
@@ -605,7 +621,7 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
         float x = 0.f;
         if (p0 + lane < hi) {
           const uint32_t i = B[p0 + lane];
-          if (iv[i] == int32_t(v + 1)) x = ptt2[i];
+          if (iv[i] == int32_t(v + 1)) x = ptt2[ord[i]];
         }
         s = ordered_add(x, hi - p0, s);
       }
@@ -613,6 +629,9 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
     }
     if (threadIdx.x == 0 && nvf == 1) sort_ind[0] = 1;
   }
+  for (uint32_t s = threadIdx.x; s < nt; s += blockDim.x)
+    if (ord[s] >= nvf) nn_out[ord[s]] = nn[s];
+  for (uint32_t v = threadIdx.x; v < nvf; v += blockDim.x) nn_out[v] = S.vnd[v];
   __syncthreads();
   if (threadIdx.x == 0) {
     E.n_vtx = nvf;
@@ -620,118 +639,96 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
   }
 }
 
-// zeroes the event's vertex products and selects its tracks (load_tracks, :51-82: >= 4 hits, loose,
-// pt >= 0.5, in tuple order); returns their number. A warp looks at 128 consecutive tuples per step,
-// its loads in flight together.
-__device__ __forceinline__ uint32_t vertex_tracks(const Dev& d, EvInfo& E, int e, uint32_t* sh) {
-  const uint64_t tb = E.tuple_base;
-  const uint32_t ntu = E.n_tuples;
-  int32_t* nn = d.ndof + tb + size_t(e) * kMaxVtx;  // length n_tuples + 1024
-  for (uint32_t v = threadIdx.x; v < uint32_t(kMaxVtx); v += blockDim.x) {
-    const size_t g = size_t(e) * kMaxVtx + v;
-    d.zv[g] = 0; d.wv[g] = 0; d.vchi2[g] = 0; d.ptv2[g] = 0; d.sort_ind[g] = 0;
-  }
-  for (uint32_t t = threadIdx.x; t < ntu + kMaxVtx; t += blockDim.x) nn[t] = 0;
-  for (uint32_t t = threadIdx.x; t < ntu; t += blockDim.x) d.idv[tb + t] = -1;
-  constexpr int kStep = 4;
-  const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  uint32_t nt = 0;
-  for (uint32_t b = 0; b < ntu; b += kStep * blockDim.x) {
-    const uint32_t t0 = b + wid * (32 * kStep) + lane;
-    uint32_t n[kStep];
-    uint8_t q[kStep];
-    float pt[kStep];
-#pragma unroll
-    for (int u = 0; u < kStep; ++u) {
-      const uint32_t t = t0 + 32 * u;
-      n[u] = 0;
-      if (t < ntu) {
-        n[u] = d.tuple_off[tb + t + 1] - d.tuple_off[tb + t];
-        q[u] = d.quality[tb + t];
-        pt[u] = d.t_pt[tb + t];
-      }
+// load_tracks (:51-82): the event's tracks of >= 4 hits, loose, pt >= 0.5, in tuple order. Each of
+// the event's blocks lists those of its range of tuples (vws_list, vtx_cnt); it also clears the range's
+// vertex ids and, with the first block, the event's vertex products.
+__global__ void __launch_bounds__(256) k_vertex_select(Dev d) {
+  const int e = blockIdx.y;
+  const EvInfo& E = d.ev[e];
+  __shared__ uint32_t sh[33];
+  if (blockIdx.x == 0)
+    for (uint32_t v = threadIdx.x; v < uint32_t(kMaxVtx); v += blockDim.x) {
+      const size_t g = size_t(e) * kMaxVtx + v;
+      d.zv[g] = 0; d.wv[g] = 0; d.vchi2[g] = 0; d.ptv2[g] = 0; d.sort_ind[g] = 0;
     }
-    uint32_t m[kStep], cnt = 0;
-#pragma unroll
-    for (int u = 0; u < kStep; ++u) {
-      m[u] = __ballot_sync(0xffffffffu, n[u] >= 4 && q[u] == 2 && !(pt[u] < 0.5f));
-      cnt += __popc(m[u]);
+  const uint64_t tb = E.tuple_base;
+  const uint32_t per = (E.n_tuples + gridDim.x - 1) / gridDim.x;
+  const uint32_t lo = min(E.n_tuples, blockIdx.x * per), hi = min(E.n_tuples, lo + per);
+  uint32_t n = 0;
+  for (uint32_t b = lo; b < hi; b += blockDim.x) {
+    const uint32_t t = b + threadIdx.x;
+    bool sel = false;
+    if (t < hi) {
+      d.idv[tb + t] = -1;
+      sel = d.tuple_off[tb + t + 1] - d.tuple_off[tb + t] >= 4 && d.quality[tb + t] == 2 && !(d.t_pt[tb + t] < 0.5f);
     }
     uint32_t tot;
-    const uint32_t ex = block_excl_scan(lane == 0 ? cnt : 0u, sh, &tot);
-    uint32_t i0 = nt + __shfl_sync(0xffffffffu, ex, 0);
-#pragma unroll
-    for (int u = 0; u < kStep; ++u) {
-      if ((m[u] >> lane) & 1u) {
-        const uint32_t t = t0 + 32 * u;
-        const uint64_t i = tb + i0 + __popc(m[u] & lt);
-        d.vws_itrk[i] = t;
-        d.vws_zt[i] = d.t_state[5 * (tb + t) + 4];
-        d.vws_ezt2[i] = d.t_cov[15 * (tb + t) + 14];
-        d.vws_ptt2[i] = __fmul_rn(pt[u], pt[u]);
-      }
-      i0 += __popc(m[u]);
-    }
-    nt += tot;
+    const uint32_t r = n + block_excl_scan(sel ? 1u : 0u, sh, &tot);
+    if (sel) d.vws_list[tb + lo + r] = t;
+    n += tot;
   }
-  if (threadIdx.x == 0) E.n_vtx_tracks = nt;
-  __syncthreads();
-  return nt;
+  if (threadIdx.x == 0) d.vtx_cnt[e * gridDim.x + blockIdx.x] = n;
 }
 
-// Events e of the grid's stride. kSelect: the launch selects the tracks (else an earlier one did)
-// and takes the events of at most kCap tracks, and with kAll those above in global memory too;
-// without kSelect it takes the events above kVtxNarrowTracks.
-template <int kThreads, uint32_t kCap, bool kSelect, bool kAll>
-__global__ void __launch_bounds__(kThreads, 1) k_vertices(Dev d) {
+// Events of the grid's stride with more than `above` selected tracks, and at most kCap (kAll: those
+// above too, in global memory). parts: blocks of k_vertex_select per event.
+template <int kThreads, uint32_t kCap, bool kAll>
+__global__ void __launch_bounds__(kThreads, kAll ? 1 : 4) k_vertices(Dev d, int parts, uint32_t above) {
   extern __shared__ __align__(16) uint8_t s_vtx[];
   VtxShared& S = *reinterpret_cast<VtxShared*>(s_vtx);
   float* s_zt = reinterpret_cast<float*>(s_vtx + (sizeof(VtxShared) + 15) / 16 * 16);
   float* s_ezt2 = s_zt + kCap;
   int16_t* s_iv = reinterpret_cast<int16_t*>(s_ezt2 + kCap);
   int16_t* s_nn = s_iv + kCap;
-  uint16_t* s_b = reinterpret_cast<uint16_t*>(s_nn + kCap);
+  uint16_t* s_ord = reinterpret_cast<uint16_t*>(s_nn + kCap);
+  uint16_t* s_b = s_ord + kCap;
   uint16_t* s_c = s_b + kCap;
   uint8_t* s_izt = reinterpret_cast<uint8_t*>(s_c + kCap);
   for (int e = blockIdx.x; e < d.E; e += gridDim.x) {
     EvInfo& E = d.ev[e];
     const uint64_t tb = E.tuple_base;
+    // the blocks' lists, one after the other
     uint32_t nt;
-    if (kSelect) {
-      nt = vertex_tracks(d, E, e, S.sh);
-      if (!kAll && nt > kCap) continue;
-    } else {
-      nt = E.n_vtx_tracks;
-      if (nt <= kVtxNarrowTracks) continue;
+    const uint32_t c = threadIdx.x < uint32_t(parts) ? d.vtx_cnt[e * parts + threadIdx.x] : 0u;
+    const uint32_t first = block_excl_scan(c, S.sh, &nt);
+    if (threadIdx.x < uint32_t(parts)) S.off[threadIdx.x] = first;
+    __syncthreads();
+    if (nt <= above && above > 0) continue;
+    if (!kAll && nt > kCap) continue;
+    const uint32_t per = (E.n_tuples + parts - 1) / parts;
+    for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
+      uint32_t a = 0, b = uint32_t(parts);
+      while (b - a > 1) {
+        const uint32_t m = (a + b) >> 1;
+        if (S.off[m] <= i) a = m; else b = m;
+      }
+      const uint32_t t = d.vws_list[tb + a * per + (i - S.off[a])];
+      const uint64_t g = tb + t;
+      const float pt = d.t_pt[g];
+      d.vws_itrk[tb + i] = t;
+      d.vws_zt[tb + i] = d.t_state[5 * g + 4];
+      d.vws_ezt2[tb + i] = d.t_cov[15 * g + 14];
+      d.vws_ptt2[tb + i] = __fmul_rn(pt, pt);
     }
-    if (threadIdx.x == 0) S.warn = 0;
+    if (threadIdx.x == 0) { E.n_vtx_tracks = nt; S.warn = 0; }
+    __syncthreads();
     float* zv = d.zv + size_t(e) * kMaxVtx;
     float* wv = d.wv + size_t(e) * kMaxVtx;
     float* vchi2 = d.vchi2 + size_t(e) * kMaxVtx;
     float* ptv2 = d.ptv2 + size_t(e) * kMaxVtx;
     uint16_t* sort_ind = d.sort_ind + size_t(e) * kMaxVtx;
-    int32_t* nn = d.ndof + tb + size_t(e) * kMaxVtx;
+    int32_t* nn_out = d.ndof + tb + size_t(e) * kMaxVtx;  // length n_tuples + 1024
+    const float* gz = d.vws_zt + tb;
+    const float* ge = d.vws_ezt2 + tb;
     const float* ptt2 = d.vws_ptt2 + tb;
     const uint32_t* itrk = d.vws_itrk + tb;
     if (nt <= kCap) {
-      for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
-        s_zt[i] = d.vws_zt[tb + i];
-        s_ezt2[i] = d.vws_ezt2[tb + i];
-      }
-      // neighbour counts of the tracks, then ndof of the vertices: the reference's nn array
-      const uint32_t nz = nt > uint32_t(kMaxVtx) ? nt : uint32_t(kMaxVtx);
-      for (uint32_t i = threadIdx.x; i < nz; i += blockDim.x) s_nn[i] = 0;
-      __syncthreads();
-      const VtxTracks<int16_t, uint16_t> A{s_zt, s_ezt2, s_iv, s_nn, s_b, s_c, s_izt};
-      vertex_core(d, E, nt, A, ptt2, itrk, zv, wv, vchi2, ptv2, sort_ind, S);
-      const uint32_t nw = nt > S.nv ? nt : S.nv;
-      for (uint32_t i = threadIdx.x; i < nw; i += blockDim.x) nn[i] = s_nn[i];
+      const VtxTracks<int16_t, uint16_t> A{s_zt, s_ezt2, s_iv, s_nn, s_ord, s_b, s_c, s_izt};
+      vertex_core(d, E, nt, A, gz, ge, ptt2, itrk, zv, wv, vchi2, ptv2, sort_ind, nn_out, S);
     } else if (kAll) {
-      __syncthreads();
-      const VtxTracks<int32_t, uint32_t> A{d.vws_zt + tb, d.vws_ezt2 + tb, d.vws_iv + tb, nn, d.vws_bins + tb,
-                                           d.vws_list + tb, d.vws_izt + tb};
-      vertex_core(d, E, nt, A, ptt2, itrk, zv, wv, vchi2, ptv2, sort_ind, S);
+      const VtxTracks<int32_t, uint32_t> A{d.vws_zs + tb, d.vws_es + tb, d.vws_iv + tb, d.vws_nn + tb,
+                                           d.vws_ord + tb, d.vws_bins + tb, d.vws_list + tb, d.vws_izt + tb};
+      vertex_core(d, E, nt, A, gz, ge, ptt2, itrk, zv, wv, vchi2, ptv2, sort_ind, nn_out, S);
     }
     __syncthreads();
   }
@@ -757,23 +754,25 @@ void launch_classify(const Dev& d, const Launch& L) {
 }
 
 int prepare_select_kernels() {
-  const int wide = int(vtx_smem_bytes(kVtxWideTracks));
-  cudaError_t err = cudaFuncSetAttribute(k_vertices<kVtxWideThreads, kVtxWideTracks, true, true>,
+  const int wide = int(vtx_smem_bytes(kVtxWideTracks)), narrow = int(vtx_smem_bytes(kVtxNarrowTracks));
+  cudaError_t err = cudaFuncSetAttribute(k_vertices<kVtxWideThreads, kVtxWideTracks, true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, wide);
   if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_vertices<kVtxWideThreads, kVtxWideTracks, false, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, wide);
+    err = cudaFuncSetAttribute(k_vertices<kVtxNarrowThreads, kVtxNarrowTracks, false>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, narrow);
   return err == cudaSuccess ? 0 : -1;
 }
 
 void launch_vertices(const Dev& d, const Launch& L) {
   const size_t wide = vtx_smem_bytes(kVtxWideTracks), narrow = vtx_smem_bytes(kVtxNarrowTracks);
+  const int parts = event_blocks(d.E, kVtxSelectBlocks, kVtxParts);
+  k_vertex_select<<<dim3(parts, d.E), 256, 0, L.s>>>(d);
   if (d.E <= 148) {  // at most one event per SM: the wide form for all
-    k_vertices<kVtxWideThreads, kVtxWideTracks, true, true><<<d.E, kVtxWideThreads, wide, L.s>>>(d);
+    k_vertices<kVtxWideThreads, kVtxWideTracks, true><<<d.E, kVtxWideThreads, wide, L.s>>>(d, parts, 0u);
   } else {
-    k_vertices<kVtxNarrowThreads, kVtxNarrowTracks, true, false><<<d.E, kVtxNarrowThreads, narrow, L.s>>>(d);
+    k_vertices<kVtxNarrowThreads, kVtxNarrowTracks, false><<<d.E, kVtxNarrowThreads, narrow, L.s>>>(d, parts, 0u);
     if (d.tuples_per_event > kVtxNarrowTracks)
-      k_vertices<kVtxWideThreads, kVtxWideTracks, false, true><<<148, kVtxWideThreads, wide, L.s>>>(d);
+      k_vertices<kVtxWideThreads, kVtxWideTracks, true><<<148, kVtxWideThreads, wide, L.s>>>(d, parts, kVtxNarrowTracks);
   }
   L.mark("vertices");
 }

@@ -217,6 +217,7 @@ int alloc_batch(PxlCtx* ctx) {
   int rc = 0;
 #define A(ptr, n) do { rc = dalloc(ctx, &d.ptr, (n)); if (rc) return rc; } while (0)
   A(ev, E + 1);
+  CK(cudaMemset(d.ev, 0, size_t(E + 1) * sizeof(EvInfo)));  // counts and warnings read before any run
   A(fed_src, E * NF); A(fed_nw, E * NF); A(fed_wo, E * NF); A(fed_nmod, E * NF + kFedParts);
   A(xx, d.cap_words); A(yy, d.cap_words); A(adc, d.cap_words); A(mid, d.cap_words); A(clus, d.cap_words);
   A(pdigi, d.cap_words); A(rawid, d.cap_words);
@@ -257,6 +258,8 @@ int alloc_batch(PxlCtx* ctx) {
   A(dup_et, d.cap_tuple_hits); A(dup_ek, d.cap_tuple_hits); A(dup_death0, d.cap_tuples); A(dup_death1, d.cap_tuples);
   A(vws_zt, d.cap_tuples); A(vws_ezt2, d.cap_tuples); A(vws_ptt2, d.cap_tuples); A(vws_iv, d.cap_tuples);
   A(vws_itrk, d.cap_tuples); A(vws_izt, d.cap_tuples); A(vws_bins, d.cap_tuples); A(vws_list, d.cap_tuples);
+  A(vws_zs, d.cap_tuples); A(vws_es, d.cap_tuples); A(vws_ord, d.cap_tuples); A(vws_nn, d.cap_tuples);
+  A(vtx_cnt, E + kVtxSelectBlocks);
   A(idv, d.cap_tuples); A(zv, E * 1024); A(wv, E * 1024); A(vchi2, E * 1024); A(ptv2, E * 1024);
   A(ndof, d.cap_tuples + E * 1024); A(sort_ind, E * 1024);
   int64_t st = scan_tmp_elems(std::max({d.cap_words, d.cap_items, d.cap_cells, d.cap_hits, d.cap_tuples}) + 1);

@@ -36,6 +36,7 @@ constexpr int kMaxActiveColumns = 512 * 1024 / 8;  // MAX_NUM_OF_ACTIVE_DOUBLETS
 constexpr uint32_t kHitIdBits = 21;                // event-local hit ids are below 2^21
 constexpr uint32_t kMaxHitsPerEvent = 1u << kHitIdBits;
 constexpr int kMaxFedSlots = 160;
+constexpr int kVtxSelectBlocks = 148 * 4;  // blocks that select the tracks of a small batch
 constexpr int kFedParts = 148 * 32;  // warps over the FED slots of a small batch
 constexpr int kWarpModulePix = 256;  // modules up to this many digis are clustered by one warp
 
@@ -231,6 +232,8 @@ struct Dev {
   int16_t* idv;            // [cap_tuples] per tuple (global tuple index), -1 when unused
   float* vws_zt; float* vws_ezt2; float* vws_ptt2;  // [cap_tuples] vertex-finder workspace per selected track
   int32_t* vws_iv; uint32_t* vws_itrk; uint8_t* vws_izt; uint32_t* vws_bins; uint32_t* vws_list;
+  float* vws_zs; float* vws_es; uint32_t* vws_ord; int32_t* vws_nn;
+  uint32_t* vtx_cnt;       // [E + kVtxSelectBlocks] selected tracks per block of k_vertex_select
   float* zv; float* wv; float* vchi2; float* ptv2;  // [E][1024]
   int32_t* ndof;           // [cap_tuples] per event slot region (same packing as tuples)
   uint16_t* sort_ind;      // [E][1024]

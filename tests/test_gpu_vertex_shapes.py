@@ -1,6 +1,6 @@
 """The vertex finder's three forms against the oracle: one wide CTA per event for small batches,
 the narrow form with the wide one behind it for the events above 2048 selected tracks, and global
-memory above 12288. Integer products and ordered FP32 sums are compared exactly."""
+memory above the wide form's tracks. Integer products and ordered FP32 sums are compared exactly."""
 import numpy as np
 import pytest
 
