@@ -88,6 +88,7 @@ __device__ __forceinline__ void adjoint_track(const AdjArgs& A, int32_t t) {
 // 502 and 575 us when the call is waited for; four: 477 us. Before the shared reciprocals and
 // with a launch per hit count it was 966 us.
 __global__ void __launch_bounds__(kFitThreads, 3) k_bl_adjoint(AdjArgs A) {
+  pdl_sync();
   for_bucket_track(*A.plan, [&](auto n, int32_t t) { adjoint_track<decltype(n)::value>(A, t); });
 }
 
@@ -126,7 +127,9 @@ extern "C" int32_t pxl_bl_fit_adjoint(const double* hits, const float* hits_ge, 
     if (rc) return rc;
     AdjArgs A{hits, hits_ge, offs, plan, b_field, hit_module, module_pos, align, n_modules, chi2, grad_hits,
               want_align ? acc : nullptr};
-    k_bl_adjoint<<<fit_blocks(n), kFitThreads, 0, s>>>(A);
+    Launch L{s};
+    L.pdl = true;
+    L.run(k_bl_adjoint, fit_blocks(n), kFitThreads, 0, A);
   }
   if (want_align) k_align_out<<<std::max(1, (6 * n_modules + 255) / 256), 256, 0, s>>>(acc, 6 * n_modules, grad_align, grad_align64);
   return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;

@@ -50,18 +50,46 @@ struct HitView {
 };
 
 // ---------------------------------------------------------------- doublets
-// per event: cumulative inner-layer sizes over the pairs, number of work items
-__global__ void k_items(Dev d, uint32_t* pair_cum) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= d.E) return;
-  const uint32_t* hls = d.hits_layer_start + size_t(e) * 11;
-  uint32_t acc = 0;
-  for (int p = 0; p < kNPairs; ++p) {
-    const int li = c_layer_pairs[2 * p];
-    acc += hls[li + 1] - hls[li];
-    pair_cum[size_t(e) * kNPairs + p] = acc;
+// Block 0, per event: cumulative inner-layer sizes over the pairs and the number of work items, with
+// their scan. The other blocks clear what the kernels of the stage count in: the cells ending on each
+// hit (the per-cell counters are cleared by the doublet fill that writes the cells), the pools and lists.
+__global__ void __launch_bounds__(1024) k_items(Dev d, uint32_t* pair_cum) {
+  pdl_sync(d);
+  if (blockIdx.x > 0) {
+    const uint32_t i0 = (blockIdx.x - 1) * blockDim.x + threadIdx.x, stride = (gridDim.x - 1) * blockDim.x;
+    const uint32_t nh = d.ev[d.E].n_hits;
+    for (uint32_t i = i0; i < nh; i += stride) d.ohc_cur[i] = 0;
+    for (uint32_t i = i0; i < uint32_t(kTpParts); i += stride) d.tp_ctr[i * kTpStride] = 0;
+    if (i0 == 0) {
+      d.tp_ctr[kTpParts * kTpStride] = 0;
+      *d.dbl_pool_ctr = 0;
+      *d.cn_pair_ctr = 0;
+      d.long_ctr[0] = 0;
+      d.long_ctr[1] = 0;
+    }
+    return;
   }
-  d.ev[e].n_items = d.ev[e].n_hits ? acc : 0u;
+  __shared__ uint32_t sh[33];
+  uint32_t carry = 0;
+  for (int b = 0; b < d.E; b += blockDim.x) {
+    const int e = b + threadIdx.x;
+    uint32_t n = 0;
+    if (e < d.E) {
+      const uint32_t* hls = d.hits_layer_start + size_t(e) * 11;
+      uint32_t acc = 0;
+      for (int p = 0; p < kNPairs; ++p) {
+        const int li = c_layer_pairs[2 * p];
+        acc += hls[li + 1] - hls[li];
+        pair_cum[size_t(e) * kNPairs + p] = acc;
+      }
+      n = d.ev[e].n_hits ? acc : 0u;
+    }
+    uint32_t tot;
+    const uint32_t lo = carry + block_excl_scan(n, sh, &tot);
+    if (e < d.E) { d.ev[e].n_items = n; d.ev[e].item_base = lo; }
+    carry += tot;
+  }
+  if (threadIdx.x == 0) { d.ev[d.E].n_items = carry; d.ev[d.E].item_base = carry; }
 }
 
 // layer pair and event-local 0-based inner hit of work item j
@@ -278,6 +306,7 @@ constexpr int kDblQueue = 64;
 
 template <bool kQ>
 __global__ void __launch_bounds__(256) k_doublets_count(Dev d, const uint32_t* __restrict__ pair_cum, WorkQueue q) {
+  pdl_sync(d);
   __shared__ uint32_t s_cum[kNPairs];
   __shared__ uint32_t s_hls[11];
   __shared__ uint4 s_rng[8][32];   // per compacted item: lo0, n0, lo1, first candidate
@@ -408,6 +437,7 @@ __global__ void __launch_bounds__(256) k_doublets_count(Dev d, const uint32_t* _
 // inner hit, pair and inner z / r of each cell's item from shared memory.
 template <bool kQ>
 __global__ void __launch_bounds__(256) k_doublets_fill(Dev d, const uint32_t* __restrict__ pair_cum, WorkQueue q) {
+  pdl_sync(d);
   __shared__ uint32_t s_cum[kNPairs];
   __shared__ uint32_t s_hls[11];
   __shared__ uint32_t s_pos[8][33];
@@ -478,24 +508,44 @@ __global__ void __launch_bounds__(256) k_doublets_fill(Dev d, const uint32_t* __
   });
 }
 
-// per event: cell base, raw and capped counts
-__global__ void k_cell_bases(Dev d) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= d.E) return;
-  EvInfo& E = d.ev[e];
-  const uint32_t lo = d.item_cnt[E.item_base], hi = d.item_cnt[E.item_base + E.n_items];
-  E.n_cols_nb = 0;
-  E.n_cols_tr = 0;
-  uint32_t n = hi - lo;  // doublets found; the reference keeps the first doublets_per_event
-  if (n > d.doublets_per_event) { n = d.doublets_per_event; E.warnings |= kWarnDoublets; }
-  E.n_cells = n;
-}
-
-// after the event scan of n_cells: events past the buffer are emptied, regions fixed
-__global__ void k_cell_regions(Dev d) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e > d.E) return;
-  d.ev[e].n_cells_raw = d.ev[e].n_cells;
+// per event: capped doublet count, its scan into the cell bases, and events past the cell buffer
+// emptied (as k_ev_scan does it); one block
+__global__ void __launch_bounds__(1024) k_cell_bases(Dev d) {
+  pdl_sync(d);
+  __shared__ uint32_t sh[33];
+  uint32_t carry = 0;
+  for (int b = 0; b < d.E; b += blockDim.x) {
+    const int e = b + threadIdx.x;
+    uint32_t n = 0;
+    if (e < d.E) {
+      EvInfo& E = d.ev[e];
+      n = d.item_cnt[E.item_base + E.n_items] - d.item_cnt[E.item_base];
+      E.n_cols_nb = 0;
+      E.n_cols_tr = 0;
+      // the reference keeps the first doublets_per_event
+      if (n > d.doublets_per_event) { n = d.doublets_per_event; E.warnings |= kWarnDoublets; }
+    }
+    uint32_t tot;
+    const uint32_t lo = carry + block_excl_scan(n, sh, &tot);
+    if (e < d.E) {
+      EvInfo& E = d.ev[e];
+      if (int64_t(lo) + int64_t(n) > d.cap_cells) {
+        n = 0;
+        E.warnings |= kWarnBuffer;
+        atomicOr(d.status, kWarnBuffer);
+      }
+      E.cell_base = lo;
+      E.n_cells = n;
+      E.n_cells_raw = n;
+    }
+    carry += tot;
+  }
+  if (threadIdx.x == 0) {
+    EvInfo& T = d.ev[d.E];
+    T.cell_base = carry;
+    T.n_cells = int64_t(carry) > d.cap_cells ? uint32_t(d.cap_cells) : carry;
+    T.n_cells_raw = T.n_cells;
+  }
 }
 
 // ---------------------------------------------------------------- outer-hit lists
@@ -503,6 +553,7 @@ __global__ void k_cell_regions(Dev d) {
 constexpr int kOhcUnroll = 4;  // cells (list entries) per thread and step, loads independent
 
 __global__ void k_ohc_fill(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint64_t cb = E.cell_base;
@@ -580,14 +631,17 @@ __device__ __forceinline__ void sort_list(uint32_t* a, uint32_t n) {
 
 // lists above the short-sort limit, sorted afterwards by k_sort_long (a list of n entries
 // needs n > 8, so the buffer of cap_long = entries / 9 entries cannot overflow)
-__device__ __forceinline__ void push_long_list(const Dev& d, uint32_t lo, uint32_t n) {
-  const uint32_t slot = atomicAdd(d.long_ctr, 1u);
+__device__ __forceinline__ void push_long_list(const Dev& d, int kind, uint32_t lo, uint32_t n) {
+  const uint32_t slot = atomicAdd(&d.long_ctr[kind], 1u);
   if (slot < uint32_t(d.cap_long)) d.long_lists[slot] = make_uint2(lo, n);
   else atomicOr(d.status, kWarnBuffer);
 }
 
-__global__ void __launch_bounds__(256) k_sort_long(Dev d, uint32_t* list) {
-  uint32_t nl = *d.long_ctr;
+constexpr int kSortLongBlocks = 148 * 4;
+
+__global__ void __launch_bounds__(256) k_sort_long(Dev d, int kind, uint32_t* list) {
+  pdl_sync(d);
+  uint32_t nl = d.long_ctr[kind];
   if (nl > uint32_t(d.cap_long)) nl = uint32_t(d.cap_long);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += gridDim.x * blockDim.x) {
     const uint2 l = d.long_lists[i];
@@ -619,6 +673,7 @@ __device__ __forceinline__ void sort_list_warp(uint32_t* a, uint32_t n) {
 // longer ones together (an insertion sort by one thread, kept above 128 entries, made the kernel
 // 248 us for one event of pileup 170).
 __global__ void k_sort_hit_lists(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint32_t hb = E.hit_base, nh = E.n_hits;
@@ -684,6 +739,7 @@ __device__ __forceinline__ bool are_aligned(float r1, float z1, float ri, float 
 
 // connect's candidates of each outer-hit list entry, gathered once per entry
 __global__ void __launch_bounds__(256) k_ohc_records(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint32_t hb = E.hit_base;
@@ -722,6 +778,7 @@ constexpr int kConnQueue = 64;
 
 template <bool kQ>
 __global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
+  pdl_sync(d);
   __shared__ float4 s_rz[kConnWarps][32];  // inner r, z and outer r, z of each cell
   __shared__ float4 s_xy[kConnWarps][32];  // inner x, y and outer x, y
   __shared__ uint32_t s_lo[kConnWarps][32];
@@ -827,6 +884,7 @@ __global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
 
 // neighbour lists from the pair list: each passing (candidate o, cell c) appends c to o's list
 __global__ void __launch_bounds__(256) k_connect_fill(Dev d) {
+  pdl_sync(d);
   uint32_t np = *d.cn_pair_ctr;
   if (np > uint32_t(d.cap_pairs)) np = uint32_t(d.cap_pairs);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
@@ -838,6 +896,7 @@ __global__ void __launch_bounds__(256) k_connect_fill(Dev d) {
 // per-cell lists: neighbours (kind 0) or tracks (kind 1), sorted ascending; flags overflow
 template <int kKind>
 __global__ void k_sort_cell_lists(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint64_t cb = E.cell_base;
@@ -855,7 +914,7 @@ __global__ void k_sort_cell_lists(Dev d) {
     if (uint64_t(hi) > lcap) hi = uint32_t(lcap);
     if (hi > lo) {
       ++cols;
-      if (!sort_short<8>(list + lo, hi - lo)) push_long_list(d, lo, hi - lo);
+      if (!sort_short<8>(list + lo, hi - lo)) push_long_list(d, kKind, lo, hi - lo);
       if (hi - lo > uint32_t(kCellRows)) atomic_or_warn(&d.ev[e], kWarnLists);
     }
     // cells with two or more tracks, for the duplicate remover
@@ -874,6 +933,7 @@ __global__ void k_sort_cell_lists(Dev d) {
 // ---------------------------------------------------------------- fishbone
 template <bool kQ>
 __global__ void __launch_bounds__(128) k_fishbone(Dev d, WorkQueue q) {
+  pdl_sync(d);
   for_each_vblock<kQ>(q, [&](int e, uint32_t bx, uint32_t nbx) {
   const EvInfo& E = d.ev[e];
   if (E.n_hits <= 1) return;
@@ -1048,6 +1108,7 @@ constexpr int kNtupQueue = 64;
 
 template <bool kFill, bool kQ>
 __global__ void __launch_bounds__(32 * kNtupWarps) k_ntuplets(Dev d, WorkQueue q) {
+  pdl_sync(d);
   __shared__ uint32_t s_queue[kNtupWarps][kNtupQueue];
   // the fill walks only when the count pass could not keep every tuple's record
   if (kFill && d.tp_ctr[kTpParts * kTpStride] == 0) return;
@@ -1107,62 +1168,65 @@ __global__ void __launch_bounds__(32 * kNtupWarps) k_ntuplets(Dev d, WorkQueue q
 constexpr int kPoolBlocksPerPart = 2;  // measured faster than one (1000 PU50 events: 1.01 / 1.05 ms)
 
 __global__ void __launch_bounds__(256) k_tuples_from_pool(Dev d) {
+  pdl_sync(d);
   if (d.tp_ctr[kTpParts * kTpStride]) return;  // a part overflowed: k_ntuplets<true> walks
-  const uint32_t r = blockIdx.x / kPoolBlocksPerPart;
-  uint32_t n = d.tp_ctr[r * kTpStride];
-  if (n > d.tp_part) n = d.tp_part;
-  for (uint32_t i = threadIdx.x + (blockIdx.x % kPoolBlocksPerPart) * blockDim.x; i < n;
-       i += kPoolBlocksPerPart * blockDim.x) {
-    const uint64_t s = uint64_t(r) * d.tp_part + i;
-    const uint4 h = d.tp_hdr[s];
-    const uint4 c0 = d.tp_cells[2 * s], c1 = d.tp_cells[2 * s + 1];
-    const uint32_t cells[kMaxDepth] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-    const int e = int(h.w >> 4);
-    const uint32_t nh = h.w & 15u;
-    const int depth = int(nh) - 2;  // index of the tuple's last doublet
-    const uint64_t v = d.tstart_cnt[h.x];
-    const uint64_t g = (v >> 32) + h.y;
-    const uint64_t hp = (v & 0xFFFFFFFFull) + h.z;
-    if (!(g < uint64_t(d.cap_tuples) && hp + nh <= uint64_t(d.cap_tuple_hits))) continue;
-    const EvInfo& E = d.ev[e];
-    const uint32_t hbase = E.hit_base;
-    uint32_t ih[kMaxDepth];
-    uint32_t top = 0;
-#pragma unroll
-    for (int k = 0; k < kMaxDepth; ++k) {
-      ih[k] = k <= depth ? d.cell_inner[cells[k]] : 0u;
-      if (k == depth) top = cells[k];
-    }
-    const uint32_t oh = d.cell_outer[top];
-    int16_t det[kMaxDepth];
-#pragma unroll
-    for (int k = 0; k < kMaxDepth; ++k)
-      if (k <= depth) det[k] = d.detind[hbase + ih[k]];
-    const int16_t det_o = d.detind[hbase + oh];
-    d.tuple_off[g] = uint32_t(hp);
-#pragma unroll
-    for (int k = 0; k < kMaxDepth; ++k)
-      if (k <= depth) {
-        d.tuple_hits[hp + k] = ih[k];
-        d.tuple_det[hp + k] = uint16_t(det[k]);
+  for (uint32_t r = blockIdx.x / kPoolBlocksPerPart; r < uint32_t(kTpParts); r += gridDim.x / kPoolBlocksPerPart) {
+    uint32_t n = d.tp_ctr[r * kTpStride];
+    if (n > d.tp_part) n = d.tp_part;
+    for (uint32_t i = threadIdx.x + (blockIdx.x % kPoolBlocksPerPart) * blockDim.x; i < n;
+         i += kPoolBlocksPerPart * blockDim.x) {
+      const uint64_t s = uint64_t(r) * d.tp_part + i;
+      const uint4 h = d.tp_hdr[s];
+      const uint4 c0 = d.tp_cells[2 * s], c1 = d.tp_cells[2 * s + 1];
+      const uint32_t cells[kMaxDepth] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+      const int e = int(h.w >> 4);
+      const uint32_t nh = h.w & 15u;
+      const int depth = int(nh) - 2;  // index of the tuple's last doublet
+      const uint64_t v = d.tstart_cnt[h.x];
+      const uint64_t g = (v >> 32) + h.y;
+      const uint64_t hp = (v & 0xFFFFFFFFull) + h.z;
+      if (!(g < uint64_t(d.cap_tuples) && hp + nh <= uint64_t(d.cap_tuple_hits))) continue;
+      const EvInfo& E = d.ev[e];
+      const uint32_t hbase = E.hit_base;
+      uint32_t ih[kMaxDepth];
+      uint32_t top = 0;
+  #pragma unroll
+      for (int k = 0; k < kMaxDepth; ++k) {
+        ih[k] = k <= depth ? d.cell_inner[cells[k]] : 0u;
+        if (k == depth) top = cells[k];
       }
-    d.tuple_hits[hp + depth + 1] = oh;
-    d.tuple_det[hp + depth + 1] = uint16_t(det_o);
-    d.quality[g] = 0;
-    // cell -> track pairs only for the tuples the event keeps (as the walking fill)
-    if (g - E.tuple_base < E.n_tuples) {
-      const uint64_t pp = hp - g;
-#pragma unroll
+      const uint32_t oh = d.cell_outer[top];
+      int16_t det[kMaxDepth];
+  #pragma unroll
+      for (int k = 0; k < kMaxDepth; ++k)
+        if (k <= depth) det[k] = d.detind[hbase + ih[k]];
+      const int16_t det_o = d.detind[hbase + oh];
+      d.tuple_off[g] = uint32_t(hp);
+  #pragma unroll
       for (int k = 0; k < kMaxDepth; ++k)
         if (k <= depth) {
-          d.tuple_cell[pp + k] = cells[k];
-          atomicAdd(&d.ct_cur[cells[k]], 1u);
+          d.tuple_hits[hp + k] = ih[k];
+          d.tuple_det[hp + k] = uint16_t(det[k]);
         }
+      d.tuple_hits[hp + depth + 1] = oh;
+      d.tuple_det[hp + depth + 1] = uint16_t(det_o);
+      d.quality[g] = 0;
+      // cell -> track pairs only for the tuples the event keeps (as the walking fill)
+      if (g - E.tuple_base < E.n_tuples) {
+        const uint64_t pp = hp - g;
+  #pragma unroll
+        for (int k = 0; k < kMaxDepth; ++k)
+          if (k <= depth) {
+            d.tuple_cell[pp + k] = cells[k];
+            atomicAdd(&d.ct_cur[cells[k]], 1u);
+          }
+      }
     }
   }
 }
 
 __global__ void k_tuple_bases(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e > d.E) return;
   if (e == d.E) {
@@ -1197,6 +1261,7 @@ __global__ void k_tuple_bases(Dev d) {
 // container (hist_to_container.jl:150-161): the offset after the last kept tuple is set to that
 // tuple's start, so the last kept tuple shows no hits (its doublets still list it).
 __global__ void k_tuple_ends(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= d.E) return;
   EvInfo& E = d.ev[e];
@@ -1217,7 +1282,12 @@ __global__ void k_tuple_ends(Dev d) {
 
 // cell -> tuple lists: fill from the (cell, tuple) pairs of the kept tuples
 __global__ void k_cell_tracks_fill(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
+  // the bitmap that the track lists' sort sets
+  for (uint32_t w = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x, n = d.ev[d.E].n_cells_raw / 32 + 2; w < n;
+       w += gridDim.y * gridDim.x * blockDim.x)
+    d.dup_bits[w] = 0;
   const EvInfo& E = d.ev[e];
   const uint64_t tb = E.tuple_base;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < E.n_tuples; t += gridDim.x * blockDim.x) {
@@ -1235,6 +1305,7 @@ __global__ void k_cell_tracks_fill(Dev d) {
 
 // kernel_early_duplicate_remover (…_impl.jl:143-166)
 __global__ void k_early_dup(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   if (E.n_cells == 0) return;
@@ -1278,6 +1349,7 @@ __global__ void k_early_dup(Dev d) {
 // counts and the last one forms the offsets (one block per event took 180 us for the 51 k tuples of
 // an event of pileup 170, most of it on nine shared counters).
 __global__ void __launch_bounds__(256) k_multiplicity(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   EvInfo& E = d.ev[e];
   __shared__ uint32_t s_cnt[9];
@@ -1334,109 +1406,93 @@ int prepare_ca_kernels(int ctas[kTuneCount]) {
   return 0;
 }
 
-// a list-sorting kernel followed by the sort of the lists it left long
-template <class F>
-void launch_sorted(const Dev& d, const Launch& L, uint32_t* list, F&& sort_kernel) {
-  cudaMemsetAsync(d.long_ctr, 0, sizeof(uint32_t), L.s);
-  sort_kernel(L.s);
-  k_sort_long<<<148 * 4, 256, 0, L.s>>>(d, list);
-}
-
 void launch_ca(const Dev& d, const Launch& L) {
   auto g = [&](int seg) { return dim3(L.bpe_of(seg), d.E); };
   const int eb = div_up(d.E + 1, 128);
   uint32_t* pair_cum = d.pair_cum;
-  // counters of the cells ending on each hit (the per-cell counters are cleared by the
-  // doublet fill that writes the cells)
-  cudaMemsetAsync(d.ohc_cur, 0, size_t(d.cap_hits) * sizeof(uint32_t), L.s);
-  k_items<<<div_up(d.E, 128), 128, 0, L.s>>>(d, pair_cum);
-  launch_ev_scan(d, L.s, int(offsetof(EvInfo, n_items)), int(offsetof(EvInfo, item_base)));
+  L.run(k_items, 1 + int(std::min<int64_t>(148, div_up(d.cap_hits, 1024))), 1024, 0, d, pair_cum);
   L.mark("doublet_items");
-  cudaMemsetAsync(d.dbl_pool_ctr, 0, sizeof(uint32_t), L.s);
   // the per-event stages run on their static grid or from a work queue (Launch::queue_of):
   // virtual blocks of (strides x block size) work units, events by decreasing hit count
-  launch_wq_order(d, L.s);
+  if (L.queue_of(kTuneDoublets) || L.queue_of(kTuneConnect) || L.queue_of(kTuneFishbone) || L.queue_of(kTuneNtuplets))
+    launch_wq_order(d, L);
   auto plan = [&](int seg, int count_off, int threads) {
     return launch_wq_plan(d, L, count_off, uint32_t(L.queue_of(seg)) * uint32_t(threads));
   };
   const int ctas_dbl = L.queue_of(kTuneDoublets) ? L.wq_ctas[kTuneDoublets] : 0;
   if (ctas_dbl) {
     const WorkQueue q = plan(kTuneDoublets, int(offsetof(EvInfo, n_items)), 256);
-    k_doublets_count<true><<<ctas_dbl, 256, 0, L.s>>>(d, pair_cum, q);
+    L.run(k_doublets_count<true>, ctas_dbl, 256, 0, d, pair_cum, q);
   } else {
-    k_doublets_count<false><<<g(kTuneDoublets), 256, 0, L.s>>>(d, pair_cum, WorkQueue{});
+    L.run(k_doublets_count<false>, g(kTuneDoublets), 256, 0, d, pair_cum, WorkQueue{});
   }
   L.mark("doublets_count");
-  excl_scan_u32(d.item_cnt, d.cap_items, &d.ev[d.E].n_items, d.scan_tmp, L.s);
-  k_cell_bases<<<eb, 128, 0, L.s>>>(d);
-  launch_ev_scan(d, L.s, int(offsetof(EvInfo, n_cells)), int(offsetof(EvInfo, cell_base)));
-  launch_ev_clamp(d, L.s, int(offsetof(EvInfo, n_cells)), int(offsetof(EvInfo, cell_base)), d.cap_cells);
-  k_cell_regions<<<eb, 128, 0, L.s>>>(d);
+  excl_scan_u32(d.item_cnt, d.cap_items, &d.ev[d.E].n_items, d.scan_tmp, L);
+  L.run(k_cell_bases, 1, 1024, 0, d);
   L.mark("doublets_scan");
   if (ctas_dbl) {
     const WorkQueue q = plan(kTuneDoublets, int(offsetof(EvInfo, n_items)), 256);
-    k_doublets_fill<true><<<ctas_dbl, 256, 0, L.s>>>(d, pair_cum, q);
+    L.run(k_doublets_fill<true>, ctas_dbl, 256, 0, d, pair_cum, q);
   } else {
-    k_doublets_fill<false><<<g(kTuneDoublets), 256, 0, L.s>>>(d, pair_cum, WorkQueue{});
+    L.run(k_doublets_fill<false>, g(kTuneDoublets), 256, 0, d, pair_cum, WorkQueue{});
   }
   L.mark("doublets_fill");
   // cells ending on each hit (counted by the doublet fill)
-  excl_scan_shift_u32(d.ohc_cur, d.ohc_cnt, d.cap_hits, &d.ev[d.E].n_hits, d.scan_tmp, L.s);
-  k_ohc_fill<<<g(kTuneHitLists), 256, 0, L.s>>>(d);
-  k_sort_hit_lists<<<g(kTuneHitLists), 256, 0, L.s>>>(d);
-  k_ohc_records<<<g(kTuneHitLists), 256, 0, L.s>>>(d);
+  excl_scan_shift_u32(d.ohc_cur, d.ohc_cnt, d.cap_hits, &d.ev[d.E].n_hits, d.scan_tmp, L);
+  L.run(k_ohc_fill, g(kTuneHitLists), 256, 0, d);
+  L.run(k_sort_hit_lists, g(kTuneHitLists), 256, 0, d);
+  L.run(k_ohc_records, g(kTuneHitLists), 256, 0, d);
   L.mark("outer_hit_lists");
   // connection and neighbour lists
-  cudaMemsetAsync(d.cn_pair_ctr, 0, sizeof(uint32_t), L.s);
   if (L.queue_of(kTuneConnect)) {
     const WorkQueue q = plan(kTuneConnect, int(offsetof(EvInfo, n_cells)), 256);
-    k_connect_test<true><<<L.wq_ctas[kTuneConnect], 256, 0, L.s>>>(d, q);
+    L.run(k_connect_test<true>, L.wq_ctas[kTuneConnect], 256, 0, d, q);
   } else {
-    k_connect_test<false><<<g(kTuneConnect), 256, 0, L.s>>>(d, WorkQueue{});
+    L.run(k_connect_test<false>, g(kTuneConnect), 256, 0, d, WorkQueue{});
   }
   L.mark("connect");
-  excl_scan_shift_u32(d.cn_cur, d.cn_cnt, d.cap_cells, &d.ev[d.E].n_cells_raw, d.scan_tmp, L.s);
-  k_connect_fill<<<148 * 8, 256, 0, L.s>>>(d);
-  launch_sorted(d, L, d.cn_list, [&](cudaStream_t s) { k_sort_cell_lists<0><<<g(kTuneCellLists), 256, 0, s>>>(d); });
+  excl_scan_shift_u32(d.cn_cur, d.cn_cnt, d.cap_cells, &d.ev[d.E].n_cells_raw, d.scan_tmp, L);
+  L.run(k_connect_fill, 148 * 8, 256, 0, d);
+  L.run(k_sort_cell_lists<0>, g(kTuneCellLists), 256, 0, d);
+  L.run(k_sort_long, kSortLongBlocks, 256, 0, d, 0, d.cn_list);
   L.mark("neighbour_lists");
   if (L.queue_of(kTuneFishbone)) {
     const WorkQueue q = plan(kTuneFishbone, int(offsetof(EvInfo, n_hits)), 128);
-    k_fishbone<true><<<L.wq_ctas[kTuneFishbone], 128, 0, L.s>>>(d, q);
+    L.run(k_fishbone<true>, L.wq_ctas[kTuneFishbone], 128, 0, d, q);
   } else {
-    k_fishbone<false><<<g(kTuneFishbone), 128, 0, L.s>>>(d, WorkQueue{});
+    L.run(k_fishbone<false>, g(kTuneFishbone), 128, 0, d, WorkQueue{});
   }
   L.mark("fishbone");
   // ntuplets: the count pass keeps each tuple's record in the pool; the fill moves the records
   // into place, or walks again when the pool overflowed
-  cudaMemsetAsync(d.tp_ctr, 0, size_t(kTpParts * kTpStride + 1) * sizeof(uint32_t), L.s);
   const int ctas_nt = L.queue_of(kTuneNtuplets) ? L.wq_ctas[kTuneNtuplets] : 0;
   if (ctas_nt) {
     const WorkQueue q = plan(kTuneNtuplets, int(offsetof(EvInfo, n_cells)), 32 * kNtupWarps);
-    k_ntuplets<false, true><<<ctas_nt, 32 * kNtupWarps, 0, L.s>>>(d, q);
+    L.run(k_ntuplets<false, true>, ctas_nt, 32 * kNtupWarps, 0, d, q);
   } else {
-    k_ntuplets<false, false><<<g(kTuneNtuplets), 32 * kNtupWarps, 0, L.s>>>(d, WorkQueue{});
+    L.run(k_ntuplets<false, false>, g(kTuneNtuplets), 32 * kNtupWarps, 0, d, WorkQueue{});
   }
   L.mark("ntuplets_count");
-  excl_scan_u64(d.tstart_cnt, d.cap_cells, &d.ev[d.E].n_cells_raw, d.scan_tmp64, L.s);
-  k_tuple_bases<<<eb, 128, 0, L.s>>>(d);
-  k_tuples_from_pool<<<kTpParts * kPoolBlocksPerPart, 256, 0, L.s>>>(d);
+  excl_scan_u64(d.tstart_cnt, d.cap_cells, &d.ev[d.E].n_cells_raw, d.scan_tmp64, L);
+  L.run(k_tuple_bases, eb, 128, 0, d);
+  // all parts advance together in a batch; a few events' records sit in few parts
+  L.run(k_tuples_from_pool, d.E <= 16 ? 148 * 8 : kTpParts * kPoolBlocksPerPart, 256, 0, d);
   if (ctas_nt) {
     const WorkQueue q = plan(kTuneNtuplets, int(offsetof(EvInfo, n_cells)), 32 * kNtupWarps);
-    k_ntuplets<true, true><<<ctas_nt, 32 * kNtupWarps, 0, L.s>>>(d, q);
+    L.run(k_ntuplets<true, true>, ctas_nt, 32 * kNtupWarps, 0, d, q);
   } else {
     // the walking fill returns at once unless the pool overflowed: a few blocks per event
-    k_ntuplets<true, false><<<dim3(std::min(L.bpe_of(kTuneNtuplets), 8), d.E), 32 * kNtupWarps, 0, L.s>>>(
-        d, WorkQueue{});
+    L.run(k_ntuplets<true, false>, dim3(std::min(L.bpe_of(kTuneNtuplets), 8), d.E), 32 * kNtupWarps, 0, d, WorkQueue{});
   }
-  k_tuple_ends<<<div_up(d.E, 128), 128, 0, L.s>>>(d);
+  L.run(k_tuple_ends, div_up(d.E, 128), 128, 0, d);
   L.mark("ntuplets_fill");
-  excl_scan_shift_u32(d.ct_cur, d.ct_cnt, d.cap_cells, &d.ev[d.E].n_cells_raw, d.scan_tmp, L.s);
-  k_cell_tracks_fill<<<g(kTuneCellTracks), 256, 0, L.s>>>(d);
-  cudaMemsetAsync(d.dup_bits, 0, size_t(d.cap_cells / 32 + 2) * sizeof(uint32_t), L.s);
-  launch_sorted(d, L, d.ct_list, [&](cudaStream_t s) { k_sort_cell_lists<1><<<g(kTuneCellTracks), 256, 0, s>>>(d); });
+  excl_scan_shift_u32(d.ct_cur, d.ct_cnt, d.cap_cells, &d.ev[d.E].n_cells_raw, d.scan_tmp, L);
+  L.run(k_cell_tracks_fill, g(kTuneCellTracks), 256, 0, d);
+  L.run(k_sort_cell_lists<1>, g(kTuneCellTracks), 256, 0, d);
+  L.run(k_sort_long, kSortLongBlocks, 256, 0, d, 1, d.ct_list);
   L.mark("cell_tracks");
-  k_early_dup<<<g(kTuneEarlyDup), 256, 0, L.s>>>(d);
-  k_multiplicity<<<dim3(event_blocks(d.E, 148 * 4, 64), d.E), 256, 0, L.s>>>(d);
+  L.run(k_early_dup, g(kTuneEarlyDup), 256, 0, d);
+  L.run(k_multiplicity, dim3(event_blocks(d.E, 148 * 4, 64), d.E), 256, 0, d);
   L.mark("dup_multiplicity");
 }
 

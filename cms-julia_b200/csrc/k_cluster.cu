@@ -403,6 +403,7 @@ __device__ __forceinline__ void cluster_module_thread(const Dev& d, int e, uint3
 // every module position of the batch: modules of <= kThreadPix digis here, one thread
 // each; larger ones to the work lists of the warp (<= 32, <= kWarpPix digis) and CTA paths
 __global__ void __launch_bounds__(128, 6) k_find_clus_tiny(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint32_t nmod = E.n_modules;
@@ -420,6 +421,7 @@ __global__ void __launch_bounds__(128, 6) k_find_clus_tiny(Dev d) {
 
 // modules of kThreadPix+1 .. 32 digis (work list), one warp each, one digi per lane
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_find_clus_small(Dev d) {
+  pdl_sync(d);
   __shared__ WarpSmem<1> smem[kWarpsPerBlock];
   const unsigned wib = threadIdx.x >> 5;
   const uint32_t nl = list_size(d, kListClusSmall);
@@ -436,6 +438,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_find_clus_small(Dev d) 
 constexpr int kMidWarps = 4;  // 7.8 KB of shared memory per warp
 
 __global__ void __launch_bounds__(32 * kMidWarps) k_find_clus_mid(Dev d) {
+  pdl_sync(d);
   __shared__ WarpSmem<kWarpSlots> smem[kMidWarps];
   __shared__ WarpHist hist[kMidWarps];
   const unsigned wib = threadIdx.x >> 5;
@@ -594,6 +597,7 @@ __device__ void cluster_module_block(const Dev& d, int e, uint32_t m, BlockSmem&
 
 // the modules the warp path handed over: (event << 11 | module position) entries
 __global__ void __launch_bounds__(256) k_find_clus_block(Dev d) {
+  pdl_sync(d);
   __shared__ BlockSmem S;
   const uint32_t n = list_size(d, kListClusBig);
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
@@ -614,6 +618,7 @@ __global__ void __launch_bounds__(256) k_find_clus_block(Dev d) {
 // A cluster id past 1024 in the sums or the renumbering (the reference indexes out of bounds and
 // raises) sets the clusters warning and is skipped.
 __global__ void __launch_bounds__(32) k_charge_cut_serial(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.x;
   const EvInfo& E = d.ev[e];
   if (!d.apply_charge_cut || !E.repeated_ids) return;
@@ -710,6 +715,7 @@ __global__ void __launch_bounds__(32) k_charge_cut_serial(Dev d) {
 
 // fill_hits_module_start + nClusters, one block per event
 __global__ void k_hits_module_start(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.x;
   __shared__ uint32_t sh[33];
   uint32_t* cim = d.clus_in_module + size_t(e) * kMaxNumModules;
@@ -764,19 +770,18 @@ static int mid_wave_ctas() {
 }
 
 void launch_cluster(const Dev& d, const Launch& L) {
-  cudaMemsetAsync(d.big_list, 0, kListHeader * sizeof(uint32_t), L.s);
   // enough warps that a few events fill the GPU, at least 8 modules per warp otherwise
   // one thread per module position (at most 2000 per event)
-  k_find_clus_tiny<<<dim3(div_up(kMaxNumModules, 128), d.E), 128, 0, L.s>>>(d);
+  L.run(k_find_clus_tiny, dim3(div_up(kMaxNumModules, 128), d.E), 128, 0, d);
   L.mark("find_clus_tiny");
-  k_find_clus_small<<<148 * 64, 32 * kWarpsPerBlock, 0, L.s>>>(d);
+  L.run(k_find_clus_small, std::min(148 * 64, div_up(int64_t(d.E) * kMaxNumModules, kWarpsPerBlock)), 32 * kWarpsPerBlock, 0, d);
   L.mark("find_clus_small");
-  k_find_clus_mid<<<mid_wave_ctas(), 32 * kMidWarps, 0, L.s>>>(d);
+  L.run(k_find_clus_mid, mid_wave_ctas(), 32 * kMidWarps, 0, d);
   L.mark("find_clus_mid");
-  k_find_clus_block<<<148 * 2, 256, 0, L.s>>>(d);
+  L.run(k_find_clus_block, 148 * 2, 256, 0, d);
   L.mark("find_clus_block");
-  k_charge_cut_serial<<<d.E, 32, 0, L.s>>>(d);
-  k_hits_module_start<<<d.E, 1024, 0, L.s>>>(d);
+  L.run(k_charge_cut_serial, d.E, 32, 0, d);
+  L.run(k_hits_module_start, d.E, 1024, 0, d);
   L.mark("hits_module_start");
 }
 

@@ -31,6 +31,7 @@ __device__ __forceinline__ uint2 export_range(uint32_t n) {
 
 // loose tracks per block, vertices per event
 __global__ void __launch_bounds__(kExpThreads) k_export_count(Dev d, ExportSet x) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint2 r = export_range(E.n_tuples);
@@ -48,6 +49,7 @@ __global__ void __launch_bounds__(kExpThreads) k_export_count(Dev d, ExportSet x
 // first track of each block, first track and first vertex of each event (one block); row E holds
 // the totals
 __global__ void __launch_bounds__(1024) k_export_scan(Dev d, ExportSet x, int nb) {
+  pdl_sync(d);
   __shared__ uint32_t sh[33];
   uint32_t ct = 0, cv = 0;
   for (int b = 0; b < d.E * nb; b += blockDim.x) {
@@ -78,6 +80,7 @@ __global__ void __launch_bounds__(1024) k_export_scan(Dev d, ExportSet x, int nb
 // the event's loose tracks in tuple order, and its vertices. The tracks of 256 tuples are listed
 // in shared memory and their rows copied word by word, so that the stores coalesce.
 __global__ void __launch_bounds__(kExpThreads) k_export_fill(Dev d, ExportSet x) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   __shared__ uint32_t sh[33];
@@ -170,11 +173,14 @@ int export_run(PxlCtx* ctx, const PxlExport* out, cudaStream_t s, cudaStream_t c
     return PXL_ERR_CUDA;
   Dev dd = d;
   dd.E = E;
+  Launch L{s};
+  L.pdl = E <= kPdlEvents;
+  dd.pdl = L.pdl;
   const int nb = event_blocks(E, kExpBlocks, 64);
   const dim3 grid(nb, E);
-  k_export_count<<<grid, kExpThreads, 0, s>>>(dd, x);
-  k_export_scan<<<1, 1024, 0, s>>>(dd, x, nb);
-  k_export_fill<<<grid, kExpThreads, 0, s>>>(dd, x);
+  L.run(k_export_count, grid, kExpThreads, 0, dd, x);
+  L.run(k_export_scan, 1, 1024, 0, dd, x, nb);
+  L.run(k_export_fill, grid, kExpThreads, 0, dd, x);
   if (cudaGetLastError() != cudaSuccess || cudaEventRecord(x.ready, s) != cudaSuccess ||
       cudaStreamWaitEvent(cs, x.ready, 0) != cudaSuccess)
     return PXL_ERR_CUDA;

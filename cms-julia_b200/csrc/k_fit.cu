@@ -62,6 +62,7 @@ __device__ bool fit_tuple(const Dev& d, uint64_t g, uint32_t hb, const uint32_t*
 // event has blocks as event_blocks gives them (one block took 580 us for the 51 k tuples of an event
 // of pileup 170); its counters are cleared before the launch.
 __global__ void __launch_bounds__(256) k_fit_list(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   EvInfo& E = d.ev[e];
   __shared__ uint32_t s_n[2], s_base[2];
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(256) k_fit_list(Dev d) {
 // bytes to L1 but runs twice the warps, which hides more of its FP64 latency.
 template <int N, class T>
 __global__ void __launch_bounds__(128, 4) k_fit_tuples(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint64_t tb = E.tuple_base;
@@ -145,6 +147,7 @@ __global__ void __launch_bounds__(128, 4) k_fit_tuples(Dev d) {
 // FP64 refits of the mixed-precision fits that asked for one (same list layout as fit_list)
 template <int N>
 __global__ void __launch_bounds__(128, 4) k_refit_tuples(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint64_t tb = E.tuple_base;
@@ -260,6 +263,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_fit_plan_fill(const int32_t* _
 
 __global__ void __launch_bounds__(1024) k_fit_plan_one(const int32_t* __restrict__ offs, int32_t n, FitPlan* plan,
                                                        int32_t* status) {
+  pdl_trigger();
   __shared__ uint32_t s_cnt[kFitMaxN + 1], s_cur[kFitMaxN + 1];
   if (threadIdx.x <= kFitMaxN) s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -296,6 +300,7 @@ __global__ void __launch_bounds__(kFitThreads, kFitResident) k_fit_buckets(const
                                                     const int32_t* __restrict__ offs, const FitPlan* __restrict__ plan,
                                                     double B, float* state, float* cov, float* chi2, float* pt,
                                                     float* eta, int32_t* status) {
+  pdl_sync();
   for_bucket_track(*plan, [&](auto n, int32_t t) {
     standalone_fit<decltype(n)::value, T>(hits, ge, offs[t], B, state, cov, chi2, pt, eta, status, t);
   });
@@ -308,27 +313,27 @@ static_assert(offsetof(EvInfo, n_refit4) == offsetof(EvInfo, n_fit3) + 3 * sizeo
 void launch_fit(const Dev& d, const Launch& L) {
   // the events' n_fit3, n_fit4, n_refit3, n_refit4
   cudaMemset2DAsync(&d.ev[0].n_fit3, sizeof(EvInfo), 0, 4 * sizeof(uint32_t), size_t(d.E), L.s);
-  k_fit_list<<<dim3(event_blocks(d.E, 148 * 4, 64), d.E), 256, 0, L.s>>>(d);
+  L.run(k_fit_list, dim3(event_blocks(d.E, 148 * 4, 64), d.E), 256, 0, d);
   L.mark("fit_list");
   // about 7000 fits per PU50 event: enough CTAs for every SM with few events
   const int bx = (L.tune && L.tune[kTuneFitTuples] > 0) ? L.tune[kTuneFitTuples]
                                                          : std::max(2, std::min(64, (148 * 16) / std::max(1, int(d.E))));
   // FP64 as the reference fits (broken_line_fit_on_gpu.jl:28-30), or the mixed-precision fit
   if (d.fit_precision == 1) {
-    k_fit_tuples<3, float><<<dim3(bx, d.E), 128, 0, L.s>>>(d);
+    L.run(k_fit_tuples<3, float>, dim3(bx, d.E), 128, 0, d);
     L.mark("broken_line_fit_3");
-    k_fit_tuples<4, float><<<dim3(bx, d.E), 128, 0, L.s>>>(d);
+    L.run(k_fit_tuples<4, float>, dim3(bx, d.E), 128, 0, d);
     L.mark("broken_line_fit_4");
     // about 1 % of the fits: one block per event and hit count, more where an event has the GPU
     // to itself (a block's fits follow one another)
     const dim3 gr(event_blocks(d.E, 148, 16), d.E);
-    k_refit_tuples<3><<<gr, 128, 0, L.s>>>(d);
-    k_refit_tuples<4><<<gr, 128, 0, L.s>>>(d);
+    L.run(k_refit_tuples<3>, gr, 128, 0, d);
+    L.run(k_refit_tuples<4>, gr, 128, 0, d);
     L.mark("broken_line_refit_fp64");
   } else {
-    k_fit_tuples<3, double><<<dim3(bx, d.E), 128, 0, L.s>>>(d);
+    L.run(k_fit_tuples<3, double>, dim3(bx, d.E), 128, 0, d);
     L.mark("broken_line_fit_3");
-    k_fit_tuples<4, double><<<dim3(bx, d.E), 128, 0, L.s>>>(d);
+    L.run(k_fit_tuples<4, double>, dim3(bx, d.E), 128, 0, d);
     L.mark("broken_line_fit_4");
   }
 }
@@ -338,14 +343,15 @@ int64_t fit_plan_bytes(int32_t n_tracks) {
 }
 
 int fit_plan_build(const int32_t* offs, int32_t n, FitPlan* plan, int32_t* status, cudaStream_t s) {
+  const Launch L{s};
   if (n <= kPlanOneCta) {
     // one launch instead of a clear, a count and a fill; above, one CTA takes longer than they do
-    k_fit_plan_one<<<1, 1024, 0, s>>>(offs, n, plan, status);
+    L.run(k_fit_plan_one, 1, 1024, 0, offs, n, plan, status);
   } else {
     if (cudaMemsetAsync(plan, 0, sizeof(FitPlan) - sizeof(plan->list), s) != cudaSuccess) return PXL_ERR_CUDA;
     const int blocks = div_up(n, kPlanThreads * kPlanPerThread);
-    k_fit_plan_count<<<blocks, kPlanThreads, 0, s>>>(offs, n, plan, status);
-    k_fit_plan_fill<<<blocks, kPlanThreads, 0, s>>>(offs, n, plan);
+    L.run(k_fit_plan_count, blocks, kPlanThreads, 0, offs, n, plan, status);
+    L.run(k_fit_plan_fill, blocks, kPlanThreads, 0, offs, n, plan);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;
 }
@@ -366,10 +372,12 @@ extern "C" int32_t pxl_bl_fit(const double* hits, const float* hits_ge, const in
   auto* plan = static_cast<pxl::FitPlan*>(workspace);
   int rc = pxl::fit_plan_build(offs, n, plan, status, s);
   if (rc) return rc;
+  pxl::Launch L{s};
+  L.pdl = true;
   const int g = pxl::bl_fit_blocks(n);
   if (precision == 0)
-    pxl::k_fit_buckets<double><<<g, pxl::kFitThreads, 0, s>>>(hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
+    L.run(pxl::k_fit_buckets<double>, g, pxl::kFitThreads, 0, hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
   else
-    pxl::k_fit_buckets<float><<<g, pxl::kFitThreads, 0, s>>>(hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
+    L.run(pxl::k_fit_buckets<float>, g, pxl::kFitThreads, 0, hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
   return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;
 }

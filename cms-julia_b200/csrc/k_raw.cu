@@ -11,27 +11,36 @@ namespace pxl {
 
 namespace {
 
-// Single-block scan of one EvInfo count field into a base field over E events;
-// ev[E] receives the batch total in both fields.
-__global__ void k_ev_scan(EvInfo* ev, int E, int count_off, int base_off) {
+// Single-block scan of one EvInfo count field into a base field over E events; ev[E] receives the
+// batch total in both fields. With a capacity (cap >= 0), events whose region [base, base + count)
+// would pass it are emptied (count = 0, buffer warning) and the batch total is capped, so that no
+// later kernel indexes past the buffer.
+__global__ void __launch_bounds__(1024) k_ev_scan(EvInfo* ev, int E, int count_off, int base_off, int64_t cap,
+                                                  uint32_t* status) {
+  pdl_sync();
   __shared__ uint32_t sh[33];
-  __shared__ uint32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
   char* base = reinterpret_cast<char*>(ev);
+  uint32_t carry = 0;
   for (int b = 0; b < E; b += blockDim.x) {
-    int e = b + threadIdx.x;
-    uint32_t v = e < E ? *reinterpret_cast<uint32_t*>(base + size_t(e) * sizeof(EvInfo) + count_off) : 0u;
+    const int e = b + threadIdx.x;
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(base + size_t(e) * sizeof(EvInfo) + count_off);
+    const uint32_t v = e < E ? *cnt : 0u;
     uint32_t tot;
-    uint32_t ex = block_excl_scan(v, sh, &tot);
-    if (e < E) *reinterpret_cast<uint32_t*>(base + size_t(e) * sizeof(EvInfo) + base_off) = carry + ex;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += tot;
-    __syncthreads();
+    const uint32_t lo = carry + block_excl_scan(v, sh, &tot);
+    if (e < E) {
+      *reinterpret_cast<uint32_t*>(base + size_t(e) * sizeof(EvInfo) + base_off) = lo;
+      if (cap >= 0 && int64_t(lo) + int64_t(v) > cap) {
+        *cnt = 0;
+        atomicOr(&ev[e].warnings, kWarnBuffer);
+        atomicOr(status, kWarnBuffer);
+      }
+    }
+    carry += tot;
   }
   if (threadIdx.x == 0) {
     *reinterpret_cast<uint32_t*>(base + size_t(E) * sizeof(EvInfo) + base_off) = carry;
-    *reinterpret_cast<uint32_t*>(base + size_t(E) * sizeof(EvInfo) + count_off) = carry;
+    *reinterpret_cast<uint32_t*>(base + size_t(E) * sizeof(EvInfo) + count_off) =
+        cap >= 0 && int64_t(carry) > cap ? uint32_t(cap) : carry;
   }
 }
 
@@ -52,6 +61,7 @@ constexpr uint32_t kFedWindow = 96 * 1024;  // bytes per window
 constexpr int kFedHops = 256;               // records per window
 
 __global__ void __launch_bounds__(256) k_fed_table(Dev d, const int16_t* __restrict__ fed_slot_of) {
+  pdl_sync(d);
   const int e = blockIdx.x;
   const int NF = d.n_fed_slots;
   __shared__ uint64_t s_src[kMaxFedSlots];
@@ -66,7 +76,10 @@ __global__ void __launch_bounds__(256) k_fed_table(Dev d, const int16_t* __restr
   __shared__ uint32_t sh[33];
   __shared__ uint32_t s_warn;
   for (int f = threadIdx.x; f < NF; f += blockDim.x) { s_nw[f] = 0; s_src[f] = 0; s_len[f] = 0; s_last[f] = 0; }
-  if (threadIdx.x == 0) { s_warn = 0; s_p = 4; s_hop = 0; }
+  if (threadIdx.x == 0) {
+    s_warn = 0; s_p = 4; s_hop = 0;
+    if (e == 0) { *d.err_count = 0; *d.status = 0; }  // of this run: set by the kernels from here on
+  }
   __syncthreads();
   const uint64_t off0 = d.ev_off[e], off1 = d.ev_off[e + 1];
   const uint8_t* ev = d.raw + off0;
@@ -302,6 +315,7 @@ __device__ __forceinline__ void unpack_word(const Dev& d, int e, uint32_t local,
 constexpr int kUnpackWarps = 8;
 
 __global__ void __launch_bounds__(32 * kUnpackWarps) k_unpack(Dev d, uint32_t parts) {
+  pdl_sync(d);
   __shared__ __align__(16) uint32_t s_words[kUnpackWarps][128];
   const unsigned lane = threadIdx.x & 31u, wq = threadIdx.x >> 5;
   const uint32_t wid = blockIdx.x * kUnpackWarps + wq, part = wid % parts;
@@ -385,6 +399,7 @@ __device__ __forceinline__ uint2 part_words(uint32_t nw, uint32_t part, uint32_t
 }
 
 __global__ void __launch_bounds__(32 * kModWarps) k_modstart_count(Dev d, uint32_t parts) {
+  pdl_sync(d);
   const uint32_t wid = blockIdx.x * kModWarps + (threadIdx.x >> 5);
   const int f = int(wid / parts), e = blockIdx.y;
   const int NF = d.n_fed_slots;
@@ -405,6 +420,7 @@ __global__ void __launch_bounds__(32 * kModWarps) k_modstart_count(Dev d, uint32
 
 // per event: module-start offsets per part of a FED slot, n_modules; zero the cluster counters
 __global__ void k_modstart_scan(Dev d, uint32_t parts) {
+  pdl_sync(d);
   const int e = blockIdx.x;
   const int NF = d.n_fed_slots * int(parts);
   __shared__ uint32_t sh[33];
@@ -420,6 +436,7 @@ __global__ void k_modstart_scan(Dev d, uint32_t parts) {
   uint32_t* cim = d.clus_in_module + size_t(e) * kMaxNumModules;
   for (int i = threadIdx.x; i < kMaxNumModules; i += blockDim.x) cim[i] = 0;
   for (int i = threadIdx.x; i < 64; i += blockDim.x) d.id_seen[size_t(e) * 64 + i] = 0;
+  if (e == 0 && threadIdx.x < kListHeader) d.big_list[threadIdx.x] = 0;  // the clustering's work lists
   if (threadIdx.x == 0) {
     d.ev[e].repeated_ids = 0;
     uint32_t nm = carry < uint32_t(kMaxNumModules) ? carry : uint32_t(kMaxNumModules);
@@ -434,6 +451,7 @@ __global__ void k_modstart_scan(Dev d, uint32_t parts) {
 // The module starts of each part of a FED slot at the part's offset, one warp per part, in word
 // order (rank of a flag = flags of the earlier lanes plus those of the earlier steps).
 __global__ void __launch_bounds__(32 * kModWarps) k_modstart_fill(Dev d, uint32_t parts) {
+  pdl_sync(d);
   const uint32_t wid = blockIdx.x * kModWarps + (threadIdx.x >> 5);
   const int f = int(wid / parts), e = blockIdx.y;
   const int NF = d.n_fed_slots;
@@ -472,13 +490,12 @@ __global__ void __launch_bounds__(32 * kModWarps) k_modstart_fill(Dev d, uint32_
 void launch_raw(const Dev& d, const Launch& L, const int16_t* fed_slot_of) {
   const int NF = d.n_fed_slots;
   L.mark("start");
-  k_fed_table<<<d.E, 256, 0, L.s>>>(d, fed_slot_of);
-  k_ev_scan<<<1, 1024, 0, L.s>>>(d.ev, d.E, int(offsetof(EvInfo, n_words)), int(offsetof(EvInfo, word_base)));
-  launch_ev_clamp(d, L.s, int(offsetof(EvInfo, n_words)), int(offsetof(EvInfo, word_base)), d.cap_words);
+  L.run(k_fed_table, d.E, 256, 0, d, fed_slot_of);
+  launch_ev_scan(d, L, int(offsetof(EvInfo, n_words)), int(offsetof(EvInfo, word_base)), d.cap_words);
   L.mark("fed_table");
   // warps per FED slot: one, more in a batch whose slots give an SM less than a wave of warps
   const int parts = event_blocks(d.E * NF, kFedParts, 16);
-  k_unpack<<<dim3(div_up(int64_t(NF) * parts, kUnpackWarps), d.E), 32 * kUnpackWarps, 0, L.s>>>(d, uint32_t(parts));
+  L.run(k_unpack, dim3(div_up(int64_t(NF) * parts, kUnpackWarps), d.E), 32 * kUnpackWarps, 0, d, uint32_t(parts));
   L.mark("unpack_calib");
   launch_modstart(d, L, parts);
   L.mark("module_starts");
@@ -486,37 +503,13 @@ void launch_raw(const Dev& d, const Launch& L, const int16_t* fed_slot_of) {
 
 void launch_modstart(const Dev& d, const Launch& L, int parts) {
   const dim3 gm(div_up(int64_t(d.n_fed_slots) * parts, kModWarps), d.E);
-  k_modstart_count<<<gm, 32 * kModWarps, 0, L.s>>>(d, uint32_t(parts));
-  k_modstart_scan<<<d.E, 256, 0, L.s>>>(d, uint32_t(parts));
-  k_modstart_fill<<<gm, 32 * kModWarps, 0, L.s>>>(d, uint32_t(parts));
+  L.run(k_modstart_count, gm, 32 * kModWarps, 0, d, uint32_t(parts));
+  L.run(k_modstart_scan, d.E, 256, 0, d, uint32_t(parts));
+  L.run(k_modstart_fill, gm, 32 * kModWarps, 0, d, uint32_t(parts));
 }
 
-void launch_ev_scan(const Dev& d, cudaStream_t s, int count_off, int base_off) {
-  k_ev_scan<<<1, 1024, 0, s>>>(d.ev, d.E, count_off, base_off);
-}
-
-// Events whose region [base, base + count) would pass the buffer capacity are
-// emptied (count = 0, buffer warning) and the batch total is capped, so that no
-// later kernel indexes past the buffer.
-__global__ void k_ev_clamp(EvInfo* ev, int E, int count_off, int base_off, int64_t cap, uint32_t* status) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e > E) return;
-  char* b = reinterpret_cast<char*>(ev) + size_t(e) * sizeof(EvInfo);
-  uint32_t& cnt = *reinterpret_cast<uint32_t*>(b + count_off);
-  const uint32_t base = *reinterpret_cast<const uint32_t*>(b + base_off);
-  if (e == E) {
-    if (int64_t(cnt) > cap) cnt = uint32_t(cap);
-    return;
-  }
-  if (int64_t(base) + int64_t(cnt) > cap) {
-    cnt = 0;
-    atomicOr(&ev[e].warnings, kWarnBuffer);
-    atomicOr(status, kWarnBuffer);
-  }
-}
-
-void launch_ev_clamp(const Dev& d, cudaStream_t s, int count_off, int base_off, int64_t cap) {
-  k_ev_clamp<<<div_up(d.E + 1, 128), 128, 0, s>>>(d.ev, d.E, count_off, base_off, cap, d.status);
+void launch_ev_scan(const Dev& d, const Launch& L, int count_off, int base_off, int64_t cap) {
+  L.run(k_ev_scan, 1, 1024, 0, d.ev, d.E, count_off, base_off, cap, d.status);
 }
 
 }  // namespace pxl

@@ -239,6 +239,7 @@ __device__ __forceinline__ void module_sums(const Dev& d, int e, const HitModule
     const uint32_t h = cms[hm.me] + k;
     if (h >= d.hits_per_event) continue;
     if (uint64_t(hb) + h >= uint64_t(d.cap_hits)) { atomic_or_warn(&d.ev[e], kWarnBuffer); continue; }
+    if (h >= d.ev[e].n_hits) continue;  // an event past the buffer, emptied: k_cpe takes none of its hits
     const size_t o = size_t(hb) + h;
     d.hit_sum[o] = ClusSumRec{S.minr[k], S.maxr[k], S.minc[k], S.maxc[k], S.q[k], S.qfx[k], S.qlx[k], S.qfy[k], S.qly[k]};
     d.hit_me[o] = hm.me;
@@ -250,6 +251,7 @@ __device__ __forceinline__ void module_sums(const Dev& d, int e, const HitModule
 // 130 bytes of spills, faster than four blocks without the cap; the kernel waits on its
 // digi gathers, and more warps in flight hide more of them.
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, 6) k_get_hits_warp(Dev d) {
+  pdl_sync(d);
   __shared__ WarpHitSmem smem[kWarpsPerBlock];
   const int e = blockIdx.y;
   const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
@@ -275,6 +277,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 6) k_get_hits_warp(Dev d)
 
 // CPE of the hits whose cluster sums k_get_hits_warp recorded, one hit per thread
 __global__ void __launch_bounds__(256) k_cpe(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint32_t hb = E.hit_base;
@@ -282,6 +285,7 @@ __global__ void __launch_bounds__(256) k_cpe(Dev d) {
     const size_t o = size_t(hb) + h;
     const uint32_t me = d.hit_me[o];
     if (me == 0xFFFFFFFFu) continue;
+    d.hit_me[o] = 0xFFFFFFFFu;  // no record, until the next run writes one
     const ClusSumRec r = d.hit_sum[o];
     write_hit(d, e, me, h, ClusSum{r.minr, r.maxr, r.minc, r.maxc, r.q, r.qfx, r.qlx, r.qfy, r.qly});
   }
@@ -294,6 +298,7 @@ struct BlockHitSmem {
 };
 
 __global__ void __launch_bounds__(256) k_get_hits_block(Dev d) {
+  pdl_sync(d);
   __shared__ BlockHitSmem S;
   const uint32_t nbig = list_size(d, kListHitsBig);
   for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
@@ -359,6 +364,7 @@ __device__ __forceinline__ uint32_t phi_bin_of(int16_t t, uint32_t i, const uint
 // setHitsLayerStart + fill_many_from_vector for the 10x128 phi histogram, one block per event.
 // Bins end up holding hit ids in decreasing order (the reference fill decrements the bin cursor).
 __global__ void __launch_bounds__(1024) k_phi_binner(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.x;
   __shared__ uint32_t s_off[kPhiTotBins + 3];
   __shared__ uint32_t s_hls[11];
@@ -412,6 +418,7 @@ __global__ void __launch_bounds__(1024) k_phi_binner(Dev d) {
 // windows. A thread per hit over all the event's blocks (within k_phi_binner's one block per
 // event, 85 us of one event of pileup 170 went here).
 __global__ void __launch_bounds__(256) k_phi_place(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint32_t hb = E.hit_base;
@@ -467,16 +474,15 @@ void launch_rechits(const Dev& d, const Launch& L) {
   // at least 16 blocks per event: short blocks (a dozen modules per warp) keep the tail of
   // the launch short (1.10 instead of 1.17 ms per 1000 PU50 events with 4)
   const int bx = std::max(16, std::min(250, (148 * 8 * 4) / std::max(1, int(d.E))));
-  // records of the warp-handled modules' clusters; hits of other modules keep 0xFFFFFFFF
-  cudaMemsetAsync(d.hit_me, 0xFF, size_t(d.cap_hits) * sizeof(uint32_t), L.s);
-  k_get_hits_warp<<<dim3(bx, d.E), 32 * kWarpsPerBlock, 0, L.s>>>(d);
+  // records of the warp-handled modules' clusters; hit_me of other modules' hits stays 0xFFFFFFFF
+  L.run(k_get_hits_warp, dim3(bx, d.E), 32 * kWarpsPerBlock, 0, d);
   L.mark("get_hits_warp");
-  k_cpe<<<dim3(std::max(1, std::min(64, (148 * 8 * 2) / std::max(1, int(d.E)))), d.E), 256, 0, L.s>>>(d);
+  L.run(k_cpe, dim3(std::max(1, std::min(64, (148 * 8 * 2) / std::max(1, int(d.E)))), d.E), 256, 0, d);
   L.mark("cpe");
-  k_get_hits_block<<<148 * 2, 256, 0, L.s>>>(d);
+  L.run(k_get_hits_block, 148 * 2, 256, 0, d);
   L.mark("get_hits_block");
-  k_phi_binner<<<d.E, 1024, 0, L.s>>>(d);
-  k_phi_place<<<dim3(event_blocks(d.E, 148 * 32, 128), d.E), 256, 0, L.s>>>(d);
+  L.run(k_phi_binner, d.E, 1024, 0, d);
+  L.run(k_phi_place, dim3(event_blocks(d.E, 148 * 32, 128), d.E), 256, 0, d);
   L.mark("phi_binner");
 }
 

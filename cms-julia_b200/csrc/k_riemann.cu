@@ -48,6 +48,7 @@ __device__ __forceinline__ void riemann_track(const RmArgs& A, int32_t t) {
 // uncapped, two blocks: 246 us; four: 208 us. At the launch per hit count it was 238 us.
 template <class T>
 __global__ void __launch_bounds__(kFitThreads, 3) k_riemann(RmArgs A) {
+  pdl_sync();
   for_bucket_track(*A.plan, [&](auto n, int32_t t) { riemann_track<decltype(n)::value, T>(A, t); });
 }
 
@@ -68,7 +69,8 @@ extern "C" int32_t pxl_riemann_fit(const double* hits, const float* hits_ge, con
   int rc = fit_plan_build(offs, n, plan, status, s);
   if (rc) return rc;
   RmArgs A{hits, hits_ge, offs, plan, b_field, state, chi2, pt, status};
-  if (precision == 0) k_riemann<double><<<fit_blocks(n), kFitThreads, 0, s>>>(A);
-  else k_riemann<float><<<fit_blocks(n), kFitThreads, 0, s>>>(A);
+  Launch L{s};
+  L.pdl = true;
+  L.run(precision == 0 ? k_riemann<double> : k_riemann<float>, fit_blocks(n), kFitThreads, 0, A);
   return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;
 }

@@ -20,10 +20,15 @@ constexpr float kChi2Coeff[4] = {0.68177776f, 0.74609577f, -0.08035491f, 0.00315
 
 // kernel_classify_tracks
 __global__ void k_classify(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   EvInfo& E = d.ev[e];
   const uint64_t tb = E.tuple_base;
   if (blockIdx.x == 0 && threadIdx.x == 0) { E.n_dup_cells = 0; E.n_dup_entries = 0; }  // filled by k_dup_cells
+  // the hits' tuple counts (k_hit_to_tuple)
+  for (uint32_t h = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x, n = d.ev[d.E].n_hits; h < n;
+       h += gridDim.y * gridDim.x * blockDim.x)
+    d.htt_cur[h] = 0;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < E.n_tuples; t += gridDim.x * blockDim.x) {
     const uint64_t g = tb + t;
     d.dup_death0[g] = 0xffffffffu;
@@ -62,6 +67,7 @@ __global__ void k_classify(Dev d) {
 // tracks at pileup 50): the tracks that are not loose can neither stay nor change. The cells carry
 // their index, so they are taken in any order.
 __global__ void __launch_bounds__(256) k_dup_cells(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   EvInfo& E = d.ev[e];
   if (E.n_cells == 0) return;
@@ -105,6 +111,7 @@ static_assert(kCellRows <= 64, "loose tracks of a cell as a 64-bit mask");
 // The rounds, one CTA per event; the death cells (event-local, 0xffffffff: none) start at none
 // (k_classify) and sit in global memory, of which an event uses a few KB.
 __global__ void k_dup_resolve(Dev d) {
+  pdl_sync(d);
   const EvInfo& E = d.ev[blockIdx.x];
   const uint32_t nc = E.n_dup_cells, ne = E.n_dup_entries;
   if (nc == 0) return;
@@ -169,6 +176,7 @@ __global__ void k_dup_resolve(Dev d) {
 // hit -> loose tuple lists
 template <int kPass>
 __global__ void k_hit_to_tuple(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint64_t tb = E.tuple_base;
@@ -187,6 +195,7 @@ __global__ void k_hit_to_tuple(Dev d) {
 
 // kernel_triplet_cleaner over hits; lists ordered by decreasing tuple id as the reference fills them
 __global__ void k_triplet_cleaner(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint32_t hb = E.hit_base;
@@ -643,6 +652,7 @@ __device__ __forceinline__ void vertex_core(Dev& d, EvInfo& E, uint32_t nt, cons
 // the event's blocks lists those of its range of tuples (vws_list, vtx_cnt); it also clears the range's
 // vertex ids and, with the first block, the event's vertex products.
 __global__ void __launch_bounds__(256) k_vertex_select(Dev d) {
+  pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   __shared__ uint32_t sh[33];
@@ -674,6 +684,7 @@ __global__ void __launch_bounds__(256) k_vertex_select(Dev d) {
 // above too, in global memory). parts: blocks of k_vertex_select per event.
 template <int kThreads, uint32_t kCap, bool kAll>
 __global__ void __launch_bounds__(kThreads, kAll ? 1 : 4) k_vertices(Dev d, int parts, uint32_t above) {
+  pdl_sync(d);
   extern __shared__ __align__(16) uint8_t s_vtx[];
   VtxShared& S = *reinterpret_cast<VtxShared*>(s_vtx);
   float* s_zt = reinterpret_cast<float*>(s_vtx + (sizeof(VtxShared) + 15) / 16 * 16);
@@ -738,18 +749,17 @@ __global__ void __launch_bounds__(kThreads, kAll ? 1 : 4) k_vertices(Dev d, int 
 
 void launch_classify(const Dev& d, const Launch& L) {
   auto g = [&](int seg) { return dim3(L.bpe_of(seg), d.E); };
-  k_classify<<<g(kTuneClassify), 256, 0, L.s>>>(d);
+  L.run(k_classify, g(kTuneClassify), 256, 0, d);
   L.mark("classify");
-  k_dup_cells<<<g(kTuneClassify), 256, 0, L.s>>>(d);
+  L.run(k_dup_cells, g(kTuneClassify), 256, 0, d);
   // a CTA per event: many threads where an SM has one event to itself, several events per SM else
-  k_dup_resolve<<<d.E, d.E <= 148 ? 1024 : 256, 0, L.s>>>(d);
+  L.run(k_dup_resolve, d.E, d.E <= 148 ? 1024 : 256, 0, d);
   L.mark("fast_duplicate_remover");
-  cudaMemsetAsync(d.htt_cur, 0, size_t(d.cap_hits) * sizeof(uint32_t), L.s);
-  k_hit_to_tuple<0><<<g(kTuneHitToTuple), 256, 0, L.s>>>(d);
-  excl_scan_shift_u32(d.htt_cur, d.htt_cnt, d.cap_hits, &d.ev[d.E].n_hits, d.scan_tmp, L.s);
-  k_hit_to_tuple<1><<<g(kTuneHitToTuple), 256, 0, L.s>>>(d);
+  L.run(k_hit_to_tuple<0>, g(kTuneHitToTuple), 256, 0, d);
+  excl_scan_shift_u32(d.htt_cur, d.htt_cnt, d.cap_hits, &d.ev[d.E].n_hits, d.scan_tmp, L);
+  L.run(k_hit_to_tuple<1>, g(kTuneHitToTuple), 256, 0, d);
   L.mark("hit_to_tuple");
-  k_triplet_cleaner<<<g(kTuneHitToTuple), 256, 0, L.s>>>(d);
+  L.run(k_triplet_cleaner, g(kTuneHitToTuple), 256, 0, d);
   L.mark("triplet_cleaner");
 }
 
@@ -766,13 +776,13 @@ int prepare_select_kernels() {
 void launch_vertices(const Dev& d, const Launch& L) {
   const size_t wide = vtx_smem_bytes(kVtxWideTracks), narrow = vtx_smem_bytes(kVtxNarrowTracks);
   const int parts = event_blocks(d.E, kVtxSelectBlocks, kVtxParts);
-  k_vertex_select<<<dim3(parts, d.E), 256, 0, L.s>>>(d);
+  L.run(k_vertex_select, dim3(parts, d.E), 256, 0, d);
   if (d.E <= 148) {  // at most one event per SM: the wide form for all
-    k_vertices<kVtxWideThreads, kVtxWideTracks, true><<<d.E, kVtxWideThreads, wide, L.s>>>(d, parts, 0u);
+    L.run(k_vertices<kVtxWideThreads, kVtxWideTracks, true>, d.E, kVtxWideThreads, wide, d, parts, 0u);
   } else {
-    k_vertices<kVtxNarrowThreads, kVtxNarrowTracks, false><<<d.E, kVtxNarrowThreads, narrow, L.s>>>(d, parts, 0u);
+    L.run(k_vertices<kVtxNarrowThreads, kVtxNarrowTracks, false>, d.E, kVtxNarrowThreads, narrow, d, parts, 0u);
     if (d.tuples_per_event > kVtxNarrowTracks)
-      k_vertices<kVtxWideThreads, kVtxWideTracks, true><<<148, kVtxWideThreads, wide, L.s>>>(d, parts, kVtxNarrowTracks);
+      L.run(k_vertices<kVtxWideThreads, kVtxWideTracks, true>, 148, kVtxWideThreads, wide, d, parts, kVtxNarrowTracks);
   }
   L.mark("vertices");
 }

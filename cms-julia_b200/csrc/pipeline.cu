@@ -229,6 +229,7 @@ int alloc_batch(PxlCtx* ctx) {
   A(xg, d.cap_hits); A(yg, d.cap_hits); A(zg, d.cap_hits); A(rg, d.cap_hits);
   A(iphi, d.cap_hits); A(xsize, d.cap_hits); A(ysize, d.cap_hits); A(detind, d.cap_hits); A(charge, d.cap_hits);
   A(hits_layer_start, E * 11); A(phi_off, E * kPhiTotBins); A(phi_bins, d.cap_hits); A(phi_fill, d.cap_hits); A(hit_rec, d.cap_hits); A(hit_rec_s, d.cap_hits); A(hit_u_s, d.cap_hits); A(hit_sum, d.cap_hits); A(hit_me, d.cap_hits); A(hit_xyzr, d.cap_hits);
+  CK(cudaMemset(d.hit_me, 0xFF, size_t(std::max<int64_t>(d.cap_hits, 1)) * sizeof(uint32_t)));
   A(pair_cum, E * kNPairs);
   A(item_cnt, d.cap_items + 1);
   A(item_pool, d.cap_items); A(dbl_pool, d.cap_cells); A(dbl_pool_ctr, 1);
@@ -237,7 +238,7 @@ int alloc_batch(PxlCtx* ctx) {
   A(cell_used, d.cap_cells);
   A(ohc_cnt, d.cap_hits + 1); A(ohc_cur, d.cap_hits); A(ohc_list, d.cap_cells); A(ohc_rec, d.cap_cells);
   A(cn_pairs, d.cap_pairs); A(cn_pair_ctr, 1); d.cap_long = std::max({d.cap_cells, d.cap_pairs, d.cap_tuple_hits}) / 9 + 1;
-  A(long_lists, d.cap_long); A(long_ctr, 1); A(cn_cnt, d.cap_cells + 1); A(cn_cur, d.cap_cells); A(cn_list, d.cap_pairs);
+  A(long_lists, d.cap_long); A(long_ctr, 2); A(cn_cnt, d.cap_cells + 1); A(cn_cur, d.cap_cells); A(cn_list, d.cap_pairs);
   A(tstart_cnt, d.cap_cells + 1);
   // tuple record pool: the batch's tuples plus a quarter for uneven parts
   d.tp_part = uint32_t((d.cap_tuples + d.cap_tuples / 4) / kTpParts + 64);
@@ -287,6 +288,8 @@ int run_chain(PxlCtx* ctx, uint32_t mask, cudaStream_t s) {
   if (d.E <= 0) return 0;
   Launch L{s, d.bpe, 256, (ctx->prof.on && !ctx->capturing) ? &ctx->prof : nullptr};
   L.tune = ctx->tune;
+  L.pdl = d.E <= kPdlEvents;
+  d.pdl = L.pdl;
   L.wq_ctas = ctx->wq_ctas;
   if ((mask & PXL_STAGE_DIGIS) && L.prof) ctx->prof.n = 0;
   // stages run in chain order; a producer boundary may stop after any of them and a
@@ -296,13 +299,10 @@ int run_chain(PxlCtx* ctx, uint32_t mask, cudaStream_t s) {
   const bool own_slot0 = (mask & PXL_STAGE_DIGIS) && !ctx->capturing && d.raw == ctx->d_raw[0];
   if (own_slot0) CK(cudaStreamWaitEvent(s, ctx->ev_staged[0], 0));
   if (mask & PXL_STAGE_DIGIS) {
-    CK(cudaMemsetAsync(d.err_count, 0, sizeof(uint32_t), s));
-    CK(cudaMemsetAsync(d.status, 0, sizeof(uint32_t), s));
     launch_raw(d, L, ctx->fed_slot_of);
     if (own_slot0) CK(cudaEventRecord(ctx->ev_consumed[0], s));
     launch_cluster(d, L);
-    launch_ev_scan(d, s, int(offsetof(EvInfo, n_hits)), int(offsetof(EvInfo, hit_base)));
-    launch_ev_clamp(d, s, int(offsetof(EvInfo, n_hits)), int(offsetof(EvInfo, hit_base)), d.cap_hits);
+    launch_ev_scan(d, L, int(offsetof(EvInfo, n_hits)), int(offsetof(EvInfo, hit_base)), d.cap_hits);
   }
   if (mask & PXL_STAGE_HITS) launch_rechits(d, L);
   if (mask & PXL_STAGE_TUPLES) launch_ca(d, L);
@@ -857,6 +857,7 @@ int32_t pxl_clusterize_digis(PxlCtx* ctx, const uint16_t* id, const int16_t* x, 
   uint32_t nw = uint32_t(n), zero = 0;
   CK(cudaMemcpyAsync(d.fed_nw, &nw, 4, cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(d.fed_wo, &zero, 4, cudaMemcpyHostToDevice, s));
+  d.pdl = 0;
   Launch L{s, d.bpe, 256};
   launch_modstart(d, L, 256);  // one slot, so 256 warps
   launch_cluster(d, L);

@@ -13,6 +13,7 @@
 #pragma once
 #include <cstdint>
 #include <type_traits>
+#include <utility>
 #include <cuda_runtime.h>
 
 namespace pxl {
@@ -193,7 +194,7 @@ struct Dev {
   uint32_t* cn_cur;        // [cap_cells]
   uint32_t* cn_list;       // [cap_pairs] global cell indices
   uint2* long_lists;       // [cap_long] (first entry, length) of the lists left to k_sort_long
-  uint32_t* long_ctr;      // [1]
+  uint32_t* long_ctr;      // [2] neighbour lists, track lists
   // tuples
   uint64_t* tstart_cnt;    // [cap_cells + 1] (tuples << 32 | hits) per start cell -> exclusive positions
   // tuples found by the count pass, in kTpParts parts of tp_part records each (a warp appends to
@@ -247,6 +248,7 @@ struct Dev {
   int64_t cap_big;
   // launch shape
   int32_t bpe;             // blocks per event for per-event kernels
+  int32_t pdl;             // the run's kernels are launched with Launch::pdl
   // persistent work-queue launches (workqueue.cu): events by decreasing hit count, and per
   // launch slot a pulled-block counter and the virtual-block prefix over that order
   uint32_t* wq_order;      // [E]
@@ -348,6 +350,21 @@ __device__ __forceinline__ void for_bucket_track(const FitPlan& plan, F&& f) {
 }
 
 // ---------------------------------------------------------------- helpers
+// First statement of every kernel launched by Launch::run. With Launch::pdl a kernel may start while
+// the one before it runs: here it waits until that one is complete and its writes are visible (all
+// threads, also those that then return, so that completion carries over from kernel to kernel), and
+// lets the next one start in turn. Launched plainly it may go on at once, which the chain's kernels of
+// many blocks are told by Dev::pdl (the two instructions cost a 512-event batch 1 %).
+__device__ __forceinline__ void pdl_sync() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// lets a kernel launched with Launch::pdl start (its blocks wait for this one's end)
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_sync(const Dev& d) {
+  if (d.pdl) pdl_sync();
+}
+
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
   const unsigned lane = threadIdx.x & 31u;
 #pragma unroll
@@ -447,16 +464,37 @@ enum TuneSeg : int {
   kTuneEarlyDup, kTuneClassify, kTuneHitToTuple, kTuneFitTuples, kTuneCount
 };
 
+// Largest batch whose kernels overlap their launches (Launch::pdl). 111 uneven events on three streams:
+// 9.3 ms without, 13.7 ms with it: the blocks that wait hold SM resources of the other streams' kernels.
+constexpr int kPdlEvents = 8;
+
 struct Launch {
   cudaStream_t s;
-  int bpe;        // blocks per event
-  int tpb;        // threads per block
+  int bpe = 0;    // blocks per event
+  int tpb = 0;    // threads per block
   Prof* prof = nullptr;
   // [kTuneCount] launch shape per stage: > 0 blocks per event (static grid), < 0 persistent
   // work queue with -value loop strides per virtual block, 0 the default
   const int* tune = nullptr;
   const int* wq_ctas = nullptr;  // [kTuneCount] CTAs of one persistent wave per stage (0: none)
   mutable int wq_slot = 0;       // next work-queue slot of the run
+  // Let a kernel's launch and its blocks' start overlap the end of the one before it. The chain of a
+  // single event is some 65 kernels of a few microseconds, which wait for one another's launch.
+  bool pdl = false;
+  template <class... P, class... A>
+  void run(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) const {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+  }
   int bpe_of(int seg) const {
     const int b = (tune && tune[seg] > 0) ? tune[seg] : bpe;
     return b > 0 ? b : 64;
@@ -475,14 +513,15 @@ struct Launch {
 // workqueue.cu: the event order of the run (most hits first, once the hits are known), and the
 // plan of one persistent launch: virtual blocks per event = ceil(count / units_per_block) with
 // count the EvInfo field at count_off
-void launch_wq_order(const Dev& d, cudaStream_t s);
+void launch_wq_order(const Dev& d, const Launch& L);
 WorkQueue launch_wq_plan(const Dev& d, const Launch& L, int count_off, uint32_t units_per_block);
 
 void launch_raw(const Dev& d, const Launch& L, const int16_t* fed_slot_of);  // a1-a4
 // a4 only (digis already in place); parts: warps per FED slot, fed_nmod holds parts counts per slot
 void launch_modstart(const Dev& d, const Launch& L, int parts);
-void launch_ev_scan(const Dev& d, cudaStream_t s, int count_off, int base_off);
-void launch_ev_clamp(const Dev& d, cudaStream_t s, int count_off, int base_off, int64_t cap);
+// scan of a count field of EvInfo into a base field; events whose region [base, base + count) would
+// pass cap are emptied (cap < 0: no limit)
+void launch_ev_scan(const Dev& d, const Launch& L, int count_off, int base_off, int64_t cap);
 void launch_cluster(const Dev& d, const Launch& L);   // a5-a7
 void launch_rechits(const Dev& d, const Launch& L);   // a8-a9
 void launch_ca(const Dev& d, const Launch& L);        // a10-a14
@@ -494,12 +533,12 @@ void launch_vertices(const Dev& d, const Launch& L);  // a18-a20
 
 // global scans over packed arrays (scan.cu)
 // In place exclusive scan of data[0..n), n = min(ncap, *n_dev) (n_dev may be null); data[n] = total.
-void excl_scan_u32(uint32_t* data, int64_t ncap, const uint32_t* n_dev, uint32_t* tmp, cudaStream_t s);
-void excl_scan_u64(uint64_t* data, int64_t ncap, const uint32_t* n_dev, uint64_t* tmp, cudaStream_t s);
+void excl_scan_u32(uint32_t* data, int64_t ncap, const uint32_t* n_dev, uint32_t* tmp, const Launch& L);
+void excl_scan_u64(uint64_t* data, int64_t ncap, const uint32_t* n_dev, uint64_t* tmp, const Launch& L);
 // out[0] = 0, out[i + 1] = exclusive prefix of in[i]: offsets of lists filled by
 // atomicAdd(&out[key + 1], 1) (scan.cu)
 void excl_scan_shift_u32(const uint32_t* in, uint32_t* out, int64_t ncap, const uint32_t* n_dev, uint32_t* tmp,
-                         cudaStream_t s);
+                         const Launch& L);
 int64_t scan_tmp_elems(int64_t n);
 
 }  // namespace pxl

@@ -1,5 +1,7 @@
 // Device-wide exclusive scans over packed arrays (three passes: tile sums,
-// scan of the tile sums in one block, tile scan with the tile's offset).
+// scan of the tile sums in one block, tile scan with the tile's offset; up to
+// kDirectTiles tiles the tile scan adds up the sums before it itself, which at
+// that size costs less than the launch in between).
 // In place: data[0..n) becomes the exclusive prefix and data[n] the total.
 // The tile passes move every element with coalesced global loads and stores and
 // hand each thread its kItems consecutive elements through shared memory padded
@@ -14,6 +16,7 @@ namespace {
 constexpr int kTpb = 256;
 constexpr int kItems = 8;
 constexpr int kTile = kTpb * kItems;
+constexpr int kDirectTiles = 1024;
 constexpr int kSumItems = 4;  // tile sums per thread in the single-block pass
 
 // shared-memory slot of tile element j: one padding element per 128 bytes
@@ -47,8 +50,9 @@ __device__ __forceinline__ int64_t live_n(int64_t n, const uint32_t* n_dev) {
   return n_dev ? (int64_t(*n_dev) < n ? int64_t(*n_dev) : n) : n;
 }
 
-template <class T>
+template <class T, bool kDirect>
 __global__ void k_tile_sums(const T* __restrict__ data, int64_t ncap, const uint32_t* n_dev, T* __restrict__ sums) {
+  if constexpr (kDirect) pdl_sync();
   int64_t n = live_n(ncap, n_dev);
   int64_t base = int64_t(blockIdx.x) * kTile;
   if (base >= n && base > 0) return;
@@ -122,8 +126,27 @@ __global__ void __launch_bounds__(1024) k_scan_sums(T* __restrict__ sums, int64_
   if (threadIdx.x == 0) sums[nt] = carry;
 }
 
-template <class T>
+// the tile's offset: the scanned sums' entry, or the sum of the ones before it
+template <class T, bool kDirect>
+__device__ __forceinline__ T tile_offset(const T* __restrict__ sums) {
+  if constexpr (!kDirect) {
+    return sums[blockIdx.x];
+  } else {
+    __shared__ T s_part[kTpb / 32];
+    T v = 0;
+    for (unsigned i = threadIdx.x; i < blockIdx.x; i += kTpb) v += sums[i];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    T r = 0;
+    for (int k = 0; k < kTpb / 32; ++k) r += s_part[k];
+    return r;
+  }
+}
+
+template <class T, bool kDirect>
 __global__ void k_tile_scan(T* __restrict__ data, int64_t ncap, const uint32_t* n_dev, const T* __restrict__ sums) {
+  if constexpr (kDirect) pdl_sync();
   int64_t n = live_n(ncap, n_dev);
   int64_t nt = (n + kTile - 1) / kTile;
   int64_t base = int64_t(blockIdx.x) * kTile;
@@ -151,7 +174,7 @@ __global__ void k_tile_scan(T* __restrict__ data, int64_t ncap, const uint32_t* 
   }
   __syncthreads();
   // a thread rewrites only the slots it read, so no barrier is needed before
-  T run = sums[blockIdx.x] + sh[wid] + inc - tsum;
+  T run = tile_offset<T, kDirect>(sums) + sh[wid] + inc - tsum;
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
     s_tile[pad_idx<T>(int(threadIdx.x) * kItems + k)] = run;
@@ -163,16 +186,18 @@ __global__ void k_tile_scan(T* __restrict__ data, int64_t ncap, const uint32_t* 
     const int j = k * kTpb + int(threadIdx.x);
     if (base + j < n) data[base + j] = s_tile[pad_idx<T>(j)];
   }
-  if (int64_t(blockIdx.x) == nt - 1 && threadIdx.x == 0) data[n] = sums[nt];
+  // the last thread of the last tile has passed all elements
+  if (int64_t(blockIdx.x) == nt - 1 && threadIdx.x == kTpb - 1) data[n] = run;
 }
 
 // Shifted form for lists filled by atomic increments: out[0] = 0 and out[i + 1] = the
 // exclusive prefix of in[i]. A fill that takes slot atomicAdd(&out[i + 1], 1) for each of
 // the in[i] entries of key i leaves out[i] = start of key i and out[n] = total: the
 // offsets of the filled lists, with no second counter array to clear.
-template <class T>
+template <class T, bool kDirect>
 __global__ void k_tile_scan_shift(const T* __restrict__ in, T* __restrict__ out, int64_t ncap, const uint32_t* n_dev,
                                   const T* __restrict__ sums) {
+  if constexpr (kDirect) pdl_sync();
   int64_t n = live_n(ncap, n_dev);
   int64_t nt = (n + kTile - 1) / kTile;
   int64_t base = int64_t(blockIdx.x) * kTile;
@@ -195,7 +220,7 @@ __global__ void k_tile_scan_shift(const T* __restrict__ in, T* __restrict__ out,
     if (lane < kTpb / 32) sh[lane] = si - s;
   }
   __syncthreads();
-  T run = sums[blockIdx.x] + sh[wid] + inc - tsum;
+  T run = tile_offset<T, kDirect>(sums) + sh[wid] + inc - tsum;
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
     s_tile[pad_idx<T>(int(threadIdx.x) * kItems + k)] = run;
@@ -209,35 +234,47 @@ __global__ void k_tile_scan_shift(const T* __restrict__ in, T* __restrict__ out,
   }
 }
 
+// The three-pass form is launched plainly: its kernels (tens of thousands of blocks) do not wait as
+// Launch::pdl asks of those it is set for.
 template <class T>
-void excl_scan_shift(const T* in, T* out, int64_t ncap, const uint32_t* n_dev, T* tmp, cudaStream_t s) {
-  int64_t nt = ncap > 0 ? (ncap + kTile - 1) / kTile : 1;
-  k_tile_sums<T><<<unsigned(nt), kTpb, 0, s>>>(in, ncap, n_dev, tmp);
-  k_scan_sums<T><<<1, 1024, 0, s>>>(tmp, ncap, n_dev);
-  k_tile_scan_shift<T><<<unsigned(nt), kTpb, 0, s>>>(in, out, ncap, n_dev, tmp);
+void excl_scan_shift(const T* in, T* out, int64_t ncap, const uint32_t* n_dev, T* tmp, const Launch& L) {
+  const int64_t nt = ncap > 0 ? (ncap + kTile - 1) / kTile : 1;
+  if (nt <= kDirectTiles) {
+    L.run(k_tile_sums<T, true>, unsigned(nt), kTpb, 0, in, ncap, n_dev, tmp);
+    L.run(k_tile_scan_shift<T, true>, unsigned(nt), kTpb, 0, in, out, ncap, n_dev, tmp);
+    return;
+  }
+  k_tile_sums<T, false><<<unsigned(nt), kTpb, 0, L.s>>>(in, ncap, n_dev, tmp);
+  k_scan_sums<T><<<1, 1024, 0, L.s>>>(tmp, ncap, n_dev);
+  k_tile_scan_shift<T, false><<<unsigned(nt), kTpb, 0, L.s>>>(in, out, ncap, n_dev, tmp);
 }
 
 template <class T>
-void excl_scan(T* data, int64_t ncap, const uint32_t* n_dev, T* tmp, cudaStream_t s) {
-  int64_t nt = ncap > 0 ? (ncap + kTile - 1) / kTile : 1;
-  k_tile_sums<T><<<unsigned(nt), kTpb, 0, s>>>(data, ncap, n_dev, tmp);
-  k_scan_sums<T><<<1, 1024, 0, s>>>(tmp, ncap, n_dev);
-  k_tile_scan<T><<<unsigned(nt), kTpb, 0, s>>>(data, ncap, n_dev, tmp);
+void excl_scan(T* data, int64_t ncap, const uint32_t* n_dev, T* tmp, const Launch& L) {
+  const int64_t nt = ncap > 0 ? (ncap + kTile - 1) / kTile : 1;
+  if (nt <= kDirectTiles) {
+    L.run(k_tile_sums<T, true>, unsigned(nt), kTpb, 0, data, ncap, n_dev, tmp);
+    L.run(k_tile_scan<T, true>, unsigned(nt), kTpb, 0, data, ncap, n_dev, tmp);
+    return;
+  }
+  k_tile_sums<T, false><<<unsigned(nt), kTpb, 0, L.s>>>(data, ncap, n_dev, tmp);
+  k_scan_sums<T><<<1, 1024, 0, L.s>>>(tmp, ncap, n_dev);
+  k_tile_scan<T, false><<<unsigned(nt), kTpb, 0, L.s>>>(data, ncap, n_dev, tmp);
 }
 
 }  // namespace
 
 int64_t scan_tmp_elems(int64_t n) { return (n + kTile - 1) / kTile + 2; }
 
-void excl_scan_u32(uint32_t* data, int64_t ncap, const uint32_t* n_dev, uint32_t* tmp, cudaStream_t s) {
-  excl_scan<uint32_t>(data, ncap, n_dev, tmp, s);
+void excl_scan_u32(uint32_t* data, int64_t ncap, const uint32_t* n_dev, uint32_t* tmp, const Launch& L) {
+  excl_scan<uint32_t>(data, ncap, n_dev, tmp, L);
 }
-void excl_scan_u64(uint64_t* data, int64_t ncap, const uint32_t* n_dev, uint64_t* tmp, cudaStream_t s) {
-  excl_scan<uint64_t>(data, ncap, n_dev, tmp, s);
+void excl_scan_u64(uint64_t* data, int64_t ncap, const uint32_t* n_dev, uint64_t* tmp, const Launch& L) {
+  excl_scan<uint64_t>(data, ncap, n_dev, tmp, L);
 }
 void excl_scan_shift_u32(const uint32_t* in, uint32_t* out, int64_t ncap, const uint32_t* n_dev, uint32_t* tmp,
-                         cudaStream_t s) {
-  excl_scan_shift<uint32_t>(in, out, ncap, n_dev, tmp, s);
+                         const Launch& L) {
+  excl_scan_shift<uint32_t>(in, out, ncap, n_dev, tmp, L);
 }
 
 }  // namespace pxl

@@ -13,6 +13,7 @@ constexpr int kOrderMax = 4096;  // events sorted in one block; larger batches k
 // events by decreasing hit count (ties by index): a bitonic sort of (count, index) keys in
 // shared memory
 __global__ void __launch_bounds__(1024) k_wq_order(const EvInfo* __restrict__ ev, int E, uint32_t* order) {
+  pdl_sync();
   __shared__ unsigned long long s_key[kOrderMax];
   if (E > kOrderMax) {
     for (int e = threadIdx.x; e < E; e += blockDim.x) order[e] = uint32_t(e);
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(1024) k_wq_order(const EvInfo* __restrict__ ev
 // launch's counter cleared; one block
 __global__ void __launch_bounds__(1024) k_wq_plan(const EvInfo* __restrict__ ev, int E, const uint32_t* order,
                                                   int count_off, uint32_t units, uint32_t* prefix, uint32_t* head) {
+  pdl_sync();
   __shared__ uint32_t sh[33];
   uint32_t carry = 0;
   const char* base = reinterpret_cast<const char*>(ev);
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(1024) k_wq_plan(const EvInfo* __restrict__ ev,
 
 }  // namespace
 
-void launch_wq_order(const Dev& d, cudaStream_t s) { k_wq_order<<<1, 1024, 0, s>>>(d.ev, d.E, d.wq_order); }
+void launch_wq_order(const Dev& d, const Launch& L) { L.run(k_wq_order, 1, 1024, 0, d.ev, d.E, d.wq_order); }
 
 WorkQueue launch_wq_plan(const Dev& d, const Launch& L, int count_off, uint32_t units_per_block) {
   const int slot = L.wq_slot++ % kWqSlots;
@@ -73,7 +75,7 @@ WorkQueue launch_wq_plan(const Dev& d, const Launch& L, int count_off, uint32_t 
   q.prefix = d.wq_prefix + size_t(slot) * (size_t(d.E) + 1);
   q.head = d.wq_head + slot;
   q.n = uint32_t(d.E);
-  k_wq_plan<<<1, 1024, 0, L.s>>>(d.ev, d.E, d.wq_order, count_off, units_per_block < 1 ? 1u : units_per_block,
+  L.run(k_wq_plan, 1, 1024, 0, d.ev, d.E, d.wq_order, count_off, units_per_block < 1 ? 1u : units_per_block,
                                  const_cast<uint32_t*>(q.prefix), q.head);
   return q;
 }
