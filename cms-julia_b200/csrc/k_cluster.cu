@@ -609,6 +609,58 @@ __global__ void __launch_bounds__(256) k_find_clus_block(Dev d) {
   }
 }
 
+// The three work lists in one launch, for small batches: a single event has a few hundred modules in
+// them, so each of the three kernels is as long as its longest module (17, 57 and 70 us for an event of
+// pileup 170), and together they are as long as the longest. The first blocks take the large modules; of
+// the others, four warps of each take the mid-size ones, then all warps the small ones.
+constexpr int kListBlocksBig = 148, kListBlocksWarp = 148 * 2;
+
+union ListSmem {
+  BlockSmem block;
+  struct {
+    WarpSmem<kWarpSlots> smem[kMidWarps];
+    WarpHist hist[kMidWarps];
+  } mid;
+  WarpSmem<1> small[8];
+};
+
+__global__ void __launch_bounds__(256) k_find_clus_lists(Dev d) {
+  pdl_sync(d);
+  __shared__ __align__(16) uint8_t s_raw[sizeof(ListSmem)];
+  ListSmem& S = *reinterpret_cast<ListSmem*>(s_raw);
+  if (blockIdx.x < uint32_t(kListBlocksBig)) {
+    const uint32_t n = list_size(d, kListClusBig);
+    for (uint32_t i = blockIdx.x; i < n; i += kListBlocksBig) {
+      const uint32_t v = list_entry(d, kListClusBig, i);
+      const int e = int(v >> 11);
+      const EvInfo& E = d.ev[e];
+      if (E.word_base + uint64_t(E.n_words) > uint64_t(d.cap_words)) continue;
+      cluster_module_block(d, e, v & 2047u, S.block);
+    }
+    return;
+  }
+  const uint32_t b = blockIdx.x - kListBlocksBig, wib = threadIdx.x >> 5;
+  if (wib < uint32_t(kMidWarps)) {
+    const uint32_t n = list_size(d, kListClusMid);
+    for (uint32_t i = b + wib * kListBlocksWarp; i < n; i += kListBlocksWarp * kMidWarps) {
+      const uint32_t v = list_entry(d, kListClusMid, i);
+      const int e = int(v >> 11);
+      ModRange r;
+      if (!module_range(d, e, v & 2047u, r)) continue;
+      cluster_module_warp<kWarpSlots>(d, e, v & 2047u, r, S.mid.smem[wib], &S.mid.hist[wib]);
+    }
+  }
+  __syncthreads();
+  const uint32_t n = list_size(d, kListClusSmall);
+  for (uint32_t i = b + wib * kListBlocksWarp; i < n; i += kListBlocksWarp * 8) {
+    const uint32_t v = list_entry(d, kListClusSmall, i);
+    const int e = int(v >> 11);
+    ModRange r;
+    if (!module_range(d, e, v & 2047u, r)) continue;
+    cluster_module_warp<1>(d, e, v & 2047u, r, S.small[wib], nullptr);
+  }
+}
+
 // cluster_charge_cut (gpu_cluster_charge_cut.jl:14-104) in the reference's serial order, for the
 // events where a module id starts more than one run: there a run's cut reads the count the id's
 // LAST run left (find_clus writes every count first), as changed by the cuts of its earlier
@@ -774,12 +826,17 @@ void launch_cluster(const Dev& d, const Launch& L) {
   // one thread per module position (at most 2000 per event)
   L.run(k_find_clus_tiny, dim3(div_up(kMaxNumModules, 128), d.E), 128, 0, d);
   L.mark("find_clus_tiny");
-  L.run(k_find_clus_small, std::min(148 * 64, div_up(int64_t(d.E) * kMaxNumModules, kWarpsPerBlock)), 32 * kWarpsPerBlock, 0, d);
-  L.mark("find_clus_small");
-  L.run(k_find_clus_mid, mid_wave_ctas(), 32 * kMidWarps, 0, d);
-  L.mark("find_clus_mid");
-  L.run(k_find_clus_block, 148 * 2, 256, 0, d);
-  L.mark("find_clus_block");
+  if (d.E <= kPdlEvents) {
+    L.run(k_find_clus_lists, kListBlocksBig + kListBlocksWarp, 256, 0, d);
+    L.mark("find_clus_lists");
+  } else {
+    L.run(k_find_clus_small, 148 * 64, 32 * kWarpsPerBlock, 0, d);
+    L.mark("find_clus_small");
+    L.run(k_find_clus_mid, mid_wave_ctas(), 32 * kMidWarps, 0, d);
+    L.mark("find_clus_mid");
+    L.run(k_find_clus_block, 148 * 2, 256, 0, d);
+    L.mark("find_clus_block");
+  }
   L.run(k_charge_cut_serial, d.E, 32, 0, d);
   L.run(k_hits_module_start, d.E, 1024, 0, d);
   L.mark("hits_module_start");
