@@ -141,7 +141,7 @@ def segment_bytes(name: str, c: dict) -> float | None:
         "neighbour_lists": 16 * C,                 # pair list in, lists filled and sorted
         "ntuplets_fill": 5 * T + 6 * TH,           # tuple offsets, hits, detector indices out
         "fast_duplicate_remover": 12 * T,          # qualities in and out, cell track lists in
-        "broken_line_fit_4": 22 * TH + 4 * TH + 8 * T + 93 * T,
+        "broken_line_fit": 22 * TH + 4 * TH + 8 * T + 93 * T,
         "vertices": 4 * T + 80 * T,
     }
     return table.get(name)
@@ -503,7 +503,7 @@ def chain_fit_precision(chain, conds, blob, offs, E: int, params, n_check: int =
             ch.run_batch(blob, offs)
             segs = dict(ch.profile_read())
         ch.profile(False)
-        fit_ms[name] = (segs.get("broken_line_fit_3", 0.0) + segs.get("broken_line_fit_4", 0.0) +
+        fit_ms[name] = (segs.get("broken_line_fit", 0.0) +
                         segs.get("broken_line_refit_fp64", 0.0))
     n_refit = sum(mixed.counts(e).n_fits_fp64 for e in range(E))
     n_fits = sum(int(mixed.product("fitted", e)[:mixed.counts(e).n_tuples].sum()) for e in range(E))

@@ -120,21 +120,19 @@ __global__ void __launch_bounds__(256) k_fit_list(Dev d) {
   }
 }
 
-// one hit count per launch, so that each instantiation keeps only its own registers.
-// Capped at 128 registers (four blocks per SM): the 4-hit fit spills a few hundred
-// bytes to L1 but runs twice the warps, which hides more of its FP64 latency.
-template <int N, class T>
-__global__ void __launch_bounds__(128, 4) k_fit_tuples(Dev d) {
-  pdl_sync(d);
-  const int e = blockIdx.y;
+// The event's fits of one hit count (N), listed in `list` as fit_list lists them.
+template <int N, class T, bool kRefit>
+__device__ __forceinline__ void fit_event(const Dev& d, int e) {
   const EvInfo& E = d.ev[e];
   const uint64_t tb = E.tuple_base;
   const uint32_t hb = E.hit_base;
-  const uint32_t nt = E.n_tuples, nfit = N == 3 ? E.n_fit3 : E.n_fit4;
+  const uint32_t nt = E.n_tuples;
+  const uint32_t nfit = kRefit ? (N == 3 ? E.n_refit3 : E.n_refit4) : (N == 3 ? E.n_fit3 : E.n_fit4);
+  const uint32_t* list = kRefit ? d.refit_list : d.fit_list;
   // B = Float64(Float32(bf)) as HelixFitOnGPU stores the field (ca_hit_ntuplet_generator.jl:83)
   const double B = double(d.c.b_field);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nfit; i += gridDim.x * blockDim.x) {
-    const uint32_t t = d.fit_list[N == 3 ? tb + i : tb + nt - 1 - i];
+    const uint32_t t = list[N == 3 ? tb + i : tb + nt - 1 - i];
     const uint64_t g = tb + t;
     if (!fit_tuple<N, T>(d, g, hb, d.tuple_hits + d.tuple_off[g], B)) {
       EvInfo& Ew = d.ev[e];
@@ -144,20 +142,15 @@ __global__ void __launch_bounds__(128, 4) k_fit_tuples(Dev d) {
   }
 }
 
-// FP64 refits of the mixed-precision fits that asked for one (same list layout as fit_list)
-template <int N>
-__global__ void __launch_bounds__(128, 4) k_refit_tuples(Dev d) {
+// Both hit counts in one launch (blockIdx.z), each block one of them: a small batch waits for the longer
+// one only (29 us for the two of one event, 15 together). 128 registers (four blocks per SM): the 4-hit
+// fit spills a few hundred bytes to L1 but runs twice the warps, which hides more of its FP64 latency.
+// kRefit: the FP64 refits of the mixed-precision fits that asked for one.
+template <class T, bool kRefit>
+__global__ void __launch_bounds__(128, 4) k_fit_tuples(Dev d) {
   pdl_sync(d);
-  const int e = blockIdx.y;
-  const EvInfo& E = d.ev[e];
-  const uint64_t tb = E.tuple_base;
-  const uint32_t hb = E.hit_base;
-  const uint32_t nt = E.n_tuples, nfit = N == 3 ? E.n_refit3 : E.n_refit4;
-  const double B = double(d.c.b_field);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nfit; i += gridDim.x * blockDim.x) {
-    const uint64_t g = tb + d.refit_list[N == 3 ? tb + i : tb + nt - 1 - i];
-    fit_tuple<N, double>(d, g, hb, d.tuple_hits + d.tuple_off[g], B);
-  }
+  if (blockIdx.z == 0) fit_event<4, T, kRefit>(d, blockIdx.y);
+  else fit_event<3, T, kRefit>(d, blockIdx.y);
 }
 
 template <int N, class T>
@@ -319,22 +312,17 @@ void launch_fit(const Dev& d, const Launch& L) {
   const int bx = (L.tune && L.tune[kTuneFitTuples] > 0) ? L.tune[kTuneFitTuples]
                                                          : std::max(2, std::min(64, (148 * 16) / std::max(1, int(d.E))));
   // FP64 as the reference fits (broken_line_fit_on_gpu.jl:28-30), or the mixed-precision fit
+  const dim3 grid(bx, d.E, 2);
   if (d.fit_precision == 1) {
-    L.run(k_fit_tuples<3, float>, dim3(bx, d.E), 128, 0, d);
-    L.mark("broken_line_fit_3");
-    L.run(k_fit_tuples<4, float>, dim3(bx, d.E), 128, 0, d);
-    L.mark("broken_line_fit_4");
+    L.run(k_fit_tuples<float, false>, grid, 128, 0, d);
+    L.mark("broken_line_fit");
     // about 1 % of the fits: one block per event and hit count, more where an event has the GPU
     // to itself (a block's fits follow one another)
-    const dim3 gr(event_blocks(d.E, 148, 16), d.E);
-    L.run(k_refit_tuples<3>, gr, 128, 0, d);
-    L.run(k_refit_tuples<4>, gr, 128, 0, d);
+    L.run(k_fit_tuples<double, true>, dim3(event_blocks(d.E, 148, 16), d.E, 2), 128, 0, d);
     L.mark("broken_line_refit_fp64");
   } else {
-    L.run(k_fit_tuples<3, double>, dim3(bx, d.E), 128, 0, d);
-    L.mark("broken_line_fit_3");
-    L.run(k_fit_tuples<4, double>, dim3(bx, d.E), 128, 0, d);
-    L.mark("broken_line_fit_4");
+    L.run(k_fit_tuples<double, false>, grid, 128, 0, d);
+    L.mark("broken_line_fit");
   }
 }
 

@@ -697,7 +697,7 @@ int32_t pxl_autotune(PxlCtx* ctx, const int32_t* candidates, int32_t n_candidate
       {"ntuplets_count", kTuneNtuplets}, {"ntuplets_fill", kTuneNtuplets}, {"cell_tracks", kTuneCellTracks},
       {"dup_multiplicity", kTuneEarlyDup}, {"classify", kTuneClassify},
       {"hit_to_tuple", kTuneHitToTuple}, {"triplet_cleaner", kTuneHitToTuple},
-      {"broken_line_fit_3", kTuneFitTuples}, {"broken_line_fit_4", kTuneFitTuples}};
+      {"broken_line_fit", kTuneFitTuples}};
   cudaSetDevice(ctx->p.device);
   const bool prof_was = ctx->prof.on;
   int rc = pxl_profile_enable(ctx, 1);
