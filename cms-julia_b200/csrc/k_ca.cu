@@ -671,17 +671,19 @@ __device__ __forceinline__ void sort_list_warp(uint32_t* a, uint32_t n) {
 
 // A thread per hit sorts the lists of up to 32 entries in registers; the warp then takes its hits'
 // longer ones together (an insertion sort by one thread, kept above 128 entries, made the kernel
-// 248 us for one event of pileup 170).
-__global__ void k_sort_hit_lists(Dev d) {
+// 248 us for one event of pileup 170). A warp takes `hits` consecutive hits, fewer than 32 in a small
+// batch: the long lists sit next to each other, and one warp sorts them one after the other.
+__global__ void k_sort_hit_lists(Dev d, uint32_t hits) {
   pdl_sync(d);
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint32_t hb = E.hit_base, nh = E.n_hits;
   const unsigned lane = threadIdx.x & 31u;
-  for (uint32_t k0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); k0 < nh; k0 += gridDim.x * blockDim.x) {
+  const uint32_t warps = gridDim.x * (blockDim.x / 32);
+  for (uint32_t k0 = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * hits; k0 < nh; k0 += warps * hits) {
     const uint32_t k = k0 + lane;
     uint32_t lo = 0, n = 0;
-    if (k < nh) {
+    if (lane < hits && k < nh) {
       lo = d.ohc_cnt[hb + k];
       n = d.ohc_cnt[hb + k + 1] - lo;
       if (n > uint32_t(kMaxCellsPerHit)) atomic_or_warn(&d.ev[e], kWarnLists);
@@ -1444,7 +1446,8 @@ void launch_ca(const Dev& d, const Launch& L) {
   // cells ending on each hit (counted by the doublet fill)
   excl_scan_shift_u32(d.ohc_cur, d.ohc_cnt, d.cap_hits, &d.ev[d.E].n_hits, d.scan_tmp, L);
   L.run(k_ohc_fill, g(kTuneHitLists), 256, 0, d);
-  L.run(k_sort_hit_lists, g(kTuneHitLists), 256, 0, d);
+  if (d.E <= kPdlEvents) L.run(k_sort_hit_lists, dim3(event_blocks(d.E, 148 * 8, 1024), d.E), 256, 0, d, 4u);
+  else L.run(k_sort_hit_lists, g(kTuneHitLists), 256, 0, d, 32u);
   L.run(k_ohc_records, g(kTuneHitLists), 256, 0, d);
   L.mark("outer_hit_lists");
   // connection and neighbour lists
