@@ -1332,44 +1332,38 @@ __global__ void k_cell_tracks_fill(Dev d) {
 }
 
 // kernel_early_duplicate_remover (…_impl.jl:143-166)
+template <bool kPerCell>
 __global__ void k_early_dup(Dev d) {
   pdl_sync(d);
-  const int e = blockIdx.y;
-  const EvInfo& E = d.ev[e];
-  if (E.n_cells == 0) return;
-  // only cells with two or more tracks act: walk their bitmap
-  const uint64_t c_lo = E.cell_base, c_hi = c_lo + E.n_cells;
-  for (uint64_t wi = (c_lo >> 5) + blockIdx.x * blockDim.x + threadIdx.x; wi <= (c_hi - 1) >> 5;
-       wi += uint64_t(gridDim.x) * blockDim.x) {
-    for (uint32_t bits = dup_word(d, wi, c_lo, c_hi); bits; bits &= bits - 1) {
-      const uint64_t c = 32 * wi + uint32_t(__ffs(bits) - 1);
-      const uint32_t lo = d.ct_cnt[c];
-      uint32_t n = d.ct_cnt[c + 1] - lo;
-      if (n > uint32_t(kCellRows)) n = kCellRows;
-      // kListBatch entries at a time, their loads independent of one another: a cell of 64 tracks
-      // otherwise waits for 128 latencies one after the other (42 us for an event of 100 tracks)
-      uint32_t maxn = 0;
-      for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
-        uint32_t t[kListBatch], s[kListBatch];
+  const EvInfo& E = d.ev[blockIdx.y];
+  for_dup_cells<kPerCell>(d, E, [&](uint32_t k) {
+    const uint64_t c = uint64_t(E.cell_base) + k;
+    const uint32_t lo = d.ct_cnt[c];
+    uint32_t n = d.ct_cnt[c + 1] - lo;
+    if (n > uint32_t(kCellRows)) n = kCellRows;
+    // kListBatch entries at a time, their loads independent of one another: a cell of 64 tracks
+    // otherwise waits for 128 latencies one after the other (42 us for an event of 100 tracks)
+    uint32_t maxn = 0;
+    for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
+      uint32_t t[kListBatch], s[kListBatch];
 #pragma unroll
-        for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[lo + min(j0 + u, n - 1)];
+      for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[lo + min(j0 + u, n - 1)];
 #pragma unroll
-        for (int u = 0; u < kListBatch; ++u) s[u] = d.tuple_off[t[u] + 1] - d.tuple_off[t[u]];
+      for (int u = 0; u < kListBatch; ++u) s[u] = d.tuple_off[t[u] + 1] - d.tuple_off[t[u]];
 #pragma unroll
-        for (int u = 0; u < kListBatch; ++u) maxn = s[u] > maxn ? s[u] : maxn;
-      }
-      for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
-        uint32_t t[kListBatch], s[kListBatch];
-#pragma unroll
-        for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[lo + min(j0 + u, n - 1)];
-#pragma unroll
-        for (int u = 0; u < kListBatch; ++u) s[u] = d.tuple_off[t[u] + 1] - d.tuple_off[t[u]];
-#pragma unroll
-        for (int u = 0; u < kListBatch; ++u)
-          if (s[u] != maxn) d.quality[t[u]] = 1;
-      }
+      for (int u = 0; u < kListBatch; ++u) maxn = s[u] > maxn ? s[u] : maxn;
     }
-  }
+    for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
+      uint32_t t[kListBatch], s[kListBatch];
+#pragma unroll
+      for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[lo + min(j0 + u, n - 1)];
+#pragma unroll
+      for (int u = 0; u < kListBatch; ++u) s[u] = d.tuple_off[t[u] + 1] - d.tuple_off[t[u]];
+#pragma unroll
+      for (int u = 0; u < kListBatch; ++u)
+        if (s[u] != maxn) d.quality[t[u]] = 1;
+    }
+  });
 }
 
 // tuple multiplicity counts (kernel_countMultiplicity + finalize!) per event: offsets after
@@ -1520,7 +1514,7 @@ void launch_ca(const Dev& d, const Launch& L) {
   L.run(k_sort_cell_lists<1>, g(kTuneCellTracks), 256, 0, d);
   L.run(k_sort_long, kSortLongBlocks, 256, 0, d, 1, d.ct_list);
   L.mark("cell_tracks");
-  L.run(k_early_dup, g(kTuneEarlyDup), 256, 0, d);
+  L.run(d.E <= kPdlEvents ? k_early_dup<true> : k_early_dup<false>, g(kTuneEarlyDup), 256, 0, d);
   L.run(k_multiplicity, dim3(event_blocks(d.E, 148 * 4, 64), d.E), 256, 0, d);
   L.mark("dup_multiplicity");
 }

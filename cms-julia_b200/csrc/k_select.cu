@@ -66,45 +66,40 @@ __global__ void k_classify(Dev d) {
 // k_dup_cells gathers the cells with two or more loose tracks (614 of the 4160 cells with two or more
 // tracks at pileup 50): the tracks that are not loose can neither stay nor change. The cells carry
 // their index, so they are taken in any order.
+template <bool kPerCell>
 __global__ void __launch_bounds__(256) k_dup_cells(Dev d) {
   pdl_sync(d);
-  const int e = blockIdx.y;
-  EvInfo& E = d.ev[e];
-  if (E.n_cells == 0) return;
-  const uint64_t tb = E.tuple_base;
-  const uint64_t c_lo = E.cell_base, c_hi = c_lo + E.n_cells;
+  EvInfo& E = d.ev[blockIdx.y];
+  const uint64_t tb = E.tuple_base, c_lo = E.cell_base;
   uint32_t* et = d.dup_et + E.tuple_hit_base;
   uint32_t* ek = d.dup_ek + E.tuple_hit_base;
-  for (uint64_t wi = (c_lo >> 5) + blockIdx.x * blockDim.x + threadIdx.x; wi <= (c_hi - 1) >> 5;
-       wi += uint64_t(gridDim.x) * blockDim.x) {
-    for (uint32_t bits = dup_word(d, wi, c_lo, c_hi); bits; bits &= bits - 1) {
-      const uint64_t c = 32 * wi + uint32_t(__ffs(bits) - 1);
-      const uint32_t l0 = d.ct_cnt[c];
-      uint32_t n = d.ct_cnt[c + 1] - l0;
-      if (n > uint32_t(kCellRows)) n = kCellRows;
-      uint64_t loose = 0;
-      for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
-        uint32_t t[kListBatch];
+  for_dup_cells<kPerCell>(d, E, [&](uint32_t k) {
+    const uint64_t c = c_lo + k;
+    const uint32_t l0 = d.ct_cnt[c];
+    uint32_t n = d.ct_cnt[c + 1] - l0;
+    if (n > uint32_t(kCellRows)) n = kCellRows;
+    uint64_t loose = 0;
+    for (uint32_t j0 = 0; j0 < n; j0 += kListBatch) {
+      uint32_t t[kListBatch];
 #pragma unroll
-        for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[l0 + min(j0 + u, n - 1)];
-        uint32_t m = 0;
+      for (int u = 0; u < kListBatch; ++u) t[u] = d.ct_list[l0 + min(j0 + u, n - 1)];
+      uint32_t m = 0;
 #pragma unroll
-        for (int u = 0; u < kListBatch; ++u) m |= uint32_t(j0 + u < n && d.quality[t[u]] == 2) << u;
-        loose |= uint64_t(m) << j0;
-      }
-      const uint32_t m = __popcll(loose);
-      if (m < 2) continue;
-      const uint32_t slot = atomicAdd(&E.n_dup_cells, 1u);
-      uint32_t o = atomicAdd(&E.n_dup_entries, m);
-      d.dup_cell[c_lo + slot] = uint32_t(c - c_lo);
-      d.dup_rng[c_lo + slot] = make_uint2(o, m);
-      for (; loose; loose &= loose - 1, ++o) {
-        const uint32_t t = d.ct_list[l0 + uint32_t(__ffsll(loose) - 1)];
-        et[o] = uint32_t(t - tb);
-        ek[o] = __float_as_uint(fabsf(d.t_state[5 * size_t(t) + 1]));  // |tip| >= 0 orders as its bits
-      }
+      for (int u = 0; u < kListBatch; ++u) m |= uint32_t(j0 + u < n && d.quality[t[u]] == 2) << u;
+      loose |= uint64_t(m) << j0;
     }
-  }
+    const uint32_t m = __popcll(loose);
+    if (m < 2) return;
+    const uint32_t slot = atomicAdd(&E.n_dup_cells, 1u);
+    uint32_t o = atomicAdd(&E.n_dup_entries, m);
+    d.dup_cell[c_lo + slot] = k;
+    d.dup_rng[c_lo + slot] = make_uint2(o, m);
+    for (; loose; loose &= loose - 1, ++o) {
+      const uint32_t t = d.ct_list[l0 + uint32_t(__ffsll(loose) - 1)];
+      et[o] = uint32_t(t - tb);
+      ek[o] = __float_as_uint(fabsf(d.t_state[5 * size_t(t) + 1]));  // |tip| >= 0 orders as its bits
+    }
+  });
 }
 static_assert(kCellRows <= 64, "loose tracks of a cell as a 64-bit mask");
 
@@ -751,7 +746,7 @@ void launch_classify(const Dev& d, const Launch& L) {
   auto g = [&](int seg) { return dim3(L.bpe_of(seg), d.E); };
   L.run(k_classify, g(kTuneClassify), 256, 0, d);
   L.mark("classify");
-  L.run(k_dup_cells, g(kTuneClassify), 256, 0, d);
+  L.run(d.E <= kPdlEvents ? k_dup_cells<true> : k_dup_cells<false>, g(kTuneClassify), 256, 0, d);
   // a CTA per event: many threads where an SM has one event to itself, several events per SM else
   L.run(k_dup_resolve, d.E, d.E <= 148 ? 1024 : 256, 0, d);
   L.mark("fast_duplicate_remover");
