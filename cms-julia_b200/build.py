@@ -18,9 +18,9 @@ LIB = PKG / "lib"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 # Kernels whose FP32 results compare bit-exactly with the reference, which never contracts
-# a*b+c, build without FMA contraction. The track fits build with it: their results hold to
-# a tolerance, a contracted product loses nothing, and the fits are bound by the length of
-# their instruction stream.
+# a*b+c, build without FMA contraction. The track fits build with it: their FP64 results hold
+# to a tolerance, a contracted product loses nothing, and the fits are bound by the length of
+# their instruction stream. Their FP32 part rounds each operation by itself (bl::f32).
 FMA_SOURCES = {"k_fit.cu", "k_adjoint.cu", "k_riemann.cu"}
 CUDA_SOURCES = [
     "scan.cu",

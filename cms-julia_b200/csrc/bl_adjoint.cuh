@@ -102,10 +102,10 @@ BL_HD double chi2_adjoint(const double hits[3][N], const float ge[6][N], double 
     }
   }
   // ---------------------------------------------------------------- circle system
-  T ivc[N], Zc[N], wc[N], hc[N - 1];
+  T VBc[N], ivc[N], Zc[N], rn[N], wc[N], hc[N - 1];
   Band<N, true> fc;
   double uc[N + 1];
-  circle_system<N, T>(ge, G, P, iv, ivc, Zc, wc, hc, fc, uc);
+  circle_system<N, T>(ge, G, P, iv, VBc, ivc, Zc, rn, wc, hc, fc, uc);
   // ---------------------------------------------------------------- circle chi2 partials
   double gsig = 0.0;
 #pragma unroll

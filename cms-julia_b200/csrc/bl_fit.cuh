@@ -28,8 +28,11 @@
 //    once for its two kinks, and the Karimaki translations carry the direction
 //    as a unit vector, so that an angle is taken only at the end.
 // T is the working type of the hit geometry, the weights, the multiple-
-// scattering variances, the band-matrix entries and the chi2: T = double is the
-// FP64 fit, T = float the mixed-precision fit.
+// scattering variances and the chi2: T = double is the FP64 fit, T = f32 the
+// mixed-precision fit. f32 rounds every operation: the FP32 residuals and chi2 of a
+// nearly perfect track are all rounding (7e-5 of the chi2 over the fit workload),
+// so a contracted product or another order of operations would give other ones,
+// no better, and move tracks across the chain's chi2 cut. The FP64 part contracts.
 #pragma once
 #include <cmath>
 #include <cstdint>
@@ -40,21 +43,49 @@
 namespace pxl {
 namespace bl {
 
+// a float whose sums and products are rounded one by one
+struct f32 {
+  float v;
+  f32() = default;
+  BL_HD explicit f32(float x) : v(x) {}
+  BL_HD explicit f32(double x) : v(float(x)) {}
+  BL_HD explicit f32(int x) : v(float(x)) {}
+  BL_HD explicit operator float() const { return v; }
+  BL_HD explicit operator double() const { return double(v); }
+};
+#ifdef __CUDA_ARCH__
+BL_HD f32 operator+(f32 a, f32 b) { return f32(__fadd_rn(a.v, b.v)); }
+BL_HD f32 operator-(f32 a, f32 b) { return f32(__fsub_rn(a.v, b.v)); }
+BL_HD f32 operator*(f32 a, f32 b) { return f32(__fmul_rn(a.v, b.v)); }
+BL_HD f32 operator/(f32 a, f32 b) { return f32(__fdiv_rn(a.v, b.v)); }
+#else
+BL_HD f32 operator+(f32 a, f32 b) { return f32(a.v + b.v); }
+BL_HD f32 operator-(f32 a, f32 b) { return f32(a.v - b.v); }
+BL_HD f32 operator*(f32 a, f32 b) { return f32(a.v * b.v); }
+BL_HD f32 operator/(f32 a, f32 b) { return f32(a.v / b.v); }
+#endif
+BL_HD f32 operator-(f32 a) { return f32(-a.v); }
+BL_HD f32& operator+=(f32& a, f32 b) { a = a + b; return a; }
+BL_HD bool operator<(f32 a, f32 b) { return a.v < b.v; }
+BL_HD bool operator>(f32 a, f32 b) { return a.v > b.v; }
+BL_HD bool operator==(f32 a, f32 b) { return a.v == b.v; }
+BL_HD f32 fmaf(f32 a, f32 b, f32 c) { return f32(::fmaf(a.v, b.v, c.v)); }
+
 template <class T> BL_HD T s_sqrt(T x);
 template <> BL_HD double s_sqrt<double>(double x) { return sqrt(x); }
-template <> BL_HD float s_sqrt<float>(float x) { return sqrtf(x); }
+template <> BL_HD f32 s_sqrt<f32>(f32 x) { return f32(sqrtf(x.v)); }
 template <class T> BL_HD T s_atan(T x);
 template <> BL_HD double s_atan<double>(double x) { return atan(x); }
-template <> BL_HD float s_atan<float>(float x) { return atanf(x); }
+template <> BL_HD f32 s_atan<f32>(f32 x) { return f32(atanf(x.v)); }
 template <class T> BL_HD T s_log(T x);
 template <> BL_HD double s_log<double>(double x) { return log(x); }
-template <> BL_HD float s_log<float>(float x) { return logf(x); }
+template <> BL_HD f32 s_log<f32>(f32 x) { return f32(logf(x.v)); }
 // 1 / sqrt(x) (host: two operations)
-template <class T> BL_HD T s_rsqrt(T x) {
+BL_HD double s_rsqrt(double x) {
 #ifdef __CUDA_ARCH__
   return rsqrt(x);
 #else
-  return T(1) / s_sqrt<T>(x);
+  return 1.0 / sqrt(x);
 #endif
 }
 // a b, rounded (not contracted into a following sum)
@@ -65,13 +96,7 @@ BL_HD double s_mul(double a, double b) {
   return a * b;
 #endif
 }
-BL_HD float s_mul(float a, float b) {
-#ifdef __CUDA_ARCH__
-  return __fmul_rn(a, b);
-#else
-  return a * b;
-#endif
-}
+BL_HD f32 s_mul(f32 a, f32 b) { return a * b; }
 template <class T> BL_HD T s_abs(T x) { return x < T(0) ? -x : x; }
 
 constexpr double kPi = 3.141592653589793;
@@ -86,14 +111,14 @@ BL_HD T bl_atan2(T y, T x) {
   return T(NAN);
 }
 
-// multiple-scattering variance of one segment (broken_line.jl:46-57), without the factor
-// mult_scatt_scale that the segments of a track share
+// multiple-scattering variance of one segment (broken_line.jl:46-57); scale is the part that the
+// segments of a track share, lt receives 1 + 0.038 log (radiation lengths)
 template <class T>
-BL_HD T mult_scatt_len(T length, T& lt) {
+BL_HD T mult_scatt(T scale, T length, T& lt) {
   const T XXI_0 = T(0.06 / 16.0);
   const T abs_len = s_abs(length) * XXI_0;
   lt = T(1) + T(0.038) * s_log<T>(abs_len);
-  return abs_len * (lt * lt);
+  return scale * abs_len * (lt * lt);
 }
 
 template <class T>
@@ -103,6 +128,15 @@ BL_HD T mult_scatt_scale(T B, T R, T slope) {
   pt2 = pt2 * pt2;
   const T fact = T(0.7 * ((13.6 / 1000) * (13.6 / 1000)));
   return fact / (pt2 * (T(1) + slope * slope));
+}
+
+template <class T>
+BL_HD void rotation_matrix(T slope, T R[2][2]) {
+  T a;
+  if constexpr (sizeof(T) == 8) a = s_rsqrt(T(1) + slope * slope);
+  else a = T(1) / s_sqrt<T>(T(1) + slope * slope);
+  const T b = slope * a;
+  R[0][0] = a; R[0][1] = b; R[1][0] = -b; R[1][1] = a;
 }
 
 // Power of the point p with respect to the circle through the local origin whose
@@ -306,7 +340,7 @@ struct Prep {
   T cx, cy;       // fast-fit centre relative to hit 0
   T alpha;        // angle at the centre from hit 0 to the last hit
   T rx[N], ry[N]; // hit - centre
-  T irn[N];       // 1 / their lengths
+  T irn[N];       // 1 / their lengths (FP64 fit)
   T s[N];         // arc length relative to hit 0
   double s0;      // arc length of hit 0
   T S[N], Z[N];   // line-fit coordinates relative to hit 0
@@ -345,16 +379,12 @@ BL_HD void prepare(const Geo<N, T>& G, T B, Prep<N, T>& P) {
   const T xn = G.p[0][N - 1] - G.p[0][N - 2], yn = G.p[1][N - 1] - G.p[1][N - 2];
   P.q = s_mul(x1, yn) - s_mul(y1, xn) > T(0) ? -1 : 1;  // collinear hits: exactly 0
   P.slope = -T(P.q) / P.f3;
-  {
-    const T a = s_rsqrt<T>(T(1) + P.slope * P.slope);
-    const T b = P.slope * a;
-    P.Rl[0][0] = a; P.Rl[0][1] = b; P.Rl[1][0] = -b; P.Rl[1][1] = a;
-  }
+  rotation_matrix<T>(P.slope, P.Rl);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     P.rx[i] = G.p[0][i] - P.cx;
     P.ry[i] = G.p[1][i] - P.cy;
-    P.irn[i] = s_rsqrt<T>(P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i]);
+    if constexpr (sizeof(T) == 8) P.irn[i] = s_rsqrt(P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i]);
   }
   const T ux = -P.cx, uy = -P.cy, uu = ux * ux + uy * uy;
   const T fac = T(P.q) * P.R;
@@ -374,11 +404,11 @@ BL_HD void prepare(const Geo<N, T>& G, T B, Prep<N, T>& P) {
   P.VB[0] = T(0);
   P.VB[N - 1] = T(0);
   P.scale = mult_scatt_scale<T>(B, P.R, P.slope);
-  T before = P.scale * mult_scatt_len<T>(P.S[1] - P.S[0], P.lt[0]);
+  T before = mult_scatt<T>(P.scale, P.S[1] - P.S[0], P.lt[0]);
   P.ms0 = before;
 #pragma unroll
   for (int i = 1; i < N - 1; ++i) {
-    const T after = P.scale * mult_scatt_len<T>(P.S[i + 1] - P.S[i], P.lt[i]);
+    const T after = mult_scatt<T>(P.scale, P.S[i + 1] - P.S[i], P.lt[i]);
     P.VB[i] = after + before;
     before = after;
   }
@@ -410,7 +440,9 @@ BL_HD void line_weights(const float ge[6][N], const Prep<N, T>& P, T w[N]) {
     auto z = [&](float v) { return fabs(double(v)) < tol ? T(0) : T(v); };
     const T V[3][3] = {{T(ge[0][i]), z(ge[1][i]), z(ge[3][i])}, {z(ge[1][i]), T(ge[2][i]), z(ge[4][i])},
                        {z(ge[3][i]), z(ge[4][i]), T(ge[5][i])}};
-    const T tmp = P.irn[i];
+    T tmp;
+    if constexpr (sizeof(T) == 8) tmp = P.irn[i];
+    else tmp = T(1) / s_sqrt<T>(P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i]);
     const T J[2][3] = {{P.ry[i] * tmp, -P.rx[i] * tmp, T(0)}, {T(0), T(0), T(1)}};
     // second row of R J V J^T R^T
     T rj[3];
@@ -487,17 +519,23 @@ BL_HD void line_fit(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>& 
   L.par[0] = par0;
   L.par[1] = par1;
   for (int a = 0; a < 2; ++a) for (int b = 0; b < 2; ++b) L.cov[a][b] = cov[a][b];
-  double chi2 = 0;
+  T chi2 = T(0);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const double diff = double(P.Z[i]) - u[i];
-    chi2 += double(w[i]) * (diff * diff);
+    const T diff = P.Z[i] - T(u[i]);
+    chi2 += w[i] * (diff * diff);
     if (i > 0 && i < N - 1) {
-      const double t = (u[i - 1] - u[i]) * h[i - 1] + (u[i + 1] - u[i]) * h[i];
-      chi2 += (t * t) * iv[i];
+      if constexpr (sizeof(T) == 8) {
+        const T t = (u[i - 1] - u[i]) * h[i - 1] + (u[i + 1] - u[i]) * h[i];
+        chi2 += (t * t) * iv[i];
+      } else {
+        const T d1 = P.S[i] - P.S[i - 1], d2 = P.S[i + 1] - P.S[i];
+        const T t = T(u[i - 1]) / d1 - T(u[i]) * ((d1 + d2) / (d2 * d1)) + T(u[i + 1]) / d2;
+        chi2 += (t * t) / P.VB[i];
+      }
     }
   }
-  L.chi2 = chi2;
+  L.chi2 = double(chi2);
 }
 
 // Karimaki translation of (phi, d, rho) and its covariance to a point (x0, y0) (broken_line.jl:85-127);
@@ -512,7 +550,7 @@ BL_HD void translate_karimaki(double& cs, double& sn, CircleOut& c, double x0, d
   const double zeta = DO * DO + DP * DP;
   const double A = 2.0 * DO + p3 * zeta;
   const double U = sqrt(1.0 + p3 * A);
-  const double ixi = s_rsqrt<double>(BB * BB + C * C);
+  const double ixi = s_rsqrt(BB * BB + C * C);
   const double xi = ixi * ixi;
   const double v = 1.0 + p3 * DO;
   const double iu = 1.0 / (U * (1.0 + U));  // 1 / (1 + U) = U iu
@@ -528,39 +566,57 @@ BL_HD void translate_karimaki(double& cs, double& sn, CircleOut& c, double x0, d
   sandwich3(J, c.cov);
 }
 
-// circle-fit system: inverse scaled scattering variances, radial residuals, weights, inverse
-// segments, band factorisation (border = curvature correction) and solution u[N+1] (hit order).
-// iv: inverse scattering variances of the line.
+// circle-fit system: scattering variances scaled to the circle and their inverses, radial residuals,
+// hit radii, weights, inverse segments, band factorisation (border = curvature correction) and
+// solution u[N+1] (hit order). iv: inverse scattering variances of the line.
 template <int N, class T>
-BL_HD void circle_system(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>& P, const double iv[N],
-                         double ivc[N], T Z[N], T w[N], double h[N - 1], Band<N, true>& f, double u[N + 1]) {
+BL_HD void circle_system(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>& P, const double iv[N], T VB[N],
+                         double ivc[N], T Z[N], T rn[N], T w[N], double h[N - 1], Band<N, true>& f, double u[N + 1]) {
+  const T ms_scale = T(1.0) + P.slope * P.slope;
+#pragma unroll
+  for (int i = 0; i < N; ++i) VB[i] = (i > 0 && i < N - 1) ? P.VB[i] * ms_scale : T(0);
   // radial residuals of the hits to the fast-fit circle, which passes through hit 0
   const T ux = -P.cx, uy = -P.cy;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
+    const T n2 = P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i];
+    if constexpr (sizeof(T) == 8) rn[i] = n2 * P.irn[i];
+    else rn[i] = s_sqrt<T>(n2);
     const T px = G.p[0][i], py = G.p[1][i];
-    const T rn = (P.rx[i] * P.rx[i] + P.ry[i] * P.ry[i]) * P.irn[i];
-    Z[i] = power_of_point<T>(ux, uy, px, py) / (rn + P.R);
+    Z[i] = power_of_point<T>(ux, uy, px, py) / (rn[i] + P.R);
   }
   const double tol = 1e-12;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     auto z = [&](float v) { return fabs(double(v)) < tol ? T(0) : T(v); };
-    // variance along the radius: the direction is the second row of the reference's rotation
-    const T hx = P.rx[i] * P.irn[i], hy = P.ry[i] * P.irn[i];
-    const T vxy = z(ge[1][i]);
-    w[i] = T(1.0) / ((hx * z(ge[0][i]) + hy * vxy) * hx + (hx * vxy + hy * z(ge[2][i])) * hy);
+    const T vxx = z(ge[0][i]), vxy = z(ge[1][i]), vyy = z(ge[2][i]);
+    // variance along the radius, the second row of the reference's rotation
+    T hx, hy;
+    if constexpr (sizeof(T) == 8) {
+      hx = P.rx[i] * P.irn[i];
+      hy = P.ry[i] * P.irn[i];
+    } else {
+      T RR[2][2];
+      rotation_matrix<T>(-P.rx[i] / P.ry[i], RR);
+      hx = RR[1][0];
+      hy = RR[1][1];
+    }
+    const T t0 = hx * vxx + hy * vxy;
+    const T t1 = hx * vxy + hy * vyy;
+    w[i] = T(1.0) / (t0 * hx + t1 * hy);
   }
   // The system is assembled in FP64 from the FP32 weights, arc lengths, scattering variances
   // and residuals: for a stiff track the scattering terms are large and nearly cancel against
   // each other in the elimination, and FP32 entries would cost the curvature correction digits
   // (which the fast-fit curvature then cancels further when the fast fit is far off).
   double wd[N], D[N];  // D[i] = s[i+1] - s[i-1]
-  const double is = 1.0 / (1.0 + double(P.slope) * double(P.slope));
+  double is = 0.0;
+  if constexpr (sizeof(T) == 8) is = 1.0 / ms_scale;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     wd[i] = double(w[i]);
-    ivc[i] = iv[i] * is;
+    if constexpr (sizeof(T) == 8) ivc[i] = iv[i] * is;
+    else ivc[i] = (i > 0 && i < N - 1) ? 1.0 / double(VB[i]) : 0.0;
     D[i] = (i > 0 && i < N - 1) ? double(P.s[i + 1]) - double(P.s[i - 1]) : 0.0;
   }
   inverse_segments<N, T>(P.s, h);
@@ -594,15 +650,18 @@ BL_HD bool circle_fit(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>
                                            CircleOut& c, bool rot = false, double cr = 1.0, double sr = 0.0) {
   bool ok = true;
   c.q = P.q;
-  T Z[N], w[N];
+  const T ms_scale = T(1.0) + P.slope * P.slope;
+  T VB[N], Z[N], rn[N], w[N];
   Band<N, true> f;
   double u[N + 1], ivc[N], h[N - 1];
-  circle_system<N, T>(ge, G, P, iv, ivc, Z, w, h, f, u);
+  circle_system<N, T>(ge, G, P, iv, VB, ivc, Z, rn, w, h, f, u);
   double I[3][3];
   band_trailing_inverse<N, true>(f, I);
   // fitted points 0 and 1 (hit-0 frame), FP64 from here on
   const double R = double(P.R), q = double(c.q);
-  const double n0 = double(P.irn[0]), n1 = double(P.irn[1]);
+  double n0, n1;
+  if constexpr (sizeof(T) == 8) { n0 = P.irn[0]; n1 = P.irn[1]; }
+  else { n0 = 1.0 / double(rn[0]); n1 = 1.0 / double(rn[1]); }
   const double r0x = double(P.rx[0]) * n0, r0y = double(P.ry[0]) * n0;
   const double r1x = double(P.rx[1]) * n1, r1y = double(P.ry[1]) * n1;
   const double tmp1 = u[0] - double(Z[0]);
@@ -611,7 +670,7 @@ BL_HD bool circle_fit(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>
   const double ev0 = double(G.p[0][1]) + tmp2 * r1x, ev1 = double(G.p[1][1]) + tmp2 * r1y;
   const double emd0 = ev0 - dv0, emd1 = ev1 - dv1;
   const double t1 = emd0 * emd0 + emd1 * emd1;
-  const double il = s_rsqrt<double>(t1), it1 = il * il;
+  const double il = s_rsqrt(t1), it1 = il * il;
   double cs = emd0 * il, sn = emd1 * il;
   const double inner = R * R - 0.25 * t1;
   if (inner < 0) ok = false;
@@ -629,21 +688,28 @@ BL_HD bool circle_fit(const float ge[6][N], const Geo<N, T>& G, const Prep<N, T>
   c.cov[2][0] = I[2][0]; c.cov[2][1] = I[2][1]; c.cov[2][2] = I[2][2];
   sandwich3(J, c.cov);
   translate_karimaki(cs, sn, c, 0.5 * emd0, 0.5 * emd1);
-  c.cov[0][0] += double((T(1.0) + P.slope * P.slope) * P.ms0);
+  c.cov[0][0] += double(ms_scale * P.ms0);
   translate_karimaki(cs, sn, c, G.h0[0] + dv0, G.h0[1] + dv1);
   c.par[0] = rot ? bl_atan2<double>(cs * sr + sn * cr, cs * cr - sn * sr) : bl_atan2<double>(sn, cs);
-  double chi2 = 0;
+  const T* s = P.s;
+  T chi2 = T(0);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const double diff = double(Z[i]) - u[i];
-    chi2 += double(w[i]) * (diff * diff);
+    const T diff = Z[i] - T(u[i]);
+    chi2 += w[i] * (diff * diff);
     if (i > 0 && i < N - 1) {
-      const double d3 = double(P.s[i + 1]) - double(P.s[i - 1]);
-      const double t = (u[i - 1] - u[i]) * h[i - 1] + (u[i + 1] - u[i]) * h[i] + 0.5 * (d3 * u[N]);
-      chi2 += (t * t) * ivc[i];
+      const T d3 = s[i + 1] - s[i - 1];
+      if constexpr (sizeof(T) == 8) {
+        const T t = (u[i - 1] - u[i]) * h[i - 1] + (u[i + 1] - u[i]) * h[i] + 0.5 * (d3 * u[N]);
+        chi2 += (t * t) * ivc[i];
+      } else {
+        const T d1 = s[i] - s[i - 1], d2 = s[i + 1] - s[i];
+        const T t = T(u[i - 1]) / d1 - (T(u[i]) * d3) / (d1 * d2) + T(u[i + 1]) / d2 + (d3 * T(u[N])) / T(2.0);
+        chi2 += (t * t) / VB[i];
+      }
     }
   }
-  c.chi2 = chi2;
+  c.chi2 = double(chi2);
   return ok;
 }
 
@@ -683,7 +749,7 @@ BL_HD void chord_frame(const double hits[3][N], const float ge_in[6][N], bool ze
 }
 
 // full fit of one track of N hits: hits[3][N] (FP64 inputs), ge[6][N] (Float32).
-// The FP32 fit (T = float) works in the chord frame: the transverse plane turned about the
+// The FP32 fit (T = f32) works in the chord frame: the transverse plane turned about the
 // origin so that the chord from the first to the last hit lies along x. A hit's offset from
 // hit 0 then has a large component along the chord but a small one across it, of the order of
 // the sagitta; rounding the offsets to FP32 costs the across component, which carries the

@@ -276,13 +276,14 @@ __global__ void __launch_bounds__(1024) k_fit_plan_one(const int32_t* __restrict
 namespace {
 
 // One launch for all hit counts, where six launches on three streams, forked and joined by events,
-// left each kernel's tail and the event waits (1237 mixed fits 43 us, now 27; 99991 FP64 fits 98 us,
+// left each kernel's tail and the event waits (1237 mixed fits 43 us, now 28; 99991 FP64 fits 98 us,
 // now 81).
 constexpr int kFitResident = 4;  // blocks per SM: 128 registers a thread
 
 // A block per 128 tracks, long fits first, so that the blocks even out; from four waves on one wave
 // of blocks that go on to further tracks saves the blocks' starts (2^20 mixed fits 374 us instead
-// of 416), which at 1.3 waves costs more in balance than it saves (99991 FP64 fits 92 us instead of 81).
+// of 416 with contracted FP32 arithmetic; 417 us now that f32 rounds each operation), which at 1.3
+// waves costs more in balance than it saves (99991 FP64 fits 92 us instead of 81).
 inline int bl_fit_blocks(int32_t n) {
   const int all = fit_blocks(n), wave = 148 * kFitResident;
   return all < 4 * wave ? all : wave;
@@ -314,7 +315,7 @@ void launch_fit(const Dev& d, const Launch& L) {
   // FP64 as the reference fits (broken_line_fit_on_gpu.jl:28-30), or the mixed-precision fit
   const dim3 grid(bx, d.E, 2);
   if (d.fit_precision == 1) {
-    L.run(k_fit_tuples<float, false>, grid, 128, 0, d);
+    L.run(k_fit_tuples<bl::f32, false>, grid, 128, 0, d);
     L.mark("broken_line_fit");
     // about 1 % of the fits: one block per event and hit count, more where an event has the GPU
     // to itself (a block's fits follow one another)
@@ -366,6 +367,6 @@ extern "C" int32_t pxl_bl_fit(const double* hits, const float* hits_ge, const in
   if (precision == 0)
     L.run(pxl::k_fit_buckets<double>, g, pxl::kFitThreads, 0, hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
   else
-    L.run(pxl::k_fit_buckets<float>, g, pxl::kFitThreads, 0, hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
+    L.run(pxl::k_fit_buckets<pxl::bl::f32>, g, pxl::kFitThreads, 0, hits, hits_ge, offs, plan, b_field, state, cov, chi2, pt, eta, status);
   return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;
 }

@@ -71,6 +71,6 @@ extern "C" int32_t pxl_riemann_fit(const double* hits, const float* hits_ge, con
   RmArgs A{hits, hits_ge, offs, plan, b_field, state, chi2, pt, status};
   Launch L{s};
   L.pdl = true;
-  L.run(precision == 0 ? k_riemann<double> : k_riemann<float>, fit_blocks(n), kFitThreads, 0, A);
+  L.run(precision == 0 ? k_riemann<double> : k_riemann<bl::f32>, fit_blocks(n), kFitThreads, 0, A);
   return cudaGetLastError() == cudaSuccess ? 0 : PXL_ERR_CUDA;
 }

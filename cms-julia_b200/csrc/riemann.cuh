@@ -20,6 +20,7 @@
 namespace pxl {
 namespace rm {
 
+using bl::f32;
 using bl::s_sqrt;
 using bl::s_log;
 using bl::s_abs;
@@ -34,7 +35,7 @@ BL_HD void chol_inverse(const double A[N][N], double Inv[N][N]) {
     double d = A[j][j];
 #pragma unroll
     for (int k = 0; k < j; ++k) d -= L[j][k] * L[j][k];
-    const double il = bl::s_rsqrt<double>(d);
+    const double il = bl::s_rsqrt(d);
     iL[j] = il;
 #pragma unroll
     for (int i = j + 1; i < N; ++i) {
@@ -97,7 +98,7 @@ BL_HD bool min_eigen3_rqi(const double A[3][3], double v[3], double& lambda) {
   double mu = 0.0, res = 0.0;
 #pragma unroll
   for (int it = 0; it < 3; ++it) {
-    const double r = bl::s_rsqrt<double>(x * x + y * y + z * z);
+    const double r = bl::s_rsqrt(x * x + y * y + z * z);
     x *= r; y *= r; z *= r;
     const double ax = A[0][0] * x + a01 * y + a02 * z, ay = a01 * x + A[1][1] * y + a12 * z,
                  az = a02 * x + a12 * y + A[2][2] * z;
@@ -130,7 +131,7 @@ BL_HD void min_eigen3(const double Ain[3][3], double v[3], double& lambda) {
         if (A[p][q] == 0.0) continue;
         const double th = (A[q][q] - A[p][p]) / (2.0 * A[p][q]);
         const double t = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-        const double c = bl::s_rsqrt<double>(t * t + 1.0), s = t * c;
+        const double c = bl::s_rsqrt(t * t + 1.0), s = t * c;
         for (int k = 0; k < 3; ++k) {
           const double akp = A[k][p], akq = A[k][q];
           A[k][p] = c * akp - s * akq;
@@ -205,7 +206,16 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
   double Cr[N][N];
   {
     const T p_t = fR * B < T(20) ? fR * B : T(20);
-    const T ip_2 = T(0.000225) / (p_t * p_t);  // over p^2 sin^2(theta) = pT^2
+    // scattering factor 0.000225 / (p^2 sin^2(theta)), p sin(theta) = pT; in FP32 in the port's steps
+    T ip_2, pst;
+    if constexpr (sizeof(T) == 8) {
+      ip_2 = T(0.000225) / (p_t * p_t);
+    } else {
+      T theta = T(atan(double(ftan)));
+      if (theta < T(0)) theta += T(bl::kPi);
+      const T st = T(sin(double(theta)));
+      pst = p_t * p_t * (T(1) + T(1) / (ftan * ftan)) * st * st;
+    }
     const T k3 = s_sqrt<T>(T(1) + T(1) / (ftan * ftan));
     const T x0inv = T(0.06 / 16.0);
     T sv[N], sig2[N];
@@ -222,7 +232,8 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
       const T rl = (i == 0 ? sv[0] * k3 : s_abs(sv[i] * k3 - sv[i - 1] * k3)) * x0inv;
       // (1 + 0.038 ln x)^2 x -> 0 as x -> 0: the continuous value where a length rounds to 0
       const T l = rl > T(0) ? T(1) + T(0.038) * s_log<T>(rl) : T(0);
-      sig2[i] = l * l * rl * ip_2;
+      if constexpr (sizeof(T) == 8) sig2[i] = l * l * rl * ip_2;
+      else sig2[i] = l * l * rl * T(0.000225) / pst;
     }
 #pragma unroll
     for (int k = 0; k < N; ++k)
@@ -331,7 +342,7 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
   // ---------------------------------------------------------------- line fit in the rotated (s, z) plane
   // sine and cosine of the angle in [0, pi) whose tangent is -q ftan
   const double tth = -q * double(ftan);
-  double cs = bl::s_rsqrt<double>(1.0 + tth * tth), sn = tth * cs;
+  double cs = bl::s_rsqrt(1.0 + tth * tth), sn = tth * cs;
   if (tth < 0) { sn = -sn; cs = -cs; }
   const T ox = T(cx), oy = T(cy);  // centre relative to hit 0
   const T gox = T(hits[0][0] + cx), goy = T(hits[1][0] + cy);
@@ -446,7 +457,7 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
   return isfinite(o.state[0]) && isfinite(o.state[2]);
 }
 
-// The FP32 fit (T = float) runs in the chord frame of the hits (bl::chord_frame): their
+// The FP32 fit (T = bl::f32) runs in the chord frame of the hits (bl::chord_frame): their
 // offsets from hit 0, rounded to FP32, then keep the small component across the chord, which
 // carries the curvature, almost exactly. Every quantity but phi is invariant under the turn.
 template <int N, class T>
