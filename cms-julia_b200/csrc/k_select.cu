@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(256) k_dup_cells(Dev d) {
     if (m < 2) return;
     const uint32_t slot = atomicAdd(&E.n_dup_cells, 1u);
     uint32_t o = atomicAdd(&E.n_dup_entries, m);
-    d.dup_cell[c_lo + slot] = k;
-    d.dup_rng[c_lo + slot] = make_uint2(o, m);
+    d.dup_cell[E.tuple_hit_base / 2 + slot] = k;
+    d.dup_rng[E.tuple_hit_base / 2 + slot] = make_uint2(o, m);
     for (; loose; loose &= loose - 1, ++o) {
       const uint32_t t = d.ct_list[l0 + uint32_t(__ffsll(loose) - 1)];
       et[o] = uint32_t(t - tb);
@@ -111,8 +111,8 @@ __global__ void k_dup_resolve(Dev d) {
   const uint32_t nc = E.n_dup_cells, ne = E.n_dup_entries;
   if (nc == 0) return;
   const uint64_t tb = E.tuple_base;
-  const uint32_t* cell = d.dup_cell + E.cell_base;
-  const uint2* rng = d.dup_rng + E.cell_base;
+  const uint32_t* cell = d.dup_cell + E.tuple_hit_base / 2;
+  const uint2* rng = d.dup_rng + E.tuple_hit_base / 2;
   const uint32_t* et = d.dup_et + E.tuple_hit_base;
   const uint32_t* ek = d.dup_ek + E.tuple_hit_base;
   uint32_t* cur = d.dup_death0 + tb;

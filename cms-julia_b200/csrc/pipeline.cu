@@ -255,7 +255,7 @@ int alloc_batch(PxlCtx* ctx) {
   A(t_chi2, d.cap_tuples); A(t_fitted, d.cap_tuples);
   A(fit_list, d.cap_tuples); A(refit_list, d.cap_tuples);
   A(htt_cnt, d.cap_hits + 1); A(htt_cur, d.cap_hits); A(htt_list, d.cap_tuple_hits);
-  A(dup_bits, d.cap_cells / 32 + 2); A(dup_cell, d.cap_cells); A(dup_rng, d.cap_cells);
+  A(dup_bits, d.cap_cells / 32 + 2); A(dup_cell, d.cap_tuple_hits / 2 + 1); A(dup_rng, d.cap_tuple_hits / 2 + 1);
   A(dup_et, d.cap_tuple_hits); A(dup_ek, d.cap_tuple_hits); A(dup_death0, d.cap_tuples); A(dup_death1, d.cap_tuples);
   A(vws_zt, d.cap_tuples); A(vws_ezt2, d.cap_tuples); A(vws_ptt2, d.cap_tuples); A(vws_iv, d.cap_tuples);
   A(vws_itrk, d.cap_tuples); A(vws_izt, d.cap_tuples); A(vws_bins, d.cap_tuples); A(vws_list, d.cap_tuples);

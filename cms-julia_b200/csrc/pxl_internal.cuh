@@ -223,8 +223,10 @@ struct Dev {
   uint32_t* htt_list;      // [cap_tuple_hits]
   // duplicate removal, packed per event
   uint32_t* dup_bits;      // [cap_cells / 32 + 2] cells with two or more tracks, one bit each
-  uint32_t* dup_cell;      // [cap_cells] event-local index of the cells with two or more loose tracks, at the cell base
-  uint2* dup_rng;          // [cap_cells] first entry and number of entries of each of them
+  // [cap_tuple_hits / 2 + 1] at half the tuple-hit base (each of the cells has two or more of the event's
+  // entries): event-local index of the cells with two or more loose tracks; their first entry and number
+  uint32_t* dup_cell;
+  uint2* dup_rng;
   uint32_t* dup_et;        // [cap_tuple_hits] entries: event-local tuple id, at the tuple-hit base
   uint32_t* dup_ek;        // [cap_tuple_hits] entries: |tip| bits
   uint32_t* dup_death0;    // [cap_tuples] cell at which the duplicate remover drops the track (two rounds' values)
