@@ -247,7 +247,8 @@ int64_t pxl_results_async(PxlCtx* ctx, uint32_t* host_dst, int64_t max_events, v
  * the tracks of quality loose (TrackSOA, CUDADataFormats/PixelTrackHeterogeneous.jl:10-62,
  * the ones the vertex finder takes) and the vertices (ZVertexSoA, z_vertex_soa.jl:4-26) of all
  * events, packed event after event (tracks in tuple order), each array copied to host memory
- * in ONE device->host copy. The compaction kernels go on `stream` (ordered after the context's
+ * in ONE device->host copy (of its first max_tracks or max_vertices rows; a batch of up to 8 events
+ * with pinned arrays: all arrays by one kernel, which writes the rows there are). The compaction kernels go on `stream` (ordered after the context's
  * last run), the copies on `copy_stream` (NULL: the same stream); nothing synchronises the
  * host. Two device export sets alternate, so the copies of one batch overlap the next chain;
  * the host arrays must stay untouched until copy_stream reaches the copies (pinned memory for
