@@ -266,9 +266,12 @@ int alloc_batch(PxlCtx* ctx) {
   int64_t st = scan_tmp_elems(std::max({d.cap_words, d.cap_items, d.cap_cells, d.cap_hits, d.cap_tuples}) + 1);
   A(scan_tmp, st); A(scan_tmp64, st);
   A(status, 1);
+  CK(cudaMemset(d.status, 0, sizeof(uint32_t)));
   d.cap_big = E * kMaxNumModules;
   A(big_list, kListHeader + kNumLists * d.cap_big);
 #undef A
+  CK(cudaMallocHost(&ctx->h_ev, size_t(E + 1) * sizeof(EvInfo)));
+  CK(cudaMallocHost(&ctx->h_status, sizeof(uint32_t)));
   // input staging
   ctx->raw_cap = size_t(d.cap_words) * 4 + size_t(E) * (4 + 16 * 4 + size_t(d.n_fed_slots + 8) * 24) + 4096;
   for (int k = 0; k < PxlCtx::kSlots; ++k) {
@@ -321,12 +324,15 @@ int note_done(PxlCtx* ctx, cudaStream_t s) {
   return 0;
 }
 
+// The events' records and the global status bits of the last run, in one wait (through pinned memory:
+// pageable copies wait one by one).
 int fetch_ev_impl(PxlCtx* ctx) {
   if (ctx->ev_host_valid) return 0;
-  ctx->ev_host.resize(size_t(ctx->last_E) + 1);
-  CK(cudaMemcpyAsync(ctx->ev_host.data(), ctx->d.ev, ctx->ev_host.size() * sizeof(EvInfo), cudaMemcpyDeviceToHost,
-                     ctx->stream));
+  const size_t n = size_t(ctx->last_E) + 1;
+  CK(cudaMemcpyAsync(ctx->h_ev, ctx->d.ev, n * sizeof(EvInfo), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->h_status, ctx->d.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  ctx->ev_host.assign(ctx->h_ev, ctx->h_ev + n);
   ctx->ev_host_valid = true;
   return 0;
 }
@@ -533,6 +539,8 @@ int32_t pxl_ctx_destroy(PxlCtx* ctx) {
     if (x.copied) { cudaEventSynchronize(x.copied); cudaEventDestroy(x.copied); }
     if (x.ready) cudaEventDestroy(x.ready);
   }
+  if (ctx->h_ev) cudaFreeHost(ctx->h_ev);
+  if (ctx->h_status) cudaFreeHost(ctx->h_status);
   for (void* q : ctx->allocs) cudaFree(q);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -740,16 +748,13 @@ int32_t pxl_sync(PxlCtx* ctx) {
   if (!ctx) return PXL_ERR_ARG;
   cudaSetDevice(ctx->p.device);
   // waits for this context's work only (its stream is ordered after the last work it enqueued)
-  CK(cudaStreamSynchronize(ctx->stream));
-  CK(cudaGetLastError());
   ctx->ev_host_valid = false;
   int rc = fetch_ev(ctx);
   if (rc) return rc;
-  uint32_t w = 0;
+  CK(cudaGetLastError());
+  uint32_t w = *ctx->h_status;
   for (int e = 0; e < ctx->last_E; ++e) w |= ctx->ev_host[e].warnings;
-  uint32_t st = 0;
-  if (copy_dev(ctx->stream, ctx->d.status, 1, &st, 4) < 0) return PXL_ERR_CUDA;
-  return int32_t(w | st);
+  return int32_t(w);
 }
 
 int32_t pxl_event_counts(PxlCtx* ctx, int32_t e, PxlEventCounts* out) {

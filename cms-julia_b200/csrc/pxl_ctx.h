@@ -30,6 +30,8 @@ struct PxlCtx {
   uint32_t last_mask = 0;
   uint32_t done_mask = 0;
   std::vector<pxl::EvInfo> ev_host;
+  pxl::EvInfo* h_ev = nullptr;    // pinned [max_events + 1], where the device's records arrive
+  uint32_t* h_status = nullptr;   // pinned, the global status bits with them
   bool ev_host_valid = false;
   // per slot: pinned staging of the rebased offsets, device input, events staged in it,
   // an event after its copies and one after the last chain that read it
