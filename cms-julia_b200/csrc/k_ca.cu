@@ -794,7 +794,10 @@ __global__ void __launch_bounds__(256) k_ohc_records(Dev d) {
 // at most kMaxCellsPerHit entries). A warp takes 32 cells and spreads their (cell, candidate)
 // pairs over its lanes, 32 pairs per step; the cheap alignment test runs on every pair, and the
 // pairs that pass it (a few percent) queue in shared memory for the circle / DCA test, which
-// then runs on full warps. A passing pair counts one neighbour of the candidate (cn_cur), sets
+// then runs on full warps: the queue goes on over the warp's cells (emptied after every 32 of
+// them, a circle test of 150 instructions ran for five pairs: connect of 512 events of pileup 50
+// 1.33 ms, now 1.18; of 111 of pileup 25 to 170, 2.75 and 2.58 ms). A passing pair counts one
+// neighbour of the candidate (cn_cur), sets
 // both used flags and goes to the pair list that k_connect_fill turns into neighbour lists; none
 // of these depends on the evaluation order.
 constexpr int kConnWarps = 8;
@@ -803,12 +806,10 @@ constexpr int kConnQueue = 64;
 template <bool kQ>
 __global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
   pdl_sync(d);
-  __shared__ float4 s_rz[kConnWarps][32];  // inner r, z and outer r, z of each cell
-  __shared__ float4 s_xy[kConnWarps][32];  // inner x, y and outer x, y
-  __shared__ uint32_t s_lo[kConnWarps][32];
+  __shared__ float4 s_rz[kConnWarps][32];  // inner r (negative: barrel), z and outer r, z of each cell
+  __shared__ uint32_t s_first[kConnWarps][32];  // list position of the cell's pair 0, were the cells' pairs one range
   __shared__ uint32_t s_ex[kConnWarps][32];
-  __shared__ uint8_t s_barrel[kConnWarps][32];
-  __shared__ uint16_t s_queue[kConnWarps][kConnQueue];  // pair: owner lane << 8 | candidate
+  __shared__ uint2 s_queue[kConnWarps][kConnQueue];  // pair: cell, list position of the candidate
   for_each_vblock<kQ>(q, [&](int e, uint32_t bx, uint32_t nbx) {
   const EvInfo& E = d.ev[e];
   const uint64_t cb = E.cell_base;
@@ -816,25 +817,21 @@ __global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
   const float4* hxyzr = d.hit_xyzr + hb;
   const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  uint64_t c0 = 0;
+  uint32_t qn = 0;
   // circle / DCA test of the queued pairs q0 .. q0+31 (lanes past qn idle)
   auto circle_step = [&](uint32_t q0, uint32_t qn) {
     bool cut = false;
     uint32_t o = 0, c = 0;
     if (q0 + lane < qn) {
-      const uint32_t v = s_queue[w][q0 + lane];
-      const uint32_t a = v >> 8, j = v & 0xffu;
-      const uint32_t p = s_lo[w][a] + j;
-      const float4 xy = s_xy[w][a];
-      const float region = signbit(d.ohc_rec[p].x) ? kDcaInner : kDcaOuter;
-      const float4 h1 = hxyzr[d.cell_inner[d.ohc_list[p]]];  // the candidate's inner hit
-      const CircleEq eq(h1.x, h1.y, xy.x, xy.y, xy.z, xy.w);
+      const uint2 v = s_queue[w][q0 + lane];
+      c = v.x;
+      o = d.ohc_list[v.y];
+      const float region = signbit(d.ohc_rec[v.y].x) ? kDcaInner : kDcaOuter;
+      const float4 h1 = hxyzr[d.cell_inner[o]];  // the candidate's inner hit
+      const float4 hi = hxyzr[d.cell_inner[c]], ho = hxyzr[d.cell_outer[c]];
+      const CircleEq eq(h1.x, h1.y, hi.x, hi.y, ho.x, ho.y);
       if (eq.c > kHardCurv) cut = false;
       else cut = fabsf(eq.dca0()) < __fmul_rn(region, fabsf(eq.c));
-      if (cut) {
-        o = d.ohc_list[p];
-        c = uint32_t(c0 + a);
-      }
     }
     const uint32_t bal = __ballot_sync(0xffffffffu, cut);
     if (bal) {
@@ -856,42 +853,38 @@ __global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
   };
   for (uint32_t k0 = bx * blockDim.x + 32u * w; k0 < E.n_cells; k0 += nbx * blockDim.x) {
     const uint32_t k = k0 + lane;
-    c0 = cb + k0;
     const uint64_t c = cb + k;
-    uint32_t n = 0;
+    uint32_t n = 0, lo = 0;
     if (k < E.n_cells) {
       const uint32_t ih = d.cell_inner[c];
-      const uint32_t lo = d.ohc_cnt[hb + ih];
+      lo = d.ohc_cnt[hb + ih];
       n = d.ohc_cnt[hb + ih + 1] - lo;
       if (n > uint32_t(kMaxCellsPerHit)) n = kMaxCellsPerHit;
       if (n > 0) {  // geometry only for cells with candidates
         const uint32_t oh = d.cell_outer[c];
         const float4 hi = hxyzr[ih], ho = hxyzr[oh];
-        s_lo[w][lane] = lo;
-        s_rz[w][lane] = make_float4(hi.w, hi.z, ho.w, ho.z);
-        s_xy[w][lane] = make_float4(hi.x, hi.y, ho.x, ho.y);
-        s_barrel[w][lane] = d.detind[hb + ih] < 1184 ? 1 : 0;
+        s_rz[w][lane] = make_float4(d.detind[hb + ih] < 1184 ? -hi.w : hi.w, hi.z, ho.w, ho.z);
       }
     }
     const uint32_t inc = warp_incl_scan(n);
     const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
     s_ex[w][lane] = inc - n;
+    s_first[w][lane] = lo - (inc - n);
     __syncwarp();
-    uint32_t qn = 0;
     uint32_t a = 0;  // owner of this lane's pair, non-decreasing over the steps
     for (uint32_t x0 = 0; x0 < total; x0 += 32) {
       const uint32_t x = x0 + lane;
       bool al = false;
-      uint32_t j = 0;
+      uint32_t p = 0;
       if (x < total) {
         while (a < 31 && s_ex[w][a + 1] <= x) ++a;
-        j = x - s_ex[w][a];
-        const float2 rec = d.ohc_rec[s_lo[w][a] + j];  // the candidate's inner hit: r (sign: inner barrel), z
+        p = s_first[w][a] + x;
+        const float2 rec = d.ohc_rec[p];  // the candidate's inner hit: r (sign: inner barrel), z
         const float4 rz = s_rz[w][a];
-        al = are_aligned(fabsf(rec.x), rec.y, rz.x, rz.y, rz.z, rz.w, ptmin_f(), s_barrel[w][a] ? kThetaBarrel : kThetaForward);
+        al = are_aligned(fabsf(rec.x), rec.y, fabsf(rz.x), rz.y, rz.z, rz.w, ptmin_f(), signbit(rz.x) ? kThetaBarrel : kThetaForward);
       }
       const uint32_t bal = __ballot_sync(0xffffffffu, al);
-      if (al) s_queue[w][qn + __popc(bal & lt)] = uint16_t((a << 8) | j);
+      if (al) s_queue[w][qn + __popc(bal & lt)] = make_uint2(uint32_t(cb + k0 + a), p);
       qn += __popc(bal);
       __syncwarp();
       if (qn >= 32) {
@@ -900,9 +893,9 @@ __global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
         __syncwarp();
       }
     }
-    circle_step(0, qn);
     __syncwarp();
   }
+  circle_step(0, qn);
   });
 }
 
