@@ -761,6 +761,18 @@ __device__ __forceinline__ bool are_aligned(float r1, float z1, float ri, float 
   return __fmul_rn(t, p_min) <= __fmul_rn(__fmul_rn(theta_cut, d13), radius_diff);
 }
 
+// False only where are_aligned is false, without its square root: the two sides squared, the right one
+// larger by a share that covers the rounding of both (1e-6) and by a term above all underflow.
+__device__ __forceinline__ bool maybe_aligned(float r1, float z1, float ri, float zi, float ro, float zo, bool barrel) {
+  constexpr float kBarrel = float(double(kThetaBarrel) * kThetaBarrel / (0.899999976158 * 0.899999976158) * (1 + 1e-5));
+  constexpr float kForward = float(double(kThetaForward) * kThetaForward / (0.899999976158 * 0.899999976158) * (1 + 1e-5));
+  const float u = __fsub_rn(ro, r1);
+  const float t = __fadd_rn(__fadd_rn(__fmul_rn(z1, __fsub_rn(ri, ro)), __fmul_rn(zi, u)), __fmul_rn(zo, __fsub_rn(r1, ri)));
+  const float dz = __fsub_rn(z1, zo), u2 = __fmul_rn(u, u);
+  const float lim = __fmaf_rn(__fmul_rn(u2, __fmaf_rn(dz, dz, u2)), barrel ? kBarrel : kForward, 1e-30f);
+  return !(__fmul_rn(t, t) > lim);
+}
+
 // connect's candidates of each outer-hit list entry, gathered once per entry
 __global__ void __launch_bounds__(256) k_ohc_records(Dev d) {
   pdl_sync(d);
@@ -792,23 +804,26 @@ __global__ void __launch_bounds__(256) k_ohc_records(Dev d) {
 
 // Connection test of every cell with the cells ending on its inner hit (the outer-hit list,
 // at most kMaxCellsPerHit entries). A warp takes 32 cells and spreads their (cell, candidate)
-// pairs over its lanes, 32 pairs per step; the cheap alignment test runs on every pair, and the
-// pairs that pass it (a few percent) queue in shared memory for the circle / DCA test, which
-// then runs on full warps: the queue goes on over the warp's cells (emptied after every 32 of
+// pairs over its lanes, 32 pairs per step; a bound of the alignment test runs on every pair, and the
+// pairs that pass it (a few percent) queue in shared memory for that test and the circle / DCA test,
+// which then run on full warps: the queue goes on over the warp's cells (emptied after every 32 of
 // them, a circle test of 150 instructions ran for five pairs: connect of 512 events of pileup 50
-// 1.33 ms, now 1.18; of 111 of pileup 25 to 170, 2.75 and 2.58 ms). A passing pair counts one
-// neighbour of the candidate (cn_cur), sets
-// both used flags and goes to the pair list that k_connect_fill turns into neighbour lists; none
+// 1.33 ms, then 1.18; of 111 of pileup 1 to 200, 2.75 and 2.58 ms). Bound by instructions issued (67 % of
+// the issue slots): the test itself with its square root on every pair, and a search for each pair's
+// cell in place of the bit mask of the cells that start in a step, took 1.18 and 2.58 ms, now 0.94
+// and 2.16. Six blocks per SM (40 registers, two of them spilled) against five: 0.94 and 0.98 ms.
+// A passing pair counts one neighbour of the candidate (cn_cur), sets both used flags and goes to the pair list that k_connect_fill turns into neighbour lists; none
 // of these depends on the evaluation order.
 constexpr int kConnWarps = 8;
 constexpr int kConnQueue = 64;
 
 template <bool kQ>
-__global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
+__global__ void __launch_bounds__(256, 6) k_connect_test(Dev d, WorkQueue q) {
   pdl_sync(d);
-  __shared__ float4 s_rz[kConnWarps][32];  // inner r (negative: barrel), z and outer r, z of each cell
-  __shared__ uint32_t s_first[kConnWarps][32];  // list position of the cell's pair 0, were the cells' pairs one range
-  __shared__ uint32_t s_ex[kConnWarps][32];
+  // of the cells with candidates: inner r (negative: barrel), z and outer r, z; the cell; the list
+  // position of pair 0, were all cells' candidates one list
+  __shared__ float4 s_rz[kConnWarps][32];
+  __shared__ uint2 s_cell[kConnWarps][32];
   __shared__ uint2 s_queue[kConnWarps][kConnQueue];  // pair: cell, list position of the candidate
   for_each_vblock<kQ>(q, [&](int e, uint32_t bx, uint32_t nbx) {
   const EvInfo& E = d.ev[e];
@@ -827,11 +842,14 @@ __global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
       c = v.x;
       o = d.ohc_list[v.y];
       const float region = signbit(d.ohc_rec[v.y].x) ? kDcaInner : kDcaOuter;
+      const uint32_t ih = d.cell_inner[c];
       const float4 h1 = hxyzr[d.cell_inner[o]];  // the candidate's inner hit
-      const float4 hi = hxyzr[d.cell_inner[c]], ho = hxyzr[d.cell_outer[c]];
-      const CircleEq eq(h1.x, h1.y, hi.x, hi.y, ho.x, ho.y);
-      if (eq.c > kHardCurv) cut = false;
-      else cut = fabsf(eq.dca0()) < __fmul_rn(region, fabsf(eq.c));
+      const float4 hi = hxyzr[ih], ho = hxyzr[d.cell_outer[c]];
+      if (are_aligned(h1.w, h1.z, hi.w, hi.z, ho.w, ho.z, ptmin_f(), d.detind[hb + ih] < 1184 ? kThetaBarrel : kThetaForward)) {
+        const CircleEq eq(h1.x, h1.y, hi.x, hi.y, ho.x, ho.y);
+        if (eq.c > kHardCurv) cut = false;
+        else cut = fabsf(eq.dca0()) < __fmul_rn(region, fabsf(eq.c));
+      }
     }
     const uint32_t bal = __ballot_sync(0xffffffffu, cut);
     if (bal) {
@@ -854,37 +872,40 @@ __global__ void __launch_bounds__(256) k_connect_test(Dev d, WorkQueue q) {
   for (uint32_t k0 = bx * blockDim.x + 32u * w; k0 < E.n_cells; k0 += nbx * blockDim.x) {
     const uint32_t k = k0 + lane;
     const uint64_t c = cb + k;
-    uint32_t n = 0, lo = 0;
+    uint32_t n = 0, lo = 0, ih = 0;
     if (k < E.n_cells) {
-      const uint32_t ih = d.cell_inner[c];
+      ih = d.cell_inner[c];
       lo = d.ohc_cnt[hb + ih];
       n = d.ohc_cnt[hb + ih + 1] - lo;
       if (n > uint32_t(kMaxCellsPerHit)) n = kMaxCellsPerHit;
-      if (n > 0) {  // geometry only for cells with candidates
-        const uint32_t oh = d.cell_outer[c];
-        const float4 hi = hxyzr[ih], ho = hxyzr[oh];
-        s_rz[w][lane] = make_float4(d.detind[hb + ih] < 1184 ? -hi.w : hi.w, hi.z, ho.w, ho.z);
-      }
     }
-    const uint32_t inc = warp_incl_scan(n);
-    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-    s_ex[w][lane] = inc - n;
-    s_first[w][lane] = lo - (inc - n);
+    const uint32_t ex = warp_incl_scan(n) - n;
+    const uint32_t total = __shfl_sync(0xffffffffu, ex + n, 31);
+    const uint32_t busy = __ballot_sync(0xffffffffu, n > 0);
+    if (n > 0) {  // geometry only for cells with candidates
+      const uint32_t oh = d.cell_outer[c], a = __popc(busy & lt);
+      const float4 hi = hxyzr[ih], ho = hxyzr[oh];
+      s_rz[w][a] = make_float4(d.detind[hb + ih] < 1184 ? -hi.w : hi.w, hi.z, ho.w, ho.z);
+      s_cell[w][a] = make_uint2(uint32_t(c), lo - ex);
+    }
     __syncwarp();
-    uint32_t a = 0;  // owner of this lane's pair, non-decreasing over the steps
+    const uint32_t start = n > 0 ? ex : 0xffffffffu;
+    int cur = -1;  // owner of the pair before the step
     for (uint32_t x0 = 0; x0 < total; x0 += 32) {
-      const uint32_t x = x0 + lane;
+      const uint32_t starts = __reduce_or_sync(0xffffffffu, start - x0 < 32u ? 1u << (start - x0) : 0u);
+      const uint32_t a = uint32_t(cur + int(__popc(starts & ((lt << 1) | 1u))));
+      cur += int(__popc(starts));
       bool al = false;
-      uint32_t p = 0;
-      if (x < total) {
-        while (a < 31 && s_ex[w][a + 1] <= x) ++a;
-        p = s_first[w][a] + x;
-        const float2 rec = d.ohc_rec[p];  // the candidate's inner hit: r (sign: inner barrel), z
+      uint2 pair = make_uint2(0, 0);
+      if (x0 + lane < total) {
+        pair = s_cell[w][a];
+        pair.y += x0 + lane;
+        const float2 rec = d.ohc_rec[pair.y];  // the candidate's inner hit: r (sign: inner barrel), z
         const float4 rz = s_rz[w][a];
-        al = are_aligned(fabsf(rec.x), rec.y, fabsf(rz.x), rz.y, rz.z, rz.w, ptmin_f(), signbit(rz.x) ? kThetaBarrel : kThetaForward);
+        al = maybe_aligned(fabsf(rec.x), rec.y, fabsf(rz.x), rz.y, rz.z, rz.w, signbit(rz.x));
       }
       const uint32_t bal = __ballot_sync(0xffffffffu, al);
-      if (al) s_queue[w][qn + __popc(bal & lt)] = make_uint2(uint32_t(cb + k0 + a), p);
+      if (al) s_queue[w][qn + __popc(bal & lt)] = pair;
       qn += __popc(bal);
       __syncwarp();
       if (qn >= 32) {
