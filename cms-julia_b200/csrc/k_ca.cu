@@ -238,12 +238,12 @@ __device__ __forceinline__ bool doublet_pass_b(int pid, float me_z, float me_r, 
   return true;
 }
 
-// doublet_pass_a without the dphi cut, for candidates that pass it by construction
-__device__ __forceinline__ bool doublet_pass_z(int pid, float me_z, float me_r, const HitRec& hr) {
-  if (hr.det() > 2000) return false;
-  const float dr = __fsub_rn(hr.r, me_r);
-  return !(dr > c_max_rf[pid] || dr < 0 ||
-           fabsf(__fsub_rn(__fmul_rn(me_z, hr.r), __fmul_rn(me_r, hr.z))) > __fmul_rn(12.f, dr));
+// doublet_pass_a without the dphi cut, for candidates that pass it by construction, and without the
+// module's, which the few that pass here take afterwards
+__device__ __forceinline__ bool doublet_pass_z(float max_r, float me_z, float me_r, float r, float z) {
+  const float dr = __fsub_rn(r, me_r);
+  return !(dr > max_r || dr < 0 ||
+           fabsf(__fsub_rn(__fmul_rn(me_z, r), __fmul_rn(me_r, z))) > __fmul_rn(12.f, dr));
 }
 
 // Reference order of a passing outer hit among its item's cells: the window's bins in order
@@ -304,7 +304,9 @@ constexpr int kGroupCells = 768;  // outer hits one 32-item group stages in shar
 // doublets are complete go to the pool and the current item's move to the front (groups above 768
 // doublets are common from pileup 100 on; the fill pass, which searches again what the count could not
 // keep, item by item, took 1.48 ms for 111 uneven events). An item that fills the staging alone, or a
-// full pool, records kNoPool and the fill pass searches again.
+// full pool, records kNoPool and the fill pass searches again. Bound by instructions issued (68 % of the
+// issue slots at 512 events of pileup 50); with the first cut's constants staged per item and the
+// module cut left to the survivors 1.37 ms, before 1.44.
 constexpr int kDblQueue = 64;
 
 template <bool kQ>
@@ -312,7 +314,9 @@ __global__ void __launch_bounds__(256, 5) k_doublets_count(Dev d, const uint32_t
   pdl_sync(d);
   __shared__ uint32_t s_cum[kNPairs];
   __shared__ uint32_t s_hls[11];
-  __shared__ uint4 s_rng[8][32];   // per compacted item: lo0, n0, lo1, first candidate
+  // per compacted item: its candidate t is hit record t + x for t < y, t + z from there on; w the pair's
+  // largest dr (float bits)
+  __shared__ uint4 s_rng[8][32];
   __shared__ uint4 s_geo[8][32];   // per compacted item: z, r (float bits), iphi | cut << 16, pid | ysize << 16
   __shared__ uint16_t s_beg[8][32], s_end[8][32];
   __shared__ uint32_t s_over[8][32];
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(256, 5) k_doublets_count(Dev d, const uint32_t
     const uint32_t ctex = warp_incl_scan(nc) - nc;
     const uint32_t total = __shfl_sync(0xffffffffu, ctex + nc, 31);
     if (nc > 0) {
-      s_rng[w][ci] = make_uint4(h.lo0, h.n0, h.lo1, ctex);
+      s_rng[w][ci] = make_uint4(h.lo0 - ctex, ctex + h.n0, h.lo1 - h.n0 - ctex, __float_as_uint(c_max_rf[h.pid]));
       s_geo[w][ci] = make_uint4(__float_as_uint(h.z), __float_as_uint(h.r),
                                 uint32_t(uint16_t(h.iphi)) | (uint32_t(uint16_t(h.cut)) << 16),
                                 uint32_t(h.pid) | (uint32_t(uint16_t(h.ysize)) << 16));
@@ -362,8 +366,8 @@ __global__ void __launch_bounds__(256, 5) k_doublets_count(Dev d, const uint32_t
         o = v >> kHitIdBits;
         const uint4 g = s_geo[w][o];
         const HitRec hr = hrec[v & (kMaxHitsPerEvent - 1u)];
-        pass = doublet_pass_b(int(g.w & 0xffu), __uint_as_float(g.x), __uint_as_float(g.y), int16_t(g.z & 0xffffu),
-                              int16_t(g.w >> 16), hr);
+        pass = hr.det() <= 2000 && doublet_pass_b(int(g.w & 0xffu), __uint_as_float(g.x), __uint_as_float(g.y),
+                                                  int16_t(g.z & 0xffffu), int16_t(g.w >> 16), hr);
         oi = (o << kOwnerShift) | cell_order_key(int16_t(g.z & 0xffffu), int16_t(g.z >> 16), hr);
       }
       const uint32_t bal = __ballot_sync(0xffffffffu, pass);
@@ -375,23 +379,24 @@ __global__ void __launch_bounds__(256, 5) k_doublets_count(Dev d, const uint32_t
       nout += __popc(bal);
       qhead += mm;
     };
+    const uint32_t start = nc > 0 ? ctex : 0xffffffffu;
     int cur = -1;       // compacted item owning the candidate before the step
     uint32_t done = 0;  // compacted items whose doublets have gone to the pool
     for (uint32_t t0 = 0;; t0 += 32) {
       const bool last = t0 >= total;
       if (!last) {
-        const uint32_t starts = __reduce_or_sync(0xffffffffu, (nc > 0 && ctex >= t0 && ctex < t0 + 32u) ? (1u << (ctex - t0)) : 0u);
+        const uint32_t starts = __reduce_or_sync(0xffffffffu, start - t0 < 32u ? 1u << (start - t0) : 0u);
         const uint32_t t = t0 + lane;
-        const uint32_t o = uint32_t(cur + int(__popc(starts & ((2u << lane) - 1u))));
+        const uint32_t o = uint32_t(cur + int(__popc(starts & ((lt << 1) | 1u))));
         cur += int(__popc(starts));
         bool pass = false;
         uint32_t p = 0;
         if (t < total) {
           const uint4 rg = s_rng[w][o];
           const uint4 g = s_geo[w][o];
-          const uint32_t k = t - rg.w;
-          p = k < rg.y ? rg.x + k : rg.z + (k - rg.y);
-          pass = doublet_pass_z(int(g.w & 0xffu), __uint_as_float(g.x), __uint_as_float(g.y), hrec[p]);
+          p = t + (t < rg.y ? rg.x : rg.z);
+          const float2 zr = *reinterpret_cast<const float2*>(hrec + p);  // z, r
+          pass = doublet_pass_z(__uint_as_float(rg.w), __uint_as_float(g.x), __uint_as_float(g.y), zr.y, zr.x);
         }
         const uint32_t bal = __ballot_sync(0xffffffffu, pass);
         if (pass) s_q[w][(qtail + __popc(bal & lt)) % kDblQueue] = (o << kHitIdBits) | p;
