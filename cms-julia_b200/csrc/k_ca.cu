@@ -640,6 +640,15 @@ __device__ __forceinline__ bool sort_short(uint32_t* a, uint32_t n) {
   return false;
 }
 
+__device__ __forceinline__ void insertion_sort(uint32_t* a, uint32_t n) {
+  for (uint32_t p = 1; p < n; ++p) {
+    const uint32_t v = a[p];
+    uint32_t q = p;
+    while (q > 0 && a[q - 1] > v) { a[q] = a[q - 1]; --q; }
+    a[q] = v;
+  }
+}
+
 // sort a short list in place (ascending; entries are ids below 0xffffffff): one load and
 // one store per entry through a register network up to 32 entries, insertion sort above
 __device__ __forceinline__ void sort_list(uint32_t* a, uint32_t n) {
@@ -648,12 +657,7 @@ __device__ __forceinline__ void sort_list(uint32_t* a, uint32_t n) {
   if (n <= 8) { sort_regs<8>(a, n); return; }
   if (n <= 16) { sort_regs<16>(a, n); return; }
   if (n <= 32) { sort_regs<32>(a, n); return; }
-  for (uint32_t p = 1; p < n; ++p) {
-    const uint32_t v = a[p];
-    uint32_t q = p;
-    while (q > 0 && a[q - 1] > v) { a[q] = a[q - 1]; --q; }
-    a[q] = v;
-  }
+  insertion_sort(a, n);
 }
 
 // lists above the short-sort limit, sorted afterwards by k_sort_long (a list of n entries
@@ -676,50 +680,79 @@ __global__ void __launch_bounds__(256) k_sort_long(Dev d, int kind, uint32_t* li
   }
 }
 
-// Sorts a list of 33..128 entries with a whole warp: each lane holds four entries and counts, for
-// each, the entries below it as they go round by shuffles (entries differ).
-__device__ __forceinline__ void sort_list_warp(uint32_t* a, uint32_t n) {
-  const unsigned lane = threadIdx.x & 31u;
-  uint32_t v[4], r[4] = {0, 0, 0, 0};
-#pragma unroll
-  for (int u = 0; u < 4; ++u) v[u] = lane + 32u * u < n ? a[lane + 32u * u] : 0xffffffffu;
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    for (uint32_t k = 0; k < 32 && 32u * q + k < n; ++k) {
-      const uint32_t x = __shfl_sync(0xffffffffu, v[q], int(k));
-#pragma unroll
-      for (int u = 0; u < 4; ++u) r[u] += x < v[u];
-    }
-  __syncwarp();
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-    if (lane + 32u * u < n) a[r[u]] = v[u];
-}
+// Sorts the outer-hit lists (ascending) and gathers connect's candidate of each entry. A warp takes
+// `hits` consecutive hits, fewer than 32 in a small batch. Their lists lie end to end: as many whole lists
+// as fit are staged, a lane takes an entry, and its place is the number of entries of its list that are
+// below it (entries differ). Reads and writes stay on the region's lines; a lane per list, with register
+// networks by length up to 32 and a warp per longer one, loaded and stored a line per lane and entry (fill,
+// sort and gather, the latter in a kernel of its own: 512 events of pileup 50 693 us, 111 of pileup 1 to 200
+// 925; now 620 and 615). 512 staged entries per warp: with 1024 the shared memory leaves no L1 (706 and
+// 685 us), with 256 more groups are cut (628 and 636). Lists above the staging (none at pileup 200, whose longest has 125 entries) are sorted by one lane.
+constexpr int kRankBuf = 512;
 
-// A thread per hit sorts the lists of up to 32 entries in registers; the warp then takes its hits'
-// longer ones together (an insertion sort by one thread, kept above 128 entries, made the kernel
-// 248 us for one event of pileup 170). A warp takes `hits` consecutive hits, fewer than 32 in a small
-// batch: the long lists sit next to each other, and one warp sorts them one after the other.
-__global__ void k_sort_hit_lists(Dev d, uint32_t hits) {
+__global__ void __launch_bounds__(256) k_sort_hit_lists(Dev d, uint32_t hits) {
   pdl_sync(d);
+  __shared__ uint32_t s_list[8][kRankBuf];
+  __shared__ uint32_t s_beg[8][33];  // first staged entry of each staged list, and one past the last
   const int e = blockIdx.y;
   const EvInfo& E = d.ev[e];
   const uint32_t hb = E.hit_base, nh = E.n_hits;
-  const unsigned lane = threadIdx.x & 31u;
+  const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
   const uint32_t warps = gridDim.x * (blockDim.x / 32);
-  for (uint32_t k0 = (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32) * hits; k0 < nh; k0 += warps * hits) {
+  uint32_t* sl = s_list[w];
+  uint32_t* sb = s_beg[w];
+  auto put = [&](uint32_t pos, uint32_t cell, uint32_t ih) {
+    const float4 h = d.hit_xyzr[hb + ih];
+    const int16_t det = d.detind[hb + ih];
+    d.ohc_list[pos] = cell;
+    d.ohc_rec[pos] = make_float2(det < 96 ? -h.w : h.w, h.z);
+  };
+  for (uint32_t k0 = (blockIdx.x * (blockDim.x / 32) + w) * hits; k0 < nh; k0 += warps * hits) {
     const uint32_t k = k0 + lane;
-    uint32_t lo = 0, n = 0;
+    const uint32_t first = d.ohc_cnt[hb + k0];
+    uint32_t ex = 0, n = 0;  // first entry of the lane's list from `first` on, entries
     if (lane < hits && k < nh) {
-      lo = d.ohc_cnt[hb + k];
+      const uint32_t lo = d.ohc_cnt[hb + k];
       n = d.ohc_cnt[hb + k + 1] - lo;
+      ex = lo - first;
       if (n > uint32_t(kMaxCellsPerHit)) atomic_or_warn(&d.ev[e], kWarnLists);
     }
-    const bool together = n > 32 && n <= 128;
-    if (!together) sort_list(d.ohc_list + lo, n);
-    for (uint32_t m = __ballot_sync(0xffffffffu, together); m; m &= m - 1) {
-      const int src = __ffs(m) - 1;
-      sort_list_warp(d.ohc_list + __shfl_sync(0xffffffffu, lo, src), __shfl_sync(0xffffffffu, n, src));
+    const uint32_t total = __reduce_max_sync(0xffffffffu, n > 0 ? ex + n : 0u);
+    for (uint32_t c0 = 0; c0 < total;) {
+      const bool in = n > 0 && ex >= c0 && ex + n <= c0 + uint32_t(kRankBuf);
+      const uint32_t m = __ballot_sync(0xffffffffu, in);
+      if (m == 0) {  // the next list exceeds the staging
+        const bool mine = n > 0 && ex == c0;
+        if (mine) {
+          insertion_sort(d.ohc_list + first + ex, n);
+          for (uint32_t p = first + ex; p < first + ex + n; ++p) put(p, d.ohc_list[p], d.cell_inner[d.ohc_list[p]]);
+        }
+        c0 += __reduce_max_sync(0xffffffffu, mine ? n : 0u);
+        continue;
+      }
+      const uint32_t len = __reduce_max_sync(0xffffffffu, in ? ex + n - c0 : 0u);
+      if (in) sb[__popc(m & lt)] = ex - c0;
+      if (lane == 0) sb[__popc(m)] = len;
+      for (uint32_t x = lane; x < len; x += 32) sl[x] = d.ohc_list[first + c0 + x];
+      __syncwarp();
+      const uint32_t start = in ? ex - c0 : 0xffffffffu;
+      int cur = -1;
+      for (uint32_t x0 = 0; x0 < len; x0 += 32) {
+        const uint32_t starts = __reduce_or_sync(0xffffffffu, start - x0 < 32u ? 1u << (start - x0) : 0u);
+        const uint32_t a = uint32_t(cur + int(__popc(starts & ((lt << 1) | 1u))));
+        cur += int(__popc(starts));
+        if (x0 + lane < len) {
+          const uint32_t v = sl[x0 + lane];
+          const uint32_t ih = d.cell_inner[v];
+          const uint32_t b0 = sb[a], b1 = sb[a + 1];
+          uint32_t rank = 0;
+#pragma unroll 4
+          for (uint32_t y = b0; y < b1; ++y) rank += sl[y] < v;
+          put(first + c0 + b0 + rank, v, ih);
+        }
+      }
+      __syncwarp();
+      c0 += len;
     }
   }
 }
@@ -776,35 +809,6 @@ __device__ __forceinline__ bool maybe_aligned(float r1, float z1, float ri, floa
   const float dz = __fsub_rn(z1, zo), u2 = __fmul_rn(u, u);
   const float lim = __fmaf_rn(__fmul_rn(u2, __fmaf_rn(dz, dz, u2)), barrel ? kBarrel : kForward, 1e-30f);
   return !(__fmul_rn(t, t) > lim);
-}
-
-// connect's candidates of each outer-hit list entry, gathered once per entry
-__global__ void __launch_bounds__(256) k_ohc_records(Dev d) {
-  pdl_sync(d);
-  const int e = blockIdx.y;
-  const EvInfo& E = d.ev[e];
-  const uint32_t hb = E.hit_base;
-  const uint32_t lo = d.ohc_cnt[hb], hi = d.ohc_cnt[uint64_t(hb) + E.n_hits];
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t p0 = lo + blockIdx.x * blockDim.x + threadIdx.x; p0 < hi; p0 += kOhcUnroll * stride) {
-    uint32_t ih[kOhcUnroll];
-#pragma unroll
-    for (int u = 0; u < kOhcUnroll; ++u) ih[u] = p0 + u * stride < hi ? d.ohc_list[p0 + u * stride] : 0xffffffffu;
-#pragma unroll
-    for (int u = 0; u < kOhcUnroll; ++u)
-      if (ih[u] != 0xffffffffu) ih[u] = d.cell_inner[ih[u]];
-    float4 h[kOhcUnroll];
-    int16_t det[kOhcUnroll];
-#pragma unroll
-    for (int u = 0; u < kOhcUnroll; ++u)
-      if (p0 + u * stride < hi) {
-        h[u] = d.hit_xyzr[hb + ih[u]];
-        det[u] = d.detind[hb + ih[u]];
-      }
-#pragma unroll
-    for (int u = 0; u < kOhcUnroll; ++u)
-      if (p0 + u * stride < hi) d.ohc_rec[p0 + u * stride] = make_float2(det[u] < 96 ? -h[u].w : h[u].w, h[u].z);
-  }
 }
 
 // Connection test of every cell with the cells ending on its inner hit (the outer-hit list,
@@ -1483,7 +1487,6 @@ void launch_ca(const Dev& d, const Launch& L) {
   L.run(k_ohc_fill, g(kTuneHitLists), 256, 0, d);
   if (d.E <= kPdlEvents) L.run(k_sort_hit_lists, dim3(event_blocks(d.E, 148 * 8, 1024), d.E), 256, 0, d, 4u);
   else L.run(k_sort_hit_lists, g(kTuneHitLists), 256, 0, d, 32u);
-  L.run(k_ohc_records, g(kTuneHitLists), 256, 0, d);
   L.mark("outer_hit_lists");
   // connection and neighbour lists
   if (L.queue_of(kTuneConnect)) {
