@@ -31,7 +31,6 @@ namespace {
 constexpr int kNPix = 4096;  // >= 4001, the largest range find_clus processes
 constexpr int kNBins = 418;
 constexpr int kWarpPix = kWarpModulePix;  // digis per module handled by one warp
-constexpr int kWarpSlots = kWarpPix / 32;
 constexpr int kWarpsPerBlock = 8;
 
 __device__ __forceinline__ int cc_find(volatile int32_t* lab, int x) {
@@ -98,194 +97,64 @@ __device__ __forceinline__ void write_module_record(const Dev& d, int e, uint32_
   if (warn) atomic_or_warn(&d.ev[e], warn);
 }
 
+// x (16 bits) | column << 16 of a digi, 0xffffffff when not clustered. A column past the 418-bin
+// histogram makes the reference's histogram assert fail; such a digi is flagged and kept out of the
+// clustering.
+struct DigiXY {
+  uint32_t xy, warn;
+};
+
+__device__ __forceinline__ DigiXY load_digi(const Dev& d, uint64_t g) {
+  const int16_t id = d.mid[g];
+  const uint32_t x = uint16_t(d.xx[g]), yb = uint32_t(uint16_t(d.yy[g])) & 511u;
+  const bool in_hist = yb + 2u <= uint32_t(kNBins), there = id != int16_t(kInvId);
+  return DigiXY{there && in_hist ? x | (yb << 16) : 0xffffffffu, there && !in_hist ? uint32_t(kWarnPixels) : 0u};
+}
+
 // ------------------------------------------------------------ warp per module
-constexpr int kHistWords = 448;  // >= 420 column bins, 14 per lane
-
-template <int kSlots>
-struct WarpSmem {
-  int32_t lab[32 * kSlots];
-  int32_t charge[32 * kSlots];
-  uint16_t cid[32 * kSlots];   // cluster number (1-based) of each root
-  uint16_t newc[32 * kSlots];  // cluster number after the charge cut
-};
-
-// column histogram of one module for the larger warp-clustered modules
-struct WarpHist {
-  uint32_t start[kHistWords];  // first sorted position of each column bin
-  uint32_t cur[kHistWords];
-  uint32_t xy[kWarpPix];       // x | column bin << 16 of each digi
-  uint8_t sorted[kWarpPix];    // digi indices ordered by column bin
-};
-
-// One module of at most 32 * kSlots digis, clustered by one warp with its digis in
-// registers (kSlots per lane; shared-memory store for up to 32 * kStore digis).
-template <int kSlots, int kStore>
-__device__ __forceinline__ void cluster_module_warp(const Dev& d, int e, uint32_t m, const ModRange& r,
-                                                    WarpSmem<kStore>& S, WarpHist* H) {
-  static_assert(kSlots <= kStore, "slots beyond the shared-memory store");
+// Cluster numbers and charge cut of one module whose labels are final (lab[k] the smallest digi of k's
+// cluster, negative for digis outside the clustering), by one warp; charge holds as many entries as
+// digis, adc(k) is digi k's charge.
+template <class F>
+__device__ __forceinline__ void finish_module_warp(const Dev& d, int e, uint32_t m, const ModRange& r, int crun, uint32_t warn,
+                                                   const int32_t* lab, int32_t* charge, uint16_t* cid, uint16_t* newc, F&& adc) {
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt = (1u << lane) - 1u;
   const int n = r.n;
-  uint32_t xy[kSlots];  // x (16 bits) | column bin << 16; 0xffffffff when not clustered
-  int32_t q[kSlots];
-  uint32_t warn = 0;
-  int crun = n;
-#pragma unroll
-  for (int j = 0; j < kSlots; ++j) {
-    const int k = int(lane) + 32 * j;
-    xy[j] = 0xffffffffu;
-    q[j] = 0;
-    if (k < n) {
-      const uint64_t g = r.g0 + k;
-      const int16_t id = d.mid[g];
-      const int16_t x = d.xx[g], y = d.yy[g];
-      q[j] = d.adc[g];
-      const uint32_t yb = uint32_t(uint16_t(y)) & 511u;
-      // a column past the 418-bin histogram makes the reference's histogram assert
-      // fail; such a digi is flagged and kept out of the clustering
-      const bool in_hist = yb + 2u <= uint32_t(kNBins);
-      if (id != int16_t(kInvId) && !in_hist) warn |= kWarnPixels;
-      const bool valid = id != int16_t(kInvId) && in_hist;
-      if (valid) xy[j] = uint32_t(uint16_t(x)) | (yb << 16);
-      else crun = crun < k ? crun : k;
-      S.lab[k] = valid ? k : -1;
-    }
-  }
-  crun = int(__reduce_min_sync(0xffffffffu, uint32_t(crun)));
-  warn = __reduce_or_sync(0xffffffffu, warn);
-  __syncwarp();
-  // histogram path: neighbour pairs (digi indices < 256) listed in the charge / cluster-number
-  // store, which is free until the labels are final; pairs past its capacity are joined at once
-  uint16_t* pairs = reinterpret_cast<uint16_t*>(S.charge);
-  constexpr uint32_t kPairCap = 32u * kStore * (sizeof(int32_t) + 2 * sizeof(uint16_t)) / sizeof(uint16_t);
-  uint32_t np = 0;
-  if (H) {
-    // neighbour pairs through a column histogram (count, warp scan, scatter); each digi
-    // then looks at its own and the next column only, as the CTA path does
-    for (int w = int(lane); w < kHistWords; w += 32) H->start[w] = 0;
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < kSlots; ++j) {
-      const int k = int(lane) + 32 * j;
-      if (k < n) H->xy[k] = xy[j];
-      if (xy[j] != 0xffffffffu) atomicAdd(&H->start[(xy[j] >> 16) + 1u], 1u);
-    }
-    __syncwarp();
-    constexpr int kPer = kHistWords / 32;
-    uint32_t cnt[kPer], tot = 0;
-#pragma unroll
-    for (int w = 0; w < kPer; ++w) { cnt[w] = H->start[lane * kPer + w]; tot += cnt[w]; }
-    uint32_t run = warp_incl_scan(tot) - tot;
-#pragma unroll
-    for (int w = 0; w < kPer; ++w) {
-      H->start[lane * kPer + w] = run;
-      H->cur[lane * kPer + w] = run;
-      run += cnt[w];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < kSlots; ++j)
-      if (xy[j] != 0xffffffffu) H->sorted[atomicAdd(&H->cur[(xy[j] >> 16) + 1u], 1u)] = uint8_t(lane + 32 * j);
-    __syncwarp();
-    uint32_t& npairs = H->cur[0];  // the scatter cursors are free again
-    if (lane == 0) npairs = 0;
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < kSlots; ++j) {
-      const int k = int(lane) + 32 * j;
-      if (k >= n || xy[j] == 0xffffffffu) continue;
-      const int xk = int(int16_t(xy[j] & 0xffffu));
-      const uint32_t bn = (xy[j] >> 16) + 1u;
-      const uint32_t p1 = H->start[bn + 2u];
-      for (uint32_t pp = H->start[bn]; pp < p1; ++pp) {
-        const int mm = H->sorted[pp];
-        if (mm == k) continue;
-        const uint32_t vm = H->xy[mm];
-        if ((vm >> 16) == (xy[j] >> 16) && mm < k) continue;  // each same-column pair once
-        const int dx = int(int16_t(vm & 0xffffu)) - xk;
-        if (dx > 1 || dx < -1) continue;
-        const uint32_t slot = atomicAdd(&npairs, 1u);
-        if (slot < kPairCap) pairs[slot] = uint16_t(k | (mm << 8));
-        else cc_union(S.lab, k, mm);
-      }
-    }
-    __syncwarp();
-    np = npairs < kPairCap ? npairs : kPairCap;
-  } else {
-    // neighbour pairs (|dx| <= 1, |dcolumn| <= 1) by broadcasting every digi, each pair
-    // once from its smaller index
-#pragma unroll
-    for (int jb = 0; jb < kSlots; ++jb) {
-      const int base = 32 * jb;
-      if (base >= n) break;
-      const uint32_t v = xy[jb];
-      const int tmax = n - base < 32 ? n - base : 32;
-      for (int t = 0; t < tmax; ++t) {
-        const uint32_t vm = __shfl_sync(0xffffffffu, v, t);
-        if (vm == 0xffffffffu) continue;
-        const int mm = base + t;
-        const int xm = int(int16_t(vm & 0xffffu)), ym = int(vm >> 16);
-#pragma unroll
-        for (int j = 0; j <= jb; ++j) {
-          const int k = int(lane) + 32 * j;
-          if (k >= mm || xy[j] == 0xffffffffu) continue;
-          const int dx = int(int16_t(xy[j] & 0xffffu)) - xm;
-          const int dy = int(xy[j] >> 16) - ym;
-          if (dx <= 1 && dx >= -1 && dy <= 1 && dy >= -1) cc_union(S.lab, k, mm);
-        }
-      }
-    }
-  }
-  // the neighbour pairs, joined 32 at a time (any order gives the same components, each
-  // rooted at its smallest digi index)
-  for (uint32_t p = lane; p < np; p += 32) cc_union(S.lab, pairs[p] & 0xff, pairs[p] >> 8);
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < kSlots; ++j) {
-    const int k = int(lane) + 32 * j;
-    if (k < n && xy[j] != 0xffffffffu) S.lab[k] = cc_find(S.lab, k);
-  }
-  __syncwarp();
   // number the roots in index order
   uint32_t nclus = 0;
-#pragma unroll
-  for (int j = 0; j < kSlots; ++j) {
-    const int k = int(lane) + 32 * j;
-    if (32 * j >= n) break;
-    const bool root = k < n && S.lab[k] == k;
+  for (int k0 = 0; k0 < n; k0 += 32) {
+    const int k = k0 + int(lane);
+    const bool root = k < n && lab[k] == k;
     const unsigned b = __ballot_sync(0xffffffffu, root);
-    if (root) S.cid[k] = uint16_t(nclus + __popc(b & lt) + 1);
+    if (root) {
+      const uint32_t c = nclus + __popc(b & lt);
+      cid[k] = uint16_t(c + 1);
+      charge[c] = 0;
+    }
     nclus += __popc(b);
   }
-  for (uint32_t c = lane; c < nclus; c += 32) S.charge[c] = 0;
   __syncwarp();
   // cluster_charge_cut: charge sums stop at the first invalid digi
-#pragma unroll
-  for (int j = 0; j < kSlots; ++j) {
-    const int k = int(lane) + 32 * j;
-    if (k < crun) atomicAdd(&S.charge[S.cid[S.lab[k]] - 1], q[j]);
-  }
+  for (int k = int(lane); k < crun; k += 32) atomicAdd(&charge[cid[lab[k]] - 1], adc(k));
   __syncwarp();
   const int32_t cut = r.this_id < 96 ? 2000 : 4000;
   uint32_t last_new = 0;
   for (uint32_t base = 0; base < nclus; base += 32) {
     const uint32_t c = base + lane;
-    const bool ok = c < nclus && S.charge[c] > cut;
+    const bool ok = c < nclus && charge[c] > cut;
     const unsigned b = __ballot_sync(0xffffffffu, ok);
-    if (c < nclus) S.newc[c] = ok ? uint16_t(last_new + __popc(b & lt) + 1) : uint16_t(kInvId);
+    if (c < nclus) newc[c] = ok ? uint16_t(last_new + __popc(b & lt) + 1) : uint16_t(kInvId);
     last_new += __popc(b);
   }
   __syncwarp();
   const bool changed = d.apply_charge_cut && !d.ev[e].repeated_ids && nclus > 0 && last_new != nclus;
-#pragma unroll
-  for (int j = 0; j < kSlots; ++j) {
-    const int k = int(lane) + 32 * j;
-    if (k >= n) continue;
+  for (int k = int(lane); k < n; k += 32) {
     const uint64_t g = r.g0 + k;
-    if (xy[j] == 0xffffffffu) { d.clus[g] = -9999; continue; }
-    const uint32_t cl = S.cid[S.lab[k]];
+    if (lab[k] < 0) { d.clus[g] = -9999; continue; }
+    const uint32_t cl = cid[lab[k]];
     if (changed) {
-      const uint16_t nc = S.newc[cl - 1];
+      const uint16_t nc = newc[cl - 1];
       d.clus[g] = int32_t(nc);
       if (nc == kInvId) d.mid[g] = int16_t(kInvId);
     } else {
@@ -294,6 +163,147 @@ __device__ __forceinline__ void cluster_module_warp(const Dev& d, int e, uint32_
   }
   if (lane == 0) write_module_record(d, e, m, r.this_id, changed ? last_new : nclus, warn);
   __syncwarp();
+}
+
+struct SmallSmem {
+  int32_t lab[32], charge[32];
+  uint16_t cid[32], newc[32];  // cluster number (1-based) of each root, and after the charge cut
+};
+
+// One module of at most 32 digis: each lane holds a digi, and the neighbour pairs (|dx| <= 1,
+// |dcolumn| <= 1) come from broadcasting every digi, each pair once from its smaller index.
+__device__ __forceinline__ void cluster_module_small(const Dev& d, int e, uint32_t m, const ModRange& r, SmallSmem& S) {
+  const int k = int(threadIdx.x & 31u);
+  uint32_t xy = 0xffffffffu, warn = 0, crun = r.n;
+  int32_t q = 0;
+  if (k < r.n) {
+    const DigiXY v = load_digi(d, r.g0 + k);
+    q = d.adc[r.g0 + k];
+    xy = v.xy;
+    warn = v.warn;
+    if (xy == 0xffffffffu) crun = k;
+    S.lab[k] = xy != 0xffffffffu ? k : -1;
+  }
+  crun = __reduce_min_sync(0xffffffffu, crun);
+  warn = __reduce_or_sync(0xffffffffu, warn);
+  __syncwarp();
+  for (int mm = 0; mm < r.n; ++mm) {
+    const uint32_t vm = __shfl_sync(0xffffffffu, xy, mm);
+    if (vm == 0xffffffffu || k >= mm || xy == 0xffffffffu) continue;
+    const int dx = int(int16_t(xy & 0xffffu)) - int(int16_t(vm & 0xffffu));
+    const int dy = int(xy >> 16) - int(vm >> 16);
+    if (dx <= 1 && dx >= -1 && dy <= 1 && dy >= -1) cc_union(S.lab, k, mm);
+  }
+  __syncwarp();
+  if (xy != 0xffffffffu) S.lab[k] = cc_find(S.lab, k);
+  __syncwarp();
+  finish_module_warp(d, e, m, r, int(crun), warn, S.lab, S.charge, S.cid, S.newc, [&](int) { return q; });
+}
+
+constexpr int kHistWords = 224;  // two column bins per word, >= 420 bins; seven words per lane
+
+struct MidSmem {
+  int32_t lab[kWarpPix];
+  int32_t charge[kWarpPix];
+  uint16_t cid[kWarpPix];     // cluster number (1-based) of each root
+  uint16_t newc[kWarpPix];    // cluster number after the charge cut
+  uint32_t xy[kWarpPix];      // x | column << 16 of each digi; 0xffffffff when not clustered
+  uint32_t sorted[kWarpPix];  // the digis by column: x | digi << 16 | column parity << 24
+  uint32_t bins[kHistWords];  // counts of the columns' digis, then first sorted position, then one past the last
+  uint32_t npairs;
+  // entry of column bin b; add(b) returns it and adds one (at most 256: the halves do not carry)
+  __device__ uint32_t get(uint32_t b) const { return (bins[b >> 1] >> (16 * (b & 1))) & 0xffffu; }
+  __device__ uint32_t add(uint32_t b) {
+    return (atomicAdd(&bins[b >> 1], 1u << (16 * (b & 1))) >> (16 * (b & 1))) & 0xffffu;
+  }
+};
+
+// One module of at most kWarpPix digis: neighbour pairs through a column histogram (count, warp scan,
+// scatter); each digi then looks at its own and the next column only, as the CTA path does. The pairs
+// are listed in the charge / cluster-number store, which is free until the labels are final, and joined
+// 32 at a time; pairs past its capacity are joined at once.
+// Bound by latency: the loops run over the digis there are, with all state in shared memory. Unrolled over
+// the eight digis per lane of the largest module and held in registers they took 69 registers (seven
+// blocks per SM) and 832 us for 512 events of pileup 50, now 590 (nine blocks); instances for up to 64, 128
+// and 256 digis 950 us, their code does not fit the instruction cache together.
+__device__ __forceinline__ void cluster_module_mid(const Dev& d, int e, uint32_t m, const ModRange& r, MidSmem& S) {
+  const unsigned lane = threadIdx.x & 31u;
+  const int n = r.n;
+  uint32_t warn = 0, crun = n;
+  for (int w = int(lane); w < kHistWords; w += 32) S.bins[w] = 0;
+  if (lane == 0) S.npairs = 0;
+  __syncwarp();
+  for (int k0 = 0; k0 < n; k0 += 64) {
+    DigiXY v[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int k = k0 + int(lane) + 32 * u;
+      if (k < n) v[u] = load_digi(d, r.g0 + k);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int k = k0 + int(lane) + 32 * u;
+      if (k >= n) continue;
+      const bool valid = v[u].xy != 0xffffffffu;
+      warn |= v[u].warn;
+      S.xy[k] = v[u].xy;
+      S.lab[k] = valid ? k : -1;
+      if (valid) S.add((v[u].xy >> 16) + 1u);
+      else crun = min(crun, uint32_t(k));
+    }
+  }
+  crun = __reduce_min_sync(0xffffffffu, crun);
+  warn = __reduce_or_sync(0xffffffffu, warn);
+  __syncwarp();
+  constexpr int kPer = kHistWords / 32;
+  uint32_t cnt[kPer], tot = 0;
+#pragma unroll
+  for (int w = 0; w < kPer; ++w) {
+    cnt[w] = S.bins[lane * kPer + w];
+    tot += (cnt[w] & 0xffffu) + (cnt[w] >> 16);
+  }
+  uint32_t run = warp_incl_scan(tot) - tot;
+#pragma unroll
+  for (int w = 0; w < kPer; ++w) {
+    const uint32_t odd = run + (cnt[w] & 0xffffu);
+    S.bins[lane * kPer + w] = run | (odd << 16);
+    run = odd + (cnt[w] >> 16);
+  }
+  __syncwarp();
+  for (int k = int(lane); k < n; k += 32) {
+    const uint32_t v = S.xy[k];
+    if (v != 0xffffffffu) S.sorted[S.add((v >> 16) + 1u)] = (v & 0xffffu) | (uint32_t(k) << 16) | ((v & 0x10000u) << 8);
+  }
+  __syncwarp();
+  uint16_t* pairs = reinterpret_cast<uint16_t*>(S.charge);
+  constexpr uint32_t kPairCap = kWarpPix * (sizeof(int32_t) + 2 * sizeof(uint16_t)) / sizeof(uint16_t);
+  for (int k = int(lane); k < n; k += 32) {
+    const uint32_t v = S.xy[k];
+    if (v == 0xffffffffu) continue;
+    const int xk = int(int16_t(v & 0xffffu));
+    const uint32_t bn = (v >> 16) + 1u;
+    const uint32_t p1 = S.get(bn + 1u);  // a bin's entry is now where the next one begins
+    for (uint32_t pp = S.get(bn - 1u); pp < p1; ++pp) {
+      const uint32_t vm = S.sorted[pp];
+      const int mm = int((vm >> 16) & 0xffu);
+      if (((vm >> 8) & 0x10000u) == (v & 0x10000u) && mm <= k) continue;  // each same-column pair once
+      const int dx = int(int16_t(vm & 0xffffu)) - xk;
+      if (dx > 1 || dx < -1) continue;
+      const uint32_t slot = atomicAdd(&S.npairs, 1u);
+      if (slot < kPairCap) pairs[slot] = uint16_t(k | (mm << 8));
+      else cc_union(S.lab, k, mm);
+    }
+  }
+  __syncwarp();
+  // any order gives the same components, each rooted at its smallest digi index
+  const uint32_t np = min(S.npairs, kPairCap);
+  for (uint32_t p = lane; p < np; p += 32) cc_union(S.lab, pairs[p] & 0xff, pairs[p] >> 8);
+  __syncwarp();
+  for (int k = int(lane); k < n; k += 32)
+    if (S.xy[k] != 0xffffffffu) S.lab[k] = cc_find(S.lab, k);
+  __syncwarp();
+  finish_module_warp(d, e, m, r, int(crun), warn, S.lab, S.charge, S.cid, S.newc,
+                     [&](int k) { return d.adc[r.g0 + k]; });
 }
 
 // every module position of the batch: modules of <= 32 digis here (one digi per lane),
@@ -422,7 +432,7 @@ __global__ void __launch_bounds__(128, 6) k_find_clus_tiny(Dev d) {
 // modules of kThreadPix+1 .. 32 digis (work list), one warp each, one digi per lane
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_find_clus_small(Dev d) {
   pdl_sync(d);
-  __shared__ WarpSmem<1> smem[kWarpsPerBlock];
+  __shared__ SmallSmem smem[kWarpsPerBlock];
   const unsigned wib = threadIdx.x >> 5;
   const uint32_t nl = list_size(d, kListClusSmall);
   for (uint32_t i = blockIdx.x * kWarpsPerBlock + wib; i < nl; i += gridDim.x * kWarpsPerBlock) {
@@ -430,17 +440,16 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_find_clus_small(Dev d) 
     const int e = int(v >> 11);
     ModRange r;
     if (!module_range(d, e, v & 2047u, r)) continue;
-    cluster_module_warp<1>(d, e, v & 2047u, r, smem[wib], nullptr);
+    cluster_module_small(d, e, v & 2047u, r, smem[wib]);
   }
 }
 
-// the mid-size modules (33..256 digis), one warp each, eight digis per lane
-constexpr int kMidWarps = 4;  // 7.8 KB of shared memory per warp
+// the mid-size modules (33..256 digis), one warp each
+constexpr int kMidWarps = 4;  // 5.9 KB of shared memory per warp
 
 __global__ void __launch_bounds__(32 * kMidWarps) k_find_clus_mid(Dev d) {
   pdl_sync(d);
-  __shared__ WarpSmem<kWarpSlots> smem[kMidWarps];
-  __shared__ WarpHist hist[kMidWarps];
+  __shared__ MidSmem smem[kMidWarps];
   const unsigned wib = threadIdx.x >> 5;
   const uint32_t nl = list_size(d, kListClusMid);
   for (uint32_t i = blockIdx.x * kMidWarps + wib; i < nl; i += gridDim.x * kMidWarps) {
@@ -448,7 +457,7 @@ __global__ void __launch_bounds__(32 * kMidWarps) k_find_clus_mid(Dev d) {
     const int e = int(v >> 11);
     ModRange r;
     if (!module_range(d, e, v & 2047u, r)) continue;
-    cluster_module_warp<kWarpSlots>(d, e, v & 2047u, r, smem[wib], &hist[wib]);
+    cluster_module_mid(d, e, v & 2047u, r, smem[wib]);
   }
 }
 
@@ -617,11 +626,8 @@ constexpr int kListBlocksBig = 148, kListBlocksWarp = 148 * 2;
 
 union ListSmem {
   BlockSmem block;
-  struct {
-    WarpSmem<kWarpSlots> smem[kMidWarps];
-    WarpHist hist[kMidWarps];
-  } mid;
-  WarpSmem<1> small[8];
+  MidSmem mid[kMidWarps];
+  SmallSmem small[8];
 };
 
 __global__ void __launch_bounds__(256) k_find_clus_lists(Dev d) {
@@ -647,7 +653,7 @@ __global__ void __launch_bounds__(256) k_find_clus_lists(Dev d) {
       const int e = int(v >> 11);
       ModRange r;
       if (!module_range(d, e, v & 2047u, r)) continue;
-      cluster_module_warp<kWarpSlots>(d, e, v & 2047u, r, S.mid.smem[wib], &S.mid.hist[wib]);
+      cluster_module_mid(d, e, v & 2047u, r, S.mid[wib]);
     }
   }
   __syncthreads();
@@ -657,7 +663,7 @@ __global__ void __launch_bounds__(256) k_find_clus_lists(Dev d) {
     const int e = int(v >> 11);
     ModRange r;
     if (!module_range(d, e, v & 2047u, r)) continue;
-    cluster_module_warp<1>(d, e, v & 2047u, r, S.small[wib], nullptr);
+    cluster_module_small(d, e, v & 2047u, r, S.small[wib]);
   }
 }
 
