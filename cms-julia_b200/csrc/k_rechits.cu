@@ -189,7 +189,7 @@ struct WarpHitSmem {
 // digi count rounded up to a power-of-two number of warp slots). The sums go to the hit's
 // record; the CPE of all records then runs one hit per thread in k_cpe.
 template <int kS>
-__device__ __forceinline__ void module_sums(const Dev& d, int e, const HitModule& hm, const uint32_t* cms,
+__device__ __forceinline__ void module_sums(const Dev& d, int e, const HitModule& hm, uint32_t first_hit,
                                             WarpHitSmem& S) {
   const unsigned lane = threadIdx.x & 31u;
   const EvInfo& E = d.ev[e];
@@ -211,18 +211,20 @@ __device__ __forceinline__ void module_sums(const Dev& d, int e, const HitModule
     if (i < hm.end0) {
       const uint64_t g = eb + i;
       const int16_t id = d.mid[g];
-      const int32_t cl = d.clus[g];
-      if (id != int16_t(kInvId) && uint32_t(int32_t(id)) == hm.me && cl >= 1 && uint32_t(cl) <= nclus) {
-        cls[j] = cl;
-        xs[j] = uint32_t(int32_t(d.xx[g]));
-        ys[j] = uint32_t(int32_t(d.yy[g]));
-        const int32_t a = d.adc[g];
-        chs[j] = a < 65535 ? a : 65535;
-        atomicMin(&S.minr[cl - 1], xs[j]); atomicMax(&S.maxr[cl - 1], xs[j]);
-        atomicMin(&S.minc[cl - 1], ys[j]); atomicMax(&S.maxc[cl - 1], ys[j]);
-      }
+      const int32_t cl = d.clus[g], a = d.adc[g];
+      xs[j] = uint32_t(int32_t(d.xx[g]));
+      ys[j] = uint32_t(int32_t(d.yy[g]));
+      chs[j] = a < 65535 ? a : 65535;
+      if (id != int16_t(kInvId) && uint32_t(int32_t(id)) == hm.me && cl >= 1 && uint32_t(cl) <= nclus) cls[j] = cl;
     }
   }
+#pragma unroll
+  for (int j = 0; j < kS; ++j)
+    if (cls[j] != 0) {
+      const int k = cls[j] - 1;
+      atomicMin(&S.minr[k], xs[j]); atomicMax(&S.maxr[k], xs[j]);
+      atomicMin(&S.minc[k], ys[j]); atomicMax(&S.maxc[k], ys[j]);
+    }
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < kS; ++j) {
@@ -236,10 +238,10 @@ __device__ __forceinline__ void module_sums(const Dev& d, int e, const HitModule
   }
   __syncwarp();
   for (uint32_t k = lane; k < nclus; k += 32) {
-    const uint32_t h = cms[hm.me] + k;
+    const uint32_t h = first_hit + k;
     if (h >= d.hits_per_event) continue;
     if (uint64_t(hb) + h >= uint64_t(d.cap_hits)) { atomic_or_warn(&d.ev[e], kWarnBuffer); continue; }
-    if (h >= d.ev[e].n_hits) continue;  // an event past the buffer, emptied: k_cpe takes none of its hits
+    if (h >= E.n_hits) continue;  // an event past the buffer, emptied: k_cpe takes none of its hits
     const size_t o = size_t(hb) + h;
     d.hit_sum[o] = ClusSumRec{S.minr[k], S.maxr[k], S.minc[k], S.maxc[k], S.q[k], S.qfx[k], S.qlx[k], S.qfy[k], S.qly[k]};
     d.hit_me[o] = hm.me;
@@ -247,9 +249,10 @@ __device__ __forceinline__ void module_sums(const Dev& d, int e, const HitModule
   __syncwarp();
 }
 
-// Six blocks per SM (the most its 37 KB of shared memory allows): 40 registers and about
-// 130 bytes of spills, faster than four blocks without the cap; the kernel waits on its
-// digi gathers, and more warps in flight hide more of them.
+// Six blocks per SM (the most its 37 KB of shared memory allows): 40 registers and 116
+// bytes of spills, faster than four blocks without the cap; the kernel waits on its
+// digi gathers, and more warps in flight hide more of them. Two instances of the sums: with four
+// (up to 32, 64, 128 and 256 digis) 490 us.
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, 6) k_get_hits_warp(Dev d) {
   pdl_sync(d);
   __shared__ WarpHitSmem smem[kWarpsPerBlock];
@@ -260,18 +263,30 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 6) k_get_hits_warp(Dev d)
   const uint32_t nmod = E.n_modules;
   if (E.word_base + uint64_t(E.n_words) > uint64_t(d.cap_words)) return;
   const uint32_t* cms = d.clus_module_start + size_t(e) * (kMaxNumModules + 1);
-  for (uint32_t m = blockIdx.x * kWarpsPerBlock + wib; m < nmod; m += gridDim.x * kWarpsPerBlock) {
-    HitModule hm;
-    if (!hit_module(d, e, m, hm)) continue;
-    const uint32_t nd = hm.end0 - hm.first0;
-    if (nd > uint32_t(kWarpModulePix) || hm.nclus > uint32_t(kWarpClus)) {
-      if (lane == 0) push_module(d, kListHitsBig, e, m);
-      continue;
+  const uint32_t warps = gridDim.x * kWarpsPerBlock;
+  for (uint32_t m0 = blockIdx.x * kWarpsPerBlock + wib; m0 < nmod; m0 += 32u * warps) {
+    // the lanes look up the warp's next 32 modules together: one after the other, with the digis' coordinates
+    // loaded only once their cluster was known, 512 events of pileup 50 took 590 us, now 470
+    const uint32_t m = m0 + lane * warps;
+    HitModule hm{};
+    uint32_t first_hit = 0;
+    bool ok = m < nmod && hit_module(d, e, m, hm);
+    if (ok && (hm.end0 - hm.first0 > uint32_t(kWarpModulePix) || hm.nclus > uint32_t(kWarpClus))) {
+      push_module(d, kListHitsBig, e, m);
+      ok = false;
     }
-    if (nd <= 32) module_sums<1>(d, e, hm, cms, S);
-    else if (nd <= 64) module_sums<2>(d, e, hm, cms, S);
-    else if (nd <= 128) module_sums<4>(d, e, hm, cms, S);
-    else module_sums<kWarpSlots>(d, e, hm, cms, S);
+    if (ok) first_hit = cms[hm.me];
+    for (uint32_t todo = __ballot_sync(0xffffffffu, ok); todo; todo &= todo - 1) {
+      const int src = __ffs(int(todo)) - 1;
+      HitModule a;
+      a.me = __shfl_sync(0xffffffffu, hm.me, src);
+      a.nclus = __shfl_sync(0xffffffffu, hm.nclus, src);
+      a.first0 = __shfl_sync(0xffffffffu, hm.first0, src);
+      a.end0 = __shfl_sync(0xffffffffu, hm.end0, src);
+      const uint32_t h0 = __shfl_sync(0xffffffffu, first_hit, src), nd = a.end0 - a.first0;
+      if (nd <= 64) module_sums<2>(d, e, a, h0, S);
+      else module_sums<kWarpSlots>(d, e, a, h0, S);
+    }
   }
 }
 
