@@ -840,7 +840,9 @@ void launch_cluster(const Dev& d, const Launch& L) {
     L.mark("find_clus_small");
     L.run(k_find_clus_mid, mid_wave_ctas(), 32 * kMidWarps, 0, d);
     L.mark("find_clus_mid");
-    L.run(k_find_clus_block, 148 * 2, 256, 0, d);
+    // four blocks per SM (45 KB of shared memory each): 111 events of pileup 1 to 200 289 us, two 464; five 263,
+    // which takes the L1 from the other batches' kernels (9.49 ms with batches alone, 6.21 in flight; 9.46, 6.22)
+    L.run(k_find_clus_block, 148 * 4, 256, 0, d);
     L.mark("find_clus_block");
   }
   L.run(k_charge_cut_serial, d.E, 32, 0, d);

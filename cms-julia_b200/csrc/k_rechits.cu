@@ -494,7 +494,8 @@ void launch_rechits(const Dev& d, const Launch& L) {
   L.mark("get_hits_warp");
   L.run(k_cpe, dim3(std::max(1, std::min(64, (148 * 8 * 2) / std::max(1, int(d.E)))), d.E), 256, 0, d);
   L.mark("cpe");
-  L.run(k_get_hits_block, 148 * 2, 256, 0, d);
+  // four blocks per SM: 111 events of pileup 1 to 200 66 us, two 118
+  L.run(k_get_hits_block, 148 * 4, 256, 0, d);
   L.mark("get_hits_block");
   L.run(k_phi_binner, d.E, 1024, 0, d);
   L.run(k_phi_place, dim3(event_blocks(d.E, 148 * 32, 128), d.E), 256, 0, d);
