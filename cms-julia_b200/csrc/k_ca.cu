@@ -460,16 +460,16 @@ __global__ void __launch_bounds__(256, 5) k_doublets_count(Dev d, const uint32_t
 
 // Fill pass over the same 32-item groups: cells of a group are contiguous, so the warp
 // writes them with consecutive lanes on consecutive cells, outer hits from the pool and the
-// inner hit, pair and inner z / r of each cell's item from shared memory.
+// inner hit and pair of each cell's item from shared memory. Bound by its 22 bytes of stores and one
+// atomic per cell; the items that own a step's cells come from a bit mask (with a binary search per cell 512
+// events of pileup 50 took 474 us, now 457; one of pileup 170 45 and 40).
 template <bool kQ>
 __global__ void __launch_bounds__(256) k_doublets_fill(Dev d, const uint32_t* __restrict__ pair_cum, WorkQueue q) {
   pdl_sync(d);
   __shared__ uint32_t s_cum[kNPairs];
   __shared__ uint32_t s_hls[11];
-  __shared__ uint32_t s_pos[8][33];
-  __shared__ uint32_t s_pool[8][32];  // where the item's pool range would put the group's cell 0
-  __shared__ uint32_t s_hit[8][32];
-  __shared__ uint8_t s_pid[8][32];
+  // of the items with doublets: where the item's pool range would put the group's cell 0, its hit, its pair
+  __shared__ uint4 s_item[8][32];
   for_each_vblock<kQ>(q, [&](int e, uint32_t bx, uint32_t nbx) {
   const EvInfo& E = d.ev[e];
   const uint32_t n = E.n_items;
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(256) k_doublets_fill(Dev d, const uint32_t* __
   const uint32_t raw_lo = d.item_cnt[ib];
   const uint64_t cell_lo = E.cell_base;
   const uint32_t keep = E.n_cells;
-  const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
   for (uint32_t j0 = bx * blockDim.x + 32u * w; j0 < n; j0 += nbx * blockDim.x) {
     const uint32_t j = j0 + lane;
     const bool valid = j < n;
@@ -504,28 +504,26 @@ __global__ void __launch_bounds__(256) k_doublets_fill(Dev d, const uint32_t* __
     const uint32_t base = __shfl_sync(0xffffffffu, pos, 0);
     uint32_t i = 0;
     const int pid = valid ? item_pair(j, s_cum, s_hls, &i) : 0;
-    s_pos[w][lane] = inc - cnt;
-    s_pool[w][lane] = pool - (inc - cnt);
-    if (cnt > 0) {
-      s_hit[w][lane] = i;
-      s_pid[w][lane] = uint8_t(pid);
-    }
+    const uint32_t busy = __ballot_sync(0xffffffffu, cnt > 0);
+    if (cnt > 0) s_item[w][__popc(busy & lt)] = make_uint4(pool - (inc - cnt), i, uint32_t(pid), 0);
     __syncwarp();
-    for (uint32_t x = lane; x < total; x += 32) {
-      const uint32_t local = base + x;
-      if (local >= keep) break;
-      uint32_t a = 0, b = 32;
-      while (b - a > 1) {
-        const uint32_t m = (a + b) >> 1;
-        if (s_pos[w][m] <= x) a = m; else b = m;
-      }
-      const uint64_t g = cell_lo + local;
-      d.cell_inner[g] = s_hit[w][a];
-      const uint32_t oh = d.dbl_pool[s_pool[w][a] + x];
+    const uint32_t start = cnt > 0 ? inc - cnt : 0xffffffffu;
+    const uint32_t m = base < keep ? min(total, keep - base) : 0u;
+    int cur = -1;  // item owning the cell before the step
+    for (uint32_t x0 = 0; x0 < m; x0 += 32) {
+      const uint32_t starts = __reduce_or_sync(0xffffffffu, start - x0 < 32u ? 1u << (start - x0) : 0u);
+      const uint32_t a = uint32_t(cur + int(__popc(starts & ((lt << 1) | 1u))));
+      cur += int(__popc(starts));
+      const uint32_t x = x0 + lane;
+      if (x >= m) continue;
+      const uint4 it = s_item[w][a];
+      const uint64_t g = cell_lo + base + x;
+      d.cell_inner[g] = it.y;
+      const uint32_t oh = d.dbl_pool[it.x + x];
       d.cell_outer[g] = oh;
       atomicAdd(&d.ohc_cur[hb + oh], 1u);  // cells ending on each hit
-      d.cell_pair[g] = s_pid[w][a];
-      d.cell_id[g] = int32_t(local + 1);
+      d.cell_pair[g] = uint8_t(it.z);
+      d.cell_id[g] = int32_t(base + x + 1);
       d.cell_used[g] = 0;
       d.cn_cur[g] = 0;
       d.ct_cur[g] = 0;
