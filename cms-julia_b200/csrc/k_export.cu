@@ -128,13 +128,14 @@ __global__ void __launch_bounds__(kExpThreads) k_export_fill(Dev d, ExportSet x)
   }
 }
 
-constexpr int kExpBlocks = 148 * 4;  // blocks of a small batch (event_blocks)
+constexpr int kExpBlocks = 148 * 16;  // blocks of the export's kernels (event_blocks); 148 * 4 left 111 uneven
+                                       // events five each: their export 1110 us, now 898; 148 * 32: 886
 
 // The packed arrays to host memory that the device can write (pinned), the rows there are and no more.
 // For small batches, in place of a copy of each array's whole capacity: 14 copies of 3.2 MB in all take
 // 100 us for the 145 KB of tracks of one event of pileup 50 (its chain and export: 684 us, now 588;
-// an event of 100 tracks: 461, now 366). Larger batches keep the copy engine,
-// which leaves the SMs to the next chain.
+// an event of 100 tracks: 461, now 366; the export of eight events of pileup 200, 4.6 MB, 1056, now 136).
+// Larger batches keep the copy engine, which leaves the SMs to the next chain.
 __device__ __forceinline__ void copy_rows(void* dst, const void* src, size_t bytes) {
   if (!dst) return;
   const size_t first = blockIdx.x * size_t(blockDim.x) + threadIdx.x, stride = size_t(gridDim.x) * blockDim.x;
