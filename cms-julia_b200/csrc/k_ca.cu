@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cstddef>
 
+#include "doublet_staging.cuh"
 #include "pxl_internal.cuh"
 
 namespace pxl {
@@ -293,7 +294,6 @@ __device__ __forceinline__ void write_item_doublets(const Dev& d, const ItemHead
 }
 
 constexpr uint32_t kNoPool = 0xffffffffu;
-constexpr int kGroupCells = 768;  // outer hits one 32-item group stages in shared memory
 
 // Count pass over groups of 32 consecutive items (one warp). The candidates of the group's
 // items are laid end to end and take the first cuts 32 at a time on all lanes; the survivors
@@ -303,8 +303,8 @@ constexpr int kGroupCells = 768;  // outer hits one 32-item group stages in shar
 // contiguous range of the pool and copies them there. When the staging is nearly full, the items whose
 // doublets are complete go to the pool and the current item's move to the front (groups above 768
 // doublets are common from pileup 100 on; the fill pass, which searches again what the count could not
-// keep, item by item, took 1.48 ms for 111 uneven events). An item that fills the staging alone, or a
-// full pool, records kNoPool and the fill pass searches again. Bound by instructions issued (68 % of the
+// keep, item by item, took 1.48 ms for 111 uneven events). An item that fills the staging alone and the ones
+// after it in the group (doublet_staging.cuh), or a full pool, record kNoPool and the fill pass searches again. Bound by instructions issued (68 % of the
 // issue slots at 512 events of pileup 50); with the first cut's constants staged per item and the
 // module cut left to the survivors 1.37 ms, before 1.44.
 constexpr int kDblQueue = 64;
@@ -407,11 +407,11 @@ __global__ void __launch_bounds__(256, 5) k_doublets_count(Dev d, const uint32_t
         stage_b(last ? qtail - qhead : 32u);
         __syncwarp();
       }
-      if (!last && nout + 32 <= uint32_t(kGroupCells)) continue;
+      if (!last && !staging_near_full(nout)) continue;
       // the staged outputs are in item order, so each item's are one run; the items before `keep` are complete
       const uint32_t nst = nout < uint32_t(kGroupCells) ? nout : uint32_t(kGroupCells);
       const uint32_t keep = last ? 32u : s_out[w][nst - 1] >> kOwnerShift;
-      if (!last && keep == done) continue;  // one item's doublets fill the staging: it overflows
+      if (!last && !staging_hands_over(nout, keep, done)) continue;
       s_beg[w][lane] = 0; s_end[w][lane] = 0;
       __syncwarp();
       for (uint32_t x = lane; x < nst; x += 32) {
