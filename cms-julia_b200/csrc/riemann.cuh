@@ -340,10 +340,14 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
   const int q = (double(px[1]) * (cy - double(py[0])) - double(py[1]) * (cx - double(px[0]))) > 0 ? -1 : 1;
   o.chi2_circle = fabs(lam) * renorm / ((2.0 * v[2] * uvr2 * s) * (2.0 * v[2] * uvr2 * s));
   // ---------------------------------------------------------------- line fit in the rotated (s, z) plane
-  // sine and cosine of the angle in [0, pi) whose tangent is -q ftan
+  // Sine and cosine of the angle in [0, pi) whose tangent is -q ftan: from the tangent or, where it is above 1, from
+  // its inverse (the tangent of hits at equal z is infinite).
   const double tth = -q * double(ftan);
-  double cs = bl::s_rsqrt(1.0 + tth * tth), sn = tth * cs;
-  if (tth < 0) { sn = -sn; cs = -cs; }
+  const bool flat = fabs(tth) > 1.0;
+  const double t = flat ? 1.0 / tth : tth;
+  const double ca = bl::s_rsqrt(1.0 + t * t), sa = t * ca;
+  double sn = flat ? ca : sa, cs = flat ? sa : ca;
+  if (!flat && tth < 0) { sn = -sn; cs = -cs; }
   const T ox = T(cx), oy = T(cy);  // centre relative to hit 0
   const T gox = T(hits[0][0] + cx), goy = T(hits[1][0] + cy);
   T sarc[N], cov_zz[N];

@@ -1,0 +1,36 @@
+"""Tracks at the edges of the fits' formulas."""
+import numpy as np
+
+B_FIELD = 0.0114256972711507
+RADII = (2.9, 6.8, 10.9, 16.0, 20.0, 24.0, 28.0, 32.0)
+
+
+def _errors(hits):
+    """Covariances of 10 um along r-phi and 20 um along z."""
+    r = np.hypot(hits[:, 0], hits[:, 1])
+    s, c = hits[:, 1] / r, hits[:, 0] / r
+    ge = np.zeros((len(hits), 6), np.float32)
+    ge[:, 0], ge[:, 1], ge[:, 2] = 1e-6 * s * s, -1e-6 * s * c, 1e-6 * c * c
+    ge[:, 5] = 4e-6
+    return ge
+
+
+def flat_tracks(count: int = 6, seed: int = 1):
+    """Helices across the beam whose first and last hit have the same z, or nearly so: [(hits, ge)], 3, 4 and 8 hits,
+    both charges, measured with the errors of the covariances."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for n in (3, 4, 8):
+        for dz in (0.0, 1e-9, -1e-9, 1e-300, 1e-4):
+            for k in range(count):
+                r, sign = np.array(RADII[:n]), (1, -1)[k % 2]
+                radius = rng.uniform(60, 900)
+                a = 2 * np.arcsin(r / (2 * radius))
+                x, y = radius * np.sin(a), sign * radius * (1 - np.cos(a))
+                y = y + rng.normal(0, 1e-3, n)
+                phi = rng.uniform(-np.pi, np.pi)
+                z = rng.uniform(-20, 20) + rng.normal(0, 2e-3, n)
+                z[-1] = z[0] + dz
+                hits = np.stack([x * np.cos(phi) - y * np.sin(phi), x * np.sin(phi) + y * np.cos(phi), z], 1)
+                out.append((hits, _errors(hits)))
+    return out
