@@ -93,7 +93,8 @@ BL_HD double s_mul(double a, double b) {
 #ifdef __CUDA_ARCH__
   return __dmul_rn(a, b);
 #else
-  return a * b;
+  volatile double p = a * b;
+  return p;
 #endif
 }
 BL_HD f32 s_mul(f32 a, f32 b) { return a * b; }
@@ -174,6 +175,15 @@ BL_HD T diff_of_products(T a, T d, T b, T c) {
     const T f = fmaf(a, d, -w);
     return f + e;
   }
+}
+
+// The same for the two chords of a fast fit, 0 where they are parallel: in FP64 both products are
+// rounded, so that equal ones cancel and the fit of collinear hits is refused (contracted, the
+// rounding error of one of them is left, and with it a circle of 1e16 cm).
+template <class T>
+BL_HD T chord_product(T a, T d, T b, T c) {
+  if constexpr (sizeof(T) == 8) return s_mul(a, d) - s_mul(b, c);
+  else return diff_of_products<T>(a, d, b, c);
 }
 
 // --------------------------------------------------------------- band solver
@@ -358,7 +368,7 @@ BL_HD void fast_fit(const Geo<N, T>& G, Prep<N, T>& P) {
   const T a1 = G.p[0][mid], a2 = G.p[1][mid];
   const T b1 = G.p[0][N - 1] - G.p[0][mid], b2 = G.p[1][N - 1] - G.p[1][mid];
   const T c1 = -G.p[0][N - 1], c2 = -G.p[1][N - 1];
-  const T ca = diff_of_products<T>(c1, a2, c2, a1);
+  const T ca = chord_product<T>(c1, a2, c2, a1);
   const T nc = c1 * c1 + c2 * c2, na = a1 * a1 + a2 * a2;
   const T tmp = T(0.5) / ca;
   P.cx = -(a2 * nc + c2 * na) * tmp;
@@ -734,7 +744,7 @@ BL_HD void chord_frame(const double hits[3][N], const float ge_in[6][N], bool ze
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     hr[0][i] = cr * hits[0][i] + sr * hits[1][i];
-    hr[1][i] = cr * hits[1][i] - sr * hits[0][i];
+    hr[1][i] = s_mul(cr, hits[1][i]) - s_mul(sr, hits[0][i]);  // equal for collinear hits along the chord
     hr[2][i] = hits[2][i];
     auto z = [&](float v) { return zero_tiny && fabs(double(v)) < 1e-12 ? 0.0 : double(v); };
     const double xx = z(ge_in[0][i]), xy = z(ge_in[1][i]), yy = z(ge_in[2][i]);

@@ -185,7 +185,7 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
     const T b2 = b0 * b0 + b1 * b1, c2 = c0 * c0 + c1 * c1;
     const bool flip = s_abs(b0) < s_abs(b1);
     const T bx = flip ? b1 : b0, by = flip ? b0 : b1, cx = flip ? c1 : c0, cy = flip ? c0 : c1;
-    const T div = T(2) * bl::diff_of_products<T>(cx, by, bx, cy);
+    const T div = T(2) * bl::chord_product<T>(cx, by, bx, cy);
     const T Y0 = (cx * b2 - bx * c2) / div;
     const T X0 = (T(0.5) * b2 - Y0 * by) / bx;
     fx = flip ? Y0 : X0;

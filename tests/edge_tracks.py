@@ -34,3 +34,17 @@ def flat_tracks(count: int = 6, seed: int = 1):
                 hits = np.stack([x * np.cos(phi) - y * np.sin(phi), x * np.sin(phi) + y * np.cos(phi), z], 1)
                 out.append((hits, _errors(hits)))
     return out
+
+
+def straight_tracks(count: int = 8, seed: int = 2):
+    """Collinear hits, whose circle has no centre: [(hits, ge)], 3, 4 and 8 hits, along directions in which the
+    products of the chords' components are equal but not representable."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for n in (3, 4, 8):
+        for dx, dy in ((1, 1), (1, -1), (1, 0.25), (-0.5, 1), (-1, -4), (1, 0), (0, -1)):
+            for _ in range(count):
+                s = np.array(RADII[:n]) + rng.uniform(0, 0.1, n)
+                hits = np.stack([dx * s, dy * s, 1.0 + 0.3 * s], 1)
+                out.append((hits, _errors(hits)))
+    return out
