@@ -559,12 +559,14 @@ BL_HD void translate_karimaki(double& cs, double& sn, CircleOut& c, double x0, d
   const double BB = p3 * x0 + uu * sn;
   const double zeta = DO * DO + DP * DP;
   const double A = 2.0 * DO + p3 * zeta;
-  const double U = sqrt(1.0 + p3 * A);
-  const double ixi = s_rsqrt(BB * BB + C * C);
-  const double xi = ixi * ixi;
+  // U = sqrt(1 + rho A), in which 1 + rho A = B^2 + C^2: as a sum of squares it does not round below 0 where
+  // the point is the circle's centre
+  const double n2 = BB * BB + C * C;
+  const double ixi = s_rsqrt(n2);
+  const double xi = ixi * ixi, U = n2 * ixi;
   const double v = 1.0 + p3 * DO;
-  const double iu = 1.0 / (U * (1.0 + U));  // 1 / (1 + U) = U iu
-  const double au = A * (U * iu);           // A / (1 + U)
+  const double iu = 1.0 / (U * (1.0 + U));       // 1 / (1 + U) = U iu
+  const double au = U > 0 ? A * (U * iu) : A;  // A / (1 + U)
   const double lambda = 0.5 * au * iu;
   const double mu = iu + p3 * lambda;
   const double J[3][3] = {{xi * uu * v, -xi * (p3 * p3) * DP, xi * DP},

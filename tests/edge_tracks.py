@@ -48,3 +48,17 @@ def straight_tracks(count: int = 8, seed: int = 2):
                 hits = np.stack([dx * s, dy * s, 1.0 + 0.3 * s], 1)
                 out.append((hits, _errors(hits)))
     return out
+
+
+def centred_tracks(count: int = 12, seed: int = 3):
+    """Hits on circles about the beam line, whose impact parameter is the radius: [(hits, ge, radius)], 3, 4 and 8 hits."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for n in (3, 4, 8):
+        for r in (2.9, 6.8, 7.0, 10.0):
+            for _ in range(count):
+                a = np.sort(rng.uniform(0, 2, n))
+                z = rng.uniform(-5, 5) + rng.uniform(-1, 1) * r * a + rng.normal(0, 2e-3, n)
+                hits = np.stack([r * np.cos(a), r * np.sin(a), z], 1)
+                out.append((hits, _errors(hits), r))
+    return out
