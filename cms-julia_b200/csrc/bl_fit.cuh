@@ -739,13 +739,13 @@ template <int N>
 BL_HD void chord_frame(const double hits[3][N], const float ge_in[6][N], bool zero_tiny, double hr[3][N],
                        float ge[6][N], double& cr, double& sr) {
   const double dx = hits[0][N - 1] - hits[0][0], dy = hits[1][N - 1] - hits[1][0];
-  const double l = sqrt(dx * dx + dy * dy);
+  const double l = sqrt(s_mul(dx, dx) + s_mul(dy, dy));
   cr = 1.0;
   sr = 0.0;
   if (l > 0) { cr = dx / l; sr = dy / l; }
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    hr[0][i] = cr * hits[0][i] + sr * hits[1][i];
+    hr[0][i] = s_mul(cr, hits[0][i]) + s_mul(sr, hits[1][i]);
     hr[1][i] = s_mul(cr, hits[1][i]) - s_mul(sr, hits[0][i]);  // equal for collinear hits along the chord
     hr[2][i] = hits[2][i];
     auto z = [&](float v) { return zero_tiny && fabs(double(v)) < 1e-12 ? 0.0 : double(v); };

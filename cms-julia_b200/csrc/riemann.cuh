@@ -182,12 +182,13 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
   T fx, fy, fR, ftan;  // centre relative to hit 0, radius, tan(theta)
   {
     const T b0 = px[mid], b1 = py[mid], c0 = px[N - 1], c1 = py[N - 1];
-    const T b2 = b0 * b0 + b1 * b1, c2 = c0 * c0 + c1 * c1;
+    // products rounded one by one, so that the equal ones of collinear hits cancel
+    const T b2 = bl::s_mul(b0, b0) + bl::s_mul(b1, b1), c2 = bl::s_mul(c0, c0) + bl::s_mul(c1, c1);
     const bool flip = s_abs(b0) < s_abs(b1);
     const T bx = flip ? b1 : b0, by = flip ? b0 : b1, cx = flip ? c1 : c0, cy = flip ? c0 : c1;
     const T div = T(2) * bl::chord_product<T>(cx, by, bx, cy);
-    const T Y0 = (cx * b2 - bx * c2) / div;
-    const T X0 = (T(0.5) * b2 - Y0 * by) / bx;
+    const T Y0 = (bl::s_mul(cx, b2) - bl::s_mul(bx, c2)) / div;
+    const T X0 = (T(0.5) * b2 - bl::s_mul(Y0, by)) / bx;
     fx = flip ? Y0 : X0;
     fy = flip ? X0 : Y0;
     fR = s_sqrt<T>(X0 * X0 + Y0 * Y0);
@@ -204,6 +205,7 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
   const T gcx = T(hits[0][0]) + fx, gcy = T(hits[1][0]) + fy;
   // ---------------------------------------------------------------- circle weights
   double Cr[N][N];
+  bool none = false;  // a hit's variance has no value
   {
     const T p_t = fR * B < T(20) ? fR * B : T(20);
     // scattering factor 0.000225 / (p^2 sin^2(theta)), p sin(theta) = pT; in FP32 in the port's steps
@@ -256,9 +258,12 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
       } else {
         const double ax = hits[0][i], ay = hits[1][i];
         const double bx = ax - double(gcx), by = ay - double(gcy);
-        const double x2 = ax * bx + ay * by, y2 = ax * by - ay * bx;
-        // at the tangent -y2 / x2
+        const double x2 = bl::s_mul(ax, bx) + bl::s_mul(ay, by), y2 = ax * by - ay * bx;
+        // At the tangent -y2 / x2. Where it is infinite the port's expression in the tangent has no value, and
+        // that is how straight tracks are refused whose circle is rounding error (a radius of 1e16 cm: both
+        // products of x2, rounded, are then as large and cancel).
         d = (vxx * x2 * x2 + vyy * y2 * y2 - 2.0 * vxy * x2 * y2) / (x2 * x2 + y2 * y2);
+        none |= x2 == 0;
       }
       Cr[i][i] += d;
     }
@@ -270,7 +275,7 @@ BL_HD bool riemann_fit_frame(const double hits[3][N], const float ge[6][N], cons
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) renorm += G[i][j];
-  const double irenorm = 1.0 / renorm;
+  const double irenorm = none ? double(NAN) : 1.0 / renorm;
   double wgt[N];
 #pragma unroll
   for (int j = 0; j < N; ++j) {

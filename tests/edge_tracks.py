@@ -62,3 +62,14 @@ def centred_tracks(count: int = 12, seed: int = 3):
                 hits = np.stack([r * np.cos(a), r * np.sin(a), z], 1)
                 out.append((hits, _errors(hits), r))
     return out
+
+
+def rounded_straight_tracks(count: int = 400, seed: int = 4):
+    """Straight tracks in any direction: collinear up to the rounding of their hits, which decides whether the fast
+    fit's circle has a radius of 1e16 cm or none."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for t in range(count):
+        hits = np.outer(RADII[:(3, 4, 8)[t % 3]], rng.normal(size=3))
+        out.append((hits, _errors(hits)))
+    return out
