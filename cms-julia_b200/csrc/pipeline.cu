@@ -47,7 +47,7 @@ int upload(PxlCtx* c, const T** dst, const std::vector<T>& v) {
   T* q = nullptr;
   int rc = dalloc(c, &q, int64_t(v.size()));
   if (rc) return rc;
-  if (!v.empty()) CK(cudaMemcpy(q, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+  if (!v.empty()) CK(cudaMemcpyAsync(q, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
   *dst = q;
   return 0;
 }
@@ -217,7 +217,7 @@ int alloc_batch(PxlCtx* ctx) {
   int rc = 0;
 #define A(ptr, n) do { rc = dalloc(ctx, &d.ptr, (n)); if (rc) return rc; } while (0)
   A(ev, E + 1);
-  CK(cudaMemset(d.ev, 0, size_t(E + 1) * sizeof(EvInfo)));  // counts and warnings read before any run
+  CK(cudaMemsetAsync(d.ev, 0, size_t(E + 1) * sizeof(EvInfo), ctx->stream));  // counts and warnings read before any run
   A(fed_src, E * NF); A(fed_nw, E * NF); A(fed_wo, E * NF); A(fed_nmod, E * NF + kFedParts);
   A(xx, d.cap_words); A(yy, d.cap_words); A(adc, d.cap_words); A(mid, d.cap_words); A(clus, d.cap_words);
   A(pdigi, d.cap_words); A(rawid, d.cap_words);
@@ -229,7 +229,7 @@ int alloc_batch(PxlCtx* ctx) {
   A(xg, d.cap_hits); A(yg, d.cap_hits); A(zg, d.cap_hits); A(rg, d.cap_hits);
   A(iphi, d.cap_hits); A(xsize, d.cap_hits); A(ysize, d.cap_hits); A(detind, d.cap_hits); A(charge, d.cap_hits);
   A(hits_layer_start, E * 11); A(phi_off, E * kPhiTotBins); A(phi_bins, d.cap_hits); A(phi_fill, d.cap_hits); A(hit_rec, d.cap_hits); A(hit_rec_s, d.cap_hits); A(hit_u_s, d.cap_hits); A(hit_sum, d.cap_hits); A(hit_me, d.cap_hits); A(hit_xyzr, d.cap_hits);
-  CK(cudaMemset(d.hit_me, 0xFF, size_t(std::max<int64_t>(d.cap_hits, 1)) * sizeof(uint32_t)));
+  CK(cudaMemsetAsync(d.hit_me, 0xFF, size_t(std::max<int64_t>(d.cap_hits, 1)) * sizeof(uint32_t), ctx->stream));
   A(pair_cum, E * kNPairs);
   A(item_cnt, d.cap_items + 1);
   A(item_pool, d.cap_items); A(dbl_pool, d.cap_cells); A(dbl_pool_ctr, 1);
@@ -266,7 +266,7 @@ int alloc_batch(PxlCtx* ctx) {
   int64_t st = scan_tmp_elems(std::max({d.cap_words, d.cap_items, d.cap_cells, d.cap_hits, d.cap_tuples}) + 1);
   A(scan_tmp, st); A(scan_tmp64, st);
   A(status, 1);
-  CK(cudaMemset(d.status, 0, sizeof(uint32_t)));
+  CK(cudaMemsetAsync(d.status, 0, sizeof(uint32_t), ctx->stream));
   d.cap_big = E * kMaxNumModules;
   A(big_list, kListHeader + kNumLists * d.cap_big);
 #undef A
@@ -517,6 +517,9 @@ int32_t pxl_ctx_create(const PxlConditions* cond, const PxlParams* params, PxlCt
   int rc = (prepare_select_kernels() || prepare_ca_kernels(ctx->wq_ctas)) ? PXL_ERR_CUDA : 0;
   if (!rc) rc = load_conditions(ctx, cond);
   if (!rc) rc = alloc_batch(ctx);
+  // what was copied and cleared is there before a run on any stream (the context's stream, and with it these
+  // commands, does not wait for the default stream's work, nor would a run on it wait for the default stream)
+  if (!rc && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = PXL_ERR_CUDA;
   if (rc) { pxl_ctx_destroy(ctx); return rc; }
   *out = ctx;
   return 0;
