@@ -63,15 +63,16 @@ def build_cuda(force: bool = False, verbose: bool = False) -> Path:
     LIB.mkdir(exist_ok=True)
     out = LIB / "libpxl_b200.so"
     srcs = [CSRC / s for s in CUDA_SOURCES if (CSRC / s).exists()]
-    deps = srcs + list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "pxl.h"]
-    if not force and _newer(out, deps):
+    # the headers, and this file, which decides the flags
+    common = [*CSRC.glob("*.cuh"), *CSRC.glob("*.h"), PKG.parent / "include" / "pxl.h", Path(__file__)]
+    if not force and _newer(out, srcs + common):
         return out
     objdir = PKG / "_build"
     objdir.mkdir(exist_ok=True)
     objs = []
     for s in srcs:
         o = objdir / (s.stem + ".o")
-        if force or not _newer(o, [s] + list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "pxl.h"]):
+        if force or not _newer(o, [s, *common]):
             cmd = [_nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", *flags(s.name), "-Xcompiler", "-fPIC",
                    "-Xptxas", "-v" if verbose else "-O3", "-c", str(s), "-o", str(o)]
             if verbose:
