@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/pxl.h"
+#include "batch_shape.cuh"
 #include "pxl_ctx.h"
 #include "pxl_internal.cuh"
 
@@ -402,11 +403,13 @@ int stage_input(PxlCtx* ctx, const uint8_t* blob, const uint64_t* offs, int32_t 
   if (on_device) {
     ctx->d.raw = blob;
     ctx->d.ev_off = offs;
+    ctx->in_words = 0;
   } else {
     int rc = stage_slot(ctx, 0, blob, offs, n, s);
     if (rc) return rc;
     ctx->d.raw = ctx->d_raw[0];
     ctx->d.ev_off = ctx->d_ev_off[0];
+    ctx->in_words = (offs[n] - offs[0]) / 4;
   }
   ctx->d.E = n;
   ctx->last_E = n;
@@ -417,12 +420,7 @@ int stage_input(PxlCtx* ctx, const uint8_t* blob, const uint64_t* offs, int32_t 
 int choose_shape(PxlCtx* ctx) {
   Dev& d = ctx->d;
   if (ctx->p.blocks_per_event > 0) { d.bpe = ctx->p.blocks_per_event; return 0; }
-  // Blocks per event: enough for eight waves of eight blocks per SM, at least 32, at most 256. Events differ
-  // in size and the blocks of one share its work, so a batch cut to one wave (1184 / E blocks, at least 4)
-  // waited for its largest events: 111 events of pileup 1 to 200 13.2 ms, now 9.3; 24 of them 3.9 and 3.7.
-  // Of equal events, whose blocks only become shorter: 512 of pileup 50 12.7 and 12.1 ms, 64 2.34 and
-  // 2.32. Twice as many blocks again: 9.1 ms (111 uneven), but 3.36 instead of 3.28 ms for 111 equal ones.
-  d.bpe = std::max(32, std::min(256, 148 * 64 / std::max(1, d.E)));
+  d.bpe = blocks_per_event(d.E, ctx->in_words);
   return 0;
 }
 

@@ -40,6 +40,7 @@ struct PxlCtx {
   uint64_t* d_ev_off[kSlots] = {};
   uint8_t* d_raw[kSlots] = {};
   int32_t slot_E[kSlots] = {};
+  uint64_t in_words = 0;  // 32-bit words of the current input, 0 where it is on the device
   cudaEvent_t ev_staged[kSlots] = {};
   cudaEvent_t ev_consumed[kSlots] = {};
   // per-kernel timing of non-graph runs
