@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cstddef>
 
+#include "alignment.cuh"
 #include "doublet_staging.cuh"
 #include "pxl_internal.cuh"
 
@@ -35,10 +36,7 @@ __constant__ double c_max_z[kNPairs] = {20., 30., 0., 22., 30., -10., 70., 70., 
 __constant__ float c_max_rf[kNPairs] = {20.f, 9.f, 9.f, 20.f, 7.f, 7.f, 5.f, 5.f, 20.f, 6.f, 6.f,
                                         5.f, 5.f, 20.f, 20.f, 9.f, 9.f, 9.f, 9.f};
 
-// CA parameters (ca_hit_ntuplet_generator.jl:9-30), Float32 as Params stores them
-__device__ __forceinline__ float ptmin_f() { return 0.899999976158f; }
-constexpr float kThetaBarrel = 0.00200000009499f;
-constexpr float kThetaForward = 0.00300000002608f;
+// CA parameters (ca_hit_ntuplet_generator.jl:9-30), Float32 as Params stores them; the others in alignment.cuh
 constexpr float kHardCurv = 0.0328407224959f;
 constexpr float kDcaInner = 0.15000000596f;
 constexpr float kDcaOuter = 0.25f;
@@ -786,29 +784,6 @@ struct CircleEq {
   }
 };
 
-__device__ __forceinline__ bool are_aligned(float r1, float z1, float ri, float zi, float ro, float zo, float ptmin,
-                                            float theta_cut) {
-  const float radius_diff = fabsf(__fsub_rn(r1, ro));
-  const float dz = __fsub_rn(z1, zo);
-  const float d13 = __fadd_rn(__fmul_rn(radius_diff, radius_diff), __fmul_rn(dz, dz));
-  const float p_min = __fmul_rn(ptmin, __fsqrt_rn(d13));
-  const float t = fabsf(__fadd_rn(__fadd_rn(__fmul_rn(z1, __fsub_rn(ri, ro)), __fmul_rn(zi, __fsub_rn(ro, r1))),
-                                  __fmul_rn(zo, __fsub_rn(r1, ri))));
-  return __fmul_rn(t, p_min) <= __fmul_rn(__fmul_rn(theta_cut, d13), radius_diff);
-}
-
-// False only where are_aligned is false, without its square root: the two sides squared, the right one
-// larger by a share that covers the rounding of both (1e-6) and by a term above all underflow.
-__device__ __forceinline__ bool maybe_aligned(float r1, float z1, float ri, float zi, float ro, float zo, bool barrel) {
-  constexpr float kBarrel = float(double(kThetaBarrel) * kThetaBarrel / (0.899999976158 * 0.899999976158) * (1 + 1e-5));
-  constexpr float kForward = float(double(kThetaForward) * kThetaForward / (0.899999976158 * 0.899999976158) * (1 + 1e-5));
-  const float u = __fsub_rn(ro, r1);
-  const float t = __fadd_rn(__fadd_rn(__fmul_rn(z1, __fsub_rn(ri, ro)), __fmul_rn(zi, u)), __fmul_rn(zo, __fsub_rn(r1, ri)));
-  const float dz = __fsub_rn(z1, zo), u2 = __fmul_rn(u, u);
-  const float lim = __fmaf_rn(__fmul_rn(u2, __fmaf_rn(dz, dz, u2)), barrel ? kBarrel : kForward, 1e-30f);
-  return !(__fmul_rn(t, t) > lim);
-}
-
 // Connection test of every cell with the cells ending on its inner hit (the outer-hit list,
 // at most kMaxCellsPerHit entries). A warp takes 32 cells and spreads their (cell, candidate)
 // pairs over its lanes, 32 pairs per step; a bound of the alignment test runs on every pair, and the
@@ -852,7 +827,7 @@ __global__ void __launch_bounds__(256, 6) k_connect_test(Dev d, WorkQueue q) {
       const uint32_t ih = d.cell_inner[c];
       const float4 h1 = hxyzr[d.cell_inner[o]];  // the candidate's inner hit
       const float4 hi = hxyzr[ih], ho = hxyzr[d.cell_outer[c]];
-      if (are_aligned(h1.w, h1.z, hi.w, hi.z, ho.w, ho.z, ptmin_f(), d.detind[hb + ih] < 1184 ? kThetaBarrel : kThetaForward)) {
+      if (are_aligned(h1.w, h1.z, hi.w, hi.z, ho.w, ho.z, d.detind[hb + ih] < 1184 ? kThetaBarrel : kThetaForward)) {
         const CircleEq eq(h1.x, h1.y, hi.x, hi.y, ho.x, ho.y);
         if (eq.c > kHardCurv) cut = false;
         else cut = fabsf(eq.dca0()) < __fmul_rn(region, fabsf(eq.c));
