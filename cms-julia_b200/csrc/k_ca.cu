@@ -302,9 +302,9 @@ constexpr uint32_t kNoPool = 0xffffffffu;
 // doublets are complete go to the pool and the current item's move to the front (groups above 768
 // doublets are common from pileup 100 on; the fill pass, which searches again what the count could not
 // keep, item by item, took 1.48 ms for 111 uneven events). An item that fills the staging alone and the ones
-// after it in the group (doublet_staging.cuh), or a full pool, record kNoPool and the fill pass searches again. Bound by instructions issued (68 % of the
-// issue slots at 512 events of pileup 50); with the first cut's constants staged per item and the
-// module cut left to the survivors 1.37 ms, before 1.44.
+// after it in the group (doublet_staging.cuh), or a full pool, record kNoPool and the fill pass searches again. Bound by
+// instructions issued (75 % of the cycles at 300 events of pileup 50); with the first cut's constants staged per
+// item and the module cut left to the survivors 512 events take 1.37 ms, before 1.44.
 constexpr int kDblQueue = 64;
 
 template <bool kQ>
@@ -683,7 +683,8 @@ __global__ void __launch_bounds__(256) k_sort_long(Dev d, int kind, uint32_t* li
 // networks by length up to 32 and a warp per longer one, loaded and stored a line per lane and entry (fill,
 // sort and gather, the latter in a kernel of its own: 512 events of pileup 50 693 us, 111 of pileup 1 to 200
 // 925; now 620 and 615). 512 staged entries per warp: with 1024 the shared memory leaves no L1 (706 and
-// 685 us), with 256 more groups are cut (628 and 636). Lists above the staging (none at pileup 200, whose longest has 125 entries) are sorted by one lane.
+// 685 us), with 256 more groups are cut (628 and 636). Lists above the staging
+// (none at pileup 200, whose longest has 125 entries) are sorted by one lane.
 constexpr int kRankBuf = 512;
 
 __global__ void __launch_bounds__(256) k_sort_hit_lists(Dev d, uint32_t hits) {
@@ -790,8 +791,8 @@ struct CircleEq {
 // pairs that pass it (a few percent) queue in shared memory for that test and the circle / DCA test,
 // which then run on full warps: the queue goes on over the warp's cells (emptied after every 32 of
 // them, a circle test of 150 instructions ran for five pairs: connect of 512 events of pileup 50
-// 1.33 ms, then 1.18; of 111 of pileup 1 to 200, 2.75 and 2.58 ms). Bound by instructions issued (67 % of
-// the issue slots): the test itself with its square root on every pair, and a search for each pair's
+// 1.33 ms, then 1.18; of 111 of pileup 1 to 200, 2.75 and 2.58 ms). Bound by instructions issued (78 % of
+// the cycles at 300 events of pileup 50): the test itself with its square root on every pair, and a search for each pair's
 // cell in place of the bit mask of the cells that start in a step, took 1.18 and 2.58 ms, now 0.94
 // and 2.16. Six blocks per SM (40 registers, two of them spilled) against five: 0.94 and 0.98 ms.
 // A passing pair counts one neighbour of the candidate (cn_cur), sets both used flags and goes to the pair list that k_connect_fill turns into neighbour lists; none

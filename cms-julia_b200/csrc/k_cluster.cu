@@ -14,10 +14,10 @@
 //  * one thread per module for modules of at most 16 digis (about three quarters
 //    of them at PU50): neighbour sets as bitmasks, components grown from the
 //    smallest digi left, all in registers;
-//  * one warp per module for modules of at most kWarpPix digis, from work lists.
-//    The warp keeps its digis in registers, finds neighbour pairs by broadcasting
-//    every digi (up to 32 digis) or through a column histogram (up to kWarpPix),
-//    joins them with the union-find, and scans with ballots;
+//  * one warp per module for modules of at most kWarpPix digis, from work lists: up
+//    to 32 digis one per lane, neighbour pairs by broadcasting every digi; above in
+//    shared memory, pairs through a column histogram. The pairs are joined with the
+//    union-find and the roots numbered with ballots;
 //  * one CTA per module for larger modules: pixels are binned by column in shared
 //    memory and only the same and the next column are searched.
 #include <algorithm>
@@ -306,8 +306,6 @@ __device__ __forceinline__ void cluster_module_mid(const Dev& d, int e, uint32_t
                      [&](int k) { return d.adc[r.g0 + k]; });
 }
 
-// every module position of the batch: modules of <= 32 digis here (one digi per lane),
-// larger ones to the mid-size list (<= kWarpPix) or the CTA list
 // ------------------------------------------------------------ thread per module
 constexpr int kThreadPix = 16;  // modules of at most this many digis: one thread each
 
@@ -828,7 +826,6 @@ static int mid_wave_ctas() {
 }
 
 void launch_cluster(const Dev& d, const Launch& L) {
-  // enough warps that a few events fill the GPU, at least 8 modules per warp otherwise
   // one thread per module position (at most 2000 per event)
   L.run(k_find_clus_tiny, dim3(div_up(kMaxNumModules, 128), d.E), 128, 0, d);
   L.mark("find_clus_tiny");

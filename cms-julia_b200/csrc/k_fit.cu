@@ -282,7 +282,7 @@ constexpr int kFitResident = 4;  // blocks per SM: 128 registers a thread
 
 // A block per 128 tracks, long fits first, so that the blocks even out; from four waves on one wave
 // of blocks that go on to further tracks saves the blocks' starts (2^20 mixed fits 374 us instead
-// of 416 with contracted FP32 arithmetic; 417 us now that f32 rounds each operation), which at 1.3
+// of 416 with contracted FP32 arithmetic; 408 us with f32, which rounds each operation), which at 1.3
 // waves costs more in balance than it saves (99991 FP64 fits 92 us instead of 81).
 inline int bl_fit_blocks(int32_t n) {
   const int all = fit_blocks(n), wave = 148 * kFitResident;

@@ -44,8 +44,9 @@ __device__ __forceinline__ void riemann_track(const RmArgs& A, int32_t t) {
   A.status[t] = ok ? 0 : 1;
 }
 
-// Latency bound like the broken-line fit. Three blocks per SM (168 registers): 2^18 FP64 fits 206 us;
-// uncapped, two blocks: 246 us; four: 208 us. At the launch per hit count it was 238 us.
+// Latency bound like the broken-line fit. Three blocks per SM (168 registers): 2^18 FP64 fits 206 us with Jacobi
+// sweeps for the eigenvector; uncapped, two blocks: 246 us; four: 208 us; with a launch per hit count 238 us. With
+// the Rayleigh quotient iteration, three blocks: 153 us.
 template <class T>
 __global__ void __launch_bounds__(kFitThreads, 3) k_riemann(RmArgs A) {
   pdl_sync();

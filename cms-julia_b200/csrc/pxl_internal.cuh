@@ -482,8 +482,12 @@ enum TuneSeg : int {
   kTuneEarlyDup, kTuneClassify, kTuneHitToTuple, kTuneFitTuples, kTuneCount
 };
 
-// Largest batch whose kernels overlap their launches (Launch::pdl). 111 uneven events on three streams:
-// 9.3 ms without, 13.7 ms with it: the blocks that wait hold SM resources of the other streams' kernels.
+// Largest batch whose kernels overlap their launches (Launch::pdl) and that takes the forms for few events: one
+// launch for the clustering lists, four hits per warp in the outer-hit sort, a cell per thread in the duplicate
+// removers, the export by one kernel. 8 events of pileup 50 take 654 us, 9 take 827. Batches run alone would gain
+// from a higher limit (at 32: 9 events 685 us, 16 1007 -> 903, 32 1405 -> 1376; of 100 tracks 9 events 502 -> 322, 32
+// 606 -> 478), but blocks that wait hold SM resources of the kernels on other streams: 111 uneven events on three
+// streams 9.3 ms without, 13.7 ms with it. Where between 8 and 111 that turns is not measured.
 constexpr int kPdlEvents = 8;
 
 struct Launch {
