@@ -91,8 +91,8 @@ typedef struct PxlParams {
   int32_t fits_per_multiplicity;     /* 24576 (MAX_NUM_OF_CONCURRENT_FITS) */
   int32_t include_errors;            /* 1 */
   int32_t use_quality;               /* 1 */
-  int32_t blocks_per_event;          /* launch shape; 0 = chosen by the autotuner */
-  int32_t threads_per_block;         /* launch shape; 0 = chosen by the autotuner */
+  int32_t blocks_per_event;          /* launch shape; 0 = the autotuner's, or by the batch */
+  int32_t threads_per_block;         /* launch shape; 0 = the autotuner's, or by the batch */
   int32_t columns_per_event;         /* 65536 (MAX_NUM_OF_ACTIVE_DOUBLETS): cells with a neighbour or
                                         track list; a warning (PXL_WARN_COLUMNS) above it */
   int32_t fit_precision;             /* broken-line fits of the chain: 0 = FP64 as the reference
