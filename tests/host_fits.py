@@ -1,11 +1,13 @@
 """The fit headers built for the host, so that single tracks can be fitted without a GPU."""
 import ctypes
+import shutil
 import subprocess
 from pathlib import Path
 
 import numpy as np
 
 ROOT = Path(__file__).resolve().parents[1]
+NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 
 SOURCE = r"""
 #include "bl_fit.cuh"
@@ -57,7 +59,7 @@ def _build(directory: Path) -> ctypes.CDLL:
     """With contracted products, as the device code is built."""
     (directory / "host_fits.cu").write_text(SOURCE)
     so = directory / "host_fits.so"
-    subprocess.run(["nvcc", "-std=c++17", "-O2", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler",
+    subprocess.run([NVCC, "-std=c++17", "-O2", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler",
                     "-fPIC,-mfma,-ffp-contract=fast", "-I", str(ROOT / "cms-julia_b200" / "csrc"),
                     str(directory / "host_fits.cu"), "-o", str(so)], check=True)
     lib = ctypes.CDLL(str(so))

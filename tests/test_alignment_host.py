@@ -7,6 +7,8 @@ from pathlib import Path
 import numpy as np
 import pytest
 
+from host_fits import NVCC
+
 CSRC = Path(__file__).resolve().parents[1] / "cms-julia_b200" / "csrc"
 SOURCE = """
 #include "alignment.cuh"
@@ -25,7 +27,7 @@ extern "C" void both(const float* a, long n, int barrel, unsigned char* cut, uns
 def both(tmp_path_factory):
     d = tmp_path_factory.mktemp("alignment")
     (d / "a.cu").write_text(SOURCE)
-    subprocess.run(["nvcc", "-std=c++17", "-O2", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler",
+    subprocess.run([NVCC, "-std=c++17", "-O2", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler",
                     "-fPIC,-ffp-contract=off", "-I", str(CSRC), str(d / "a.cu"), "-o", str(d / "a.so")], check=True)
     lib = ctypes.CDLL(str(d / "a.so"))
     lib.both.argtypes = [ctypes.c_void_p, ctypes.c_long, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
